@@ -14,6 +14,7 @@
 #include <math.h>
 
 #include "nh_cnn_item.cuh"
+#include "nh_cnn_mma.cuh"
 #include "nh_common.cuh"
 
 namespace nh {
@@ -93,6 +94,39 @@ __global__ void __launch_bounds__(TH) cnn_kernel(CnnArgs<T> a) {
   }
 }
 
+// FP64 features on the FP64 matrix instruction (cnn_layers_mma), mode 1 only.
+template <int TH>
+__global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) cnn_mma_kernel(CnnArgs<double> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int N = a.N, C = a.C, M2 = 2 * N, d = C / 2;
+  const int PS = mma_plane(a.Lx, a.Ly), W = a.Ly + 2;
+  double* act = reinterpret_cast<double*>(smem_raw);
+  double* wsm = act + (size_t)C * PS;
+  int* simg = reinterpret_cast<int*>(wsm + 9 * C * C);
+  int* occl = simg + M2;
+  int* wbuf = occl + M2;
+  const int G = a.cl.G;
+  const int n_work = a.slot_item ? *a.slot_count
+                                 : (a.cl.n_cfg_dev ? *a.cl.n_cfg_dev : a.cl.n_cfg) * G;
+  for (int slot = blockIdx.x; slot < n_work; slot += gridDim.x) {
+    const int item = a.slot_item ? a.slot_item[slot] : slot;
+    const int c = item / G, g = item - c * G;
+    const int smp = a.cl.sample ? a.cl.sample[c] : c;
+    const int fr = a.cl.from ? a.cl.from[c] : -1;
+    const int to = a.cl.from ? a.cl.to[c] : -1;
+    __syncthreads();  // previous item's readers of simg/act are done
+    cnn_layers_mma<4, TH>(a.wp, a.b, a.Lx, a.Ly, a.layers, a.cl.spins + (int64_t)smp * M2, fr, to,
+                          g, act, wsm, simg);
+    auto feat_of = [&](int sg, int aa, int site) {
+      const int x = site / a.Ly;
+      return act[(sg * d + aa) * PS + (x + 1) * W + site - x * a.Ly + 1];
+    };
+    write_occupied_rows<double, decltype(feat_of), TH>(
+        simg, occl, wbuf, N, a.n, d, g, a.Lx, a.Ly, a.Y + (int64_t)slot * a.n * d,
+        a.idx + (int64_t)slot * a.n, a.item_sign + item, feat_of);
+  }
+}
+
 // packed[l][ci][tap][co] = conv_w[l][co][ci][tap]
 __global__ void pack_kernel(const float* __restrict__ w, int C, int layers, float* packed) {
   const int total = 18 * C + (layers - 1) * 9 * C * C;
@@ -156,6 +190,24 @@ int launch_cnn_t(const CnnLaunch& q, int N, int C, cudaStream_t st) {
   return check_launch(sizeof(T) == 8 ? "cnn_kernel<double>" : "cnn_kernel<float>");
 }
 
+template <int TH>
+int launch_cnn_mma(const CnnLaunch& q, int N, int C, size_t smem, cudaStream_t st) {
+  const nh_backflow_params& p = *q.p;
+  const int slots = q.slot_item ? q.max_slots : q.cl->n_cfg * q.cl->G;
+  if (slots <= 0) return NH_OK;
+  int grid = num_sms() * (smem <= 113 * 1024 ? 2 : 1);
+  if (grid > slots) grid = slots;
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      cnn_mma_kernel<TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  if (attr != cudaSuccess) return check_cuda(attr, "cnn smem attribute");
+  CnnArgs<double> a{*q.cl, p.conv_w_packed, p.conv_b, p.Lx, p.Ly, N, C, p.layers,
+                    p.n_up + p.n_dn, q.mode, q.slot_item, q.slot_count, q.max_slots,
+                    nullptr, static_cast<double*>(q.Y), q.idx, q.item_sign, nullptr};
+  ProfScope prof_scope(NH_K_CNN64, st);
+  cnn_mma_kernel<TH><<<grid, TH, smem, st>>>(a);
+  return check_launch("cnn_mma_kernel");
+}
+
 size_t cnn_scratch_bytes(int N, int C) {
   if (cnn_smem<double>(N, C) <= 227 * 1024) return 0;
   return (size_t)num_sms() * kCnnBigPerSm * 2 * C * (N + 1) * sizeof(double);
@@ -170,9 +222,18 @@ int launch_cnn(const CnnLaunch& q, cudaStream_t st) {
                 C, p.layers, N);
   if (!p.conv_w_packed)
     return fail(NH_ERR_INVALID, "cnn: conv_w_packed is null (call nh_pack_cnn_weights)");
-  if (q.fp64)
+  if (q.fp64) {
+    // Up to 256 sites and 32 channels: the matrix-instruction form; two 256-thread CTAs per SM
+    // where they fit (lattices up to about 100 sites), else one of 512 threads.
+    const size_t mma = sizeof(double) * cnn_mma_doubles(p.Lx, p.Ly, C) +
+                       sizeof(int) * (4 * (size_t)N + 4 * p.Lx + 32);
+    if (q.mode == 1 && mma <= 113 * 1024 && cnn_mma_fits(p.Lx, p.Ly, C, 256))
+      return launch_cnn_mma<256>(q, N, C, mma, st);
+    if (q.mode == 1 && mma <= 227 * 1024 && cnn_mma_fits(p.Lx, p.Ly, C, 512))
+      return launch_cnn_mma<512>(q, N, C, mma, st);
     return cnn_smem<double>(N, C) <= 227 * 1024 ? launch_cnn_t<double, false, 512>(q, N, C, st)
                                                  : launch_cnn_t<double, true>(q, N, C, st);
+  }
   return cnn_smem<float>(N, C) <= 227 * 1024 ? launch_cnn_t<float, false>(q, N, C, st)
                                               : launch_cnn_t<float, true>(q, N, C, st);
 }
