@@ -17,33 +17,44 @@
 // F[p, q] = sum_a (Y[p, a] Y[q, a]) Wt[2 s_p + s_q, r(p, q), a], in the same order of operations
 // as the FP32 gather so that the FP32 matrix is reproduced bit for bit.
 //
-// One CTA (256 threads) per SM.  Phase 1 stages the Wt table and the item's features in shared
-// memory and writes the permuted lower triangle to a per-CTA slice of global scratch (L2
-// resident); phase 2 loads it into shared memory as FP64 (row a at roff(a), rows 16-byte
-// aligned); phase 3 eliminates.  n <= kRefineMaxN (224: the FP64 triangle takes 200 KB).
+// One CTA of 512 threads per SM (two of 256 where the lattice is small).  Phase 1 fills the permuted
+// lower triangle in shared memory, stored as 8 x 8 FP64 tiles (tile (I, J <= I) at index
+// I (I + 1) / 2 + J; 16-byte chunks swizzled inside a tile, see toff); phase 2 eliminates panels of
+// 8 columns: one warp factorises the 8 x 8 pivot block, one thread per row solves the panel, and
+// the trailing tiles take P W^T as two m8n8k4 FP64 products each.  The next panel's column is
+// updated first, so that its pivot block (a serial chain) is factorised by warp 0 while the other
+// warps update the rest.  n <= kRefineMaxN (224: the tiles take 203 KB).
 #include <math.h>
 
 #include <algorithm>
 
 #include "nh_cnn_item.cuh"
+#include "nh_cnn_mma.cuh"
 #include "nh_common.cuh"
 
 namespace nh {
 namespace {
 
-constexpr int kRThreads = 256;
-constexpr int kRWarps = kRThreads / 32;
 constexpr int kPW = 8;  // panel width: 4 elimination steps
 
-// Row a of the padded lower triangle starts at roff(a) (even, so FP64 pairs are 16-byte aligned).
+// Modes 1 and 3 (FP32 entries): row a of a packed lower triangle in the CTA's slice starts at
+// roff(a).
 __host__ __device__ __forceinline__ int roff(int a) { return (a * (a - 1)) / 2 + a / 2; }
-// Elements of a whole triangle, rounded up to a multiple of 4 so that every per-CTA slice (FP32
-// or FP64) and every 16-byte vector of the copies stays aligned.
-__host__ __device__ __forceinline__ int tri_elems(int n) { return (roff(n) + 3) & ~3; }
-// Bytes of one CTA's slice: the FP64 triangle, or an item's FP64 rows and modes (modes 3, 4),
-// whichever is larger; a multiple of 16.
+__host__ __device__ __forceinline__ int tile_rows(int n) { return (n + 7) >> 3; }
+__host__ __device__ __forceinline__ int tile_base(int I) { return (I * (I + 1)) >> 1; }
+// Bytes of the tiles of rows < I.
+__host__ __device__ __forceinline__ size_t tile_bytes(int I) { return 512 * (size_t)tile_base(I); }
+// Offset of element (r, c) in an 8 x 8 tile: the row's four 16-byte chunks are XOR-ed with the bit
+// reversal of r / 2, so that 8 rows of one chunk (the panel solve), 2 rows of all chunks (an MMA
+// accumulator) and 4 rows x 4 columns of doubles (an MMA operand) all hit distinct banks.
+__device__ __forceinline__ int toff(int r, int c) {
+  const int f = (r & 2) | ((r >> 2) & 1);
+  return r * 8 + ((((c >> 1) ^ f) << 1) | (c & 1));
+}
+// Bytes of one CTA's slice: the tiles, the packed FP32 triangle, or an item's rows and modes
+// (mode 3), whichever is largest; a multiple of 16.
 __host__ __device__ __forceinline__ size_t slice_stride(int n, int d) {
-  const size_t tri = 8 * (size_t)tri_elems(n), rows = 8 * (size_t)n * d + 4 * (size_t)n;
+  const size_t tri = tile_bytes(tile_rows(n)), rows = 8 * (size_t)n * d + 4 * (size_t)n;
   return ((tri > rows ? tri : rows) + 15) & ~(size_t)15;
 }
 
@@ -61,7 +72,7 @@ struct RefineArgs {
   const int32_t* idx;
   const void* Wt;
   int Lx, Ly, D;
-  bool stage_wt;  // Wt fits in shared memory with the features
+  bool stage_wt;  // Wt (modes 2, 4: one spin block of it) fits in shared memory with the rows
   const int32_t* list;   // slot -> item
   const int32_t* count;  // device number of slots
   const uint16_t* perm;  // per item: perm[0, n) logical -> physical, [n] relabelling parity
@@ -71,6 +82,10 @@ struct RefineArgs {
   double* logabs;
   int32_t* flags;
   void* slice;  // per CTA: slice_stride(n, D) bytes
+  // modes 2, 4 (byte offsets in dynamic shared memory): rows Y, packed modes, one spin block of
+  // Wt64 (stage_wt); tiles of rows >= keep overlap them and go through the slice.
+  int y_off, info_off, wt_off, keep;
+  bool rows_slice;  // mode 4: no room for Y above the CNN, its rows pass through the slice
 };
 
 template <typename T>
@@ -86,12 +101,12 @@ struct Vec2<double> {
   using V = double2;
 };
 
-// Phase 1: logical lower triangle A[p][q] = F[perm p][perm q] of one item into the CTA's slice
+// Phase 1 of modes 1 and 3: logical lower triangle A[p][q] = F[perm p][perm q] of one item into the CTA's slice
 // (element type T).  Warp <-> 32 consecutive logical columns q (their features in registers
 // when small), rows p > q in turn (the row's features broadcast); each element reads one Wt row.
-template <typename T, int D, int kRegBytes = 64>
+template <typename T, int D, int TH, int kRegBytes = 64>
 __device__ void gather_permuted(const RefineArgs& a, const T* Yg, const int32_t* ig,
-                                const int* perm, unsigned char* smem, T* slice) {
+                                const uint16_t* perm, unsigned char* smem, T* slice) {
   const int n = a.n, N = a.Lx * a.Ly;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   constexpr int DP = D + (sizeof(T) == 4 ? 4 : 2);
@@ -107,17 +122,17 @@ __device__ void gather_permuted(const RefineArgs& a, const T* Yg, const int32_t*
   auto stage = [&](const T* src, T* dst, int rows, bool nc) {
     constexpr int VPR = D / VK;  // vectors per row
     const int nv = rows * VPR;
-    for (int v0 = tid; v0 < nv; v0 += 4 * kRThreads) {
+    for (int v0 = tid; v0 < nv; v0 += 4 * TH) {
       V buf[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const int v = v0 + u * kRThreads;
+        const int v = v0 + u * TH;
         if (v < nv) buf[u] = nc ? __ldg(reinterpret_cast<const V*>(src) + v)
                                 : reinterpret_cast<const V*>(src)[v];
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const int v = v0 + u * kRThreads;
+        const int v = v0 + u * TH;
         if (v < nv) {
           const int r = v / VPR;
           *reinterpret_cast<V*>(dst + r * DP + (v - r * VPR) * VK) = buf[u];
@@ -126,7 +141,7 @@ __device__ void gather_permuted(const RefineArgs& a, const T* Yg, const int32_t*
     }
   };
   stage(Yg, ys, n, false);
-  for (int p = tid; p < n; p += kRThreads) {
+  for (int p = tid; p < n; p += TH) {
     const int m = ig[p];
     const int sp = m >= N ? 1 : 0, site = m - sp * N, x = site / a.Ly;
     info[p] = (sp << 16) | (x << 8) | (site - x * a.Ly);
@@ -140,7 +155,7 @@ __device__ void gather_permuted(const RefineArgs& a, const T* Yg, const int32_t*
   constexpr bool kRegs = D * sizeof(T) <= kRegBytes;
   T yj[kRegs ? D : 1];
 #pragma unroll 1
-  for (int u = wid; u < total; u += kRWarps, rem += kRWarps) {
+  for (int u = wid; u < total; u += (TH / 32), rem += (TH / 32)) {
     while (rem >= n - 32 * qb - 1) {
       rem -= n - 32 * qb - 1;
       ++qb;
@@ -192,315 +207,469 @@ __device__ void gather_permuted(const RefineArgs& a, const T* Yg, const int32_t*
   }
 }
 
-// The CTA's slice (tot = tri_elems(n) values, a multiple of 4) into the FP64 triangle, 16-byte
-// vectors with four in flight per thread.
-__device__ __forceinline__ void copy_slice(const float* sl, double* S, int tot) {
-  const int nv = tot / 4;
-  for (int v0 = threadIdx.x; v0 < nv; v0 += 4 * kRThreads) {
-    float4 buf[4];
+// Phase 1 of modes 2 and 4: F[i][j] = sum_a (Y[i, a] Y[j, a]) Wt[2 s_i + s_j, r(i, j), a] of the
+// physical pairs i > j, scattered with its sign to the logical tile.  LPR lanes share a pair, each
+// with D / LPR of the a; a table row is then one contiguous 16 LPR-byte read (no bank conflicts,
+// where one lane per pair read 32 scattered rows), the column's features stay in registers, the
+// row's are a broadcast, and LPR rows are reduced together (each lane ends with one of them).
+// The table is staged one spin block at a time (uu, du, dd: the modes ascend, so rows and columns
+// of a block are ranges); unsorted mode lists (a wrong particle number) and lattices whose block
+// does not fit read it from global memory.
+template <int D, int TH>
+__device__ void gather_tiles(const RefineArgs& a, const double* Ys, const int* info,
+                             const uint16_t* iperm, int nu, bool sorted, unsigned char* smem,
+                             double* S, double* slice) {
+  constexpr int LPR = D / 2 < 8 ? D / 2 : 8, CPL = D / (2 * LPR);  // lanes per pair, chunks per lane
+  constexpr int GR = 32 / LPR, JW = 2 * GR;                        // column groups, columns per warp
+  constexpr int WARPS = TH / 32;
+  const int n = a.n, N = a.Lx * a.Ly;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int grp = lane / LPR, c = lane % LPR;
+  const double* Wg = static_cast<const double*>(a.Wt);
+  double* wts = reinterpret_cast<double*>(smem + a.wt_off);
+  const bool stage = a.stage_wt && sorted;
+  for (int ph = 0; ph < (stage ? 3 : 1); ++ph) {
+    // uu, du, dd; without staging every pair at once
+    const int i0 = stage && ph > 0 ? nu : 0, i1 = stage && ph == 0 ? nu : n;
+    const int j0 = stage && ph == 2 ? nu : 0, j1 = stage && ph < 2 ? nu : n;
+    const bool tri = !(stage && ph == 1);
+    if (stage) {
+      const double2* src =
+          reinterpret_cast<const double2*>(Wg + (size_t)(ph == 0 ? 0 : ph + 1) * N * D);
+      __syncthreads();  // the previous block's readers are done
+      if (i1 > i0 && j1 > j0)
+        for (int v0 = tid; v0 < N * (D / 2); v0 += 4 * TH) {
+          double2 buf[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-      if (v0 + u * kRThreads < nv) buf[u] = reinterpret_cast<const float4*>(sl)[v0 + u * kRThreads];
+          for (int u = 0; u < 4; ++u)
+            if (v0 + u * TH < N * (D / 2)) buf[u] = __ldg(src + v0 + u * TH);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int v = v0 + u * kRThreads;
-      if (v < nv) {
-        reinterpret_cast<double2*>(S)[2 * v] = make_double2(buf[u].x, buf[u].y);
-        reinterpret_cast<double2*>(S)[2 * v + 1] = make_double2(buf[u].z, buf[u].w);
+          for (int u = 0; u < 4; ++u)
+            if (v0 + u * TH < N * (D / 2)) reinterpret_cast<double2*>(wts)[v0 + u * TH] = buf[u];
+        }
+      __syncthreads();
+    }
+    const int nr = i1 - i0, nc = j1 - j0;
+    if (nr <= 0 || nc <= 0) continue;
+    const int nrb = (nr + LPR - 1) / LPR, ncg = (nc + JW - 1) / JW;
+    // column groups of row block rb that hold a pair (i > j for the triangular blocks)
+    auto groups = [&](int rb) {
+      return tri ? min(ncg, (rb * LPR + LPR - 1 + JW - 1) / JW) : ncg;
+    };
+    int rb = 0, rem = wid;
+    for (;; rem += WARPS) {
+      while (rb < nrb && rem >= groups(rb)) {
+        rem -= groups(rb);
+        ++rb;
       }
+      if (rb >= nrb) break;
+      int j[2], infj[2];
+      double2 yj[2][CPL];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        j[q] = j0 + rem * JW + q * GR + grp;
+        const int jj = min(j[q], j1 - 1);
+        infj[q] = info[jj];
+#pragma unroll
+        for (int x = 0; x < CPL; ++x)
+          yj[q][x] = *reinterpret_cast<const double2*>(Ys + jj * D + 2 * (c + LPR * x));
+      }
+      const int ib = i0 + rb * LPR;
+      double part[2][LPR];
+#pragma unroll
+      for (int u = 0; u < LPR; ++u) {
+        const int i = min(ib + u, i1 - 1);
+        const int infi = info[i];
+        double2 yi[CPL];
+#pragma unroll
+        for (int x = 0; x < CPL; ++x)
+          yi[x] = *reinterpret_cast<const double2*>(Ys + i * D + 2 * (c + LPR * x));
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          int dx = ((infi >> 8) & 0xFF) - ((infj[q] >> 8) & 0xFF);
+          int dy = (infi & 0xFF) - (infj[q] & 0xFF);
+          dx += dx < 0 ? a.Lx : 0;
+          dy += dy < 0 ? a.Ly : 0;
+          const int r = dx * a.Ly + dy;
+          double acc = 0.0;
+          const int blk = 2 * (infi >> 16) + (infj[q] >> 16);
+          const double2* wr = stage ? reinterpret_cast<const double2*>(wts + r * D) + c
+                                    : reinterpret_cast<const double2*>(Wg + (size_t)(blk * N + r) * D) + c;
+#pragma unroll
+          for (int x = 0; x < CPL; ++x) {
+            const double2 w = wr[LPR * x];
+            acc = fma(yi[x].x * yj[q][x].x, w.x, acc);
+            acc = fma(yi[x].y * yj[q][x].y, w.y, acc);
+          }
+          part[q][u] = acc;
+        }
+      }
+      // Sum over the LPR lanes, row u ending in lane c = u: halves of the rows are exchanged.
+#pragma unroll
+      for (int h = LPR / 2; h; h >>= 1) {
+        const bool up = c & h;
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+#pragma unroll
+          for (int u = 0; u < h; ++u) {
+            const double keep = up ? part[q][u + h] : part[q][u];
+            const double send = up ? part[q][u] : part[q][u + h];
+            part[q][u] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+          }
+      }
+      const int i = ib + c;
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        if (i < i1 && j[q] < j1 && (!tri || i > j[q])) {
+          const int p = iperm[i], lq = iperm[j[q]];
+          const int hi = max(p, lq), lo = min(p, lq), I = hi >> 3;
+          const int o = (tile_base(I) + (lo >> 3)) * 64 + toff(hi & 7, lo & 7);
+          const double v = p > lq ? part[q][0] : -part[q][0];
+          if (I < a.keep)
+            S[o] = v;
+          else
+            slice[o] = v;
+        }
     }
   }
-}
-__device__ __forceinline__ void copy_slice(const double* sl, double* S, int tot) {
-  const int nv = tot / 2;
-  for (int v0 = threadIdx.x; v0 < nv; v0 += 4 * kRThreads) {
+  __syncthreads();  // the staged rows and table are dead: the slice's tiles take their place
+  const int T = tile_rows(n), o0 = tile_base(a.keep) * 32, o1 = tile_base(T) * 32;
+  for (int v0 = o0 + tid; v0 < o1; v0 += 4 * TH) {
     double2 buf[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (v0 + u * kRThreads < nv) buf[u] = reinterpret_cast<const double2*>(sl)[v0 + u * kRThreads];
+      if (v0 + u * TH < o1) buf[u] = reinterpret_cast<const double2*>(slice)[v0 + u * TH];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (v0 + u * kRThreads < nv) reinterpret_cast<double2*>(S)[v0 + u * kRThreads] = buf[u];
+      if (v0 + u * TH < o1) reinterpret_cast<double2*>(S)[v0 + u * TH] = buf[u];
   }
 }
 
-// Modes 3 and 4: the features of the item's configuration (CNN in shared memory) written as its
-// occupied rows Y (n, d) and modes to global memory (the CTA's slice, read back by the gather's
-// staging before the gather overwrites it).
-template <typename T>
+// Modes 3 and 4: the features of the item's configuration (CNN in shared memory) as its occupied
+// rows Y (n, d) and modes: mode 3 to the CTA's slice (read back by the gather's staging), mode 4
+// to the staging area above the CNN's shared memory.
+template <typename T, int TH>
 __device__ void features_to(const RefineArgs& a, int item, unsigned char* smem, T* Ydst,
-                            int32_t* idst) {
-  const int N = a.Lx * a.Ly, C = a.C, M2 = 2 * N, NS = N + 1;
+                            int32_t* idst, float* sign_dummy) {
+  const int N = a.Lx * a.Ly, C = a.C, M2 = 2 * N, NS = N + 1, d = C / 2;
   const int G = a.cl.G;
   const int c = item / G, g = item - c * G;
   const int smp = a.cl.sample ? a.cl.sample[c] : c;
   const int fr = a.cl.from ? a.cl.from[c] : -1;
   const int to = a.cl.from ? a.cl.to[c] : -1;
   const int8_t* base = a.cl.spins + (int64_t)smp * M2;
-  __shared__ float sign_dummy;
   int* simg = reinterpret_cast<int*>(smem);
   int* occl = simg + M2;
   int* wbuf = occl + M2;
   const size_t ints = 4 * (size_t)N + 4 * a.Lx + 32;
   T* actA = reinterpret_cast<T*>(smem + ((sizeof(int) * ints + 15) & ~(size_t)15));
+  __syncthreads();
+  if constexpr (sizeof(T) == 8) {
+    if (cnn_mma_fits(a.Lx, a.Ly, C, TH)) {
+      const int PS = mma_plane(a.Lx, a.Ly), W = a.Ly + 2;
+      cnn_layers_mma<4, TH>(a.cnn_w, a.cnn_b, a.Lx, a.Ly, a.layers, base, fr, to, g, actA,
+                            actA + (size_t)C * PS, simg);
+      auto feat = [&](int sg, int aa, int site) {
+        const int x = site / a.Ly;
+        return actA[(sg * d + aa) * PS + (x + 1) * W + site - x * a.Ly + 1];
+      };
+      write_occupied_rows<T, decltype(feat), TH>(simg, occl, wbuf, N, a.n, d, g, a.Lx, a.Ly, Ydst,
+                                                 idst, sign_dummy, feat);
+      __syncthreads();
+      return;
+    }
+  }
   T* actB = actA + C * NS;
   T* wsm = actB + C * NS;
   wsm = reinterpret_cast<T*>((reinterpret_cast<uintptr_t>(wsm) + 15) & ~(uintptr_t)15);
   T* bsm = wsm + C * C * 9;
-  __syncthreads();
-  const T* in = cnn_layers<T>(a.cnn_w, a.cnn_b, a.Lx, a.Ly, C, a.layers, base, fr, to, g, actA,
-                              actB, wsm, bsm, simg);
-  const int d = C / 2;
-  write_occupied_rows(simg, occl, wbuf, N, a.n, d, g, a.Lx, a.Ly, Ydst, idst, &sign_dummy,
-                      [&](int sg, int aa, int site) { return in[(sg * d + aa) * NS + site]; });
+  const T* in = cnn_layers<T, TH>(a.cnn_w, a.cnn_b, a.Lx, a.Ly, C, a.layers, base, fr, to, g, actA,
+                                  actB, wsm, bsm, simg);
+  auto feat = [&](int sg, int aa, int site) { return in[(sg * d + aa) * NS + site]; };
+  write_occupied_rows<T, decltype(feat), TH>(simg, occl, wbuf, N, a.n, d, g, a.Lx, a.Ly, Ydst, idst,
+                                             sign_dummy, feat);
   __syncthreads();
 }
 
-// Shared memory of the in-kernel CNN (modes 3, 4).
-size_t features_smem(int N, int C, int Lx, int elt) {
-  const size_t ints = 4 * (size_t)N + 4 * Lx + 32;
-  const size_t act = ((sizeof(int) * ints + 15) & ~(size_t)15) + (size_t)elt * 2 * C * (N + 1);
+// Shared memory of the in-kernel CNN (modes 3, 4) with TH threads.
+size_t features_smem(int Lx, int Ly, int C, int elt, int TH) {
+  const size_t N = (size_t)Lx * Ly, ints = 4 * N + 4 * Lx + 32;
+  const size_t act0 = (sizeof(int) * ints + 15) & ~(size_t)15;
+  if (elt == 8 && cnn_mma_fits(Lx, Ly, C, TH)) return act0 + 8 * cnn_mma_doubles(Lx, Ly, C);
+  const size_t act = act0 + (size_t)elt * 2 * C * (N + 1);
   return ((act + 15) & ~(size_t)15) + (size_t)elt * ((size_t)C * C * 9 + C);
+}
+
+// Pivot block of panel p (w <= 8 columns) by one warp: lane r holds row r, row[c] = B[r][c]
+// (c < r); each step's columns k, k+1 go through shared memory to every lane.  Writes the block
+// multipliers Lm, the reciprocal pivots xinv and the pivots to piv[0, w / 2).
+__device__ __forceinline__ void factor_block(const double* D, int w, double* Lm, double* xinv,
+                                             double (*xy)[kPW], double* piv) {
+  const int lane = threadIdx.x & 31;
+  double row[kPW];
+#pragma unroll
+  for (int c = 0; c < kPW; ++c) row[c] = (lane < w && c < lane) ? D[toff(lane & 7, c)] : 0.0;
+#pragma unroll
+  for (int t = 0; t < kPW / 2; ++t) {
+    if (2 * t < w) {
+      const int k = 2 * t;
+      const double xr = row[k], yr = row[k + 1];  // B[r][k], B[r][k+1] (lanes r > k+1)
+      if (lane < kPW) {
+        xy[0][lane] = xr;
+        xy[1][lane] = yr;
+      }
+      __syncwarp();
+      const double x = -xy[0][k + 1];  // B[k][k+1] = -B[k+1][k]
+      const double inv = 1.0 / x;
+      if (lane == 0) {
+        piv[t] = x;
+        xinv[t] = inv;
+      }
+      const double yi = yr * inv, xi = xr * inv;
+      if (lane >= k + 2 && lane < w) {
+        Lm[lane * kPW + k] = yi;
+        Lm[lane * kPW + k + 1] = -xi;
+      }
+#pragma unroll
+      for (int c = 0; c < kPW; ++c)
+        if (c >= k + 2 && c < lane && lane < w) row[c] += yi * xy[0][c] - xi * xy[1][c];
+      __syncwarp();
+    }
+  }
+}
+
+// Tile update C += P W^T: P and W are 8 x 8 tiles (rows x panel columns).
+struct Operand {
+  double k0, k1;
+};
+__device__ __forceinline__ Operand load_operand(const double* t) {
+  const int lane = threadIdx.x & 31;
+  return Operand{t[toff(lane >> 2, lane & 3)], t[toff(lane >> 2, 4 + (lane & 3))]};
+}
+__device__ __forceinline__ double2* acc_ptr(double* t) {
+  const int lane = threadIdx.x & 31;
+  return reinterpret_cast<double2*>(t + toff(lane >> 2, 2 * (lane & 3)));
+}
+__device__ __forceinline__ double2 tile_mma(double2 v, const Operand& p, const Operand& w) {
+  double c[2] = {v.x, v.y};
+  mma_f64(c, p.k0, w.k0);
+  mma_f64(c, p.k1, w.k1);
+  return make_double2(c[0], c[1]);
 }
 
 // MODE is a.mode as a template argument, so that each instance holds only its own phase-1 code
 // (the register allocation of the elimination is then not shaped by the other modes).
-template <int D, int MODE>
-__global__ void __launch_bounds__(kRThreads, 1) refine_kernel(RefineArgs a) {
+template <int D, int MODE, int TH>
+__global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int perm_s[kRefineMaxN];
-  __shared__ double Lm[kPW * kPW];  // block multipliers L[r][c] of the current panel
-  __shared__ double xs[kPW / 2];    // its FP64 pivots
-  __shared__ double xinv[kPW / 2];  // and their reciprocals
-  __shared__ double xy[2][kPW];     // pivot-block columns k, k+1 of the current step
-  const int n = a.n;
+  __shared__ uint16_t perm_s[kRefineMaxN];  // logical -> physical (modes 2, 4: physical -> logical)
+  __shared__ double Lm[kPW * kPW];          // block multipliers L[r][c] of the current panel
+  __shared__ double xinv[kPW / 2];          // reciprocals of its pivots
+  __shared__ double xy[2][kPW];             // pivot-block columns k, k+1 of the current step
+  __shared__ int nu_s;                      // up modes of the item; bit 31: list not sorted by spin
+  constexpr int WARPS = TH / 32;
+  const int n = a.n, T = tile_rows(n);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   double* S = reinterpret_cast<double*>(smem);
+  double* Wb = S + (size_t)tile_base(T) * 64;  // W tiles of the current panel, one per tile row
   const int n_work = *a.count;
   for (int slot = blockIdx.x; slot < n_work; slot += gridDim.x) {
     const int item = a.list[slot];
     const uint16_t* pr = a.perm + (size_t)item * a.perm_stride;
     __syncthreads();
-    for (int p = tid; p < n; p += kRThreads) perm_s[p] = pr[p];
+    for (int p = tid; p < n; p += TH) {
+      const int v = pr[p];
+      if (MODE == 2 || MODE == 4)
+        perm_s[v < n ? v : 0] = (uint16_t)p;
+      else
+        perm_s[p] = (uint16_t)v;
+    }
+    if (tid == 0) nu_s = 0;
     __syncthreads();
-    // Phases 1 and 2: the permuted lower triangle in FP64 shared memory.
+    // Phase 1: the permuted lower triangle in FP64 tiles.
+    unsigned char* slb = static_cast<unsigned char*>(a.slice) + (size_t)blockIdx.x * slice_stride(n, D);
     if constexpr (MODE == 0) {
       const float* F = a.F + (size_t)item * n * n;
-      for (int p = wid; p < n; p += kRWarps) {
+      for (int p = wid; p < n; p += WARPS) {
         const int i = perm_s[p];
         for (int q = lane; q < p; q += 32) {
           const int j = perm_s[q];
-          S[roff(p) + q] = i > j ? (double)__ldg(F + (size_t)i * n + j)
-                                 : -(double)__ldg(F + (size_t)j * n + i);
+          S[(tile_base(p >> 3) + (q >> 3)) * 64 + toff(p & 7, q & 7)] =
+              i > j ? (double)__ldg(F + (size_t)i * n + j) : -(double)__ldg(F + (size_t)j * n + i);
         }
       }
+    } else if constexpr (MODE == 1 || MODE == 3) {
+      float* sl = reinterpret_cast<float*>(slb);
+      const float* Yg = static_cast<const float*>(a.Y) + (size_t)item * n * D;
+      const int32_t* ig = a.idx + (size_t)item * n;
+      if constexpr (MODE == 3) {  // the item's FP32 features, rows and modes to the slice
+        features_to<float, TH>(a, item, smem, sl, reinterpret_cast<int32_t*>(sl + n * D),
+                               reinterpret_cast<float*>(xinv));
+        Yg = sl;
+        ig = reinterpret_cast<const int32_t*>(sl + n * D);
+      }
+      gather_permuted<float, D, TH>(a, Yg, ig, perm_s, smem, sl);
+      __syncthreads();  // slice written; the staging area is dead
+      for (int p = wid; p < n; p += WARPS)
+        for (int q = lane; q < p; q += 32)
+          S[(tile_base(p >> 3) + (q >> 3)) * 64 + toff(p & 7, q & 7)] = (double)sl[roff(p) + q];
     } else {
-      const int tot = tri_elems(n);  // a multiple of 4
-      unsigned char* slb = static_cast<unsigned char*>(a.slice) + (size_t)blockIdx.x * slice_stride(n, D);
-      if constexpr (MODE == 1 || MODE == 3) {
-        float* sl = reinterpret_cast<float*>(slb);
-        const float* Yg = static_cast<const float*>(a.Y) + (size_t)item * n * D;
-        const int32_t* ig = a.idx + (size_t)item * n;
-        if constexpr (MODE == 3) {  // the item's FP32 features, rows and modes to the slice
-          features_to(a, item, smem, sl, reinterpret_cast<int32_t*>(sl + n * D));
-          Yg = sl;
-          ig = reinterpret_cast<const int32_t*>(sl + n * D);
-        }
-        gather_permuted<float, D>(a, Yg, ig, perm_s, smem, sl);
-        __syncthreads();  // slice written; the staging area is dead
-        copy_slice(sl, S, tot);
-      } else {
-        double* sl = reinterpret_cast<double*>(slb);
-        const double* Yg = static_cast<const double*>(a.Y) + (size_t)slot * n * D;
-        const int32_t* ig = a.idx + (size_t)slot * n;
-        if constexpr (MODE == 4) {
-          features_to(a, item, smem, sl, reinterpret_cast<int32_t*>(sl + n * D));
-          Yg = sl;
-          ig = reinterpret_cast<const int32_t*>(sl + n * D);
-        }
-        // mode 2 keeps each column's FP64 features in registers (its instance has the room)
-        gather_permuted<double, D, MODE == 2 ? 128 : 64>(a, Yg, ig, perm_s, smem, sl);
-        __syncthreads();
-        copy_slice(sl, S, tot);
+      double* Ys = reinterpret_cast<double*>(smem + a.y_off);
+      int* info = reinterpret_cast<int*>(smem + a.info_off);
+      const int N = a.Lx * a.Ly;
+      const double* Yg = static_cast<const double*>(a.Y) + (size_t)slot * n * D;
+      const int32_t* ig = a.idx + (size_t)slot * n;
+      if constexpr (MODE == 4) {
+        double* Yd = a.rows_slice ? reinterpret_cast<double*>(slb) : Ys;
+        int32_t* id = a.rows_slice ? reinterpret_cast<int32_t*>(Yd + n * D) : info;
+        features_to<double, TH>(a, item, smem, Yd, id, reinterpret_cast<float*>(xinv));
+        Yg = Yd;
+        ig = id;
       }
+      if (MODE == 2 || a.rows_slice) {
+        const double2* src = reinterpret_cast<const double2*>(Yg);
+        for (int v = tid; v < n * (D / 2); v += TH) reinterpret_cast<double2*>(Ys)[v] = src[v];
+        for (int p = tid; p < n; p += TH) info[p] = ig[p];
+        __syncthreads();
+      }
+      int mode_p = 0, mode_n = 0;
+      if (tid < n) {
+        mode_p = info[tid];
+        mode_n = tid + 1 < n ? info[tid + 1] : 2 * N;
+      }
+      __syncthreads();
+      if (tid < n) {
+        const int sp = mode_p >= N ? 1 : 0, site = mode_p - sp * N, x = site / a.Ly;
+        info[tid] = (sp << 16) | (x << 8) | (site - x * a.Ly);
+        if (sp == 0) atomicAdd(&nu_s, 1);
+        if (sp == 1 && mode_n < N) atomicOr(&nu_s, (int)0x80000000);
+      }
+      __syncthreads();
+      const int nus = nu_s;
+      gather_tiles<D, TH>(a, Ys, info, perm_s, nus & 0x7FFFFFFF, nus >= 0, smem, S,
+                          reinterpret_cast<double*>(slb));
     }
     __syncthreads();
 
-    // Phase 3: static-pivot blocked elimination.
-    double mant = 1.0;  // thread 0: running product of |x_t| as mantissa and exponent
-    int expo = 0, neg = 0, bad = 0;
-    for (int k0 = 0; k0 < n; k0 += kPW) {
-      const int w = min(kPW, n - k0), steps = w >> 1;
-      if (wid == 0) {
-        // (1) factorise the w x w pivot block: lane r holds row r, row[c] = B[r][c] (c < r);
-        // each step's columns k, k+1 go through shared memory to every lane.
-        double row[kPW];
-#pragma unroll
-        for (int c = 0; c < kPW; ++c)
-          row[c] = (lane < w && c < lane) ? S[roff(k0 + lane) + k0 + c] : 0.0;
-#pragma unroll
-        for (int t = 0; t < kPW / 2; ++t) {
-          if (t < steps) {
-            const int k = 2 * t;
-            const double xr = row[k], yr = row[k + 1];  // B[r][k], B[r][k+1] (lanes r > k+1)
-            if (lane < kPW) {
-              xy[0][lane] = xr;
-              xy[1][lane] = yr;
-            }
-            __syncwarp();
-            const double piv = -xy[0][k + 1];  // B[k][k+1] = -B[k+1][k]
-            const double inv = 1.0 / piv;
-            if (lane == 0) {
-              xs[t] = piv;
-              xinv[t] = inv;
-            }
-            if (lane >= k + 2 && lane < w) {
-              Lm[lane * kPW + k] = yr * inv;
-              Lm[lane * kPW + k + 1] = -xr * inv;
-            }
-            const double yi = yr * inv, xi = xr * inv;
-#pragma unroll
-            for (int c = 0; c < kPW; ++c)
-              if (c >= k + 2 && c < lane && lane < w) row[c] += yi * xy[0][c] - xi * xy[1][c];
-            __syncwarp();
-          }
-        }
-      }
-      __syncthreads();
-      if (tid == 0) {
-        for (int t = 0; t < steps; ++t) {
-          const double x = xs[t];
-          if (x < 0.0) neg ^= 1;
-          const double ax = fabs(x);
-          if (!(ax > 0.0) || !isfinite(ax)) bad |= ax == 0.0 ? NH_FLAG_ZERO_PIVOT : NH_FLAG_NONFINITE;
-          int e;
-          mant = frexp(mant * ax, &e);
-          expo += e;
-        }
-      }
-      const int base = k0 + w;
-      const int m = n - base;
-      if (m <= 0) break;
-      // (2) rows c >= base: W[:, c] = L11^-1 A12[:, c] with A12[i][c] = -S[c][k0 + i]; the dead
-      // slots S[c][k0, k0 + w) then hold P[c][2t] = W[2t+1][c] / x_t, P[c][2t+1] = -W[2t][c] / x_t.
-      for (int c = base + tid; c < n; c += kRThreads) {
-        double* sc = S + roff(c) + k0;
+    // Phase 2: static-pivot blocked elimination.  The pivots of panel p are kept in the W tile of
+    // tile row p, which no later step reads or writes.
+    if (wid == 0) factor_block(S, min(kPW, n), Lm, xinv, xy, Wb);
+    __syncthreads();
+    for (int p = 0; p + 1 < T; ++p) {
+      // (1) rows c >= base: W[:, c] = L11^-1 A12[:, c] with A12[i][c] = -S[c][k0 + i]; the dead
+      // tiles (I, p) then hold P[c][2t] = W[2t+1][c] / x_t, P[c][2t+1] = -W[2t][c] / x_t.
+      for (int c = 8 * (p + 1) + tid; c < n; c += TH) {
+        double* sc = S + (size_t)(tile_base(c >> 3) + p) * 64;
+        double* wc = Wb + (c >> 3) * 64;
         double wv[kPW];
 #pragma unroll
         for (int i = 0; i < kPW; i += 2) {
-          if (i < w) {
-            const double2 v = *reinterpret_cast<const double2*>(sc + i);
-            wv[i] = -v.x;
-            wv[i + 1] = -v.y;
-          } else {
-            wv[i] = wv[i + 1] = 0.0;
-          }
+          const double2 v = *reinterpret_cast<const double2*>(sc + toff(c & 7, i));
+          wv[i] = -v.x;
+          wv[i + 1] = -v.y;
         }
 #pragma unroll
         for (int t = 0; t < kPW / 2; ++t) {
           const int k = 2 * t;
 #pragma unroll
           for (int r = k + 2; r < kPW; ++r)
-            if (r < w) wv[r] -= Lm[r * kPW + k] * wv[k] + Lm[r * kPW + k + 1] * wv[k + 1];
+            wv[r] -= Lm[r * kPW + k] * wv[k] + Lm[r * kPW + k + 1] * wv[k + 1];
         }
 #pragma unroll
         for (int t = 0; t < kPW / 2; ++t) {
-          if (2 * t < w) {
-            const double inv = xinv[t];
-            *reinterpret_cast<double2*>(sc + 2 * t) =
-                make_double2(wv[2 * t + 1] * inv, -wv[2 * t] * inv);
-          }
+          const double inv = xinv[t];
+          *reinterpret_cast<double2*>(sc + toff(c & 7, 2 * t)) =
+              make_double2(wv[2 * t + 1] * inv, -wv[2 * t] * inv);
+          *reinterpret_cast<double2*>(wc + toff(c & 7, 2 * t)) = make_double2(wv[2 * t], wv[2 * t + 1]);
         }
       }
       __syncthreads();
-      // (3) trailing update S[a][b] += sum_i P[a][i] W[i][b] for base <= b < a: warp <-> a pair of
-      // rows, lane <-> columns b0 = base + 64 cb + lane and b0 + 32 (their W in registers), the
-      // rows' P broadcast; four elements and two partial sums each per lane keep the FP64 pipe
-      // fed.  All loads of a unit precede its stores.
-      if (m >= 2) {
-        double xv[kPW / 2];
-#pragma unroll
-        for (int t = 0; t < kPW / 2; ++t) xv[t] = t < steps ? xs[t] : 0.0;
-        // units: (column block cb, row pair) over rows base + 64 cb + 1 .. n - 1
-        auto pairs = [&](int cb) { return (m - 64 * cb - 1 + 1) >> 1; };
-        int total = 0;
-        for (int cb = 0; 64 * cb + 1 < m; ++cb) total += pairs(cb);
-        int cb = 0, rem = wid, cur = -1;
-        double w0[kPW], w1[kPW];
-        int b0 = 0, b1 = 0;
-#pragma unroll 1
-        for (int u = wid; u < total; u += kRWarps, rem += kRWarps) {
-          while (rem >= pairs(cb)) {
-            rem -= pairs(cb);
-            ++cb;
+      // (2) the next panel's column of tiles.
+      {
+        const Operand w = load_operand(Wb + (p + 1) * 64);
+        for (int I = p + 1 + wid; I < T; I += WARPS) {
+          double* row = S + (size_t)tile_base(I) * 64;
+          double2* cp = acc_ptr(row + (p + 1) * 64);
+          *cp = tile_mma(*cp, load_operand(row + p * 64), w);
+        }
+      }
+      __syncthreads();
+      // (3) warp 0: the next pivot block; the others: the remaining tiles, 2 x 2 at a time.
+      if (wid == 0) {
+        factor_block(S + (size_t)(tile_base(p + 1) + p + 1) * 64, min(kPW, n - 8 * (p + 1)), Lm, xinv,
+                     xy, Wb + (p + 1) * 64);
+      } else {
+        const int R = T - (p + 2), SR = (R + 1) >> 1;
+        int si = 0, rem = wid - 1;
+        for (;; rem += WARPS - 1) {
+          while (si < SR && rem > si) {
+            rem -= si + 1;
+            ++si;
           }
-          if (cb != cur) {
-            cur = cb;
-            b0 = base + 64 * cb + lane;
-            b1 = b0 + 32;
-#pragma unroll
-            for (int t = 0; t < kPW / 2; ++t) {
-              double2 p0 = make_double2(0.0, 0.0), p1 = make_double2(0.0, 0.0);
-              if (b0 < n) p0 = *reinterpret_cast<const double2*>(S + roff(b0) + k0 + 2 * t);
-              if (b1 < n) p1 = *reinterpret_cast<const double2*>(S + roff(b1) + k0 + 2 * t);
-              // W[2t][b] = -P[b][2t+1] x_t, W[2t+1][b] = P[b][2t] x_t
-              w0[2 * t] = -p0.y * xv[t];
-              w0[2 * t + 1] = p0.x * xv[t];
-              w1[2 * t] = -p1.y * xv[t];
-              w1[2 * t + 1] = p1.x * xv[t];
-            }
+          if (si >= SR) break;
+          const int I0 = p + 2 + 2 * si, J0 = p + 2 + 2 * rem;
+          const bool i2 = I0 + 1 < T, up = rem < si;  // second row; tile (I0, J0 + 1) exists
+          double* r0 = S + (size_t)tile_base(I0) * 64;
+          double* r1 = S + (size_t)tile_base(i2 ? I0 + 1 : I0) * 64;
+          const bool c2 = up || i2;  // column J0 + 1 is needed
+          const Operand a0 = load_operand(r0 + p * 64), a1 = load_operand(r1 + p * 64);
+          const Operand b0 = load_operand(Wb + J0 * 64);
+          const Operand b1 = load_operand(Wb + (c2 ? J0 + 1 : J0) * 64);
+          double2 *p00 = acc_ptr(r0 + J0 * 64), *p01 = acc_ptr(r0 + (up ? J0 + 1 : J0) * 64);
+          double2 *p10 = acc_ptr(r1 + J0 * 64), *p11 = acc_ptr(r1 + (c2 ? J0 + 1 : J0) * 64);
+          const double2 v00 = tile_mma(*p00, a0, b0);
+          const double2 v01 = tile_mma(*p01, a0, b1);
+          const double2 v10 = tile_mma(*p10, a1, b0);
+          const double2 v11 = tile_mma(*p11, a1, b1);
+          *p00 = v00;
+          if (up) *p01 = v01;
+          if (i2) {
+            *p10 = v10;
+            *p11 = v11;
           }
-          const int ra = base + 64 * cb + 1 + 2 * rem;  // rows ra and ra + 1
-          const int rb = ra + 1 < n ? ra + 1 : ra;
-          double* rowa = S + roff(ra);
-          double* rowb = S + roff(rb);
-          const bool a0 = b0 < ra, a1 = b1 < ra, c0 = rb != ra && b0 < rb, c1 = rb != ra && b1 < rb;
-          double acc[4][2];
-          acc[0][0] = a0 ? rowa[b0] : 0.0;
-          acc[1][0] = a1 ? rowa[b1] : 0.0;
-          acc[2][0] = c0 ? rowb[b0] : 0.0;
-          acc[3][0] = c1 ? rowb[b1] : 0.0;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) acc[e][1] = 0.0;
-#pragma unroll
-          for (int i = 0; i < kPW; i += 2) {
-            const double2 pa = *reinterpret_cast<const double2*>(rowa + k0 + i);
-            const double2 pb = *reinterpret_cast<const double2*>(rowb + k0 + i);
-            const int h = (i >> 1) & 1;
-            acc[0][h] = fma(pa.x, w0[i], acc[0][h]);
-            acc[1][h] = fma(pa.x, w1[i], acc[1][h]);
-            acc[2][h] = fma(pb.x, w0[i], acc[2][h]);
-            acc[3][h] = fma(pb.x, w1[i], acc[3][h]);
-            acc[0][h] = fma(pa.y, w0[i + 1], acc[0][h]);
-            acc[1][h] = fma(pa.y, w1[i + 1], acc[1][h]);
-            acc[2][h] = fma(pb.y, w0[i + 1], acc[2][h]);
-            acc[3][h] = fma(pb.y, w1[i + 1], acc[3][h]);
-          }
-          if (a0) rowa[b0] = acc[0][0] + acc[0][1];
-          if (a1) rowa[b1] = acc[1][0] + acc[1][1];
-          if (c0) rowb[b0] = acc[2][0] + acc[2][1];
-          if (c1) rowb[b1] = acc[3][0] + acc[3][1];
         }
       }
       __syncthreads();
     }
-    if (tid == 0) {
-      float s = a.item_sign ? a.item_sign[item] : 1.0f;
-      if (pr[n] & 1) s = -s;
-      if (neg) s = -s;
-      int f = a.flags ? a.flags[item] : 0;
-      f &= ~(kFlagNeedRefine | NH_FLAG_ZERO_PIVOT | NH_FLAG_NONFINITE);
-      double la = log(mant) + (double)expo * 0.6931471805599453;
-      if (isnan(s)) f |= NH_FLAG_NONFINITE;
-      if (bad & NH_FLAG_ZERO_PIVOT) {
-        s = 0.0f;
-        la = -INFINITY;
+    // log|pf| = sum of log|x_t| as one product per lane (mantissa and exponent), then a butterfly.
+    if (wid == 0) {
+      double mant = 1.0;
+      int expo = 0, neg = 0, bad = 0;
+      for (int t = lane; t < n / 2; t += 32) {
+        const double x = Wb[(t >> 2) * 64 + (t & 3)];
+        if (x < 0.0) neg ^= 1;
+        const double ax = fabs(x);
+        if (!(ax > 0.0) || !isfinite(ax)) bad |= ax == 0.0 ? NH_FLAG_ZERO_PIVOT : NH_FLAG_NONFINITE;
+        int e;
+        mant = frexp(mant * ax, &e);
+        expo += e;
       }
-      if (!isfinite(la) && s != 0.0f) bad |= NH_FLAG_NONFINITE;
-      f |= bad | NH_FLAG_REFINED;
-      a.sign[item] = s;
-      a.logabs[item] = s == 0.0f ? -INFINITY : la;
-      if (a.flags) a.flags[item] = f;
+#pragma unroll
+      for (int o = 16; o; o >>= 1) {
+        int e;
+        mant = frexp(mant * __shfl_xor_sync(0xffffffffu, mant, o), &e);
+        expo += __shfl_xor_sync(0xffffffffu, expo, o) + e;
+        neg ^= __shfl_xor_sync(0xffffffffu, neg, o);
+        bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+      }
+      if (lane == 0) {
+        float s = a.item_sign ? a.item_sign[item] : 1.0f;
+        if (pr[n] & 1) s = -s;
+        if (neg) s = -s;
+        int f = a.flags ? a.flags[item] : 0;
+        f &= ~(kFlagNeedRefine | NH_FLAG_ZERO_PIVOT | NH_FLAG_NONFINITE);
+        double la = log(mant) + (double)expo * 0.6931471805599453;
+        if (isnan(s)) f |= NH_FLAG_NONFINITE;
+        if (bad & NH_FLAG_ZERO_PIVOT) {
+          s = 0.0f;
+          la = -INFINITY;
+        }
+        if (!isfinite(la) && s != 0.0f) bad |= NH_FLAG_NONFINITE;
+        f |= bad | NH_FLAG_REFINED;
+        a.sign[item] = s;
+        a.logabs[item] = s == 0.0f ? -INFINITY : la;
+        if (a.flags) a.flags[item] = f;
+      }
     }
   }
 }
@@ -510,41 +679,83 @@ size_t stage_bytes(int n, int N, int D, int elt, bool wt) {
   return (size_t)elt * n * DP + sizeof(int) * ((n + 3) & ~3) + (wt ? (size_t)elt * 4 * N * DP : 0);
 }
 
+// Shared memory of one launch with TH threads (modes 2, 4: and the staging offsets); 0: too large.
 template <int D>
-int launch_refine_d(RefineArgs a, int max_slots, cudaStream_t st) {
-  const int N = a.Lx * a.Ly;
-  const size_t tri = sizeof(double) * tri_elems(a.n);
-  size_t smem = tri;
-  if (a.mode != 0) {
-    const int elt = (a.mode == 1 || a.mode == 3) ? 4 : 8;
-    a.stage_wt = stage_bytes(a.n, N, D, elt, true) <= kRefineSmemLimit;
-    smem = std::max(smem, stage_bytes(a.n, N, D, elt, a.stage_wt));
-    if (a.mode >= 3) smem = std::max(smem, features_smem(N, a.C, a.Lx, elt));
+size_t refine_smem(RefineArgs& a, int TH) {
+  const int N = a.Lx * a.Ly, n = a.n, T = tile_rows(n);
+  const size_t elim = tile_bytes(T) + 512 * (size_t)T;
+  size_t smem = elim;
+  if (a.mode == 1 || a.mode == 3) {
+    a.stage_wt = stage_bytes(n, N, D, 4, true) <= kRefineSmemLimit;
+    smem = std::max(smem, stage_bytes(n, N, D, 4, a.stage_wt));
+    if (a.mode == 3) smem = std::max(smem, features_smem(a.Lx, a.Ly, a.C, 4, TH));
+  } else if (a.mode != 0) {
+    const size_t y = 8 * (size_t)n * D, inf = (4 * (size_t)n + 15) & ~(size_t)15, wt = 8 * (size_t)N * D;
+    const size_t feat = a.mode == 4 ? (features_smem(a.Lx, a.Ly, a.C, 8, TH) + 15) & ~(size_t)15 : 0;
+    if (feat > kRefineSmemLimit) return 0;
+    a.rows_slice = feat + y + inf > kRefineSmemLimit;
+    smem = std::max(smem, a.rows_slice ? std::max(feat, y + inf) : feat + y + inf);
+    // One spin block of the table above the tiles' first rows, where it fits at all.
+    a.stage_wt = wt + y + inf <= kRefineSmemLimit;
+    if (a.stage_wt) smem = std::max(smem, wt + y + inf);
+    smem = (smem + 15) & ~(size_t)15;
+    a.info_off = (int)(smem - inf);
+    a.y_off = (int)(smem - inf - y);
+    a.wt_off = a.stage_wt ? (int)(smem - inf - y - wt) : a.y_off;
+    a.keep = T;
+    while (a.keep > 0 && tile_bytes(a.keep) > (size_t)a.wt_off) --a.keep;
   }
-  if (smem > kRefineSmemLimit)
-    return fail(NH_ERR_UNSUPPORTED, "refine: n=%d needs %zu B of shared memory", a.n, smem);
-  static bool configured[5] = {false, false, false, false, false};
-  auto kern = a.mode == 0 ? refine_kernel<D, 0> : a.mode == 1 ? refine_kernel<D, 1>
-            : a.mode == 2 ? refine_kernel<D, 2> : a.mode == 3 ? refine_kernel<D, 3>
-                                                 : refine_kernel<D, 4>;
-  if (!configured[a.mode]) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kRefineSmemLimit);
-    if (e != cudaSuccess) return check_cuda(e, "refine smem attribute");
-    configured[a.mode] = true;
-  }
-  int grid = num_sms();
+  return smem <= kRefineSmemLimit ? smem : 0;
+}
+
+template <int D, int MODE, int TH>
+int launch_refine_k(const RefineArgs& a, int max_slots, size_t smem, cudaStream_t st) {
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(refine_kernel<D, MODE, TH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)kRefineSmemLimit);
+  if (attr != cudaSuccess) return check_cuda(attr, "refine smem attribute");
+  int grid = num_sms() * (TH <= 256 ? 2 : 1);
   if (grid > max_slots) grid = max_slots;
   if (grid <= 0) return NH_OK;
   ProfScope prof_scope(NH_K_REFINE, st);
-  kern<<<grid, kRThreads, smem, st>>>(a);
+  refine_kernel<D, MODE, TH><<<grid, TH, smem, st>>>(a);
   return check_launch("refine_kernel");
+}
+
+// Two CTAs of 256 threads per SM where shared memory holds both (small lattices, whose phases are
+// latency-bound), else one of 512.
+constexpr size_t kTwoCtaSmem = 111 * 1024;  // dynamic, beside the static arrays
+
+template <int D, int MODE>
+int launch_refine_m(RefineArgs a, int max_slots, cudaStream_t st) {
+  const bool small = MODE != 4 || cnn_mma_fits(a.Lx, a.Ly, a.C, 256);
+  const size_t s256 = refine_smem<D>(a, 256);
+  if (small && s256 && s256 <= kTwoCtaSmem)
+    return launch_refine_k<D, MODE, 256>(a, max_slots, s256, st);
+  const size_t s512 = refine_smem<D>(a, 512);
+  if (!s512)
+    return fail(NH_ERR_UNSUPPORTED, "refine: n=%d does not fit in shared memory", a.n);
+  return launch_refine_k<D, MODE, 512>(a, max_slots, s512, st);
+}
+
+template <int D>
+int launch_refine_d(const RefineArgs& a, int max_slots, cudaStream_t st) {
+  switch (a.mode) {
+    case 1: return launch_refine_m<D, 1>(a, max_slots, st);
+    case 2: return launch_refine_m<D, 2>(a, max_slots, st);
+    case 3: return launch_refine_m<D, 3>(a, max_slots, st);
+    default: return launch_refine_m<D, 4>(a, max_slots, st);
+  }
 }
 
 }  // namespace
 
 size_t refine_slice_bytes(int n, int d) {
-  return (n > 0 && n <= kRefineMaxN) ? (size_t)num_sms() * slice_stride(n, d < 8 ? 8 : d) : 0;
+  if (n <= 0 || n > kRefineMaxN) return 0;
+  // one slice per CTA: two CTAs per SM only where the elimination alone leaves room for both
+  const int T = tile_rows(n);
+  const size_t per_sm = tile_bytes(T) + 512 * (size_t)T <= kTwoCtaSmem ? 2 : 1;
+  return per_sm * num_sms() * slice_stride(n, d < 8 ? 8 : d);
 }
 
 int launch_refine(const RefineLaunch& q, cudaStream_t st) {
@@ -579,7 +790,8 @@ int launch_refine(const RefineLaunch& q, cudaStream_t st) {
   a.layers = q.layers;
   if (q.mode >= 3 && (!q.cnn_w || !q.cnn_b || q.C % 16 || q.d * 2 != q.C))
     return fail(NH_ERR_INVALID, "refine: in-kernel features need the CNN weights");
-  switch (q.mode == 0 ? 16 : q.d) {
+  if (q.mode == 0) return launch_refine_m<16, 0>(a, q.max_slots, st);
+  switch (q.d) {
     case 8: return launch_refine_d<8>(a, q.max_slots, st);
     case 16: return launch_refine_d<16>(a, q.max_slots, st);
     case 32: return launch_refine_d<32>(a, q.max_slots, st);

@@ -14,11 +14,20 @@ import torch
 import neuralhubbard_b200 as nh
 from oracle import bcs as obcs
 from oracle import lattice as olat
+from oracle import pfaffian as opf
 from oracle import projection as oproj
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 TOL = 1e-8
+
+
+def log_error(la, l0):
+    """Largest difference of the finite logarithms; the infinite ones (a sum that vanishes by
+    symmetry) have to be the same."""
+    fin = np.isfinite(l0)
+    assert np.array_equal(la[~fin], l0[~fin])
+    return np.max(np.abs(la[fin] - l0[fin]), initial=0.0)
 
 
 def params_for(Lx, Ly, seed, ansatz="pfaffian"):
@@ -49,4 +58,68 @@ def test_fp64_features_through_bcs(Lx, Ly):
     model = nh.BCSBackflow(Lx, Ly, ne, ne, params=p, cond_tau=1.0)
     sg, la = nh.Variational(model)(s).numpy()
     assert np.array_equal(sg, s0)
-    assert np.max(np.abs(la - l0)) < TOL
+    assert log_error(la, l0) < TOL
+
+
+@pytest.mark.parametrize("n", [2, 6, 8, 10, 56, 110, 142, 222, 224])
+def test_refine_dense(n):
+    """Static-pivot FP64 factorisation of dense matrices: partial last panels (n mod 8 != 0), one
+    panel only, both thread counts and the largest n."""
+    rng = np.random.default_rng(n)
+    A = rng.normal(size=(5, n, n)).astype(np.float32)
+    A = A - np.swapaxes(A, 1, 2)
+    s0, l0 = opf.slogpf(A.astype(np.float64))
+    sg, la, _ = nh.slogpf(torch.from_numpy(A).to(DEV), cond_tau=1.0)
+    assert np.array_equal(sg.cpu().numpy(), s0)
+    assert np.max(np.abs(la.cpu().numpy() - l0)) < 1e-9
+
+
+# n = 2 and n = 224; a partial tile; unequal spins; few sites per block; a lattice whose FP64
+# features take the scalar path (16x17); 16 channels (d = 8).
+@pytest.mark.parametrize("Lx,Ly,up,dn,symm,channels", [
+    (3, 4, 1, 1, True, 32), (4, 4, 5, 3, True, 32), (8, 8, 28, 28, True, 32),
+    (5, 6, 0, 8, False, 32), (9, 12, 50, 44, False, 32), (10, 14, 61, 59, False, 32),
+    (16, 16, 112, 112, False, 32), (16, 17, 100, 98, False, 32), (8, 10, 35, 35, False, 16)])
+def test_refine_gather(Lx, Ly, up, dn, symm, channels):
+    """FP64 features, gather and factorisation of every image (cond_tau = 1), the fused form."""
+    N = Lx * Ly
+    p = nh.init_params(Lx, Ly, channels=channels, layers=4, std=0.1, seed=N + up)
+    s = olat.random_configs(np.random.default_rng(N), 3, N, up, dn)
+    s0, l0 = oproj.projected_amplitude(s, oracle_params(p, Lx, Ly), symm=symm)
+    model = nh.PfaffianBackflow(Lx, Ly, up, dn, params=p, cond_tau=1.0)
+    sg, la = nh.Variational(model, symm=symm)(s).numpy()
+    assert np.array_equal(sg, s0)
+    assert log_error(la, l0) < TOL
+
+
+def test_refine_refuses_wide_cnn():
+    """64 channels: the FP64 weights of a layer alone exceed shared memory."""
+    p = nh.init_params(6, 8, channels=64, layers=4, std=0.1, seed=1)
+    s = olat.random_configs(np.random.default_rng(1), 3, 48, 20, 22)
+    model = nh.PfaffianBackflow(6, 8, 20, 22, params=p, cond_tau=1.0)
+    with pytest.raises(nh.NativeLibraryError):
+        nh.Variational(model)(s)
+
+
+@pytest.mark.parametrize("cnn_mode", [0, 2])
+def test_refine_stored_features(cnn_mode):
+    """The unfused gather from stored FP64 rows (tensor-core CNN form; the residual network's
+    d = 32 with its wider rows), projected."""
+    L, N, ne = 16, 256, 112
+    rng = np.random.default_rng(3)
+    if cnn_mode == 2:
+        p = params_for(L, L, 5)
+        op = oracle_params(p, L, L)
+    else:
+        p = dict(net="resconv", embed=rng.normal(size=(64, 4)).astype(np.float32),
+                 conv_w=[(rng.normal(size=(64, 64, 3, 3)) * 0.04).astype(np.float32)] * 2,
+                 conv_b=[(rng.normal(size=64) * 0.1).astype(np.float32)] * 2,
+                 W=(rng.normal(size=(3, N, 32)) / np.sqrt(32)).astype(np.float32),
+                 theta=float(np.float32(0.55)))
+        op = dict(p, Lx=L, Ly=L, W=np.asarray(p["W"], np.float64))
+    s = olat.random_configs(rng, 2, N, ne, ne)
+    s0, l0 = oproj.projected_amplitude(s, op)
+    model = nh.PfaffianBackflow(L, L, ne, ne, params=p, cond_tau=1.0, cnn_mode=cnn_mode)
+    sg, la = nh.Variational(model)(s).numpy()
+    assert np.array_equal(sg, s0)
+    assert log_error(la, l0) < TOL
