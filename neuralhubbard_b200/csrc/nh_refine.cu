@@ -20,8 +20,8 @@
 // One CTA of 512 threads per SM (two of 256 where the lattice is small).  Phase 1 fills the permuted
 // lower triangle in shared memory, stored as 8 x 8 FP64 tiles (tile (I, J <= I) at index
 // I (I + 1) / 2 + J; 16-byte chunks swizzled inside a tile, see toff); phase 2 eliminates panels of
-// 8 columns: one warp factorises the 8 x 8 pivot block, one thread per row solves the panel, and
-// the trailing tiles take P W^T as two m8n8k4 FP64 products each.  The next panel's column is
+// 8 columns: one warp factorises the 8 x 8 pivot block, the panel rows are multiplied by the inverse
+// of its unit factor, and the trailing tiles take P W^T, all as m8n8k4 FP64 products.  The next panel's column is
 // updated first, so that its pivot block (a serial chain) is factorised by warp 0 while the other
 // warps update the rest.  n <= kRefineMaxN (224: the tiles take 203 KB).
 #include <math.h>
@@ -209,9 +209,10 @@ __device__ void gather_permuted(const RefineArgs& a, const T* Yg, const int32_t*
 
 // Phase 1 of modes 2 and 4: F[i][j] = sum_a (Y[i, a] Y[j, a]) Wt[2 s_i + s_j, r(i, j), a] of the
 // physical pairs i > j, scattered with its sign to the logical tile.  LPR lanes share a pair, each
-// with D / LPR of the a; a table row is then one contiguous 16 LPR-byte read (no bank conflicts,
-// where one lane per pair read 32 scattered rows), the column's features stay in registers, the
-// row's are a broadcast, and LPR rows are reduced together (each lane ends with one of them).
+// with CPL 16-byte chunks of the a; a table row is then read in contiguous pieces (no bank
+// conflicts, where one lane per pair read 32 scattered rows), the column's features stay in
+// registers, and LPR rows are reduced together.  Lane c takes the rows in the order u ^ c, so
+// that the reduction's exchanges need no selection and lane c ends with row c.
 // The table is staged one spin block at a time (uu, du, dd: the modes ascend, so rows and columns
 // of a block are ranges); unsorted mode lists (a wrong particle number) and lattices whose block
 // does not fit read it from global memory.
@@ -219,12 +220,17 @@ template <int D, int TH>
 __device__ void gather_tiles(const RefineArgs& a, const double* Ys, const int* info,
                              const uint16_t* iperm, int nu, bool sorted, unsigned char* smem,
                              double* S, double* slice) {
-  constexpr int LPR = D / 2 < 8 ? D / 2 : 8, CPL = D / (2 * LPR);  // lanes per pair, chunks per lane
-  constexpr int GR = 32 / LPR, JW = 2 * GR;                        // column groups, columns per warp
+  constexpr int LPR = D <= 16 ? 4 : 8, CPL = D / (2 * LPR);  // lanes per pair, chunks per lane
+  constexpr int GR = 32 / LPR, JW = 2 * GR;                  // column groups, columns per warp
   constexpr int WARPS = TH / 32;
   const int n = a.n, N = a.Lx * a.Ly;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int grp = lane / LPR, c = lane % LPR;
+  // Offset of chunk x of this lane in a row: with two chunks per lane, odd groups read theirs in
+  // the other order, so that the two groups of a quarter-warp use different banks.
+  int ch[CPL];
+#pragma unroll
+  for (int x = 0; x < CPL; ++x) ch[x] = 2 * (c + LPR * (CPL == 2 && LPR == 4 ? x ^ (grp & 1) : x));
   const double* Wg = static_cast<const double*>(a.Wt);
   double* wts = reinterpret_cast<double*>(smem + a.wt_off);
   const bool stage = a.stage_wt && sorted;
@@ -272,18 +278,18 @@ __device__ void gather_tiles(const RefineArgs& a, const double* Ys, const int* i
         infj[q] = info[jj];
 #pragma unroll
         for (int x = 0; x < CPL; ++x)
-          yj[q][x] = *reinterpret_cast<const double2*>(Ys + jj * D + 2 * (c + LPR * x));
+          yj[q][x] = *reinterpret_cast<const double2*>(Ys + jj * D + ch[x]);
       }
       const int ib = i0 + rb * LPR;
       double part[2][LPR];
 #pragma unroll
       for (int u = 0; u < LPR; ++u) {
-        const int i = min(ib + u, i1 - 1);
+        const int i = min(ib + (u ^ c), i1 - 1);
         const int infi = info[i];
         double2 yi[CPL];
 #pragma unroll
         for (int x = 0; x < CPL; ++x)
-          yi[x] = *reinterpret_cast<const double2*>(Ys + i * D + 2 * (c + LPR * x));
+          yi[x] = *reinterpret_cast<const double2*>(Ys + i * D + ch[x]);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           int dx = ((infi >> 8) & 0xFF) - ((infj[q] >> 8) & 0xFF);
@@ -293,30 +299,25 @@ __device__ void gather_tiles(const RefineArgs& a, const double* Ys, const int* i
           const int r = dx * a.Ly + dy;
           double acc = 0.0;
           const int blk = 2 * (infi >> 16) + (infj[q] >> 16);
-          const double2* wr = stage ? reinterpret_cast<const double2*>(wts + r * D) + c
-                                    : reinterpret_cast<const double2*>(Wg + (size_t)(blk * N + r) * D) + c;
+          const double* wr = stage ? wts + r * D : Wg + (size_t)(blk * N + r) * D;
 #pragma unroll
           for (int x = 0; x < CPL; ++x) {
-            const double2 w = wr[LPR * x];
+            const double2 w = *reinterpret_cast<const double2*>(wr + ch[x]);
             acc = fma(yi[x].x * yj[q][x].x, w.x, acc);
             acc = fma(yi[x].y * yj[q][x].y, w.y, acc);
           }
           part[q][u] = acc;
         }
       }
-      // Sum over the LPR lanes, row u ending in lane c = u: halves of the rows are exchanged.
+      // Sum over the LPR lanes: index u of lane c is row u ^ c, which its partner c ^ h holds at
+      // index u ^ h; row c stays.
 #pragma unroll
-      for (int h = LPR / 2; h; h >>= 1) {
-        const bool up = c & h;
+      for (int h = LPR / 2; h; h >>= 1)
 #pragma unroll
         for (int q = 0; q < 2; ++q)
 #pragma unroll
-          for (int u = 0; u < h; ++u) {
-            const double keep = up ? part[q][u + h] : part[q][u];
-            const double send = up ? part[q][u] : part[q][u + h];
-            part[q][u] = keep + __shfl_xor_sync(0xffffffffu, send, h);
-          }
-      }
+          for (int u = 0; u < h; ++u)
+            part[q][u] += __shfl_xor_sync(0xffffffffu, part[q][u + h], h);
       const int i = ib + c;
 #pragma unroll
       for (int q = 0; q < 2; ++q)
@@ -400,42 +401,45 @@ size_t features_smem(int Lx, int Ly, int C, int elt, int TH) {
   return ((act + 15) & ~(size_t)15) + (size_t)elt * ((size_t)C * C * 9 + C);
 }
 
-// Pivot block of panel p (w <= 8 columns) by one warp: lane r holds row r, row[c] = B[r][c]
-// (c < r); each step's columns k, k+1 go through shared memory to every lane.  Writes the block
-// multipliers Lm, the reciprocal pivots xinv and the pivots to piv[0, w / 2).
-__device__ __forceinline__ void factor_block(const double* D, int w, double* Lm, double* xinv,
-                                             double (*xy)[kPW], double* piv) {
-  const int lane = threadIdx.x & 31;
-  double row[kPW];
-#pragma unroll
-  for (int c = 0; c < kPW; ++c) row[c] = (lane < w && c < lane) ? D[toff(lane & 7, c)] : 0.0;
-#pragma unroll
-  for (int t = 0; t < kPW / 2; ++t) {
-    if (2 * t < w) {
-      const int k = 2 * t;
-      const double xr = row[k], yr = row[k + 1];  // B[r][k], B[r][k+1] (lanes r > k+1)
-      if (lane < kPW) {
-        xy[0][lane] = xr;
-        xy[1][lane] = yr;
+// Pivot block of a panel (w <= 8 columns) by one warp, two elements per lane: lane (r, q) = 4 r + q
+// holds B[r][2q], B[r][2q + 1] (the MMA accumulator layout; only c < r is used).  A step takes
+// its columns k, k + 1 from the lanes (r, k / 2) by shuffles; the same row operations applied to
+// the identity give the inverse of the block's unit lower factor, which the panel solve uses as
+// an MMA operand.  Writes Li (that inverse, a swizzled tile), the reciprocal pivots xinv and the
+// pivots to piv[0, w / 2).  The loop stays rolled (the code runs on one warp).
+__device__ __forceinline__ void factor_block(const double* D, int w, double* Li, double* xinv,
+                                             double* piv) {
+  const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
+  const double2 d = *reinterpret_cast<const double2*>(D + toff(r, 2 * q));
+  // entries outside the strict lower triangle of the w rows hold no data
+  double b0 = (r < w && 2 * q < r) ? d.x : 0.0, b1 = (r < w && 2 * q + 1 < r) ? d.y : 0.0;
+  double e0 = r == 2 * q ? 1.0 : 0.0, e1 = r == 2 * q + 1 ? 1.0 : 0.0;
+  const unsigned full = 0xffffffffu;
+#pragma unroll 1
+  for (int t = 0; 2 * t < w; ++t) {
+    const double x = -__shfl_sync(full, b0, (2 * t + 1) * 4 + t);  // B[k][k+1] = -B[k+1][k]
+    const double inv = 1.0 / x;
+    // B[r][k], B[r][k+1] of this row and of the rows 2q, 2q + 1 (this lane's columns)
+    const double xr = __shfl_sync(full, b0, (lane & 28) + t), yr = __shfl_sync(full, b1, (lane & 28) + t);
+    const double x0 = __shfl_sync(full, b0, 8 * q + t), y0 = __shfl_sync(full, b1, 8 * q + t);
+    const double x1 = __shfl_sync(full, b0, 8 * q + 4 + t), y1 = __shfl_sync(full, b1, 8 * q + 4 + t);
+    const double f0 = __shfl_sync(full, e0, 8 * t + q), f1 = __shfl_sync(full, e1, 8 * t + q);
+    const double g0 = __shfl_sync(full, e0, 8 * t + 4 + q), g1 = __shfl_sync(full, e1, 8 * t + 4 + q);
+    const double yi = yr * inv, xi = xr * inv;
+    if (r >= 2 * t + 2) {
+      if (2 * q >= 2 * t + 2) {
+        b0 = fma(yi, x0, fma(-xi, y0, b0));
+        b1 = fma(yi, x1, fma(-xi, y1, b1));
       }
-      __syncwarp();
-      const double x = -xy[0][k + 1];  // B[k][k+1] = -B[k+1][k]
-      const double inv = 1.0 / x;
-      if (lane == 0) {
-        piv[t] = x;
-        xinv[t] = inv;
-      }
-      const double yi = yr * inv, xi = xr * inv;
-      if (lane >= k + 2 && lane < w) {
-        Lm[lane * kPW + k] = yi;
-        Lm[lane * kPW + k + 1] = -xi;
-      }
-#pragma unroll
-      for (int c = 0; c < kPW; ++c)
-        if (c >= k + 2 && c < lane && lane < w) row[c] += yi * xy[0][c] - xi * xy[1][c];
-      __syncwarp();
+      e0 = fma(-yi, f0, fma(xi, g0, e0));
+      e1 = fma(-yi, f1, fma(xi, g1, e1));
+    }
+    if (lane == 0) {
+      piv[t] = x;
+      xinv[t] = inv;
     }
   }
+  *reinterpret_cast<double2*>(Li + toff(r, 2 * q)) = make_double2(e0, e1);
 }
 
 // Tile update C += P W^T: P and W are 8 x 8 tiles (rows x panel columns).
@@ -463,9 +467,8 @@ template <int D, int MODE, int TH>
 __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint16_t perm_s[kRefineMaxN];  // logical -> physical (modes 2, 4: physical -> logical)
-  __shared__ double Lm[kPW * kPW];          // block multipliers L[r][c] of the current panel
-  __shared__ double xinv[kPW / 2];          // reciprocals of its pivots
-  __shared__ double xy[2][kPW];             // pivot-block columns k, k+1 of the current step
+  __shared__ __align__(16) double Li[kPW * kPW];  // inverse unit factor of the current pivot block
+  __shared__ double xinv[kPW / 2];                // reciprocals of its pivots
   __shared__ int nu_s;                      // up modes of the item; bit 31: list not sorted by spin
   constexpr int WARPS = TH / 32;
   const int n = a.n, T = tile_rows(n);
@@ -553,34 +556,21 @@ __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArg
 
     // Phase 2: static-pivot blocked elimination.  The pivots of panel p are kept in the W tile of
     // tile row p, which no later step reads or writes.
-    if (wid == 0) factor_block(S, min(kPW, n), Lm, xinv, xy, Wb);
+    if (wid == 0) factor_block(S, min(kPW, n), Li, xinv, Wb);
     __syncthreads();
     for (int p = 0; p + 1 < T; ++p) {
-      // (1) rows c >= base: W[:, c] = L11^-1 A12[:, c] with A12[i][c] = -S[c][k0 + i]; the dead
-      // tiles (I, p) then hold P[c][2t] = W[2t+1][c] / x_t, P[c][2t+1] = -W[2t][c] / x_t.
-      for (int c = 8 * (p + 1) + tid; c < n; c += TH) {
-        double* sc = S + (size_t)(tile_base(c >> 3) + p) * 64;
-        double* wc = Wb + (c >> 3) * 64;
-        double wv[kPW];
-#pragma unroll
-        for (int i = 0; i < kPW; i += 2) {
-          const double2 v = *reinterpret_cast<const double2*>(sc + toff(c & 7, i));
-          wv[i] = -v.x;
-          wv[i + 1] = -v.y;
-        }
-#pragma unroll
-        for (int t = 0; t < kPW / 2; ++t) {
-          const int k = 2 * t;
-#pragma unroll
-          for (int r = k + 2; r < kPW; ++r)
-            wv[r] -= Lm[r * kPW + k] * wv[k] + Lm[r * kPW + k + 1] * wv[k + 1];
-        }
-#pragma unroll
-        for (int t = 0; t < kPW / 2; ++t) {
-          const double inv = xinv[t];
-          *reinterpret_cast<double2*>(sc + toff(c & 7, 2 * t)) =
-              make_double2(wv[2 * t + 1] * inv, -wv[2 * t] * inv);
-          *reinterpret_cast<double2*>(wc + toff(c & 7, 2 * t)) = make_double2(wv[2 * t], wv[2 * t + 1]);
+      // (1) tile rows I > p: W_I = -S_(I, p) Li^T (the forward substitution of every row as one
+      // product); the dead tile (I, p) then holds P[c][2t] = W[c][2t+1] / x_t, P[c][2t+1] =
+      // -W[c][2t] / x_t, both columns in this lane.
+      {
+        const Operand li = load_operand(Li);
+        const double inv = xinv[lane & 3];
+        for (int I = p + 1 + wid; I < T; I += WARPS) {
+          double* sc = S + (size_t)(tile_base(I) + p) * 64;
+          const double2 w = tile_mma(make_double2(0.0, 0.0), load_operand(sc), li);
+          __syncwarp();  // every lane has read its operand
+          *acc_ptr(sc) = make_double2(-w.y * inv, w.x * inv);
+          *acc_ptr(Wb + I * 64) = make_double2(-w.x, -w.y);
         }
       }
       __syncthreads();
@@ -596,12 +586,14 @@ __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArg
       __syncthreads();
       // (3) warp 0: the next pivot block; the others: the remaining tiles, 2 x 2 at a time.
       if (wid == 0) {
-        factor_block(S + (size_t)(tile_base(p + 1) + p + 1) * 64, min(kPW, n - 8 * (p + 1)), Lm, xinv,
-                     xy, Wb + (p + 1) * 64);
-      } else {
+        factor_block(S + (size_t)(tile_base(p + 1) + p + 1) * 64, min(kPW, n - 8 * (p + 1)), Li, xinv,
+                     Wb + (p + 1) * 64);
+      } else if (wid & 3) {
+        // not the warps of warp 0's scheduler, whose chain would queue behind their products
+        constexpr int NW = WARPS - WARPS / 4;
         const int R = T - (p + 2), SR = (R + 1) >> 1;
-        int si = 0, rem = wid - 1;
-        for (;; rem += WARPS - 1) {
+        int si = 0, rem = wid - 1 - (wid >> 2);
+        for (;; rem += NW) {
           while (si < SR && rem > si) {
             rem -= si + 1;
             ++si;
@@ -645,10 +637,9 @@ __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArg
         expo += e;
       }
 #pragma unroll
-      for (int o = 16; o; o >>= 1) {
-        int e;
-        mant = frexp(mant * __shfl_xor_sync(0xffffffffu, mant, o), &e);
-        expo += __shfl_xor_sync(0xffffffffu, expo, o) + e;
+      for (int o = 16; o; o >>= 1) {  // 32 mantissas in [1/2, 1): no underflow
+        mant *= __shfl_xor_sync(0xffffffffu, mant, o);
+        expo += __shfl_xor_sync(0xffffffffu, expo, o);
         neg ^= __shfl_xor_sync(0xffffffffu, neg, o);
         bad |= __shfl_xor_sync(0xffffffffu, bad, o);
       }
