@@ -106,6 +106,11 @@ static size_t refine_bytes(size_t items, int n, int d) {
          align256(sizeof(int32_t)) + align256(refine_slice_bytes(n, d));
 }
 
+// FP32 pairing table in chunks (the staged and fused gathers).
+static size_t wt_chunk_bytes(const nh_backflow_params& p) {
+  return sizeof(float) * 4 * (size_t)p.Lx * p.Ly * (size_t)(p.channels / 2);
+}
+
 size_t pipeline_bytes(int max_items, const nh_backflow_params& p) {
   const size_t it = (size_t)(max_items > 0 ? max_items : 1);
   const size_t n = (size_t)(p.n_up + p.n_dn), d = (size_t)(p.channels / 2);
@@ -114,7 +119,8 @@ size_t pipeline_bytes(int max_items, const nh_backflow_params& p) {
          align256(it * sizeof(int32_t)) * 2 + align256(sizeof(int32_t)) +
          align256(it * n * d * sizeof(double)) + align256(it * n * sizeof(int32_t)) +
          align256(sizeof(int32_t)) + align256(pfaffian_scratch_bytes((int)n)) +
-         align256(act_scratch_bytes(p)) + align256(it * sizeof(float)) + refine_bytes(it, (int)n, (int)d);
+         align256(act_scratch_bytes(p)) + align256(it * sizeof(float)) +
+         align256(wt_chunk_bytes(p)) + refine_bytes(it, (int)n, (int)d);
 }
 
 PipelineBuffers carve_pipeline(void* ws, int max_items, const nh_backflow_params& prm) {
@@ -142,6 +148,7 @@ PipelineBuffers carve_pipeline(void* ws, int max_items, const nh_backflow_params
   b.pf_tri = tri_bytes ? take(tri_bytes) : nullptr;
   b.cnn_act = act_bytes ? take(act_bytes) : nullptr;
   b.pf_ratio = reinterpret_cast<float*>(take(it * sizeof(float)));
+  b.wt_chunks = reinterpret_cast<float*>(take(wt_chunk_bytes(prm)));
   b.perm = nullptr;
   b.list32 = b.count32 = nullptr;
   b.slice = nullptr;
@@ -207,6 +214,7 @@ int run_pipeline(const ConfigList& cl, const nh_backflow_params& p, const Pipeli
   PfGatherArgs g{b.Y, b.idx, p.Wt, p.Lx, p.Ly, d, n, cl.n_cfg_dev, cl.G, max_items, nullptr,
                  b.item_sign, b.pf_sign, b.pf_logabs, b.pf_flags, p.cond_tau, 0, false, b.pf_tri};
   g.ratio = b.pf_ratio;
+  g.wt_chunks = b.wt_chunks;
   if (refine) {
     g.perm = b.perm;
     g.refine_tau = p.refine_tau;
@@ -269,6 +277,7 @@ struct FusedBuffers {
   uint16_t* perm;
   int32_t *list, *count, *list32, *count32, *queue;
   void* slice;
+  float* wt_chunks;
 };
 
 static bool fused_ok(const nh_backflow_params& p) {
@@ -279,7 +288,8 @@ static size_t fused_bytes(size_t items, const nh_backflow_params& p) {
   const int n = p.n_up + p.n_dn;
   return align256(items * sizeof(float)) * 3 + align256(items * sizeof(double)) +
          align256(items * sizeof(int32_t)) * 3 + align256(items * perm_stride(n) * 2) +
-         align256(sizeof(int32_t)) * 3 + align256(refine_slice_bytes(n, p.channels / 2));
+         align256(sizeof(int32_t)) * 3 + align256(refine_slice_bytes(n, p.channels / 2)) +
+         align256(wt_chunk_bytes(p));
 }
 
 static FusedBuffers carve_fused(void* ws, size_t items, const nh_backflow_params& p) {
@@ -303,6 +313,7 @@ static FusedBuffers carve_fused(void* ws, size_t items, const nh_backflow_params
   b.count32 = reinterpret_cast<int32_t*>(take(sizeof(int32_t)));
   b.queue = reinterpret_cast<int32_t*>(take(sizeof(int32_t)));
   b.slice = take(refine_slice_bytes(n, p.channels / 2));
+  b.wt_chunks = reinterpret_cast<float*>(take(wt_chunk_bytes(p)));
   return b;
 }
 
@@ -314,7 +325,7 @@ static int run_pipeline_fused(const ConfigList& cl, const nh_backflow_params& p,
   if (max_items <= 0) return NH_OK;
   int rc;
   FusedLaunch f{cl, &p, b.pf_sign, b.pf_logabs, b.pf_flags, b.pf_ratio, b.item_sign, b.perm,
-                b.queue};
+                b.queue, b.wt_chunks};
   if ((rc = launch_pfaffian_fused(f, st))) return rc;
   const bool fp64 = p.Wt64 && (p.cond_tau > 0.0 || (p.cancel_tau > 0.0 && cl.G > 1));
   if (fp64) {

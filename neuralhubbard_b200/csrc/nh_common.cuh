@@ -277,6 +277,7 @@ struct PipelineBuffers {
   int32_t* list32;    // (items,) items refined against their FP32 matrix
   int32_t* count32;   // (1,) their number
   void* slice;        // refinement: per-CTA permuted triangles (refine_slice_bytes)
+  float* wt_chunks;   // (4 N, d) FP32 pairing table in chunks (staged gather)
 };
 
 // uint16 words per item of the pivot-order record: perm[0, n) then the relabelling parity.
@@ -350,6 +351,7 @@ struct PfGatherArgs {
   uint16_t* perm = nullptr;  // when set: the pivot order of every item (perm_stride(n) words)
   double refine_tau = 0.0;   // pivot ratio above which kFlagNeedRefine is set (0: never)
   float* ratio = nullptr;    // when set: every item's pivot ratio
+  float* wt_chunks = nullptr;  // staged form: 4 N d floats for the FP32 table in chunks
 };
 
 // Launchers (return NH_OK or an error code).
@@ -377,6 +379,7 @@ struct FusedLaunch {
   float* item_sign;
   uint16_t* perm;
   int32_t* queue;
+  float* wt_chunks;  // 4 N d floats for the FP32 table in chunks
 };
 bool fused_supported(const nh_backflow_params& p);
 // The FP32 gather + Pfaffian with the item's rows copied into shared memory first (the gather

@@ -78,6 +78,7 @@ struct PfArgs {
   const void* Y;       // (slots, n, D) of T
   const int32_t* idx;  // (slots, n)
   const void* Wt;      // (4, N, D) of T
+  const float4* Wc;    // modes 2, 3: the FP32 table in chunks of four a (pair_chunks)
   int Lx, Ly;
   const int32_t* count_dev;  // work count on the device (times count_mult) or null
   int count_mult;
@@ -122,31 +123,6 @@ __host__ __device__ inline size_t cnn_phase_layout(int N, int C, int Lx, size_t*
 __device__ __forceinline__ int pack_mode(int m, int N, int Ly) {
   const int s = m >= N ? 1 : 0, site = m - s * N, x = site / Ly;
   return (s << 16) | (x << 8) | (site - x * Ly);
-}
-
-// F[p][q] (p > q) of the item from occupied rows Y (n, D, chunk-swizzled: swz_index) and packed
-// modes (pack_mode) in shared memory, the same arithmetic as pair_value:
-// sum_a (Y[p, a] Y[q, a]) Wt[2 s_p + s_q, r(p, q), a] in order of a.
-template <int D>
-__device__ __forceinline__ float pair_smem(const float* yp, int cp, const float* __restrict__ Ys,
-                                           const int* __restrict__ ids, int q, int N, int Lx,
-                                           int Ly, const float* __restrict__ Wt) {
-  const int cq = ids[q];
-  int dx = ((cp >> 8) & 0xff) - ((cq >> 8) & 0xff), dy = (cp & 0xff) - (cq & 0xff);
-  dx += dx < 0 ? Lx : 0;
-  dy += dy < 0 ? Ly : 0;
-  const float* wrow = Wt + ((size_t)(2 * (cp >> 16) + (cq >> 16)) * N + dx * Ly + dy) * D;
-  float acc = 0.0f;
-#pragma unroll
-  for (int a0 = 0; a0 < D; a0 += 4) {
-    const float4 w = __ldg(reinterpret_cast<const float4*>(wrow + a0));
-    const float4 v = *reinterpret_cast<const float4*>(Ys + swz_index<float, D>(q, a0));
-    acc = fmaf(yp[a0] * v.x, w.x, acc);
-    acc = fmaf(yp[a0 + 1] * v.y, w.y, acc);
-    acc = fmaf(yp[a0 + 2] * v.z, w.z, acc);
-    acc = fmaf(yp[a0 + 3] * v.w, w.w, acc);
-  }
-  return acc;
 }
 
 __device__ __forceinline__ int tri_off(int i) { return (i * (i - 1)) >> 1; }
@@ -210,20 +186,20 @@ __device__ void gather_lower(T* Lw, int n, const T* __restrict__ Y, const int32_
   }
 }
 
-// Load phase of modes 2 and 3: the item's occupied rows Y (n, D) and packed modes in shared memory
-// (mode 2: the CNN of its configuration in shared memory, write_occupied_rows, item sign to
-// item_sign_out; mode 3: copied from the global rows a.Y / a.idx of slot), then the gather of
-// the lower triangle from them.  Rows of the triangle that overlap Y (tail_row on) are computed
-// into registers first and stored after a barrier.
-constexpr int kTailRegs = 16;
+// Load phase of modes 2 and 3 by a TH-thread block: the item's occupied rows Y (n, D) and packed
+// modes in shared memory (mode 2: the CNN of its configuration in shared memory,
+// write_occupied_rows, item sign to item_sign_out; mode 3: copied from the global rows a.Y / a.idx
+// of slot), then the gather of the lower triangle from them.  Rows of the triangle that overlap Y
+// (tail_row on) are computed into registers first and stored after a barrier.
+constexpr int kTailElems = 4096;
 
-template <int D>
+template <int D, int TH>
 __device__ void features_to_smem(const PfArgs& a, int item, unsigned char* smem, float* Ys,
                                  int* ids);
-template <int D>
+template <int D, int TH>
 __device__ void gather_from_rows(const PfArgs& a, float* Lw, const float* Ys, const int* ids);
 
-template <int D>
+template <int D, int TH>
 __device__ void rows_and_gather(const PfArgs& a, int item, int slot, float* Lw,
                                 unsigned char* smem) {
   const int n = a.n;
@@ -235,28 +211,28 @@ __device__ void rows_and_gather(const PfArgs& a, int item, int slot, float* Lw,
                                                         (size_t)slot * n * D);
     constexpr int K = D / 4;  // 16-byte chunks per row, stored swizzled (swz_index)
     const int nv = n * K;
-    for (int v0 = tid; v0 < nv; v0 += 4 * kNumThreads) {
-      float4 buf[4];
+    for (int v0 = tid; v0 < nv; v0 += 2 * TH) {
+      float4 buf[2];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (v0 + u * kNumThreads < nv) buf[u] = __ldg(src + v0 + u * kNumThreads);
+      for (int u = 0; u < 2; ++u)
+        if (v0 + u * TH < nv) buf[u] = __ldg(src + v0 + u * TH);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int v = v0 + u * kNumThreads, row = v / K;
+      for (int u = 0; u < 2; ++u) {
+        const int v = v0 + u * TH, row = v / K;
         if (v < nv) reinterpret_cast<float4*>(Ys)[row * K + ((v % K) ^ swz_key(row, K))] = buf[u];
       }
     }
     const int N = a.Lx * a.Ly;
-    for (int p = tid; p < n; p += kNumThreads)
+    for (int p = tid; p < n; p += TH)
       ids[p] = pack_mode(__ldg(a.idx + (size_t)slot * n + p), N, a.Ly);
     __syncthreads();
   } else {
-    features_to_smem<D>(a, item, smem, Ys, ids);
+    features_to_smem<D, TH>(a, item, smem, Ys, ids);
   }
-  gather_from_rows<D>(a, Lw, Ys, ids);
+  gather_from_rows<D, TH>(a, Lw, Ys, ids);
 }
 
-template <int D>
+template <int D, int TH>
 __device__ void features_to_smem(const PfArgs& a, int item, unsigned char* smem, float* Ys,
                                  int* ids) {
   const int N = a.Lx * a.Ly, C = a.C, M2 = 2 * N, NS = N + 1;
@@ -276,74 +252,104 @@ __device__ void features_to_smem(const PfArgs& a, int item, unsigned char* smem,
   float* actB = actA + C * NS;
   float* wsm = reinterpret_cast<float*>(smem + ((act_end + 15) & ~(size_t)15));
   float* bsm = wsm + C * C * 9;
-  const float* in = cnn_layers<float>(a.cnn_w, a.cnn_b, a.Lx, a.Ly, C, a.layers, base, fr, to,
-                                      g, actA, actB, wsm, bsm, simg);
+  const float* in = cnn_layers<float, TH>(a.cnn_w, a.cnn_b, a.Lx, a.Ly, C, a.layers, base, fr, to,
+                                          g, actA, actB, wsm, bsm, simg);
   const int d = C / 2;
-  write_occupied_rows(simg, occl, wbuf, N, a.n, d, g, a.Lx, a.Ly, Ys, ids,
-                      a.item_sign_out + item,
-                      [&](int sg, int aa, int site) { return in[(sg * d + aa) * NS + site]; },
-                      true);
+  auto feat = [&](int sg, int aa, int site) { return in[(sg * d + aa) * NS + site]; };
+  write_occupied_rows<float, decltype(feat), TH>(simg, occl, wbuf, N, a.n, d, g, a.Lx, a.Ly, Ys,
+                                                 ids, a.item_sign_out + item, feat, true);
   __syncthreads();
-  for (int p = threadIdx.x; p < a.n; p += kNumThreads) ids[p] = pack_mode(ids[p], N, a.Ly);
+  for (int p = threadIdx.x; p < a.n; p += TH) ids[p] = pack_mode(ids[p], N, a.Ly);
   __syncthreads();
 }
 
+// The features of row p (chunk-swizzled rows, swz_index).
 template <int D>
+__device__ __forceinline__ void row_features(const float* Ys, int p, float* y) {
+#pragma unroll
+  for (int a0 = 0; a0 < D; a0 += 4) lds16(Ys + swz_index<float, D>(p, a0), y + a0);
+}
+
+// F[p][q] (p > q): sum_a (Y[p, a] Y[q, a]) Wt[2 s_p + s_q, r(p, q), a] in order of a (the
+// arithmetic of pair_value: the product of the features commutes).  Wc: the table in chunks,
+// Wc[(a / 4) 4 N + row] of four a, so that the lanes' neighbouring rows share cache lines.
+// yq: the column's features (a lane's registers, or nullptr to read row q of Ys).
+template <int D>
+__device__ __forceinline__ float pair_chunks(const float* Ys, int p, int cp, const float* yq, int q,
+                                             int cq, int N, int Lx, int Ly,
+                                             const float4* __restrict__ Wc) {
+  int dx = ((cp >> 8) & 0xff) - ((cq >> 8) & 0xff), dy = (cp & 0xff) - (cq & 0xff);
+  dx += dx < 0 ? Lx : 0;
+  dy += dy < 0 ? Ly : 0;
+  const float4* w4 = Wc + (2 * (cp >> 16) + (cq >> 16)) * N + dx * Ly + dy;
+  float acc = 0.0f;
+#pragma unroll
+  for (int c = 0; c < D / 4; ++c) {
+    const float4 w = __ldg(w4 + c * 4 * N);
+    float yp[4], yc[4];
+    lds16(Ys + swz_index<float, D>(p, 4 * c), yp);
+    if (yq) {
+#pragma unroll
+      for (int x = 0; x < 4; ++x) yc[x] = yq[4 * c + x];
+    } else {
+      lds16(Ys + swz_index<float, D>(q, 4 * c), yc);
+    }
+    acc = fmaf(yp[0] * yc[0], w.x, acc);
+    acc = fmaf(yp[1] * yc[1], w.y, acc);
+    acc = fmaf(yp[2] * yc[2], w.z, acc);
+    acc = fmaf(yp[3] * yc[3], w.w, acc);
+  }
+  return acc;
+}
+
+// Lane <-> column (its features in registers over the rows below), the row's features broadcast;
+// rows go to the warps in turn.  The shared-memory port bounds this loop: D / 4 broadcasts and
+// D / 4 table loads of about ten cache lines per 32 pairs.
+template <int D, int TH>
 __device__ void gather_from_rows(const PfArgs& a, float* Lw, const float* Ys, const int* ids) {
   const int n = a.n, N = a.Lx * a.Ly;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const float* Wt = static_cast<const float*>(a.Wt);
-  // rows below tail_row: straight into the triangle, warp <-> row, lane <-> two columns in flight
-  for (int p = wid; p < a.tail_row; p += kNumThreads / 32) {
-    float yp[D];
-#pragma unroll
-    for (int a0 = 0; a0 < D; a0 += 4) {
-      const float4 v = *reinterpret_cast<const float4*>(Ys + swz_index<float, D>(p, a0));
-      yp[a0] = v.x;
-      yp[a0 + 1] = v.y;
-      yp[a0 + 2] = v.z;
-      yp[a0 + 3] = v.w;
+  const float4* Wc = a.Wc;
+  int total = 0;  // (column block, row) units over the rows below tail_row
+  for (int q0 = 0; q0 + 1 < a.tail_row; q0 += 32) total += a.tail_row - q0 - 1;
+  int q0 = 0, rem = wid, cur = -1, cq = 0;
+  float yq[D];
+#pragma unroll 1
+  for (int u = wid; u < total; u += TH / 32, rem += TH / 32) {
+    while (rem >= a.tail_row - q0 - 1) {
+      rem -= a.tail_row - q0 - 1;
+      q0 += 32;
     }
-    const int mp = ids[p];
-    float* row = Lw + ((p * (p - 1)) >> 1);
-    int q = lane;
-    for (; q + 32 < p; q += 64) {
-      const float v0 = pair_smem<D>(yp, mp, Ys, ids, q, N, a.Lx, a.Ly, Wt);
-      const float v1 = pair_smem<D>(yp, mp, Ys, ids, q + 32, N, a.Lx, a.Ly, Wt);
-      row[q] = v0;
-      row[q + 32] = v1;
+    const int p = q0 + 1 + rem, q = q0 + lane;
+    if (q0 != cur) {
+      cur = q0;
+      const int qq = q < n ? q : n - 1;
+      row_features<D>(Ys, qq, yq);
+      cq = ids[qq];
     }
-    if (q < p) row[q] = pair_smem<D>(yp, mp, Ys, ids, q, N, a.Lx, a.Ly, Wt);
+    if (q < p)
+      Lw[tri_off(p) + q] = pair_chunks<D>(Ys, p, ids[p], yq, q, cq, N, a.Lx, a.Ly, Wc);
   }
   if (a.tail_row < n) {
-    // rows tail_row .. n-1 (E elements, at most kTailRegs per thread) through registers
-    const int t0 = (a.tail_row * (a.tail_row - 1)) >> 1;
-    const int E = ((n * (n - 1)) >> 1) - t0;
-    float v[kTailRegs];
+    // rows tail_row .. n-1 (E elements, at most kTailElems) through registers
+    const int t0 = tri_off(a.tail_row);
+    const int E = tri_off(n) - t0;
+    float v[kTailElems / TH];
 #pragma unroll
-    for (int k = 0; k < kTailRegs; ++k) {
-      const int e = tid + k * kNumThreads;
+    for (int k = 0; k < kTailElems / TH; ++k) {
+      const int e = tid + k * TH;
       v[k] = 0.0f;
       if (e < E) {
         int p = a.tail_row;
-        while ((((p + 1) * p) >> 1) - t0 <= e) ++p;
-        const int q = e - ((((p * (p - 1)) >> 1)) - t0);
-        float yp[D];
-#pragma unroll
-        for (int a0 = 0; a0 < D; a0 += 4) {
-          const float4 y4 = *reinterpret_cast<const float4*>(Ys + swz_index<float, D>(p, a0));
-          yp[a0] = y4.x;
-          yp[a0 + 1] = y4.y;
-          yp[a0 + 2] = y4.z;
-          yp[a0 + 3] = y4.w;
-        }
-        v[k] = pair_smem<D>(yp, ids[p], Ys, ids, q, N, a.Lx, a.Ly, Wt);
+        while (tri_off(p + 1) - t0 <= e) ++p;
+        const int q = e - (tri_off(p) - t0);
+        v[k] = pair_chunks<D>(Ys, p, ids[p], nullptr, q, ids[q], N, a.Lx, a.Ly, Wc);
       }
     }
     __syncthreads();  // every read of Y is done
 #pragma unroll
-    for (int k = 0; k < kTailRegs; ++k) {
-      const int e = tid + k * kNumThreads;
+    for (int k = 0; k < kTailElems / TH; ++k) {
+      const int e = tid + k * TH;
       if (e < E) Lw[t0 + e] = v[k];
     }
   }
@@ -386,24 +392,14 @@ __global__ void __launch_bounds__(THREADS, THREADS > kNumThreads ? 1 : (sizeof(T
   // to the lowest row.
   unsigned long long* cand = reinterpret_cast<unsigned long long*>(rkey);
   int* alist = rlog + WARPS;                       // (n) active physical rows
-  int* misc = alist + n;                            // [0] physical row of logical k, [1] item
+  int* misc = alist + n;                            // [0] physical row of logical k
 
   const int n_work = a.count_dev ? (*a.count_dev) * a.count_mult : a.n_slots;
   const T* Ybase = static_cast<const T*>(a.Y);
   const T* Wt = static_cast<const T*>(a.Wt);
-  for (int slot = blockIdx.x;; slot += gridDim.x) {
-    if (a.queue) {  // dynamic schedule: the next item comes off the work counter
-      __syncthreads();
-      if (tid == 0) misc[1] = atomicAdd(a.queue, 1);
-      __syncthreads();
-      slot = misc[1];
-    }
-    if (slot >= n_work) break;
+  for (int slot = blockIdx.x; slot < n_work; slot += gridDim.x) {
     const int item = a.slot_item ? a.slot_item[slot] : slot;
     __syncthreads();
-    if constexpr (sizeof(T) == 4 && THREADS == kNumThreads && D % 4 == 0) {
-      if (a.mode >= 2) rows_and_gather<D>(a, item, slot, Lw, smem_raw);
-    }
     if (a.mode == 0) {
       const float* F = a.F + (size_t)item * n * n;
       for (int i = wid; i < n; i += WARPS) {
@@ -415,9 +411,6 @@ __global__ void __launch_bounds__(THREADS, THREADS > kNumThreads ? 1 : (sizeof(T
       gather_lower<T, D, WARPS>(Lw, n, Ybase + (size_t)slot * n * D, a.idx + (size_t)slot * n,
                                 Wt, a.Lx, a.Ly);
     }
-    // Modes 2 and 3: the rows in shared memory can overlap the factorisation's scratch (misc
-    // among it), so every warp's gather reads end before the first scratch write.
-    if (a.mode >= 2) __syncthreads();
     if (tid == 0) misc[0] = 0;
     __syncthreads();
 
@@ -619,8 +612,7 @@ __global__ void __launch_bounds__(THREADS, THREADS > kNumThreads ? 1 : (sizeof(T
     if (tid == 0) {
       // Pfaffian = relabelling parity x product of the pivots, accumulated in FP64 as mantissa
       // and exponent; the pivot ratio flags near-nodal blocks.
-      const float* isg = a.mode == 2 ? a.item_sign_out : a.item_sign;
-      float s = isg ? isg[item] : 1.0f;
+      float s = a.item_sign ? a.item_sign[item] : 1.0f;
       double la, pmax_all = 0.0, pmin_all = 1.0;
       if (isnan(s)) flag |= NH_FLAG_NONFINITE;  // the CNN could not compute this item
       if (zero) {
@@ -713,14 +705,414 @@ int launch_pf(const PfArgs& a, cudaStream_t st) {
   return check_launch("pfaffian_kernel");
 }
 
-// FP32: the widest panel that keeps two CTAs per SM; FP64: one CTA per SM; beyond shared
-// memory (FP32 n > 256, FP64 n > 236): the large-lattice kernel.
+// ------------------------------------------------------------------ FP32, n <= 256
+// The factorisation of pfaffian_kernel (same operations in the same order, so the same bits) for
+// the matrices that fit in shared memory, organised around what bounds them: the 112 pivot steps
+// of n = 224 are latency, the trailing updates shared-memory traffic.
+//  * The active rows are compacted at the end of every panel (alist, clog: physical row and
+//    logical label in physical order), and a panel is run by ceil(m / 32) warps behind a named
+//    barrier of their own: warps without active rows do not repeat the step's work, and the last
+//    32 rows need no barrier at all.
+//  * The trailing update gives a lane four columns (their U / V in registers) where the row has
+//    them, so that a row's broadcast U / V serves 128 elements: a uniform 16-byte shared load costs
+//    two cycles of the load port (its register write), which is what bounds this phase.
+//  * The pivots are multiplied by one warp in parallel.
+constexpr int kPf32NB8MaxN = 224;  // panels of 8 up to here (two CTAs per SM), of 4 beyond
+
+struct Pf32Layout {
+  size_t us, vs, pivs, cand, rt, misc, alist, clog, end;  // byte offsets; the triangle is at 0
+};
+__host__ __device__ inline Pf32Layout pf32_layout(int n, int NB) {
+  Pf32Layout L;
+  L.us = sizeof(float) * ((((size_t)n * (n - 1)) / 2 + 3) & ~(size_t)3);
+  L.vs = L.us + sizeof(float) * (size_t)n * NB;
+  L.pivs = L.vs + sizeof(float) * (size_t)n * NB;
+  L.cand = (L.pivs + sizeof(float) * (size_t)(n / 2) + 15) & ~(size_t)15;
+  L.rt = L.cand + 8 * sizeof(unsigned long long);
+  L.misc = L.rt + 12 * sizeof(int);
+  L.alist = L.misc + 4 * sizeof(int);
+  L.clog = L.alist + n;
+  L.end = L.clog + n;
+  return L;
+}
+
+// Barrier of the PW panel warps (one warp: the warp's own).
+__device__ __forceinline__ void panel_sync(int PW) {
+  if (PW == 1)
+    __syncwarp();
+  else
+    asm volatile("bar.sync 1, %0;" ::"r"(32 * PW) : "memory");
+}
+
+// The panel values of one row: 16-byte loads of a swizzled row.
+template <int NB>
+__device__ __forceinline__ void panel_load(const float* Us, const float* Vs, int row, float* v,
+                                           float* u) {
+#pragma unroll
+  for (int q = 0; q < NB; q += 4) {
+    lds16(Vs + swz_index<float, NB>(row, q), v + q);
+    lds16(Us + swz_index<float, NB>(row, q), u + q);
+  }
+}
+
+// A[ph][q] with the panel's first j terms: panel values past j are zero on both sides.  Branch-free
+// but for the uniform half of the terms: both orientations of the element take one load.
+template <int NB>
+__device__ __forceinline__ float panel_value(const float* Lw, int ph, int off, int q, int j,
+                                             const float* U, const float* V, const float* vr,
+                                             const float* ur) {
+  float c = Lw[ph > q ? off + q : tri_off(q) + ph];
+  c = ph < q ? -c : c;
+  c = ph == q ? 0.0f : c;
+#pragma unroll
+  for (int p = 0; p < 4; ++p) c += U[p] * vr[p] - V[p] * ur[p];
+  if (NB > 4 && j > 4) {
+#pragma unroll
+    for (int p = 4; p < NB; ++p) c += U[p] * vr[p] - V[p] * ur[p];
+  }
+  return c;
+}
+
+// Panel of `steps` pivot steps from logical column k0 on the m active rows, one row per thread of
+// the first PW warps.  A step is bound by the number of instructions one warp issues in sequence
+// (about 150), so the rows are spread over the schedulers, the candidates are compared by
+// reductions and the loop stays rolled (unrolled, its code outgrows the instruction cache).
+// Measured at n = 224, two CTAs per SM: 1,350 cycles per step; two rows per thread 1,750, and one
+// barrier per step, every thread forming the next column's panel values itself, 1,500.  rt[8]
+// tells the block whether a column was exactly zero.
+template <int NB>
+__device__ __forceinline__ void panel_steps(float* Lw, float* Us, float* Vs, float* pivs,
+                                            unsigned long long* cand, int* rt, int* misc,
+                                            uint8_t* alist, uint8_t* clog, int m, int k0, int steps,
+                                            int PW, int& swaps, uint16_t* perm) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const bool has = tid < m;
+  const int ph = has ? alist[tid] : 0, off = tri_off(ph);
+  int log = has ? clog[tid] : -1;
+  if (has) {
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int p = 0; p < NB; p += 4) {
+      *reinterpret_cast<float4*>(Us + swz_index<float, NB>(ph, p)) = z;
+      *reinterpret_cast<float4*>(Vs + swz_index<float, NB>(ph, p)) = z;
+    }
+  }
+  if (wid == 0 && lane < 8) cand[lane] = 0ull;  // the slots of warps that do not run stay zero
+  panel_sync(PW);
+  bool zero = false;
+#pragma unroll 1
+  for (int j = 0; j < steps; ++j) {
+    const int k = k0 + 2 * j;
+    const int ck = misc[0];
+    float U[NB], V[NB], vr[NB], ur[NB];
+    panel_load<NB>(Us, Vs, ph, V, U);
+    panel_load<NB>(Us, Vs, ck, vr, ur);
+    const float c = panel_value<NB>(Lw, ph, off, ck, j, U, V, vr, ur);
+    // |c| bits + 1 (NaN as +inf); 0 for rows that are no longer active
+    const unsigned mag = min(__float_as_uint(c) & 0x7FFFFFFFu, 0x7F800000u);
+    const unsigned key = log > k ? mag + 1u : 0u;
+    // Maximum, ties to the lowest physical row (the rows ascend with the thread index).
+    unsigned kbest = __reduce_max_sync(0xffffffffu, key);
+    const int wl = __ffs(__ballot_sync(0xffffffffu, key == kbest)) - 1;
+    unsigned lbest = ((0xFFFFu - (unsigned)ph) << 16) | (signbit(c) ? 0x8000u : 0u) |
+                     ((unsigned)log & 0x7FFFu);
+    if (PW == 1) {
+      lbest = __shfl_sync(0xffffffffu, lbest, wl);
+    } else {
+      if (lane == wl) cand[wid] = ((unsigned long long)kbest << 32) | lbest;
+      panel_sync(PW);  // (1) pivot candidates
+      const unsigned long long w = cand[lane & 7];
+      const unsigned hi = (unsigned)(w >> 32);
+      kbest = __reduce_max_sync(0xffffffffu, hi);
+      lbest = __reduce_max_sync(0xffffffffu, hi == kbest ? (unsigned)w : 0u);
+    }
+    const float bk = kbest ? __uint_as_float(kbest - 1u) : -1.0f;
+    if (!(bk > 0.0f)) {  // exactly singular (or empty) column: pf = 0
+      zero = true;
+      panel_sync(PW);
+      break;
+    }
+    const int r = 0xFFFF - (int)(lbest >> 16);
+    const int lr = (int)(lbest & 0x7FFFu);
+    const float piv = (lbest & 0x8000u) ? bk : -bk;
+    panel_load<NB>(Us, Vs, r, vr, ur);
+    const float rp = 1.0f / piv;
+    // the row that held label k+1 takes the pivot's old label
+    log = has && ph == r ? k + 1 : (log == k + 1 ? lr : log);
+    const float u = panel_value<NB>(Lw, ph, off, r, j, U, V, vr, ur);
+    if (log > k + 1) {
+      const int o = swz_index<float, NB>(ph, j);
+      Us[o] = u;
+      Vs[o] = c * rp;
+    }
+    if (log == k + 2) misc[0] = ph;
+    if (tid == 0) pivs[k >> 1] = lr != k + 1 ? -piv : piv;
+    swaps ^= lr != k + 1 ? 1 : 0;
+    panel_sync(PW);  // (2) panel column written, next column's owner known
+  }
+  // Eliminated rows leave: their order to the record, the others compacted in physical order.
+  const int k_end = k0 + 2 * steps;
+  const unsigned bal = __ballot_sync(0xffffffffu, log >= k_end);
+  if (lane == 0) rt[wid] = __popc(bal);
+  if (perm && !zero && log >= 0 && log < k_end) perm[log] = (uint16_t)ph;
+  panel_sync(PW);
+  if (log >= k_end) {
+    int i = __popc(bal & ((1u << lane) - 1u));
+    for (int w = 0; w < wid; ++w) i += rt[w];
+    alist[i] = (uint8_t)ph;
+    clog[i] = (uint8_t)log;
+  }
+  if (tid == 0) rt[8] = zero ? 1 : 0;
+}
+
+// Trailing update of one unit: RT consecutive active rows from ia0, NC columns per lane
+// (c0 + lane + 32 i of the active list; physical rows pb, panel values ub / vb).
+template <int NB, int RT, int NC, int NCB>
+__device__ __forceinline__ void trail_unit(float* Lw, const float* Us, const float* Vs,
+                                           const uint8_t* alist, int m, int ia0, int c0,
+                                           const int (&pb)[NCB], const float (&ub)[NCB][NB],
+                                           const float (&vb)[NCB][NB]) {
+  const int lane = threadIdx.x & 31;
+  float acc[RT][NC];
+  int pa[RT], off[RT];
+#pragma unroll
+  for (int rr = 0; rr < RT; ++rr) {
+    pa[rr] = alist[ia0 + rr < m ? ia0 + rr : ia0];
+    off[rr] = tri_off(pa[rr]);
+  }
+#pragma unroll
+  for (int rr = 0; rr < RT; ++rr)
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      const bool ok = ia0 + rr < m && c0 + lane + 32 * i < ia0 + rr;
+      acc[rr][i] = ok ? Lw[off[rr] + pb[i]] : 0.0f;
+    }
+#pragma unroll
+  for (int h = 0; h < NB; h += 4) {
+    float ua[RT][4], va[RT][4];
+#pragma unroll
+    for (int rr = 0; rr < RT; ++rr) {
+      lds16(Us + swz_index<float, NB>(pa[rr], h), ua[rr]);
+      lds16(Vs + swz_index<float, NB>(pa[rr], h), va[rr]);
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+      for (int rr = 0; rr < RT; ++rr) {
+#pragma unroll
+        for (int i = 0; i < NC; ++i) acc[rr][i] = fmaf(ua[rr][p], vb[i][h + p], acc[rr][i]);
+#pragma unroll
+        for (int i = 0; i < NC; ++i) acc[rr][i] = fmaf(-va[rr][p], ub[i][h + p], acc[rr][i]);
+      }
+  }
+#pragma unroll
+  for (int rr = 0; rr < RT; ++rr)
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      const bool ok = ia0 + rr < m && c0 + lane + 32 * i < ia0 + rr;
+      if (ok) Lw[off[rr] + pb[i]] = acc[rr][i];
+    }
+}
+
+// Trailing update of the columns [c0, c0 + 32 NC) of the active list over the rows below;
+// done counts the units handed out so far, so that the warps stay evenly loaded across blocks.
+template <int NB, int NC, int WARPS>
+__device__ __forceinline__ void trail_block(float* Lw, const float* Us, const float* Vs,
+                                            const uint8_t* alist, int m, int c0, int& done) {
+  constexpr int RT = 2;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int units = (m - c0 - 1 + RT - 1) / RT;
+  const int u0 = (wid - done) & (WARPS - 1);
+  done += units;
+  if (u0 >= units) return;
+  int pb[NC];
+  float ub[NC][NB], vb[NC][NB];
+#pragma unroll
+  for (int i = 0; i < NC; ++i) {
+    const int ib = c0 + lane + 32 * i;
+    pb[i] = alist[ib < m ? ib : m - 1];
+#pragma unroll
+    for (int p = 0; p < NB; p += 4) {
+      lds16(Us + swz_index<float, NB>(pb[i], p), ub[i] + p);
+      lds16(Vs + swz_index<float, NB>(pb[i], p), vb[i] + p);
+    }
+  }
+  for (int u = u0; u < units; u += WARPS) {
+    const int ia0 = c0 + 1 + u * RT;
+    if (NC == 4 && ia0 + RT - 1 <= c0 + 64)  // no row reaches the upper half of the columns
+      trail_unit<NB, RT, NC / 2, NC>(Lw, Us, Vs, alist, m, ia0, c0, pb, ub, vb);
+    else
+      trail_unit<NB, RT, NC, NC>(Lw, Us, Vs, alist, m, ia0, c0, pb, ub, vb);
+  }
+}
+
+template <int NB, int D, int TH>
+__global__ void __launch_bounds__(TH, 512 / TH) pf32_kernel(PfArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int WARPS = TH / 32;
+  const int n = a.n;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const Pf32Layout L = pf32_layout(n, NB);
+  float* Lw = reinterpret_cast<float*>(smem_raw);
+  float* Us = reinterpret_cast<float*>(smem_raw + L.us);  // (n, NB), swizzled chunks (swz_index)
+  float* Vs = reinterpret_cast<float*>(smem_raw + L.vs);
+  float* pivs = reinterpret_cast<float*>(smem_raw + L.pivs);  // pivot A[k, k+1], negated on a swap
+  unsigned long long* cand = reinterpret_cast<unsigned long long*>(smem_raw + L.cand);
+  int* rt = reinterpret_cast<int*>(smem_raw + L.rt);        // compaction counts; [8] zero column
+  int* misc = reinterpret_cast<int*>(smem_raw + L.misc);    // [0] row of logical k, [1] item
+  uint8_t* alist = smem_raw + L.alist;
+  uint8_t* clog = smem_raw + L.clog;
+
+  const int n_work = a.count_dev ? (*a.count_dev) * a.count_mult : a.n_slots;
+  for (int slot = blockIdx.x;; slot += gridDim.x) {
+    if (a.queue) {  // dynamic schedule: the next item comes off the work counter
+      __syncthreads();
+      if (tid == 0) misc[1] = atomicAdd(a.queue, 1);
+      __syncthreads();
+      slot = misc[1];
+    }
+    if (slot >= n_work) break;
+    const int item = a.slot_item ? a.slot_item[slot] : slot;
+    __syncthreads();
+    if (a.mode >= 2) {
+      rows_and_gather<D, TH>(a, item, slot, Lw, smem_raw);
+    } else if (a.mode == 0) {
+      const float* F = a.F + (size_t)item * n * n;
+      for (int i = wid; i < n; i += WARPS) {
+        const float* src = F + (size_t)i * n;
+        float* dst = Lw + tri_off(i);
+        for (int j = lane; j < i; j += 32) dst[j] = __ldg(src + j);
+      }
+    } else {
+      gather_lower<float, D, WARPS>(Lw, n, static_cast<const float*>(a.Y) + (size_t)slot * n * D,
+                             a.idx + (size_t)slot * n, static_cast<const float*>(a.Wt), a.Lx, a.Ly);
+    }
+    __syncthreads();  // the rows in shared memory can overlap the scratch written next
+    for (int p = tid; p < n; p += TH) alist[p] = clog[p] = (uint8_t)p;
+    if (tid == 0) misc[0] = 0;
+    __syncthreads();
+
+    uint16_t* perm = a.perm ? a.perm + (size_t)item * perm_stride(n) : nullptr;
+    int swaps = 0;
+    bool zero = false;
+    for (int k0 = 0; k0 < n - 1; k0 += 2 * NB) {
+      const int steps = min(NB, (n - k0) >> 1);
+      const int m = n - k0, PW = (m + 31) >> 5;
+      if (wid < PW)
+        panel_steps<NB>(Lw, Us, Vs, pivs, cand, rt, misc, alist, clog, m, k0, steps, PW, swaps,
+                           perm);
+      __syncthreads();  // panel written, active rows compacted
+      zero = rt[8] != 0;
+      if (zero) break;
+      const int mt = m - 2 * steps;
+      if (mt >= 2) {  // then steps == NB
+        int done = 0;
+        for (int c0 = 0; c0 + 1 < mt;) {
+          if (mt - c0 > 64) {
+            trail_block<NB, 4, WARPS>(Lw, Us, Vs, alist, mt, c0, done);
+            c0 += 128;
+          } else {
+            trail_block<NB, 2, WARPS>(Lw, Us, Vs, alist, mt, c0, done);
+            c0 += 64;
+          }
+        }
+        __syncthreads();  // trailing triangle updated
+      }
+    }
+    if (wid == 0) {
+      // Pfaffian = relabelling parity x product of the pivots, accumulated in FP64 as mantissa
+      // and exponent (one product per lane, then a butterfly); the pivot ratio flags near-nodal
+      // blocks.
+      int flag = 0, neg = 0, expo = 0;
+      double mant = 1.0;
+      float pmin = INFINITY, pmax = 0.0f;
+      if (!zero)
+        for (int k = lane; k < n / 2; k += 32) {
+          const float pv = pivs[k];
+          if (pv < 0.0f) neg ^= 1;
+          const float ap = fabsf(pv);
+          if (!isfinite(ap)) flag |= NH_FLAG_NONFINITE;
+          pmin = fminf(pmin, ap);
+          pmax = fmaxf(pmax, ap);
+          mant *= (double)ap;  // at most 4 FP32 magnitudes per lane
+        }
+      mant = frexp(mant, &expo);
+#pragma unroll
+      for (int o = 16; o; o >>= 1) {
+        mant *= __shfl_xor_sync(0xffffffffu, mant, o);
+        expo += __shfl_xor_sync(0xffffffffu, expo, o);
+        neg ^= __shfl_xor_sync(0xffffffffu, neg, o);
+        flag |= __shfl_xor_sync(0xffffffffu, flag, o);
+        pmin = fminf(pmin, __shfl_xor_sync(0xffffffffu, pmin, o));
+        pmax = fmaxf(pmax, __shfl_xor_sync(0xffffffffu, pmax, o));
+      }
+      if (lane == 0) {
+        const float* isg = a.mode == 2 ? a.item_sign_out : a.item_sign;
+        float s = isg ? isg[item] : 1.0f;
+        double la;
+        if (isnan(s)) flag |= NH_FLAG_NONFINITE;  // the CNN could not compute this item
+        if (zero) {
+          s = 0.0f;
+          la = -INFINITY;
+          flag |= NH_FLAG_ZERO_PIVOT;
+        } else {
+          if (neg) s = -s;
+          la = log(mant) + (double)expo * 0.6931471805599453;
+          if (!isfinite(la)) flag |= NH_FLAG_NONFINITE;
+          if (a.cond_tau > 0.0 && (double)pmax > a.cond_tau * (double)pmin) flag |= NH_FLAG_GROWTH;
+          if (a.refine_tau > 0.0 && (double)pmax > a.refine_tau * (double)pmin)
+            flag |= kFlagNeedRefine;
+        }
+        if (s == 0.0f) la = -INFINITY;
+        a.sign[item] = s;
+        a.logabs[item] = la;
+        if (a.flags) a.flags[item] = flag | a.flag_or;
+        if (a.ratio) a.ratio[item] = zero ? INFINITY : (float)((double)pmax / (double)pmin);
+        if (perm && !zero) perm[n] = (uint16_t)swaps;
+      }
+    }
+  }
+}
+
+// Launch with the panel width of n: 8 up to kPf32NB8MaxN, else 4 (the width is part of the
+// operation order, so it depends on n alone).
+template <int NB, int D, int TH>
+int launch_pf32_th(const PfArgs& a, size_t smem, int per_sm, int prof_id, cudaStream_t st) {
+  if (int rc = raise_smem_cap(pf32_kernel<NB, D, TH>, smem)) return rc;
+  int grid = num_sms() * per_sm;
+  if (grid > a.n_slots) grid = a.n_slots;
+  if (grid <= 0) return NH_OK;
+  ProfScope prof_scope(prof_id, st);
+  pf32_kernel<NB, D, TH><<<grid, TH, smem, st>>>(a);
+  return check_launch("pf32_kernel");
+}
+
+// Two CTAs of 256 threads per SM (one beyond 113 KB), or, where there are items for them, four of
+// 128 that shared memory and one row per thread allow: small matrices leave most of 256 threads
+// idle, and their steps are latency.
+template <int NB, int D>
+int launch_pf32_nb(const PfArgs& a, size_t smem, int prof_id, cudaStream_t st) {
+  if (smem > 227 * 1024)
+    return fail(NH_ERR_UNSUPPORTED, "Pfaffian: n=%d needs %zu B of shared memory", a.n, smem);
+  if (smem <= 56 * 1024 && a.n <= 128 && a.n_slots > 2 * num_sms())
+    return launch_pf32_th<NB, D, 128>(a, smem, 4, prof_id, st);
+  return launch_pf32_th<NB, D, 256>(a, smem, smem <= 113 * 1024 ? 2 : 1, prof_id, st);
+}
+
+template <int D>
+int launch_pf32(const PfArgs& a, cudaStream_t st) {
+  return a.n <= kPf32NB8MaxN
+             ? launch_pf32_nb<8, D>(a, pf32_layout(a.n, 8).end, NH_K_PFAFFIAN, st)
+             : launch_pf32_nb<4, D>(a, pf32_layout(a.n, 4).end, NH_K_PFAFFIAN, st);
+}
+
+// FP32 up to 256 rows: pf32_kernel; FP64: one CTA per SM; beyond shared memory (FP32 n > 256, FP64
+// n > 236): the large-lattice kernel.
 template <typename T, int D>
 int launch_pf_pick(const PfArgs& a, cudaStream_t st) {
   if (a.n <= kNumThreads) {
     if constexpr (sizeof(T) == 4) {
-      if (pf_smem<T, 8>(a.n) <= 113 * 1024) return launch_pf<T, 8, D>(a, st);
-      return launch_pf<T, 4, D>(a, st);
+      return launch_pf32<D>(a, st);
     } else {
       if (pf_smem<T, 4>(a.n) <= 227 * 1024) return launch_pf<T, 4, D>(a, st);
       if (pf_smem<T, 2>(a.n) <= 227 * 1024) return launch_pf<T, 2, D>(a, st);
@@ -1455,21 +1847,18 @@ int launch_pfaffian_gather(const PfGatherArgs& g, cudaStream_t st) {
 template <int NB, int D>
 int launch_fused_nb(PfArgs a, cudaStream_t st) {
   const int n = a.n, N = a.Lx * a.Ly;
-  constexpr int WARPS = kWarps;
-  const size_t pf = pf_smem<float, NB>(n);
+  const Pf32Layout L = pf32_layout(n, NB);
   size_t cnn_end = 0, act_end = 0;  // mode 3 (rows copied from global memory): no CNN phase
   if (a.mode == 2) act_end = cnn_phase_layout(N, a.C, a.Lx, &cnn_end);
-  const size_t tri_pad = ((size_t)n * (n - 1) / 2 + 3) & ~(size_t)3;
-  const size_t tri_bytes = 4 * tri_pad, y_bytes = 4 * (size_t)n * D;
+  const size_t tri_bytes = L.us, y_bytes = 4 * (size_t)n * D;
   const size_t two_cta = 113 * 1024;
   // A: rows after the triangle and the activation planes, modes after the rows.
   const size_t yA = (std::max(act_end, tri_bytes) + 15) & ~(size_t)15;
-  const size_t totA = std::max(std::max(pf, cnn_end), yA + y_bytes + 4 * (size_t)n);
-  // B: rows in the triangle's tail (rows from tail_row gathered through registers), modes in the
-  // active-row list of the factorisation.
+  const size_t totA = std::max(std::max(L.end, cnn_end), yA + y_bytes + 4 * (size_t)n);
+  // B: rows in the triangle's tail (rows from tail_row gathered through registers), modes at the
+  // end of the panel (not yet in use).
   const size_t yB = (tri_bytes - y_bytes) & ~(size_t)15;
-  const size_t alist_off = 4 * (tri_pad + 2 * (size_t)n * NB + (((size_t)n / 2 + 3) & ~(size_t)3)) +
-                           4 * (size_t)WARPS * 3;
+  const size_t idsB = L.pivs - 4 * (size_t)n;
   int tail = n;
   if (y_bytes < tri_bytes) {
     const size_t yf = yB / 4;
@@ -1477,9 +1866,9 @@ int launch_fused_nb(PfArgs a, cudaStream_t st) {
     while (tail < n && (size_t)tail * (tail - 1) / 2 + tail <= yf) ++tail;
   }
   const size_t tail_elems = (size_t)n * (n - 1) / 2 - (size_t)tail * (tail - 1) / 2;
-  const size_t totB = std::max(pf, cnn_end);
-  const bool okB = y_bytes < tri_bytes && yB >= act_end && alist_off >= act_end &&
-                   tail_elems <= (size_t)kTailRegs * kNumThreads;
+  const size_t totB = std::max(L.end, cnn_end);
+  const bool okB = y_bytes < tri_bytes && yB >= act_end && idsB >= act_end &&
+                   tail_elems <= (size_t)kTailElems;
   size_t smem;
   if (totA <= two_cta || !okB || totB > two_cta) {
     smem = totA;
@@ -1489,24 +1878,19 @@ int launch_fused_nb(PfArgs a, cudaStream_t st) {
   } else {
     smem = totB;
     a.y_off = (int)yB;
-    a.idx_off = (int)alist_off;
+    a.idx_off = (int)idsB;
     a.tail_row = tail;
   }
-  if (smem > 227 * 1024)
-    return fail(NH_ERR_UNSUPPORTED, "fused amplitude: n=%d, N=%d needs %zu B of shared memory", n,
-                N, smem);
-  if (int rc = raise_smem_cap(pfaffian_kernel<float, NB, D, kNumThreads>, smem)) return rc;
-  const int per_sm = smem <= two_cta ? 2 : 1;
-  int grid = num_sms() * per_sm;
-  if (grid > a.n_slots) grid = a.n_slots;
-  if (grid <= 0) return NH_OK;
   if (a.queue) {
     cudaError_t e = cudaMemsetAsync(a.queue, 0, sizeof(int32_t), st);
     if (e != cudaSuccess) return check_cuda(e, "fused amplitude: clear work counter");
   }
-  ProfScope prof_scope(a.mode == 2 ? NH_K_FUSED : NH_K_PFAFFIAN, st);
-  pfaffian_kernel<float, NB, D, kNumThreads><<<grid, kNumThreads, smem, st>>>(a);
-  return check_launch("pfaffian_kernel (fused features)");
+  return launch_pf32_nb<NB, D>(a, smem, a.mode == 2 ? NH_K_FUSED : NH_K_PFAFFIAN, st);
+}
+
+template <int D>
+int launch_fused_d(const PfArgs& a, cudaStream_t st) {
+  return a.n <= kPf32NB8MaxN ? launch_fused_nb<8, D>(a, st) : launch_fused_nb<4, D>(a, st);
 }
 
 int launch_pfaffian_tc(const PfGatherArgs& g, int mode, const float* F, int32_t* err,
@@ -1568,11 +1952,32 @@ bool fused_supported(const nh_backflow_params& p) {
 }
 
 bool staged_supported(const PfGatherArgs& g) {
-  return !g.fp64 && g.n <= kNumThreads && g.n % 2 == 0 && g.d % 4 == 0 && g.d <= 32 && !g.tri;
+  return !g.fp64 && g.n <= kNumThreads && g.n % 2 == 0 && g.d % 4 == 0 && g.d <= 32 && !g.tri &&
+         g.wt_chunks;
+}
+
+// Wt (rows, d) to chunks of four a: Wc[(a / 4) rows + row].
+__global__ void wt_chunk_kernel(const float4* __restrict__ Wt, int rows, int chunks,
+                                float4* __restrict__ Wc) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < rows * chunks; e += gridDim.x * blockDim.x) {
+    const int c = e / rows, row = e - c * rows;
+    Wc[e] = __ldg(Wt + (size_t)row * chunks + c);
+  }
+}
+
+static int launch_wt_chunks(const float* Wt, int N, int d, float* Wc, cudaStream_t st) {
+  const int total = 4 * N * (d / 4);
+  ProfScope prof_scope(NH_K_PACK, st);
+  wt_chunk_kernel<<<(total + 255) / 256, 256, 0, st>>>(reinterpret_cast<const float4*>(Wt), 4 * N,
+                                                       d / 4, reinterpret_cast<float4*>(Wc));
+  return check_launch("wt_chunk_kernel");
 }
 
 int launch_pfaffian_staged(const PfGatherArgs& g, cudaStream_t st) {
+  if (int rc = launch_wt_chunks(static_cast<const float*>(g.Wt), g.Lx * g.Ly, g.d, g.wt_chunks, st))
+    return rc;
   PfArgs a{};
+  a.Wc = reinterpret_cast<const float4*>(g.wt_chunks);
   a.n = g.n;
   a.mode = 3;
   a.Y = g.Y;
@@ -1593,11 +1998,10 @@ int launch_pfaffian_staged(const PfGatherArgs& g, cudaStream_t st) {
   a.perm = g.perm;
   a.refine_tau = g.refine_tau;
   a.ratio = g.ratio;
-  const bool nb8 = pf_smem<float, 8>(a.n) <= 113 * 1024;
   switch (g.d) {
-    case 8: return nb8 ? launch_fused_nb<8, 8>(a, st) : launch_fused_nb<4, 8>(a, st);
-    case 16: return nb8 ? launch_fused_nb<8, 16>(a, st) : launch_fused_nb<4, 16>(a, st);
-    case 32: return nb8 ? launch_fused_nb<8, 32>(a, st) : launch_fused_nb<4, 32>(a, st);
+    case 8: return launch_fused_d<8>(a, st);
+    case 16: return launch_fused_d<16>(a, st);
+    case 32: return launch_fused_d<32>(a, st);
     default: return fail(NH_ERR_UNSUPPORTED, "staged Pfaffian: d=%d", g.d);
   }
 }
@@ -1605,7 +2009,9 @@ int launch_pfaffian_staged(const PfGatherArgs& g, cudaStream_t st) {
 int launch_pfaffian_fused(const FusedLaunch& f, cudaStream_t st) {
   const nh_backflow_params& p = *f.p;
   if (!fused_supported(p)) return fail(NH_ERR_UNSUPPORTED, "fused amplitude: unsupported network");
+  if (int rc = launch_wt_chunks(p.Wt, p.Lx * p.Ly, p.channels / 2, f.wt_chunks, st)) return rc;
   PfArgs a{};
+  a.Wc = reinterpret_cast<const float4*>(f.wt_chunks);
   a.n = p.n_up + p.n_dn;
   a.mode = 2;
   a.Wt = p.Wt;
@@ -1628,11 +2034,10 @@ int launch_pfaffian_fused(const FusedLaunch& f, cudaStream_t st) {
   a.layers = p.layers;
   a.item_sign_out = f.item_sign;
   a.queue = f.queue;
-  const bool nb8 = pf_smem<float, 8>(a.n) <= 113 * 1024;
   switch (p.channels / 2) {
-    case 8: return nb8 ? launch_fused_nb<8, 8>(a, st) : launch_fused_nb<4, 8>(a, st);
-    case 16: return nb8 ? launch_fused_nb<8, 16>(a, st) : launch_fused_nb<4, 16>(a, st);
-    case 32: return nb8 ? launch_fused_nb<8, 32>(a, st) : launch_fused_nb<4, 32>(a, st);
+    case 8: return launch_fused_d<8>(a, st);
+    case 16: return launch_fused_d<16>(a, st);
+    case 32: return launch_fused_d<32>(a, st);
     default: return fail(NH_ERR_UNSUPPORTED, "fused amplitude: d=%d", p.channels / 2);
   }
 }
