@@ -123,3 +123,21 @@ def test_refine_stored_features(cnn_mode):
     sg, la = nh.Variational(model)(s).numpy()
     assert np.array_equal(sg, s0)
     assert log_error(la, l0) < TOL
+
+
+# 128-row blocks are the largest two CTAs share in FP32 and the largest in FP64; 33 and 65 open a
+# new column group.
+@pytest.mark.parametrize("Lx,Ly,nh_", [(4, 4, 1), (8, 8, 32), (8, 9, 33), (10, 13, 65),
+                                       (16, 16, 128)])
+def test_determinant_blocks(Lx, Ly, nh_):
+    """BCS determinant at the edges of its register blocks: all FP64 against the oracle, and the
+    default mixed path within the 1e-4 bar of the mixed forms."""
+    N = Lx * Ly
+    p = params_for(Lx, Ly, 7 * N + nh_, "bcs")
+    s = olat.random_configs(np.random.default_rng(nh_), 2, N, nh_, nh_)
+    s0, l0 = obcs.projected_amplitude(s, oracle_params(p, Lx, Ly))
+    for tau, tol in ((1.0, TOL), (5.0, 1e-4)):
+        model = nh.BCSBackflow(Lx, Ly, nh_, nh_, params=p, cond_tau=tau)
+        sg, la = nh.Variational(model)(s).numpy()
+        assert np.array_equal(sg, s0)
+        assert log_error(la, l0) < tol
