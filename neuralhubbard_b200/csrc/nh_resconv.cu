@@ -20,8 +20,10 @@
 // latency hides behind the FMAs.  Per (input channel, tap) a thread issues 4 activation loads,
 // 4 broadcast 16-byte weight loads and 64 FMAs.  The output rows Y of the occupied modes, their
 // indices and the item sign are written by the same epilogue as the plain CNN's.
+#include <cooperative_groups.h>
 #include <math.h>
 
+#include "nh_cnn_mma.cuh"
 #include "nh_common.cuh"
 
 namespace nh {
@@ -315,6 +317,240 @@ __global__ void __launch_bounds__(kRcThreads, 1) resconv_kernel(RcArgs<T> a) {
   }
 }
 
+// FP64 features on the FP64 matrix instruction, mode 1 only, lattices up to 256 sites: a cluster of
+// two CTAs per item, each with half of the output channels.  The convolutions are the implicit GEMMs
+// of nh_cnn_mma.cuh (same products in the same order as conv_pass); both CTAs keep the whole
+// input's padded planes in shared memory (166 KB at 16x16) and write their halves of every new
+// activation to both.  The residual stream x stays in registers, in the accumulator layout.  The
+// weights stream through two 9 KB chunks (4 input channels, in fragment order), the next one in
+// registers.  Half an item per CTA also halves the granularity of the last wave: the recompute
+// lists are a few items per SM.  478 items of 16 blocks at 16x16: 25.4 ms by conv_pass in FP64 with
+// its planes in global memory, 9.6 ms here (the FMA floor, evenly spread, is 7.7 ms).
+constexpr int kRmThreads = 512;
+constexpr int kRmChunk = 9 * 4 * 32;  // weights of one chunk: 36 k x 32 channels
+constexpr int kRmPre = (kRmChunk + kRmThreads - 1) / kRmThreads;
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRmThreads, 1)
+    resconv_mma_kernel(RcArgs<double> a) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double red[kRmThreads / 32];
+  __shared__ double part[2];  // both CTAs' sums of x^2
+  constexpr int NT = 4, WARPS = kRmThreads / 32;
+  const int Lx = a.Lx, Ly = a.Ly, N = a.N, M2 = 2 * N, W = Ly + 2, PS = mma_plane(Lx, Ly);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  double* act = reinterpret_cast<double*>(smem_raw);
+  double* wsm = act + (size_t)kRcC * PS;
+  int* simg = reinterpret_cast<int*>(wsm + 2 * kRmChunk);
+  int* occl = simg + M2;
+  int* wbuf = occl + M2;
+  double* act_peer = cluster.map_shared_rank(act, rank ^ 1);
+  double* part_peer = cluster.map_shared_rank(part, rank ^ 1);
+
+  const int G = a.cl.G;
+  const int n_work = a.slot_item ? *a.slot_count
+                                 : (a.cl.n_cfg_dev ? *a.cl.n_cfg_dev : a.cl.n_cfg) * G;
+  const size_t conv_floats = (size_t)kRcC * 9 * kRcC;
+  const int convs = 2 * a.blocks;
+  const double inv_cn = 1.0 / (double)(kRcC * N), out_scale = trsqrt_eps((double)(a.blocks + 1), 0.0);
+  const int co0 = 32 * rank + 2 * (lane & 3);  // this lane's channels: co0 + 8 nt, co0 + 8 nt + 1
+
+  // Site tiles warp and warp + WARPS: this lane's row is site 8 tile + lane / 4.
+  const int MT = (N + 7) >> 3;
+  const int tiles = warp + WARPS < MT ? 2 : (warp < MT ? 1 : 0);
+  int pad[2], site[2];
+  bool live[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int st = 8 * (warp + i * WARPS) + (lane >> 2);
+    live[i] = i < tiles && st < N;
+    site[i] = live[i] ? st : 0;
+    const int x = site[i] / Ly;
+    pad[i] = (x + 1) * W + site[i] - x * Ly + 1;
+  }
+  int off[9];  // operand offsets of the nine groups of four k in 4 channels x 9 taps
+#pragma unroll
+  for (int j = 0; j < 9; ++j) {
+    const int k = 4 * j + (lane & 3), tap = k % 9;
+    off[j] = (k / 9) * PS + (tap / 3) * W + tap % 3;
+  }
+  float pre[kRmPre];
+  auto prefetch = [&](const float* w) {  // w: 36 k rows of 64 channels
+#pragma unroll
+    for (int q = 0; q < kRmPre; ++q) {
+      const int i = tid + q * kRmThreads, ln = i & 31;
+      if (i < kRmChunk)
+        pre[q] = __ldg(w + (4 * (i >> 7) + (ln & 3)) * kRcC + 32 * rank + ((i >> 5) & 3) * 8 + (ln >> 2));
+    }
+  };
+  // One convolution of the planes in act; acc starts from the bias.  next: the first chunk that
+  // follows.
+  auto conv = [&](double (&acc)[2][NT][2], const float* w, const float* bias, const float* next) {
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+      const double b0 = (double)__ldg(bias + co0 + 8 * nt), b1 = (double)__ldg(bias + co0 + 8 * nt + 1);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        acc[i][nt][0] = b0;
+        acc[i][nt][1] = b1;
+      }
+    }
+    const double* a0 = act + pad[0] - W - 1;
+    const double* a1 = act + pad[1] - W - 1;
+#pragma unroll 1
+    for (int ch = 0; ch < kRcC / 4; ++ch) {
+      double* buf = wsm + (ch & 1) * kRmChunk;
+#pragma unroll
+      for (int q = 0; q < kRmPre; ++q) {
+        const int i = tid + q * kRmThreads;
+        if (i < kRmChunk) buf[i] = (double)pre[q];
+      }
+      __syncthreads();
+      prefetch(ch + 1 < kRcC / 4 ? w + (size_t)(ch + 1) * 36 * kRcC : next);
+      const double* ws = buf + lane;
+      if (tiles == 2) {
+#pragma unroll
+        for (int j = 0; j < 9; ++j) {
+          const double x0 = a0[off[j]], x1 = a1[off[j]];
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) {
+            const double b = ws[(j * NT + nt) * 32];
+            mma_f64(acc[0][nt], x0, b);
+            mma_f64(acc[1][nt], x1, b);
+          }
+        }
+      } else if (tiles == 1) {
+#pragma unroll
+        for (int j = 0; j < 9; ++j) {
+          const double x0 = a0[off[j]];
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt) mma_f64(acc[0][nt], x0, ws[(j * NT + nt) * 32]);
+        }
+      }
+      a0 += 4 * PS;
+      a1 += 4 * PS;
+    }
+  };
+  // This CTA's half of the new planes to both CTAs, then the borders of all planes.  Both CTAs have
+  // finished reading the old planes before the call.
+  auto publish = [&](auto value) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (live[i]) {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int o = (co0 + 8 * nt + h) * PS + pad[i];
+            const double v = value(i, nt, h);
+            act[o] = v;
+            act_peer[o] = v;
+          }
+      }
+    cluster.sync();
+    mma_halo<kRmThreads>(act, kRcC, PS, Lx, Ly);
+    __syncthreads();
+  };
+
+  prefetch(a.wp);
+  const int clusters = gridDim.x >> 1;
+  for (int slot = blockIdx.x >> 1; slot < n_work; slot += clusters) {
+    const int item = a.slot_item ? a.slot_item[slot] : slot;
+    const int c = item / G, g = item - c * G;
+    const int smp = a.cl.sample ? a.cl.sample[c] : c;
+    const int fr = a.cl.from ? a.cl.from[c] : -1;
+    const int to = a.cl.from ? a.cl.to[c] : -1;
+    const int8_t* base = a.cl.spins + (int64_t)smp * M2;
+    __syncthreads();  // the previous item's readers of simg are done
+    for (int m = tid; m < M2; m += kRmThreads) {
+      const int src = sym_map(m, g, Lx, Ly, N);  // image[m] = s[g(m)] (g is an involution)
+      simg[m] = move_value(src, base[src], fr, to) > 0 ? 1 : -1;
+    }
+    __syncthreads();
+    double x[2][NT][2], acc[2][NT][2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {  // occupation embedding
+      const int occ = (simg[site[i]] > 0 ? 1 : 0) + (simg[N + site[i]] > 0 ? 2 : 0);
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          x[i][nt][h] = live[i] ? (double)__ldg(a.embed + occ * kRcC + co0 + 8 * nt + h) : 0.0;
+    }
+    for (int blk = 0; blk < a.blocks; ++blk) {
+      double ss = 0.0;
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) ss = fma(x[i][nt][h], x[i][nt][h], ss);
+#pragma unroll
+      for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (lane == 0) red[warp] = ss;
+      __syncthreads();
+      if (tid == 0) {
+        double t = 0.0;
+        for (int w = 0; w < WARPS; ++w) t += red[w];
+        part[rank] = t;
+        part_peer[rank] = t;
+      }
+      cluster.sync();  // both sums known; both CTAs are done with the old planes
+      const double r = trsqrt_eps((part[0] + part[1]) * inv_cn, kRmsEps);
+      const float* w1 = a.wp + (size_t)(2 * blk) * conv_floats;
+      const float* w2 = w1 + conv_floats;
+      publish([&](int i, int nt, int h) { return gelu_tanh(x[i][nt][h] * r); });
+      conv(acc, w1, a.b + (2 * blk) * kRcC, w2);
+      cluster.sync();
+      publish([&](int i, int nt, int h) { return gelu_tanh(acc[i][nt][h]); });
+      conv(acc, w2, a.b + (2 * blk + 1) * kRcC, 2 * blk + 2 < convs ? w2 + conv_floats : a.wp);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) x[i][nt][h] = live[i] ? x[i][nt][h] + acc[i][nt][h] : 0.0;
+    }
+    cluster.sync();
+    publish([&](int i, int nt, int h) { return x[i][nt][h] * out_scale; });
+    if (rank == 0) {
+      constexpr int d = kRcC / 2;
+      auto feat = [&](int sg, int aa, int st) {
+        const int px = st / Ly;
+        return act[(sg * d + aa) * PS + (px + 1) * W + st - px * Ly + 1];
+      };
+      write_occupied_rows<double, decltype(feat), kRmThreads>(
+          simg, occl, wbuf, N, a.n, d, g, Lx, Ly, a.Y + (int64_t)slot * a.n * d,
+          a.idx + (int64_t)slot * a.n, a.item_sign + item, feat);
+    }
+  }
+  cluster.sync();  // no CTA leaves while the other may still write to it
+}
+
+size_t rm_smem(int Lx, int Ly) {
+  return sizeof(double) * ((size_t)kRcC * mma_plane(Lx, Ly) + 2 * kRmChunk) +
+         sizeof(int) * (4 * (size_t)Lx * Ly + 4 * Lx + 32);
+}
+
+int launch_resconv_mma(const CnnLaunch& q, int N, cudaStream_t st) {
+  const nh_backflow_params& p = *q.p;
+  const int slots = q.slot_item ? q.max_slots : q.cl->n_cfg * q.cl->G;
+  if (slots <= 0) return NH_OK;
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      resconv_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024);
+  if (attr != cudaSuccess) return check_cuda(attr, "resconv smem attribute");
+  int grid = num_sms() & ~1;
+  if (grid > 2 * slots) grid = 2 * slots;
+  RcArgs<double> a{*q.cl, p.conv_w_packed, p.conv_w_packed + 4 * kRcC, p.conv_b, p.Lx, p.Ly, N,
+                   p.layers, p.n_up + p.n_dn, q.mode, q.slot_item, q.slot_count, q.max_slots,
+                   nullptr, static_cast<double*>(q.Y), q.idx, q.item_sign, nullptr};
+  ProfScope prof_scope(NH_K_RESCONV64, st);
+  resconv_mma_kernel<<<grid, kRmThreads, rm_smem(p.Lx, p.Ly), st>>>(a);
+  return check_launch("resconv_mma_kernel");
+}
+
 // packed = [embed (4, C): [occ][co]] ++ per conv k [ci][tap][co];
 // conv_w = [embed (C, 4)] ++ per conv k (C, C, 3, 3).
 __global__ void resconv_pack_kernel(const float* __restrict__ w, int C, int convs,
@@ -402,7 +638,12 @@ int launch_resconv(const CnnLaunch& q, cudaStream_t st) {
                 "is null");
   if (reinterpret_cast<uintptr_t>(p.conv_w_packed) % 16)
     return fail(NH_ERR_INVALID, "resconv: conv_w_packed must be 16-byte aligned");
-  if (q.fp64) return launch_rc_t<double, true>(q, N, st);
+  if (q.fp64) {
+    // two site tiles per warp of the 512-thread CTAs, planes in shared memory
+    if (q.mode == 1 && N <= 16 * (kRmThreads / 32) && rm_smem(p.Lx, p.Ly) <= 226 * 1024)
+      return launch_resconv_mma(q, N, st);
+    return launch_rc_t<double, true>(q, N, st);
+  }
   return rc_smem<float, false>(N) <= 227 * 1024 ? launch_rc_t<float, false>(q, N, st)
                                                  : launch_rc_t<float, true>(q, N, st);
 }

@@ -141,3 +141,25 @@ def test_determinant_blocks(Lx, Ly, nh_):
         sg, la = nh.Variational(model)(s).numpy()
         assert np.array_equal(sg, s0)
         assert log_error(la, l0) < tol
+
+
+# 6 sites to a partial tile, 64 (half of the warps), 16 x 16 (the largest of the cluster form) and
+# 10 x 28 beyond it.
+@pytest.mark.parametrize("Lx,Ly,ne,blocks", [(3, 4, 3, 1), (5, 6, 10, 2), (8, 8, 28, 3),
+                                             (16, 16, 100, 2), (10, 28, 60, 1)])
+def test_resconv_fp64(Lx, Ly, ne, blocks):
+    """FP64 residual network: one cluster of two CTAs per image, more images than clusters."""
+    N = Lx * Ly
+    rng = np.random.default_rng(N)
+    p = dict(net="resconv", embed=rng.normal(size=(64, 4)).astype(np.float32),
+             conv_w=[(rng.normal(size=(64, 64, 3, 3)) * 0.04).astype(np.float32)
+                     for _ in range(2 * blocks)],
+             conv_b=[(rng.normal(size=64) * 0.1).astype(np.float32) for _ in range(2 * blocks)],
+             W=(rng.normal(size=(3, N, 32)) / np.sqrt(32)).astype(np.float32),
+             theta=float(np.float32(0.55)))
+    s = olat.random_configs(rng, 3, N, ne, ne)
+    s0, l0 = oproj.projected_amplitude(s, dict(p, Lx=Lx, Ly=Ly, W=np.asarray(p["W"], np.float64)))
+    model = nh.PfaffianBackflow(Lx, Ly, ne, ne, params=p, cond_tau=1.0)
+    sg, la = nh.Variational(model)(np.tile(s, (6, 1))).numpy()
+    assert np.array_equal(sg, np.tile(s0, 6))
+    assert log_error(la, np.tile(l0, 6)) < TOL
