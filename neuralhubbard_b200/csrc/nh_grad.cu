@@ -78,8 +78,8 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adjoint_kernel(AdjArgs a) {
   float* colbuf = tile + adjoint_region(n, NP);        // [2][NP]
   int* rho = reinterpret_cast<int*>(colbuf + 2 * NP);  // [NP] pivot row of step k
   int* rhoinv = rho + NP;                              // [NP]
-  unsigned long long* slot = reinterpret_cast<unsigned long long*>(rhoinv + NP);  // [3]
-  float* scale_s = reinterpret_cast<float*>(slot + 3);
+  unsigned long long* keys = reinterpret_cast<unsigned long long*>(rhoinv + NP);  // [2][16]
+  float* scale_s = reinterpret_cast<float*>(keys + 32);
   int* bad_s = reinterpret_cast<int*>(scale_s + 1);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
@@ -100,7 +100,6 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adjoint_kernel(AdjArgs a) {
     for (int t = 0; t < TR; ++t)
       if (warp + 16 * t >= n) used |= 1u << t;
     if (threadIdx.x == 0) {
-      slot[0] = slot[1] = 0ull;  // slot[2] is cleared after step 0's barrier
       *bad_s = 0;
       float sc = 0.5f;
       if (a.pf_sign) sc = (float)(0.5 * image_weight(a.pf_sign, a.pf_logabs, item, a.n_img));
@@ -108,13 +107,13 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adjoint_kernel(AdjArgs a) {
     }
     __syncthreads();
     int bad = 0;
-    // One barrier per step.  The key slots rotate over three (slot sl is read after the step's
-    // barrier and cleared after the next step's barrier, two steps before its next use); the
-    // column and candidate buffers alternate by parity (a warp writes step k + 2's copy only
-    // after every warp has passed step k + 1's barrier, so after every read of step k's).
-    int sl = 0;
+    // One barrier per step: the column, key and candidate buffers alternate by parity (a warp
+    // writes step k + 2's copy only after every warp has passed step k + 1's barrier, so after
+    // every read of step k's).  Each warp leaves its best key in a place of its own and reduces all
+    // 16 after the barrier (a 64-bit shared-memory maximum serialised the warps before it).
 #pragma unroll
     for (int uk = 0; uk < TC; ++uk) {
+#pragma unroll 1
       for (int lk = 0; lk < 32; ++lk) {
         const int k = uk * 32 + lk;
         if (k >= n || bad) break;  // uniform
@@ -148,23 +147,21 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adjoint_kernel(AdjArgs a) {
 #pragma unroll
                 for (int u = 0; u < TC; ++u) cw[lane + 32 * u] = A[t][u];
               }
-            if (lane == 0) atomicMax(slot + sl, key);
           }
+          if (lane == 0) keys[16 * par + warp] = key;
         }
         __syncthreads();
-        const unsigned long long win = slot[sl];
-        const int p = 0x7FFFFFFF - (int)(unsigned)(win & 0xFFFFFFFFull);
-        const float mag = __uint_as_float((unsigned)(win >> 32));
-        if (win == 0ull || !(mag > 0.0f && mag <= 3.0e38f)) {  // zero column, or non-finite
-          bad = (win == 0ull || mag == 0.0f) ? NH_FLAG_ZERO_PIVOT : NH_FLAG_NONFINITE;
-          __syncthreads();
+        const unsigned long long kw = keys[16 * par + (lane & 15)];
+        const unsigned wh = __reduce_max_sync(0xffffffffu, (unsigned)(kw >> 32));
+        const unsigned wl =
+            __reduce_max_sync(0xffffffffu, (unsigned)(kw >> 32) == wh ? (unsigned)kw : 0u);
+        const int p = 0x7FFFFFFF - (int)wl;
+        const float mag = __uint_as_float(wh);
+        if ((wh | wl) == 0u || !(mag > 0.0f && mag <= 3.0e38f)) {  // zero column, or non-finite
+          bad = ((wh | wl) == 0u || mag == 0.0f) ? NH_FLAG_ZERO_PIVOT : NH_FLAG_NONFINITE;
           break;
         }
-        if (threadIdx.x == 0) {
-          slot[sl == 0 ? 2 : sl - 1] = 0ull;
-          rho[k] = p;
-        }
-        sl = sl == 2 ? 0 : sl + 1;
+        if (threadIdx.x == 0) rho[k] = p;
         const float* prow = cand + (size_t)(par * 16 + (p & 15)) * NP;
         const float inv = 1.0f / prow[k];
         float r[TC];
@@ -230,7 +227,7 @@ template <int TC>
 size_t adjoint_smem(int n) {
   constexpr int NP = 32 * TC;
   return sizeof(float) * (adjoint_region(n, NP) + 2 * NP) + sizeof(int) * 2 * NP +
-         sizeof(unsigned long long) * 3 + 16;
+         sizeof(unsigned long long) * 32 + 16;
 }
 
 template <int TC>

@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(kRcThreads, 1) resconv_kernel(RcArgs<T> a) {
 // weights stream through two 9 KB chunks (4 input channels, in fragment order), the next one in
 // registers.  Half an item per CTA also halves the granularity of the last wave: the recompute
 // lists are a few items per SM.  478 items of 16 blocks at 16x16: 25.4 ms by conv_pass in FP64 with
-// its planes in global memory, 9.6 ms here (the FMA floor, evenly spread, is 7.7 ms).
+// its planes in global memory, 12.2 ms here (the FMA floor, evenly spread, is 7.7 ms).
 constexpr int kRmThreads = 512;
 constexpr int kRmChunk = 9 * 4 * 32;  // weights of one chunk: 36 k x 32 channels
 constexpr int kRmPre = (kRmChunk + kRmThreads - 1) / kRmThreads;
