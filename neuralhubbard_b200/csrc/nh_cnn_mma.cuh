@@ -48,12 +48,12 @@ __device__ __forceinline__ void mma_f64(double* c, double a, double b) {
       : "d"(a), "d"(b));
 }
 
-// Border cells of `planes` planes from their periodic interior cells.
+// Border cells of `planes` planes from their periodic interior cells: a lane works out a cell once
+// and copies it in the planes of its warp.
 template <int TH>
 __device__ __forceinline__ void mma_halo(double* act, int planes, int PS, int Lx, int Ly) {
   const int W = Ly + 2, H = 2 * W + 2 * Lx;
-  for (int e = threadIdx.x; e < planes * H; e += TH) {
-    const int c = e / H, h = e - c * H;
+  for (int h = threadIdx.x & 31; h < H; h += 32) {
     int x, y;  // padded coordinates of the border cell
     if (h < 2 * W) {
       x = h < W ? 0 : Lx + 1;
@@ -64,7 +64,9 @@ __device__ __forceinline__ void mma_halo(double* act, int planes, int PS, int Lx
     }
     const int sx = x == 0 ? Lx : (x == Lx + 1 ? 1 : x);
     const int sy = y == 0 ? Ly : (y == Ly + 1 ? 1 : y);
-    act[c * PS + x * W + y] = act[c * PS + sx * W + sy];
+    double* dst = act + x * W + y;
+    const double* src = act + sx * W + sy;
+    for (int c = threadIdx.x >> 5; c < planes; c += TH / 32) dst[c * PS] = src[c * PS];
   }
 }
 
