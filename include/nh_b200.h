@@ -96,8 +96,8 @@ enum {
  *                refinement is the pivoted FP64 recompute of cond_tau below.
  * cond_tau:      an item whose pivot ratio exceeds cond_tau is flagged NH_FLAG_GROWTH and, when
  *                Wt64 is set, its features are recomputed in FP64 (CNN) and its log-Pfaffian is
- *                refined against the FP64 pairing block (NH_FLAG_REFINED; n > 224: a pivoted
- *                FP64 Pfaffian); <= 0 disables both.  For projected amplitudes with
+ *                refined against the FP64 pairing block (NH_FLAG_REFINED; 224 < n <= 236: a
+ *                pivoted FP64 Pfaffian); <= 0 disables both.  For projected amplitudes with
  *                cond_tau > 1 an image whose |psi(g s)| is below 1e-3 of |psi_P(s)| is not
  *                recomputed in FP64 (its error cannot move log|psi_P| by more than ~1e-5);
  *                cond_tau <= 1 recomputes every image (the all-FP64 form).

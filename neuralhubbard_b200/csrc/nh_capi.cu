@@ -99,9 +99,10 @@ static size_t act_scratch_bytes(const nh_backflow_params& p) {
   return p.net == NH_NET_RESCONV ? resconv_scratch_bytes(N) : cnn_scratch_bytes(N, p.channels);
 }
 
-// Pivot-order records and refinement scratch: only where the FP64 refinement applies.
+// Pivot-order records, and up to kRefineMaxN the refinement's lists and scratch (beyond, it uses the
+// Pfaffian's triangles).
 static size_t refine_bytes(size_t items, int n, int d) {
-  if (n > kRefineMaxN) return 0;
+  if (n > kRefineMaxN) return align256(items * perm_stride(n) * sizeof(uint16_t));
   return align256(items * perm_stride(n) * sizeof(uint16_t)) + align256(items * sizeof(int32_t)) +
          align256(sizeof(int32_t)) + align256(refine_slice_bytes(n, d));
 }
@@ -149,11 +150,10 @@ PipelineBuffers carve_pipeline(void* ws, int max_items, const nh_backflow_params
   b.cnn_act = act_bytes ? take(act_bytes) : nullptr;
   b.pf_ratio = reinterpret_cast<float*>(take(it * sizeof(float)));
   b.wt_chunks = reinterpret_cast<float*>(take(wt_chunk_bytes(prm)));
-  b.perm = nullptr;
+  b.perm = reinterpret_cast<uint16_t*>(take(it * perm_stride((int)n) * sizeof(uint16_t)));
   b.list32 = b.count32 = nullptr;
   b.slice = nullptr;
   if ((int)n <= kRefineMaxN) {
-    b.perm = reinterpret_cast<uint16_t*>(take(it * perm_stride((int)n) * sizeof(uint16_t)));
     b.list32 = reinterpret_cast<int32_t*>(take(it * sizeof(int32_t)));
     b.count32 = reinterpret_cast<int32_t*>(take(sizeof(int32_t)));
     b.slice = take(refine_slice_bytes((int)n, prm.channels / 2));
@@ -165,7 +165,7 @@ PipelineBuffers carve_pipeline(void* ws, int max_items, const nh_backflow_params
 // items flagged ill-conditioned or cancelling -> FP64 refinement of the log-Pfaffian with the
 // FP32 pivot order (against the FP64 pairing block for those items, against the item's own FP32
 // block for the others above refine_tau) -> combination of the symmetry images (or a copy for
-// G = 1).  Beyond n = kRefineMaxN the flagged items are recomputed by the pivoted FP64 kernel.
+// G = 1).  For 224 < n <= 236 the flagged items are recomputed by the pivoted FP64 kernel.
 int run_pipeline(const ConfigList& cl, const nh_backflow_params& p, const PipelineBuffers& b,
                  float* sign, double* logabs, int32_t* flags, cudaStream_t st) {
   const int n = p.n_up + p.n_dn, d = p.channels / 2;
@@ -210,15 +210,15 @@ int run_pipeline(const ConfigList& cl, const nh_backflow_params& p, const Pipeli
     return launch_combine(b.pf_sign, b.pf_logabs, b.pf_flags, cl.G, cl.n_cfg, cl.n_cfg_dev, sign,
                           logabs, flags, p.cancel_tau, tc ? b.err : nullptr, st);
   }
-  const bool refine = b.perm != nullptr;  // n <= kRefineMaxN
+  const bool refine = n <= kRefineMaxN;
+  // beyond shared memory: the refinement's tiles take the place of the FP32 triangles
+  const bool big = !refine && b.pf_tri && refine_big_bytes(n) <= pfaffian_scratch_bytes(n);
   PfGatherArgs g{b.Y, b.idx, p.Wt, p.Lx, p.Ly, d, n, cl.n_cfg_dev, cl.G, max_items, nullptr,
                  b.item_sign, b.pf_sign, b.pf_logabs, b.pf_flags, p.cond_tau, 0, false, b.pf_tri};
   g.ratio = b.pf_ratio;
   g.wt_chunks = b.wt_chunks;
-  if (refine) {
-    g.perm = b.perm;
-    g.refine_tau = p.refine_tau;
-  }
+  if (refine || big) g.perm = b.perm;
+  if (refine) g.refine_tau = p.refine_tau;
   if (p.pf_mode == 1)
     rc = launch_pfaffian_tc(g, 1, nullptr, b.err, st);
   else if (staged_supported(g))
@@ -237,10 +237,10 @@ int run_pipeline(const ConfigList& cl, const nh_backflow_params& p, const Pipeli
     CnnLaunch c64{&cl, &p, 1, true, b.list, b.count, max_items, nullptr, b.Y64, b.idx64,
                   b.item_sign, b.cnn_act};
     if ((rc = launch_cnn(c64, st))) return rc;
-    if (refine) {
+    if (refine || big) {
       RefineLaunch r{n, d, 2, nullptr, b.Y64, b.idx64, p.Wt64, p.Lx, p.Ly, b.list, b.count,
                      max_items, b.perm, perm_stride(n), b.item_sign, b.pf_sign, b.pf_logabs,
-                     b.pf_flags, b.slice};
+                     b.pf_flags, big ? b.pf_tri : b.slice};
       if ((rc = launch_refine(r, st))) return rc;
     } else {
       PfGatherArgs g64{b.Y64, b.idx64, p.Wt64, p.Lx, p.Ly, d, n, b.count, 1, max_items, b.list,

@@ -17,7 +17,9 @@ constexpr int kMaxN = 1024;       // sites per lattice supported by the bookkeep
 constexpr int kFlagNeedRefine = 1 << 20;
 constexpr int kPublicFlags = 0xFFFF;
 // FP64 refinement with the FP32 pivot order (nh_refine.cu): its FP64 triangle lives in shared
-// memory, so n <= kRefineMaxN; beyond, flagged items are recomputed by the pivoted FP64 kernel.
+// memory up to kRefineMaxN.  Beyond, the flagged items of the amplitude pipeline are refined with
+// their triangle in global memory where the pipeline has that scratch (pfaffian_scratch_bytes,
+// n > 236), else recomputed by the pivoted FP64 kernel, which also serves dense matrices.
 constexpr int kRefineMaxN = 224;
 constexpr size_t kRefineSmemLimit = 225 * 1024;
 // Backward of the amplitude (nh_grad.cu): the Gauss-Jordan inverse keeps the matrix in registers
@@ -273,7 +275,7 @@ struct PipelineBuffers {
   void* pf_tri;       // large lattices: per-CTA Pfaffian triangles (pfaffian_scratch_bytes)
   void* cnn_act;      // large lattices: per-CTA CNN activation planes (cnn_scratch_bytes)
   float* pf_ratio;    // (items,) pivot ratio of the FP32 factorisation
-  uint16_t* perm;     // (items, perm_stride) FP32 pivot order of every item (n <= kRefineMaxN)
+  uint16_t* perm;     // (items, perm_stride) FP32 pivot order of every item
   int32_t* list32;    // (items,) items refined against their FP32 matrix
   int32_t* count32;   // (1,) their number
   void* slice;        // refinement: per-CTA permuted triangles (refine_slice_bytes)
@@ -311,6 +313,8 @@ struct RefineLaunch {
 };
 int launch_refine(const RefineLaunch& q, cudaStream_t st);
 size_t refine_slice_bytes(int n, int d);
+// n > kRefineMaxN (mode 2): bytes of the clusters' FP64 tiles, passed as the slice.
+size_t refine_big_bytes(int n);
 
 size_t pipeline_bytes(int max_items, const nh_backflow_params& p);
 PipelineBuffers carve_pipeline(void* ws, int max_items, const nh_backflow_params& p);

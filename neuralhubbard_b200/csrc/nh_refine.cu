@@ -24,6 +24,7 @@
 // of its unit factor, and the trailing tiles take P W^T, all as m8n8k4 FP64 products.  The next panel's column is
 // updated first, so that its pivot block (a serial chain) is factorised by warp 0 while the other
 // warps update the rest.  n <= kRefineMaxN (224: the tiles take 203 KB).
+#include <cooperative_groups.h>
 #include <math.h>
 
 #include <algorithm>
@@ -216,15 +217,15 @@ __device__ void gather_permuted(const RefineArgs& a, const T* Yg, const int32_t*
 // The table is staged one spin block at a time (uu, du, dd: the modes ascend, so rows and columns
 // of a block are ranges); unsorted mode lists (a wrong particle number) and lattices whose block
 // does not fit read it from global memory.
+// gw of nw: this warp among those that share the item.
 template <int D, int TH>
 __device__ void gather_tiles(const RefineArgs& a, const double* Ys, const int* info,
                              const uint16_t* iperm, int nu, bool sorted, unsigned char* smem,
-                             double* S, double* slice) {
+                             double* S, double* slice, int gw, int nw) {
   constexpr int LPR = D <= 16 ? 4 : 8, CPL = D / (2 * LPR);  // lanes per pair, chunks per lane
   constexpr int GR = 32 / LPR, JW = 2 * GR;                  // column groups, columns per warp
-  constexpr int WARPS = TH / 32;
   const int n = a.n, N = a.Lx * a.Ly;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31;
   const int grp = lane / LPR, c = lane % LPR;
   // Offset of chunk x of this lane in a row: with two chunks per lane, odd groups read theirs in
   // the other order, so that the two groups of a quarter-warp use different banks.
@@ -262,8 +263,8 @@ __device__ void gather_tiles(const RefineArgs& a, const double* Ys, const int* i
     auto groups = [&](int rb) {
       return tri ? min(ncg, (rb * LPR + LPR - 1 + JW - 1) / JW) : ncg;
     };
-    int rb = 0, rem = wid;
-    for (;; rem += WARPS) {
+    int rb = 0, rem = gw;
+    for (;; rem += nw) {
       while (rb < nrb && rem >= groups(rb)) {
         rem -= groups(rb);
         ++rb;
@@ -333,9 +334,13 @@ __device__ void gather_tiles(const RefineArgs& a, const double* Ys, const int* i
         }
     }
   }
-  __syncthreads();  // the staged rows and table are dead: the slice's tiles take their place
-  const int T = tile_rows(n), o0 = tile_base(a.keep) * 32, o1 = tile_base(T) * 32;
-  for (int v0 = o0 + tid; v0 < o1; v0 += 4 * TH) {
+}
+
+// The slice's tiles of rows >= keep into shared memory, once the staged rows and table are dead.
+template <int TH>
+__device__ void copy_tail(const RefineArgs& a, double* S, const double* slice) {
+  const int T = tile_rows(a.n), o0 = tile_base(a.keep) * 32, o1 = tile_base(T) * 32;
+  for (int v0 = o0 + threadIdx.x; v0 < o1; v0 += 4 * TH) {
     double2 buf[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
@@ -401,16 +406,21 @@ size_t features_smem(int Lx, int Ly, int C, int elt, int TH) {
   return ((act + 15) & ~(size_t)15) + (size_t)elt * ((size_t)C * C * 9 + C);
 }
 
+// A lane's two elements of a tile in the MMA accumulator layout.
+__device__ __forceinline__ double2* acc_ptr(double* t) {
+  const int lane = threadIdx.x & 31;
+  return reinterpret_cast<double2*>(t + toff(lane >> 2, 2 * (lane & 3)));
+}
+
 // Pivot block of a panel (w <= 8 columns) by one warp, two elements per lane: lane (r, q) = 4 r + q
 // holds B[r][2q], B[r][2q + 1] (the MMA accumulator layout; only c < r is used).  A step takes
 // its columns k, k + 1 from the lanes (r, k / 2) by shuffles; the same row operations applied to
 // the identity give the inverse of the block's unit lower factor, which the panel solve uses as
 // an MMA operand.  Writes Li (that inverse, a swizzled tile), the reciprocal pivots xinv and the
-// pivots to piv[0, w / 2).  The loop stays rolled (the code runs on one warp).
-__device__ __forceinline__ void factor_block(const double* D, int w, double* Li, double* xinv,
-                                             double* piv) {
+// pivots to piv[0, w / 2).  d: the lane's two elements.  The loop stays rolled (the code runs on one
+// warp).
+__device__ __forceinline__ void factor_block(double2 d, int w, double* Li, double* xinv, double* piv) {
   const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
-  const double2 d = *reinterpret_cast<const double2*>(D + toff(r, 2 * q));
   // entries outside the strict lower triangle of the w rows hold no data
   double b0 = (r < w && 2 * q < r) ? d.x : 0.0, b1 = (r < w && 2 * q + 1 < r) ? d.y : 0.0;
   double e0 = r == 2 * q ? 1.0 : 0.0, e1 = r == 2 * q + 1 ? 1.0 : 0.0;
@@ -450,15 +460,54 @@ __device__ __forceinline__ Operand load_operand(const double* t) {
   const int lane = threadIdx.x & 31;
   return Operand{t[toff(lane >> 2, lane & 3)], t[toff(lane >> 2, 4 + (lane & 3))]};
 }
-__device__ __forceinline__ double2* acc_ptr(double* t) {
-  const int lane = threadIdx.x & 31;
-  return reinterpret_cast<double2*>(t + toff(lane >> 2, 2 * (lane & 3)));
-}
 __device__ __forceinline__ double2 tile_mma(double2 v, const Operand& p, const Operand& w) {
   double c[2] = {v.x, v.y};
   mma_f64(c, p.k0, w.k0);
   mma_f64(c, p.k1, w.k1);
   return make_double2(c[0], c[1]);
+}
+
+// The item's sign, log|pf| and flags from its n / 2 pivots, by one warp: log|pf| = sum of log|x_t| as
+// one product per lane (mantissa and exponent), then a butterfly.
+template <typename Piv>
+__device__ __forceinline__ void write_result(const RefineArgs& a, int item, int swapped, Piv pivot) {
+  const int lane = threadIdx.x & 31;
+  double mant = 1.0;
+  int expo = 0, neg = 0, bad = 0;
+  for (int t = lane; t < a.n / 2; t += 32) {
+    const double x = pivot(t);
+    if (x < 0.0) neg ^= 1;
+    const double ax = fabs(x);
+    if (!(ax > 0.0) || !isfinite(ax)) bad |= ax == 0.0 ? NH_FLAG_ZERO_PIVOT : NH_FLAG_NONFINITE;
+    int e;
+    mant = frexp(mant * ax, &e);
+    expo += e;
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {  // 32 mantissas in [1/2, 1]: no underflow
+    mant *= __shfl_xor_sync(0xffffffffu, mant, o);
+    expo += __shfl_xor_sync(0xffffffffu, expo, o);
+    neg ^= __shfl_xor_sync(0xffffffffu, neg, o);
+    bad |= __shfl_xor_sync(0xffffffffu, bad, o);
+  }
+  if (lane == 0) {
+    float s = a.item_sign ? a.item_sign[item] : 1.0f;
+    if (swapped) s = -s;
+    if (neg) s = -s;
+    int f = a.flags ? a.flags[item] : 0;
+    f &= ~(kFlagNeedRefine | NH_FLAG_ZERO_PIVOT | NH_FLAG_NONFINITE);
+    double la = log(mant) + (double)expo * 0.6931471805599453;
+    if (isnan(s)) f |= NH_FLAG_NONFINITE;
+    if (bad & NH_FLAG_ZERO_PIVOT) {
+      s = 0.0f;
+      la = -INFINITY;
+    }
+    if (!isfinite(la) && s != 0.0f) bad |= NH_FLAG_NONFINITE;
+    f |= bad | NH_FLAG_REFINED;
+    a.sign[item] = s;
+    a.logabs[item] = s == 0.0f ? -INFINITY : la;
+    if (a.flags) a.flags[item] = f;
+  }
 }
 
 // MODE is a.mode as a template argument, so that each instance holds only its own phase-1 code
@@ -549,14 +598,16 @@ __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArg
       }
       __syncthreads();
       const int nus = nu_s;
-      gather_tiles<D, TH>(a, Ys, info, perm_s, nus & 0x7FFFFFFF, nus >= 0, smem, S,
-                          reinterpret_cast<double*>(slb));
+      double* sl = reinterpret_cast<double*>(slb);
+      gather_tiles<D, TH>(a, Ys, info, perm_s, nus & 0x7FFFFFFF, nus >= 0, smem, S, sl, wid, WARPS);
+      __syncthreads();
+      copy_tail<TH>(a, S, sl);
     }
     __syncthreads();
 
     // Phase 2: static-pivot blocked elimination.  The pivots of panel p are kept in the W tile of
     // tile row p, which no later step reads or writes.
-    if (wid == 0) factor_block(S, min(kPW, n), Li, xinv, Wb);
+    if (wid == 0) factor_block(*acc_ptr(S), min(kPW, n), Li, xinv, Wb);
     __syncthreads();
     for (int p = 0; p + 1 < T; ++p) {
       // (1) tile rows I > p: W_I = -S_(I, p) Li^T (the forward substitution of every row as one
@@ -586,8 +637,8 @@ __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArg
       __syncthreads();
       // (3) warp 0: the next pivot block; the others: the remaining tiles, 2 x 2 at a time.
       if (wid == 0) {
-        factor_block(S + (size_t)(tile_base(p + 1) + p + 1) * 64, min(kPW, n - 8 * (p + 1)), Li, xinv,
-                     Wb + (p + 1) * 64);
+        factor_block(*acc_ptr(S + (size_t)(tile_base(p + 1) + p + 1) * 64),
+                     min(kPW, n - 8 * (p + 1)), Li, xinv, Wb + (p + 1) * 64);
       } else if (wid & 3) {
         // not the warps of warp 0's scheduler, whose chain would queue behind their products
         constexpr int NW = WARPS - WARPS / 4;
@@ -623,45 +674,151 @@ __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArg
       }
       __syncthreads();
     }
-    // log|pf| = sum of log|x_t| as one product per lane (mantissa and exponent), then a butterfly.
-    if (wid == 0) {
-      double mant = 1.0;
-      int expo = 0, neg = 0, bad = 0;
-      for (int t = lane; t < n / 2; t += 32) {
-        const double x = Wb[(t >> 2) * 64 + (t & 3)];
-        if (x < 0.0) neg ^= 1;
-        const double ax = fabs(x);
-        if (!(ax > 0.0) || !isfinite(ax)) bad |= ax == 0.0 ? NH_FLAG_ZERO_PIVOT : NH_FLAG_NONFINITE;
-        int e;
-        mant = frexp(mant * ax, &e);
-        expo += e;
-      }
+    if (wid == 0) write_result(a, item, pr[n] & 1, [&](int t) { return Wb[(t >> 2) * 64 + (t & 3)]; });
+  }
+}
+
+// ------------------------------------------------------------------ n beyond shared memory
+// The same factorisation with the FP64 tiles in global memory (L2), one item per cluster of kBigCl
+// CTAs.  CTA r owns the tile rows I = r mod kBigCl: all updates of a row stay in one CTA, only the
+// W tiles of a panel travel, written by their owner into every CTA's shared memory (two panels'
+// worth, by parity), so a panel costs one cluster barrier.  Every CTA factorises the pivot block
+// itself, and every warp forms the one foreign W tile that the next column needs.  What bounds it
+// is the L2 traffic of the trailing tiles (1 KB per tile update) and, at the end, the panels'
+// latency.  Replaces the pivoted FP64 factorisation with its triangle in global memory, one CTA
+// per item: 44 items at n = 896 12.25 -> 2.62 ms, 98 at n = 504 3.33 -> 1.37 ms.
+constexpr int kBigTh = 512;
+constexpr int kBigCl = 4;
+constexpr int kBigWarps = kBigTh / 32;
+
+// Accumulator layout (row r, columns 2q, 2q + 1 in lane 4 r + q) to MMA operand layout.
+__device__ __forceinline__ Operand to_operand(const double2& v) {
+  const int lane = threadIdx.x & 31, src = (lane & 28) + ((lane & 3) >> 1);
+  const double x0 = __shfl_sync(0xffffffffu, v.x, src), y0 = __shfl_sync(0xffffffffu, v.y, src);
+  const double x1 = __shfl_sync(0xffffffffu, v.x, src + 2), y1 = __shfl_sync(0xffffffffu, v.y, src + 2);
+  return (lane & 1) ? Operand{y0, y1} : Operand{x0, x1};
+}
+__device__ __forceinline__ double2 ldcg2(const double* p) {
+  return __ldcg(reinterpret_cast<const double2*>(p));
+}
+
+template <int D>
+__global__ void __cluster_dims__(kBigCl, 1, 1) __launch_bounds__(kBigTh, 1)
+    refine_big_kernel(RefineArgs a, size_t item_doubles) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank();
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ __align__(16) double Li[kPW * kPW];
+  __shared__ double xinv[kPW / 2];
+  __shared__ double piv[kMaxN / 2];
+  __shared__ uint16_t iperm[kMaxN];
+  __shared__ int nu_s;
+  const int n = a.n, T = tile_rows(n), N = a.Lx * a.Ly;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  // Elimination: W tiles of two panels, then this CTA's P tiles (rows rank, rank + kBigCl, ...).
+  double* Wl = reinterpret_cast<double*>(smem);
+  double* Pl = Wl + 2 * (size_t)T * 64;
+  double* Wr[kBigCl];
 #pragma unroll
-      for (int o = 16; o; o >>= 1) {  // 32 mantissas in [1/2, 1): no underflow
-        mant *= __shfl_xor_sync(0xffffffffu, mant, o);
-        expo += __shfl_xor_sync(0xffffffffu, expo, o);
-        neg ^= __shfl_xor_sync(0xffffffffu, neg, o);
-        bad |= __shfl_xor_sync(0xffffffffu, bad, o);
-      }
-      if (lane == 0) {
-        float s = a.item_sign ? a.item_sign[item] : 1.0f;
-        if (pr[n] & 1) s = -s;
-        if (neg) s = -s;
-        int f = a.flags ? a.flags[item] : 0;
-        f &= ~(kFlagNeedRefine | NH_FLAG_ZERO_PIVOT | NH_FLAG_NONFINITE);
-        double la = log(mant) + (double)expo * 0.6931471805599453;
-        if (isnan(s)) f |= NH_FLAG_NONFINITE;
-        if (bad & NH_FLAG_ZERO_PIVOT) {
-          s = 0.0f;
-          la = -INFINITY;
-        }
-        if (!isfinite(la) && s != 0.0f) bad |= NH_FLAG_NONFINITE;
-        f |= bad | NH_FLAG_REFINED;
-        a.sign[item] = s;
-        a.logabs[item] = s == 0.0f ? -INFINITY : la;
-        if (a.flags) a.flags[item] = f;
-      }
+  for (int r = 0; r < kBigCl; ++r) Wr[r] = cluster.map_shared_rank(Wl, r);
+  const int clusters = gridDim.x / kBigCl, cid = blockIdx.x / kBigCl;
+  double* S = static_cast<double*>(a.slice) + (size_t)cid * item_doubles;
+  const int n_work = *a.count;
+  for (int slot = cid; slot < n_work; slot += clusters) {
+    const int item = a.list[slot];
+    const uint16_t* pr = a.perm + (size_t)item * a.perm_stride;
+    double* Ys = reinterpret_cast<double*>(smem + a.y_off);
+    int* info = reinterpret_cast<int*>(smem + a.info_off);
+    const double* Yg = static_cast<const double*>(a.Y) + (size_t)slot * n * D;
+    const int32_t* ig = a.idx + (size_t)slot * n;
+    __syncthreads();  // the previous item's readers are done
+    if (tid == 0) nu_s = 0;
+    for (int p = tid; p < n; p += kBigTh) {
+      const int v = pr[p];
+      iperm[v < n ? v : 0] = (uint16_t)p;
     }
+    if (!a.rows_slice) {  // rows staged in shared memory
+      const double2* src = reinterpret_cast<const double2*>(Yg);
+      for (int v = tid; v < n * (D / 2); v += kBigTh) reinterpret_cast<double2*>(Ys)[v] = __ldg(src + v);
+    }
+    __syncthreads();
+    for (int p = tid; p < n; p += kBigTh) {
+      const int m = ig[p], sp = m >= N ? 1 : 0, site = m - sp * N, x = site / a.Ly;
+      info[p] = (sp << 16) | (x << 8) | (site - x * a.Ly);
+      if (sp == 0) atomicAdd(&nu_s, 1);
+      if (sp == 1 && p + 1 < n && ig[p + 1] < N) atomicOr(&nu_s, (int)0x80000000);
+    }
+    __syncthreads();
+    const int nus = nu_s;
+    gather_tiles<D, kBigTh>(a, a.rows_slice ? Yg : Ys, info, iperm, nus & 0x7FFFFFFF, nus >= 0, smem,
+                            nullptr, S, rank * kBigWarps + wid, kBigCl * kBigWarps);
+    cluster.sync();  // every tile written; the staging areas are dead in every CTA
+    const int o = toff(lane >> 2, 2 * (lane & 3));  // this lane's elements of a tile
+    if (wid == 0) factor_block(ldcg2(S + o), min(kPW, n), Li, xinv, piv);
+    __syncthreads();
+    for (int p = 0; p + 1 < T; ++p) {
+      double* Wp = Wl + (size_t)(p & 1) * T * 64;
+      // (1) this CTA's rows I > p: W_I and P_I from tile (I, p), then tile (I, p + 1).  W of row p + 1
+      // comes from that row's own tile (its owner does not overwrite it).
+      {
+        const Operand li = load_operand(Li);
+        const double inv = xinv[lane & 3];
+        const int I0 = p + 1 + ((rank - (p + 1)) & (kBigCl - 1));
+        Operand wn{0.0, 0.0};
+        if (I0 + kBigCl * wid < T) {
+          const double2 w = tile_mma(make_double2(0.0, 0.0),
+                                     to_operand(ldcg2(S + (size_t)(tile_base(p + 1) + p) * 64 + o)),
+                                     li);
+          wn = to_operand(make_double2(-w.x, -w.y));
+        }
+        for (int I = I0 + kBigCl * wid; I < T; I += kBigCl * kBigWarps) {
+          double* row = S + (size_t)tile_base(I) * 64;
+          const double2 sv = ldcg2(row + p * 64 + o), cv = ldcg2(row + (p + 1) * 64 + o);
+          const double2 w = tile_mma(make_double2(0.0, 0.0), to_operand(sv), li);
+          const double2 pv = make_double2(-w.y * inv, w.x * inv);
+          *reinterpret_cast<double2*>(Pl + (I / kBigCl) * 64 + o) = pv;
+#pragma unroll
+          for (int r = 0; r < kBigCl; ++r)
+            *reinterpret_cast<double2*>(Wr[r] + (size_t)(p & 1) * T * 64 + I * 64 + o) =
+                make_double2(-w.x, -w.y);
+          const double2 nv = tile_mma(cv, to_operand(pv), wn);
+          __stcg(reinterpret_cast<double2*>(row + (p + 1) * 64 + o), nv);
+        }
+      }
+      cluster.sync();  // W complete everywhere, column p + 1 updated
+      // (2) warp 0: the next pivot block; the others: this CTA's rows over the columns p + 2 .. I,
+      // strips of kStrip tiles of one row with all loads in flight.
+      if (wid == 0) {
+        factor_block(ldcg2(S + (size_t)(tile_base(p + 1) + p + 1) * 64 + o),
+                     min(kPW, n - 8 * (p + 1)), Li, xinv, piv + 4 * (p + 1));
+      } else {
+        constexpr int kStrip = 6, NW = kBigWarps - 1;
+        int I = p + 2 + ((rank - (p + 2)) & (kBigCl - 1)), rem = wid - 1;
+        for (;; rem += NW) {
+          while (I < T && rem >= (I - p - 2) / kStrip + 1) {
+            rem -= (I - p - 2) / kStrip + 1;
+            I += kBigCl;
+          }
+          if (I >= T) break;
+          const int J0 = p + 2 + rem * kStrip;
+          double* row = S + (size_t)tile_base(I) * 64 + o;
+          double2 v[kStrip];
+#pragma unroll
+          for (int u = 0; u < kStrip; ++u)
+            if (J0 + u <= I) v[u] = ldcg2(row + (J0 + u) * 64);
+          const Operand pa = load_operand(Pl + (I / kBigCl) * 64);
+#pragma unroll
+          for (int u = 0; u < kStrip; ++u)
+            if (J0 + u <= I)
+              __stcg(reinterpret_cast<double2*>(row + (J0 + u) * 64),
+                     tile_mma(v[u], pa, load_operand(Wp + (J0 + u) * 64)));
+        }
+      }
+      __syncthreads();  // Li ready, this CTA's rows updated
+    }
+    if (rank == 0 && wid == 0) write_result(a, item, pr[n] & 1, [&](int t) { return piv[t]; });
+    cluster.sync();  // no CTA starts the next item's gather over tiles still being read
   }
 }
 
@@ -729,6 +886,31 @@ int launch_refine_m(RefineArgs a, int max_slots, cudaStream_t st) {
   return launch_refine_k<D, MODE, 512>(a, max_slots, s512, st);
 }
 
+// n > kRefineMaxN (mode 2 only): tiles in the scratch q.slice.
+template <int D>
+int launch_refine_big(RefineArgs a, int max_slots, cudaStream_t st) {
+  const int N = a.Lx * a.Ly, n = a.n, T = tile_rows(n);
+  const size_t inf = (4 * (size_t)n + 15) & ~(size_t)15, y = 8 * (size_t)n * D, wt = 8 * (size_t)N * D;
+  const size_t lim = 200 * 1024;
+  a.rows_slice = inf + y > lim;  // rows read from global memory
+  a.stage_wt = !a.rows_slice && inf + y + wt <= lim;
+  a.info_off = 0;
+  a.y_off = (int)inf;
+  a.wt_off = (int)(inf + y);
+  a.keep = 0;  // every tile in global memory
+  size_t smem = 512 * (2 * (size_t)T + (T + kBigCl - 1) / kBigCl);
+  smem = std::max(smem, inf + (a.rows_slice ? 0 : y) + (a.stage_wt ? wt : 0));
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      refine_big_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim);
+  if (attr != cudaSuccess) return check_cuda(attr, "refine smem attribute");
+  int clusters = num_sms() / kBigCl;
+  if (clusters > max_slots) clusters = max_slots;
+  if (clusters <= 0) return NH_OK;
+  ProfScope prof_scope(NH_K_PFAFFIAN64, st);
+  refine_big_kernel<D><<<clusters * kBigCl, kBigTh, smem, st>>>(a, tile_bytes(T) / 8);
+  return check_launch("refine_big_kernel");
+}
+
 template <int D>
 int launch_refine_d(const RefineArgs& a, int max_slots, cudaStream_t st) {
   switch (a.mode) {
@@ -741,6 +923,10 @@ int launch_refine_d(const RefineArgs& a, int max_slots, cudaStream_t st) {
 
 }  // namespace
 
+size_t refine_big_bytes(int n) {
+  return n > kRefineMaxN ? (size_t)(num_sms() / kBigCl) * tile_bytes(tile_rows(n)) : 0;
+}
+
 size_t refine_slice_bytes(int n, int d) {
   if (n <= 0 || n > kRefineMaxN) return 0;
   // one slice per CTA: two CTAs per SM only where the elimination alone leaves room for both
@@ -750,7 +936,8 @@ size_t refine_slice_bytes(int n, int d) {
 }
 
 int launch_refine(const RefineLaunch& q, cudaStream_t st) {
-  if (q.n <= 0 || q.n % 2 || q.n > kRefineMaxN)
+  const bool big = q.n > kRefineMaxN;  // stored FP64 rows only, tiles in q.slice (refine_big_bytes)
+  if (q.n <= 0 || q.n % 2 || q.n > (q.mode == 2 ? kMaxN : kRefineMaxN))
     return fail(NH_ERR_UNSUPPORTED, "refine: n=%d (even, <= %d)", q.n, kRefineMaxN);
   if (q.max_slots <= 0) return NH_OK;
   if (q.mode < 0 || q.mode > 4) return fail(NH_ERR_INVALID, "refine: mode %d", q.mode);
@@ -782,6 +969,14 @@ int launch_refine(const RefineLaunch& q, cudaStream_t st) {
   if (q.mode >= 3 && (!q.cnn_w || !q.cnn_b || q.C % 16 || q.d * 2 != q.C))
     return fail(NH_ERR_INVALID, "refine: in-kernel features need the CNN weights");
   if (q.mode == 0) return launch_refine_m<16, 0>(a, q.max_slots, st);
+  if (big) {
+    switch (q.d) {
+      case 8: return launch_refine_big<8>(a, q.max_slots, st);
+      case 16: return launch_refine_big<16>(a, q.max_slots, st);
+      case 32: return launch_refine_big<32>(a, q.max_slots, st);
+      default: return fail(NH_ERR_UNSUPPORTED, "refine: d=%d (8, 16 or 32)", q.d);
+    }
+  }
   switch (q.d) {
     case 8: return launch_refine_d<8>(a, q.max_slots, st);
     case 16: return launch_refine_d<16>(a, q.max_slots, st);

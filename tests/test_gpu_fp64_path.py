@@ -163,3 +163,19 @@ def test_resconv_fp64(Lx, Ly, ne, blocks):
     sg, la = nh.Variational(model)(np.tile(s, (6, 1))).numpy()
     assert np.array_equal(sg, np.tile(s0, 6))
     assert log_error(la, np.tile(l0, 6)) < TOL
+
+
+# 238 is the first size of the form with its tiles in global memory (236 the last of the pivoted
+# one); partial tiles; 16x17 with the table staged, 31x33 not; the largest n.
+@pytest.mark.parametrize("Lx,Ly,up,dn,symm", [(16, 17, 118, 118, False), (16, 17, 120, 118, True),
+                                              (18, 20, 121, 119, False), (20, 19, 180, 176, False),
+                                              (24, 24, 252, 252, False), (32, 32, 512, 512, False)])
+def test_refine_large(Lx, Ly, up, dn, symm):
+    N = Lx * Ly
+    p = nh.init_params(Lx, Ly, channels=32, layers=4, std=0.05, seed=N + up)
+    s = olat.random_configs(np.random.default_rng(N), 2, N, up, dn)
+    s0, l0 = oproj.projected_amplitude(s, oracle_params(p, Lx, Ly), symm=symm)
+    model = nh.PfaffianBackflow(Lx, Ly, up, dn, params=p, cond_tau=1.0)
+    sg, la = nh.Variational(model, symm=symm)(np.tile(s, (30, 1))).numpy()
+    assert np.array_equal(sg, np.tile(s0, 30))
+    assert log_error(la, np.tile(l0, 30)) < TOL
