@@ -946,6 +946,61 @@ __device__ __forceinline__ void trail_block(float* Lw, const float* Us, const fl
   }
 }
 
+// The item's results from its n / 2 pivots (negated where the step swapped labels), by one warp:
+// Pfaffian = relabelling parity x product of the pivots, accumulated in FP64 as mantissa and
+// exponent (one product per lane, then a butterfly); the pivot ratio flags near-nodal blocks.
+template <typename Piv>
+__device__ __forceinline__ void write_pfaffian(const PfArgs& a, int item, bool zero, int swaps,
+                                               uint16_t* perm, const float* item_sign, Piv pivot) {
+  const int lane = threadIdx.x & 31;
+  int flag = 0, neg = 0, expo = 0;
+  double mant = 1.0;
+  float pmin = INFINITY, pmax = 0.0f;
+  if (!zero)
+    for (int k = lane; k < a.n / 2; k += 32) {
+      const float pv = pivot(k);
+      if (pv < 0.0f) neg ^= 1;
+      const float ap = fabsf(pv);
+      if (!isfinite(ap)) flag |= NH_FLAG_NONFINITE;
+      pmin = fminf(pmin, ap);
+      pmax = fmaxf(pmax, ap);
+      int e;
+      mant = frexp(mant * (double)ap, &e);
+      expo += e;
+    }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {  // 32 mantissas in [1/2, 1]: no underflow
+    mant *= __shfl_xor_sync(0xffffffffu, mant, o);
+    expo += __shfl_xor_sync(0xffffffffu, expo, o);
+    neg ^= __shfl_xor_sync(0xffffffffu, neg, o);
+    flag |= __shfl_xor_sync(0xffffffffu, flag, o);
+    pmin = fminf(pmin, __shfl_xor_sync(0xffffffffu, pmin, o));
+    pmax = fmaxf(pmax, __shfl_xor_sync(0xffffffffu, pmax, o));
+  }
+  if (lane == 0) {
+    float s = item_sign ? item_sign[item] : 1.0f;
+    double la;
+    if (isnan(s)) flag |= NH_FLAG_NONFINITE;  // the CNN could not compute this item
+    if (zero) {
+      s = 0.0f;
+      la = -INFINITY;
+      flag |= NH_FLAG_ZERO_PIVOT;
+    } else {
+      if (neg) s = -s;
+      la = log(mant) + (double)expo * 0.6931471805599453;
+      if (!isfinite(la)) flag |= NH_FLAG_NONFINITE;
+      if (a.cond_tau > 0.0 && (double)pmax > a.cond_tau * (double)pmin) flag |= NH_FLAG_GROWTH;
+      if (a.refine_tau > 0.0 && (double)pmax > a.refine_tau * (double)pmin) flag |= kFlagNeedRefine;
+    }
+    if (s == 0.0f) la = -INFINITY;
+    a.sign[item] = s;
+    a.logabs[item] = la;
+    if (a.flags) a.flags[item] = flag | a.flag_or;
+    if (a.ratio) a.ratio[item] = zero ? INFINITY : (float)((double)pmax / (double)pmin);
+    if (perm && !zero) perm[a.n] = (uint16_t)swaps;
+  }
+}
+
 template <int NB, int D, int TH>
 __global__ void __launch_bounds__(TH, 512 / TH) pf32_kernel(PfArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1019,58 +1074,369 @@ __global__ void __launch_bounds__(TH, 512 / TH) pf32_kernel(PfArgs a) {
         __syncthreads();  // trailing triangle updated
       }
     }
-    if (wid == 0) {
-      // Pfaffian = relabelling parity x product of the pivots, accumulated in FP64 as mantissa
-      // and exponent (one product per lane, then a butterfly); the pivot ratio flags near-nodal
-      // blocks.
-      int flag = 0, neg = 0, expo = 0;
-      double mant = 1.0;
-      float pmin = INFINITY, pmax = 0.0f;
-      if (!zero)
-        for (int k = lane; k < n / 2; k += 32) {
-          const float pv = pivs[k];
-          if (pv < 0.0f) neg ^= 1;
-          const float ap = fabsf(pv);
-          if (!isfinite(ap)) flag |= NH_FLAG_NONFINITE;
-          pmin = fminf(pmin, ap);
-          pmax = fmaxf(pmax, ap);
-          mant *= (double)ap;  // at most 4 FP32 magnitudes per lane
-        }
-      mant = frexp(mant, &expo);
+    if (wid == 0)
+      write_pfaffian(a, item, zero, swaps, perm, a.mode == 2 ? a.item_sign_out : a.item_sign,
+                     [&](int k) { return pivs[k]; });
+  }
+}
+
+// ------------------------------------------------------------------ FP32, n > 256
+// The same operations in the same order as pfaffian_kernel with panels of 4 (the same bits), for
+// triangles in global memory.  The trailing triangle is the traffic (8 bytes per element and
+// update, from L2 or, where 148 triangles exceed it, from HBM), so it is updated once per
+// kBbSteps = 16 pivot steps instead of once per 4: the panel values of four panels stay in
+// shared memory, a column is brought up to date when it is read (the finished panels' terms as the
+// trailing update's chain, then the running panel's), and the trailing update applies all four
+// chains to an element in registers.  A negated element takes the two products of a step in the
+// other order, so both orientations round alike.  512 threads, up to two rows each; the active
+// rows are compacted after every 16 steps.  The next column is loaded while the pivot's is used (its
+// owner is published before the step's first barrier).
+constexpr int kBbTh = 512;
+constexpr int kBbSteps = 16;
+constexpr int kBbQuads = kBbSteps / 4;
+
+struct BbLayout {
+  size_t us, vs, pivs, cand, rt, misc, alist, clog, end;
+};
+__host__ __device__ inline BbLayout bb_layout(int n, int D) {
+  BbLayout L;
+  L.us = 0;
+  L.vs = L.us + 16 * (size_t)n * kBbQuads;
+  size_t uv = L.vs + 16 * (size_t)n * kBbQuads;
+  const size_t rows = 4 * (size_t)n * D + 4 * (size_t)n;  // gather: features and modes
+  uv = (uv > rows ? uv : rows) + 15 & ~(size_t)15;
+  L.pivs = uv;
+  L.cand = (L.pivs + sizeof(float) * (size_t)(n / 2) + 15) & ~(size_t)15;
+  L.rt = L.cand + 16 * sizeof(unsigned long long);
+  L.misc = L.rt + 36 * sizeof(int);
+  L.alist = L.misc + 8 * sizeof(int);
+  L.clog = L.alist + 2 * (size_t)n;
+  L.end = L.clog + 2 * (size_t)n;
+  return L;
+}
+
+// Entry (i, q) of the matrix as of step s: the stored element `c` (already negated where the row
+// precedes the column), the chains of the finished quads, the running quad's terms.
+__device__ __forceinline__ float bb_value(float c, bool gt, int i, int qi, int n, int quad,
+                                          const float4* Us, const float4* Vs) {
+  for (int b = 0; b < quad; ++b) {
+    const float4 u = Us[b * n + i], v = Vs[b * n + i], uq = Us[b * n + qi], vq = Vs[b * n + qi];
+    if (gt) {
+      c = fmaf(u.x, vq.x, c);
+      c = fmaf(-v.x, uq.x, c);
+      c = fmaf(u.y, vq.y, c);
+      c = fmaf(-v.y, uq.y, c);
+      c = fmaf(u.z, vq.z, c);
+      c = fmaf(-v.z, uq.z, c);
+      c = fmaf(u.w, vq.w, c);
+      c = fmaf(-v.w, uq.w, c);
+    } else {
+      c = fmaf(-v.x, uq.x, c);
+      c = fmaf(u.x, vq.x, c);
+      c = fmaf(-v.y, uq.y, c);
+      c = fmaf(u.y, vq.y, c);
+      c = fmaf(-v.z, uq.z, c);
+      c = fmaf(u.z, vq.z, c);
+      c = fmaf(-v.w, uq.w, c);
+      c = fmaf(u.w, vq.w, c);
+    }
+  }
+  const float4 u = Us[quad * n + i], v = Vs[quad * n + i];
+  const float4 uq = Us[quad * n + qi], vq = Vs[quad * n + qi];
+  c += u.x * vq.x - v.x * uq.x;  // terms past the running step are zero
+  c += u.y * vq.y - v.y * uq.y;
+  c += u.z * vq.z - v.z * uq.z;
+  c += u.w * vq.w - v.w * uq.w;
+  return c;
+}
+
+// Stored element (ph, q) of the triangle in global memory, negated where ph < q.
+__device__ __forceinline__ float bb_stored(const float* Lw, int ph, int off, int q, int qoff) {
+  const float c = __ldcg(Lw + (ph > q ? off + q : (ph < q ? qoff + ph : 0)));
+  return ph > q ? c : (ph < q ? -c : 0.0f);
+}
+
+// Up to 16 pivot steps from logical column k0 on the m active rows by the first PW warps.
+__device__ __forceinline__ void bb_panel(const float* Lw, float4* Us, float4* Vs, float* pivs,
+                                         unsigned long long* cand, int* rt, int* misc,
+                                         uint16_t* alist, uint16_t* clog, int n, int m, int k0,
+                                         int steps, int PW, int& swaps, uint16_t* perm) {
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  int ph[2], off[2], log[2];
+  float next[2];  // stored entries of the column of the coming step
+  const int ck0 = misc[0], ckp0 = alist[ck0], ckoff0 = tri_off(ckp0);
 #pragma unroll
-      for (int o = 16; o; o >>= 1) {
-        mant *= __shfl_xor_sync(0xffffffffu, mant, o);
-        expo += __shfl_xor_sync(0xffffffffu, expo, o);
-        neg ^= __shfl_xor_sync(0xffffffffu, neg, o);
-        flag |= __shfl_xor_sync(0xffffffffu, flag, o);
-        pmin = fminf(pmin, __shfl_xor_sync(0xffffffffu, pmin, o));
-        pmax = fmaxf(pmax, __shfl_xor_sync(0xffffffffu, pmax, o));
+  for (int q = 0; q < 2; ++q) {
+    const int i = tid + q * kBbTh;
+    const bool has = i < m;
+    ph[q] = has ? alist[i] : 0;
+    log[q] = has ? clog[i] : -1;
+    off[q] = tri_off(ph[q]);
+    next[q] = has ? bb_stored(Lw, ph[q], off[q], ckp0, ckoff0) : 0.0f;
+  }
+  if (wid == 0 && lane < 16) cand[lane] = 0ull;
+  bool zero = false;
+  int ci = ck0;
+#pragma unroll 1
+  for (int s = 0; s < steps; ++s) {
+    const int k = k0 + 2 * s, quad = s >> 2, j = s & 3;
+    if (j == 0) {  // a new quad of panel values starts from zeros
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int i = tid + q * kBbTh;
+        if (i < m) Us[quad * n + i] = Vs[quad * n + i] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      if (lane == 0) {
-        const float* isg = a.mode == 2 ? a.item_sign_out : a.item_sign;
-        float s = isg ? isg[item] : 1.0f;
-        double la;
-        if (isnan(s)) flag |= NH_FLAG_NONFINITE;  // the CNN could not compute this item
-        if (zero) {
-          s = 0.0f;
-          la = -INFINITY;
-          flag |= NH_FLAG_ZERO_PIVOT;
-        } else {
-          if (neg) s = -s;
-          la = log(mant) + (double)expo * 0.6931471805599453;
-          if (!isfinite(la)) flag |= NH_FLAG_NONFINITE;
-          if (a.cond_tau > 0.0 && (double)pmax > a.cond_tau * (double)pmin) flag |= NH_FLAG_GROWTH;
-          if (a.refine_tau > 0.0 && (double)pmax > a.refine_tau * (double)pmin)
-            flag |= kFlagNeedRefine;
+      panel_sync(PW);
+    }
+    const int ckp = alist[ci];
+    float c[2];
+    unsigned key[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      key[q] = 0u;
+      c[q] = 0.0f;
+      if (log[q] > k) {
+        c[q] = bb_value(next[q], ph[q] > ckp, tid + q * kBbTh, ci, n, quad, Us, Vs);
+        // |c| bits + 1 (NaN as +inf)
+        key[q] = min(__float_as_uint(c[q]) & 0x7FFFFFFFu, 0x7F800000u) + 1u;
+      }
+      if (log[q] == k + 1 || log[q] == k + 2) misc[log[q] - k] = tid + q * kBbTh;
+    }
+    // Maximum, ties to the lowest physical row (rows ascend with the index, slot 0 before slot 1).
+    unsigned kbest = __reduce_max_sync(0xffffffffu, max(key[0], key[1]));
+    const unsigned h0 = __ballot_sync(0xffffffffu, key[0] == kbest);
+    const unsigned h1 = __ballot_sync(0xffffffffu, key[1] == kbest);
+    const int wq = h0 ? 0 : 1, wl = __ffs(h0 ? h0 : h1) - 1;
+    // row index, sign, label: 0x3FF - index (10 bits), 1, 10 bits
+    const unsigned mine = ((0x3FFu - (unsigned)(tid + wq * kBbTh)) << 11) |
+                          (signbit(wq ? c[1] : c[0]) ? 0x400u : 0u) |
+                          ((unsigned)(wq ? log[1] : log[0]) & 0x3FFu);
+    unsigned lbest;
+    if (PW == 1) {
+      lbest = __shfl_sync(0xffffffffu, mine, wl);
+      __syncwarp();  // misc
+    } else {
+      if (lane == wl) cand[wid] = ((unsigned long long)kbest << 32) | mine;
+      panel_sync(PW);  // (1) pivot candidates, owners of the next labels
+      const unsigned long long w = cand[lane & 15];
+      const unsigned hi = (unsigned)(w >> 32);
+      kbest = __reduce_max_sync(0xffffffffu, hi);
+      lbest = __reduce_max_sync(0xffffffffu, hi == kbest ? (unsigned)w : 0u);
+    }
+    const float bk = kbest ? __uint_as_float(kbest - 1u) : -1.0f;
+    if (!(bk > 0.0f)) {  // exactly singular (or empty) column: pf = 0
+      zero = true;
+      panel_sync(PW);
+      break;
+    }
+    const int ri = 0x3FF - (int)(lbest >> 11), lr = (int)(lbest & 0x3FFu);
+    const float piv = (lbest & 0x400u) ? bk : -bk;
+    const int rp = alist[ri], roff = tri_off(rp);
+    ci = lr == k + 2 ? misc[1] : misc[2];
+    const bool more = s + 1 < steps;
+    const int cp = more ? alist[ci] : 0, coff = tri_off(cp);
+    float dv[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (log[q] <= k) continue;
+      // the row that held label k+1 takes the pivot's old label
+      log[q] = tid + q * kBbTh == ri ? k + 1 : (log[q] == k + 1 ? lr : log[q]);
+      dv[q] = bb_stored(Lw, ph[q], off[q], rp, roff);
+      if (more) next[q] = bb_stored(Lw, ph[q], off[q], cp, coff);
+    }
+    const float rpiv = 1.0f / piv;
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      if (log[q] > k + 1) {
+        const int i = tid + q * kBbTh;
+        const float u = bb_value(dv[q], ph[q] > rp, i, ri, n, quad, Us, Vs);
+        reinterpret_cast<float*>(Us + quad * n + i)[j] = u;
+        reinterpret_cast<float*>(Vs + quad * n + i)[j] = c[q] * rpiv;
+      }
+    if (tid == 0) pivs[k >> 1] = lr != k + 1 ? -piv : piv;
+    swaps ^= lr != k + 1 ? 1 : 0;
+    panel_sync(PW);  // (2) panel column written
+  }
+  // Eliminated rows leave: their order to the record, the others compacted in physical order (with
+  // their panel values, which the trailing update reads by the new index).
+  const int k_end = k0 + 2 * steps;
+  unsigned bal[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    bal[q] = __ballot_sync(0xffffffffu, log[q] >= k_end);
+    if (lane == 0) rt[q * 16 + wid] = __popc(bal[q]);
+    if (perm && !zero && log[q] >= 0 && log[q] < k_end) perm[log[q]] = (uint16_t)ph[q];
+  }
+  if (tid == 0) rt[32] = zero ? 1 : 0;
+  panel_sync(PW);
+  int base = 0, dst[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    int before = base;
+    for (int w = 0; w < PW; ++w) {
+      before += w < wid ? rt[q * 16 + w] : 0;
+      base += rt[q * 16 + w];
+    }
+    dst[q] = log[q] >= k_end ? before + __popc(bal[q] & ((1u << lane) - 1u)) : -1;
+    if (dst[q] >= 0) {
+      alist[dst[q]] = (uint16_t)ph[q];
+      clog[dst[q]] = (uint16_t)log[q];
+      if (log[q] == k_end) misc[0] = dst[q];
+    }
+  }
+  if (!zero && base > 0) {
+#pragma unroll 1
+    for (int b = 0; b < kBbQuads; ++b) {
+      float4 u[2], v[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        if (dst[q] >= 0) {
+          u[q] = Us[b * n + tid + q * kBbTh];
+          v[q] = Vs[b * n + tid + q * kBbTh];
         }
-        if (s == 0.0f) la = -INFINITY;
-        a.sign[item] = s;
-        a.logabs[item] = la;
-        if (a.flags) a.flags[item] = flag | a.flag_or;
-        if (a.ratio) a.ratio[item] = zero ? INFINITY : (float)((double)pmax / (double)pmin);
-        if (perm && !zero) perm[n] = (uint16_t)swaps;
+      panel_sync(PW);
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        if (dst[q] >= 0) {
+          Us[b * n + dst[q]] = u[q];
+          Vs[b * n + dst[q]] = v[q];
+        }
+      panel_sync(PW);
+    }
+  }
+}
+
+// Trailing update of the m active rows by the 16 steps' panel values: units of 8 rows x 64 columns
+// (lane: two columns, their panel values in registers), all loads of a unit in flight together.
+__device__ __forceinline__ void bb_trailing(float* Lw, const float4* Us, const float4* Vs,
+                                            const uint16_t* alist, int n, int m) {
+  constexpr int RT = 8, WARPS = kBbTh / 32;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int done = 0;
+  for (int c0 = 0; c0 + 1 < m; c0 += 64) {
+    const int units = (m - c0 - 1 + RT - 1) / RT;
+    const int u0 = (wid - done) & (WARPS - 1);
+    done += units;
+    if (u0 >= units) continue;
+    int pb[2];
+    float4 ub[2][kBbQuads], vb[2][kBbQuads];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int ib = min(c0 + lane + 32 * h, m - 1);
+      pb[h] = alist[ib];
+#pragma unroll
+      for (int b = 0; b < kBbQuads; ++b) {
+        ub[h][b] = Us[b * n + ib];
+        vb[h][b] = Vs[b * n + ib];
       }
     }
+#pragma unroll 1
+    for (int u = u0; u < units; u += WARPS) {
+      const int ia0 = c0 + 1 + u * RT;
+      float acc[RT][2];
+#pragma unroll
+      for (int r = 0; r < RT; ++r) {
+        const int ia = ia0 + r, off = tri_off(alist[min(ia, m - 1)]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          acc[r][h] = ia < m && c0 + lane + 32 * h < ia ? __ldcg(Lw + off + pb[h]) : 0.0f;
+      }
+#pragma unroll
+      for (int r = 0; r < RT; ++r) {
+        const int ia = min(ia0 + r, m - 1);
+#pragma unroll
+        for (int b = 0; b < kBbQuads; ++b) {
+          const float4 ua = Us[b * n + ia], va = Vs[b * n + ia];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            float x = acc[r][h];
+            x = fmaf(ua.x, vb[h][b].x, x);
+            x = fmaf(-va.x, ub[h][b].x, x);
+            x = fmaf(ua.y, vb[h][b].y, x);
+            x = fmaf(-va.y, ub[h][b].y, x);
+            x = fmaf(ua.z, vb[h][b].z, x);
+            x = fmaf(-va.z, ub[h][b].z, x);
+            x = fmaf(ua.w, vb[h][b].w, x);
+            x = fmaf(-va.w, ub[h][b].w, x);
+            acc[r][h] = x;
+          }
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < RT; ++r) {
+        const int ia = ia0 + r, off = tri_off(alist[min(ia, m - 1)]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (ia < m && c0 + lane + 32 * h < ia) __stcg(Lw + off + pb[h], acc[r][h]);
+      }
+    }
+  }
+}
+
+template <int D>
+__global__ void __launch_bounds__(kBbTh, 1) pf32_big_kernel(PfArgs a) {
+  constexpr int WARPS = kBbTh / 32;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int n = a.n, N = a.Lx * a.Ly;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const BbLayout L = bb_layout(n, a.mode == 0 ? 0 : D);
+  float4* Us = reinterpret_cast<float4*>(smem_raw + L.us);  // [quad][compact row]
+  float4* Vs = reinterpret_cast<float4*>(smem_raw + L.vs);
+  float* pivs = reinterpret_cast<float*>(smem_raw + L.pivs);
+  unsigned long long* cand = reinterpret_cast<unsigned long long*>(smem_raw + L.cand);
+  int* rt = reinterpret_cast<int*>(smem_raw + L.rt);      // compaction counts; [32] zero column
+  int* misc = reinterpret_cast<int*>(smem_raw + L.misc);  // compact rows of labels k, k + 1, k + 2
+  uint16_t* alist = reinterpret_cast<uint16_t*>(smem_raw + L.alist);
+  uint16_t* clog = reinterpret_cast<uint16_t*>(smem_raw + L.clog);
+  float* Lw = static_cast<float*>(a.tri) + (size_t)blockIdx.x * ((tri_off(n) + 3) & ~3);
+
+  const int n_work = a.count_dev ? (*a.count_dev) * a.count_mult : a.n_slots;
+  for (int slot = blockIdx.x; slot < n_work; slot += gridDim.x) {
+    const int item = a.slot_item ? a.slot_item[slot] : slot;
+    __syncthreads();  // the previous item's readers are done
+    if (a.mode == 0) {
+      const float* F = a.F + (size_t)item * n * n;
+      for (int i = wid; i < n; i += WARPS)
+        for (int j = lane; j < i; j += 32) __stcg(Lw + tri_off(i) + j, __ldg(F + (size_t)i * n + j));
+    } else {
+      float* Ys = reinterpret_cast<float*>(smem_raw);
+      int* ids = reinterpret_cast<int*>(Ys + (size_t)n * D);
+      const float4* src = reinterpret_cast<const float4*>(static_cast<const float*>(a.Y) +
+                                                          (size_t)slot * n * D);
+      constexpr int K = D / 4;
+      for (int v = tid; v < n * K; v += kBbTh) {
+        const int row = v / K;
+        reinterpret_cast<float4*>(Ys)[row * K + ((v % K) ^ swz_key(row, K))] = __ldg(src + v);
+      }
+      for (int p = tid; p < n; p += kBbTh)
+        ids[p] = pack_mode(__ldg(a.idx + (size_t)slot * n + p), N, a.Ly);
+      __syncthreads();
+      gather_from_rows<D, kBbTh>(a, Lw, Ys, ids);
+    }
+    __syncthreads();
+    for (int p = tid; p < n; p += kBbTh) alist[p] = clog[p] = (uint16_t)p;
+    if (tid == 0) misc[0] = 0;
+    __syncthreads();
+
+    uint16_t* perm = a.perm ? a.perm + (size_t)item * perm_stride(n) : nullptr;
+    int swaps = 0;
+    bool zero = false;
+    for (int k0 = 0; k0 < n - 1; k0 += 2 * kBbSteps) {
+      const int steps = min(kBbSteps, (n - k0) >> 1);
+      const int m = n - k0, PW = min(WARPS, (m + 31) >> 5);
+      if (wid < PW)
+        bb_panel(Lw, Us, Vs, pivs, cand, rt, misc, alist, clog, n, m, k0, steps, PW, swaps, perm);
+      __syncthreads();  // panel values and active rows compacted
+      zero = rt[32] != 0;
+      if (zero) break;
+      const int mt = m - 2 * steps;  // when rows remain, steps == kBbSteps
+      if (mt >= 2) {
+        bb_trailing(Lw, Us, Vs, alist, n, mt);
+        __syncthreads();
+      }
+    }
+    if (wid == 0)
+      write_pfaffian(a, item, zero, swaps, perm, a.item_sign, [&](int k) { return pivs[k]; });
   }
 }
 
@@ -1106,8 +1472,24 @@ int launch_pf32(const PfArgs& a, cudaStream_t st) {
              : launch_pf32_nb<4, D>(a, pf32_layout(a.n, 4).end, NH_K_PFAFFIAN, st);
 }
 
-// FP32 up to 256 rows: pf32_kernel; FP64: one CTA per SM; beyond shared memory (FP32 n > 256, FP64
-// n > 236): the large-lattice kernel.
+template <int D>
+int launch_pf32_big(const PfArgs& a, cudaStream_t st) {
+  if (!a.tri)
+    return fail(NH_ERR_UNSUPPORTED, "Pfaffian: n=%d needs the large-lattice scratch", a.n);
+  const size_t smem = bb_layout(a.n, a.mode == 0 ? 0 : D).end;
+  if (smem > 227 * 1024)
+    return fail(NH_ERR_UNSUPPORTED, "Pfaffian: n=%d needs %zu B of shared memory", a.n, smem);
+  if (int rc = raise_smem_cap(pf32_big_kernel<D>, smem)) return rc;
+  int grid = num_sms();
+  if (grid > a.n_slots) grid = a.n_slots;
+  if (grid <= 0) return NH_OK;
+  ProfScope prof_scope(NH_K_PFAFFIAN, st);
+  pf32_big_kernel<D><<<grid, kBbTh, smem, st>>>(a);
+  return check_launch("pf32_big_kernel");
+}
+
+// FP32: pf32_kernel up to 256 rows, pf32_big_kernel beyond; FP64: one CTA per SM, beyond shared memory
+// (n > 236) the triangle in global memory.
 template <typename T, int D>
 int launch_pf_pick(const PfArgs& a, cudaStream_t st) {
   if (a.n <= kNumThreads) {
@@ -1118,7 +1500,10 @@ int launch_pf_pick(const PfArgs& a, cudaStream_t st) {
       if (pf_smem<T, 2>(a.n) <= 227 * 1024) return launch_pf<T, 2, D>(a, st);
     }
   }
-  return launch_pf<T, kBigNB, D, kBigThreads>(a, st);
+  if constexpr (sizeof(T) == 4)
+    return launch_pf32_big<D>(a, st);
+  else
+    return launch_pf<T, kBigNB, D, kBigThreads>(a, st);
 }
 
 template <typename T>
@@ -1815,6 +2200,23 @@ int launch_pfaffian_from_F(const float* F, int n, int batch, const int32_t* list
   return fp64 ? launch_pf_pick<double, 16>(a, st) : launch_pf_pick<float, 16>(a, st);
 }
 
+// Wt (rows, d) to chunks of four a: Wc[(a / 4) rows + row].
+__global__ void wt_chunk_kernel(const float4* __restrict__ Wt, int rows, int chunks,
+                                float4* __restrict__ Wc) {
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < rows * chunks; e += gridDim.x * blockDim.x) {
+    const int c = e / rows, row = e - c * rows;
+    Wc[e] = __ldg(Wt + (size_t)row * chunks + c);
+  }
+}
+
+static int launch_wt_chunks(const float* Wt, int N, int d, float* Wc, cudaStream_t st) {
+  const int total = 4 * N * (d / 4);
+  ProfScope prof_scope(NH_K_PACK, st);
+  wt_chunk_kernel<<<(total + 255) / 256, 256, 0, st>>>(reinterpret_cast<const float4*>(Wt), 4 * N,
+                                                       d / 4, reinterpret_cast<float4*>(Wc));
+  return check_launch("wt_chunk_kernel");
+}
+
 int launch_pfaffian_gather(const PfGatherArgs& g, cudaStream_t st) {
   if (g.n <= 0 || g.n % 2 || g.n > kBigThreads)
     return fail(NH_ERR_UNSUPPORTED, "amplitude: n=%d must be even and <= %d", g.n, kBigThreads);
@@ -1840,6 +2242,14 @@ int launch_pfaffian_gather(const PfGatherArgs& g, cudaStream_t st) {
   a.perm = g.perm;
   a.refine_tau = g.refine_tau;
   a.ratio = g.ratio;
+  if (!g.fp64 && g.n > kNumThreads) {  // pf32_big_kernel gathers from the chunked table
+    if (!g.wt_chunks) return fail(NH_ERR_INVALID, "amplitude: n=%d needs the chunked table", g.n);
+    if (int rc = launch_wt_chunks(static_cast<const float*>(g.Wt), g.Lx * g.Ly, g.d, g.wt_chunks, st))
+      return rc;
+    a.Wc = reinterpret_cast<const float4*>(g.wt_chunks);
+    a.mode = 3;
+    a.tail_row = g.n;
+  }
   return g.fp64 ? launch_pf_d<double>(a, g.d, st) : launch_pf_d<float>(a, g.d, st);
 }
 
@@ -1954,23 +2364,6 @@ bool fused_supported(const nh_backflow_params& p) {
 bool staged_supported(const PfGatherArgs& g) {
   return !g.fp64 && g.n <= kNumThreads && g.n % 2 == 0 && g.d % 4 == 0 && g.d <= 32 && !g.tri &&
          g.wt_chunks;
-}
-
-// Wt (rows, d) to chunks of four a: Wc[(a / 4) rows + row].
-__global__ void wt_chunk_kernel(const float4* __restrict__ Wt, int rows, int chunks,
-                                float4* __restrict__ Wc) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < rows * chunks; e += gridDim.x * blockDim.x) {
-    const int c = e / rows, row = e - c * rows;
-    Wc[e] = __ldg(Wt + (size_t)row * chunks + c);
-  }
-}
-
-static int launch_wt_chunks(const float* Wt, int N, int d, float* Wc, cudaStream_t st) {
-  const int total = 4 * N * (d / 4);
-  ProfScope prof_scope(NH_K_PACK, st);
-  wt_chunk_kernel<<<(total + 255) / 256, 256, 0, st>>>(reinterpret_cast<const float4*>(Wt), 4 * N,
-                                                       d / 4, reinterpret_cast<float4*>(Wc));
-  return check_launch("wt_chunk_kernel");
 }
 
 int launch_pfaffian_staged(const PfGatherArgs& g, cudaStream_t st) {
