@@ -1096,7 +1096,7 @@ constexpr int kBbSteps = 16;
 constexpr int kBbQuads = kBbSteps / 4;
 
 struct BbLayout {
-  size_t us, vs, pivs, cand, rt, misc, alist, clog, end;
+  size_t us, vs, pivs, cand, rt, misc, offs, alist, clog, end;
 };
 __host__ __device__ inline BbLayout bb_layout(int n, int D) {
   BbLayout L;
@@ -1109,7 +1109,8 @@ __host__ __device__ inline BbLayout bb_layout(int n, int D) {
   L.cand = (L.pivs + sizeof(float) * (size_t)(n / 2) + 15) & ~(size_t)15;
   L.rt = L.cand + 16 * sizeof(unsigned long long);
   L.misc = L.rt + 36 * sizeof(int);
-  L.alist = L.misc + 8 * sizeof(int);
+  L.offs = L.misc + 8 * sizeof(int);
+  L.alist = L.offs + sizeof(int) * (size_t)n;
   L.clog = L.alist + 2 * (size_t)n;
   L.end = L.clog + 2 * (size_t)n;
   return L;
@@ -1158,7 +1159,7 @@ __device__ __forceinline__ float bb_stored(const float* Lw, int ph, int off, int
 
 // Up to 16 pivot steps from logical column k0 on the m active rows by the first PW warps.
 __device__ __forceinline__ void bb_panel(const float* Lw, float4* Us, float4* Vs, float* pivs,
-                                         unsigned long long* cand, int* rt, int* misc,
+                                         unsigned long long* cand, int* rt, int* misc, int* offs,
                                          uint16_t* alist, uint16_t* clog, int n, int m, int k0,
                                          int steps, int PW, int& swaps, uint16_t* perm) {
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -1281,6 +1282,7 @@ __device__ __forceinline__ void bb_panel(const float* Lw, float4* Us, float4* Vs
     if (dst[q] >= 0) {
       alist[dst[q]] = (uint16_t)ph[q];
       clog[dst[q]] = (uint16_t)log[q];
+      offs[dst[q]] = off[q];
       if (log[q] == k_end) misc[0] = dst[q];
     }
   }
@@ -1306,13 +1308,59 @@ __device__ __forceinline__ void bb_panel(const float* Lw, float4* Us, float4* Vs
   }
 }
 
+// One unit of the trailing update: RT rows from ia0 on the lane's two columns (physical rows pb,
+// panel values ub / vb).  FULL: every row exists and reaches both columns of every lane.
+template <int RT, bool FULL>
+__device__ __forceinline__ void bb_unit(float* Lw, const float4* Us, const float4* Vs, const int* offs,
+                                        int n, int m, int ia0, int col, const int (&pb)[2],
+                                        const float4 (&ub)[2][kBbQuads],
+                                        const float4 (&vb)[2][kBbQuads]) {
+  float acc[RT][2];
+  int off[RT];
+#pragma unroll
+  for (int r = 0; r < RT; ++r) {
+    off[r] = offs[FULL ? ia0 + r : min(ia0 + r, m - 1)];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      acc[r][h] = FULL || (ia0 + r < m && col + 32 * h < ia0 + r) ? __ldcg(Lw + off[r] + pb[h]) : 0.0f;
+  }
+#pragma unroll
+  for (int r = 0; r < RT; ++r) {
+    const int ia = FULL ? ia0 + r : min(ia0 + r, m - 1);
+#pragma unroll
+    for (int b = 0; b < kBbQuads; ++b) {
+      const float4 ua = Us[b * n + ia], va = Vs[b * n + ia];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float x = acc[r][h];
+        x = fmaf(ua.x, vb[h][b].x, x);
+        x = fmaf(-va.x, ub[h][b].x, x);
+        x = fmaf(ua.y, vb[h][b].y, x);
+        x = fmaf(-va.y, ub[h][b].y, x);
+        x = fmaf(ua.z, vb[h][b].z, x);
+        x = fmaf(-va.z, ub[h][b].z, x);
+        x = fmaf(ua.w, vb[h][b].w, x);
+        x = fmaf(-va.w, ub[h][b].w, x);
+        acc[r][h] = x;
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < RT; ++r)
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (FULL || (ia0 + r < m && col + 32 * h < ia0 + r)) __stcg(Lw + off[r] + pb[h], acc[r][h]);
+}
+
 // Trailing update of the m active rows by the 16 steps' panel values: units of 8 rows x 64 columns
 // (lane: two columns, their panel values in registers), all loads of a unit in flight together.
+// offs: the rows' offsets in the triangle.
 __device__ __forceinline__ void bb_trailing(float* Lw, const float4* Us, const float4* Vs,
-                                            const uint16_t* alist, int n, int m) {
+                                            const uint16_t* alist, const int* offs, int n, int m) {
   constexpr int RT = 8, WARPS = kBbTh / 32;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int done = 0;
+#pragma unroll 1
   for (int c0 = 0; c0 + 1 < m; c0 += 64) {
     const int units = (m - c0 - 1 + RT - 1) / RT;
     const int u0 = (wid - done) & (WARPS - 1);
@@ -1333,42 +1381,10 @@ __device__ __forceinline__ void bb_trailing(float* Lw, const float4* Us, const f
 #pragma unroll 1
     for (int u = u0; u < units; u += WARPS) {
       const int ia0 = c0 + 1 + u * RT;
-      float acc[RT][2];
-#pragma unroll
-      for (int r = 0; r < RT; ++r) {
-        const int ia = ia0 + r, off = tri_off(alist[min(ia, m - 1)]);
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          acc[r][h] = ia < m && c0 + lane + 32 * h < ia ? __ldcg(Lw + off + pb[h]) : 0.0f;
-      }
-#pragma unroll
-      for (int r = 0; r < RT; ++r) {
-        const int ia = min(ia0 + r, m - 1);
-#pragma unroll
-        for (int b = 0; b < kBbQuads; ++b) {
-          const float4 ua = Us[b * n + ia], va = Vs[b * n + ia];
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            float x = acc[r][h];
-            x = fmaf(ua.x, vb[h][b].x, x);
-            x = fmaf(-va.x, ub[h][b].x, x);
-            x = fmaf(ua.y, vb[h][b].y, x);
-            x = fmaf(-va.y, ub[h][b].y, x);
-            x = fmaf(ua.z, vb[h][b].z, x);
-            x = fmaf(-va.z, ub[h][b].z, x);
-            x = fmaf(ua.w, vb[h][b].w, x);
-            x = fmaf(-va.w, ub[h][b].w, x);
-            acc[r][h] = x;
-          }
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < RT; ++r) {
-        const int ia = ia0 + r, off = tri_off(alist[min(ia, m - 1)]);
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          if (ia < m && c0 + lane + 32 * h < ia) __stcg(Lw + off + pb[h], acc[r][h]);
-      }
+      if (ia0 >= c0 + 64 && ia0 + RT <= m)
+        bb_unit<RT, true>(Lw, Us, Vs, offs, n, m, ia0, c0 + lane, pb, ub, vb);
+      else
+        bb_unit<RT, false>(Lw, Us, Vs, offs, n, m, ia0, c0 + lane, pb, ub, vb);
     }
   }
 }
@@ -1386,6 +1402,7 @@ __global__ void __launch_bounds__(kBbTh, 1) pf32_big_kernel(PfArgs a) {
   unsigned long long* cand = reinterpret_cast<unsigned long long*>(smem_raw + L.cand);
   int* rt = reinterpret_cast<int*>(smem_raw + L.rt);      // compaction counts; [32] zero column
   int* misc = reinterpret_cast<int*>(smem_raw + L.misc);  // compact rows of labels k, k + 1, k + 2
+  int* offs = reinterpret_cast<int*>(smem_raw + L.offs);  // triangle offsets of the active rows
   uint16_t* alist = reinterpret_cast<uint16_t*>(smem_raw + L.alist);
   uint16_t* clog = reinterpret_cast<uint16_t*>(smem_raw + L.clog);
   float* Lw = static_cast<float*>(a.tri) + (size_t)blockIdx.x * ((tri_off(n) + 3) & ~3);
@@ -1425,13 +1442,14 @@ __global__ void __launch_bounds__(kBbTh, 1) pf32_big_kernel(PfArgs a) {
       const int steps = min(kBbSteps, (n - k0) >> 1);
       const int m = n - k0, PW = min(WARPS, (m + 31) >> 5);
       if (wid < PW)
-        bb_panel(Lw, Us, Vs, pivs, cand, rt, misc, alist, clog, n, m, k0, steps, PW, swaps, perm);
+        bb_panel(Lw, Us, Vs, pivs, cand, rt, misc, offs, alist, clog, n, m, k0, steps, PW, swaps,
+                 perm);
       __syncthreads();  // panel values and active rows compacted
       zero = rt[32] != 0;
       if (zero) break;
       const int mt = m - 2 * steps;  // when rows remain, steps == kBbSteps
       if (mt >= 2) {
-        bb_trailing(Lw, Us, Vs, alist, n, mt);
+        bb_trailing(Lw, Us, Vs, alist, offs, n, mt);
         __syncthreads();
       }
     }
