@@ -38,6 +38,58 @@ __device__ __forceinline__ void cnn_lds8(const double* p, double* o) {
   }
 }
 
+template <int S>
+struct Sites {
+  static constexpr int value = S;
+};
+
+// One task of a periodic 3x3 cross-correlation: S sites x 8 output channels (group grp of cout / 8) of
+// cin planes of stride N + 1, weights [ci][tap][co] in shared memory, accumulated in order of
+// (ci, tap) onto acc.  With four sites a thread issues 32 FMAs per 4 loads of inputs and two
+// broadcast 16-byte weight loads (two cycles of the load port each), which is what bounds it.
+template <typename T, int S>
+__device__ __forceinline__ void conv_task(const T* in, int cin, int cout, const T* wsm, int grp,
+                                          const int (&site)[S], int Lx, int Ly, T (&acc)[S][8]) {
+  const int NS = Lx * Ly + 1;
+  int row[S][3], col[S][3];
+#pragma unroll
+  for (int k = 0; k < S; ++k) {
+    const int x = site[k] / Ly, y = site[k] - x * Ly;
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+      int xx = x + u - 1, yy = y + u - 1;
+      xx = xx < 0 ? xx + Lx : (xx >= Lx ? xx - Lx : xx);
+      yy = yy < 0 ? yy + Ly : (yy >= Ly ? yy - Ly : yy);
+      row[k][u] = xx * Ly;
+      col[k][u] = yy;
+    }
+  }
+#pragma unroll 1
+  for (int ci = 0; ci < cin; ++ci) {
+    const T* inc = in + ci * NS;
+    const T* wc = wsm + ci * 9 * cout + grp * 8;
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {
+#pragma unroll
+      for (int v = 0; v < 3; ++v) {
+        T w8[8];
+        cnn_lds8(wc + (u * 3 + v) * cout, w8);
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+          const T i0 = inc[row[k][u] + col[k][v]];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[k][j] = fma(i0, w8[j], acc[k][j]);
+        }
+      }
+    }
+  }
+}
+
+// Sites per task: four where that still gives every thread of a TH-thread block a task.
+__device__ __forceinline__ bool conv_four_sites(int N, int cout, int TH) {
+  return N % 4 == 0 && (cout / 8) * (N / 4) >= TH;
+}
+
 // Builds the item's image configuration in simg (2N ints, +-1) and runs the layers; returns the
 // activation buffer (actA or actB) that holds the last layer's output, C planes of stride N + 1.
 // wsm: C * C * 9 values, bsm: C values (shared memory); actA, actB: C (N + 1) values each
@@ -48,7 +100,7 @@ __device__ T* cnn_layers(const float* __restrict__ wp, const float* __restrict__
                          int to, int g, T* actA, T* actB, T* wsm, T* bsm, int* simg) {
   const int tid = threadIdx.x;
   const int N = Lx * Ly, NS = N + 1, M2 = 2 * N;
-  const int half = N / 2, ngroups = C / 8;
+  const int ngroups = C / 8;
   for (int m = tid; m < M2; m += TH) {
     const int src = sym_map(m, g, Lx, Ly, N);  // image[m] = s[g(m)] (g is an involution)
     const int v = move_value(src, base[src], fr, to);
@@ -67,44 +119,33 @@ __device__ T* cnn_layers(const float* __restrict__ wp, const float* __restrict__
     for (int i = tid; i < C; i += TH) bsm[i] = T(__ldg(bias + l * C + i));
     __syncthreads();
     const bool act_fn = l < layers - 1;
-    for (int task = tid; task < ngroups * half; task += TH) {
-      const int grp = task / half;
-      const int s0 = task - grp * half, s1 = s0 + half;
-      const int x0 = s0 / Ly, y0 = s0 - x0 * Ly;
-      const int x1 = s1 / Ly, y1 = s1 - x1 * Ly;
-      T acc0[8], acc1[8];
+    auto tasks = [&](auto sites) {
+      constexpr int S = decltype(sites)::value;
+      const int part = N / S;
+      for (int task = tid; task < ngroups * part; task += TH) {
+        const int grp = task / part;
+        int site[S];
+        T acc[S][8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc0[j] = acc1[j] = bsm[grp * 8 + j];
-      for (int ci = 0; ci < cin; ++ci) {
-        const T* inc = in + ci * NS;
+        for (int k = 0; k < S; ++k) {
+          site[k] = task - grp * part + k * part;
 #pragma unroll
-        for (int u = 0; u < 3; ++u) {
-          int xa = x0 + u - 1, xb = x1 + u - 1;
-          xa = xa < 0 ? xa + Lx : (xa >= Lx ? xa - Lx : xa);
-          xb = xb < 0 ? xb + Lx : (xb >= Lx ? xb - Lx : xb);
-#pragma unroll
-          for (int v = 0; v < 3; ++v) {
-            int ya = y0 + v - 1, yb = y1 + v - 1;
-            ya = ya < 0 ? ya + Ly : (ya >= Ly ? ya - Ly : ya);
-            yb = yb < 0 ? yb + Ly : (yb >= Ly ? yb - Ly : yb);
-            const T i0 = inc[xa * Ly + ya];
-            const T i1 = inc[xb * Ly + yb];
-            T w8[8];
-            cnn_lds8(wsm + (ci * 9 + u * 3 + v) * C + grp * 8, w8);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              acc0[j] = fma(i0, w8[j], acc0[j]);
-              acc1[j] = fma(i1, w8[j], acc1[j]);
-            }
-          }
+          for (int j = 0; j < 8; ++j) acc[k][j] = bsm[grp * 8 + j];
         }
-      }
+        conv_task<T, S>(in, cin, C, wsm, grp, site, Lx, Ly, acc);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        out[(grp * 8 + j) * NS + s0] = act_fn ? gelu_tanh_dev(acc0[j]) : acc0[j];
-        out[(grp * 8 + j) * NS + s1] = act_fn ? gelu_tanh_dev(acc1[j]) : acc1[j];
+        for (int k = 0; k < S; ++k)
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            out[(grp * 8 + j) * NS + site[k]] = act_fn ? gelu_tanh_dev(acc[k][j]) : acc[k][j];
       }
-    }
+    };
+    if (sizeof(T) == 4 && conv_four_sites(N, C, TH))
+      tasks(Sites<4>{});
+    else if (sizeof(T) == 4 && ngroups * N <= TH)  // small lattices: every thread a task
+      tasks(Sites<1>{});
+    else
+      tasks(Sites<2>{});
     wl += C * cin * 9;
     cin = C;
     T* t = in;
