@@ -85,12 +85,12 @@ __global__ void __launch_bounds__(kDetThreads, sizeof(T) == 4 && TC <= 4 ? 2 : 1
   int* inv_s = rho + NP;                           // [16] inversions of the warps' rows, mod 2
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const T* Yb = static_cast<const T*>(a.Y);
-  const V* Wud = reinterpret_cast<const V*>(static_cast<const T*>(a.Wt) + (size_t)N * D);
+  const T* Wud = static_cast<const T*>(a.Wt) + (size_t)N * D;
   const int n_work = a.count_dev ? (*a.count_dev) * a.count_mult : a.n_slots;
   if ((int)blockIdx.x < n_work)
-    for (int e = threadIdx.x; e < N * K; e += kDetThreads) {
-      const int row = e / K;
-      wsm[(e - row * K) * N + row] = __ldg(Wud + e);
+    for (int e = threadIdx.x; e < N * D; e += kDetThreads) {  // scalar: any alignment of the table
+      const int row = e / D, c = e - row * D;
+      reinterpret_cast<T*>(wsm)[((c / E) * N + row) * E + c % E] = __ldg(Wud + e);
     }
 
   for (int slot_i = blockIdx.x; slot_i < n_work; slot_i += gridDim.x) {
