@@ -487,9 +487,10 @@ int launch_pf_adjoint(const float* F, float* G, int n, int batch, const float* p
                       const double* pf_logabs, int n_img, int32_t* flags, cudaStream_t st);
 // Per item dY (may be null) and, with jac null, per item dWt (items, 4, N, d); with jac set the
 // images' dWt of each sample are summed and chained through build_wtilde's backward into
-// jac[sample * ld + off_w + (3 N d W values, theta)].
+// jac[sample * ld + off_w + (3 N d W values, theta)].  wt_chunks: Wt in chunks of four a
+// (launch_pfaffian_staged leaves it in its buffer), or null.
 int launch_pairing_vjp(const float* G, const float* Y, const int32_t* idx, const float* Wt,
-                       int Lx, int Ly, int d, int n, int n_img, int samples, float* dY,
+                       const float* wt_chunks, int Lx, int Ly, int d, int n, int n_img, int samples, float* dY,
                        float* dWt, float* jac, int64_t ld, int64_t off_w, float theta,
                        cudaStream_t st);
 // Convolution weight and bias cotangents of every sample's images, summed into jac[sample * ld].

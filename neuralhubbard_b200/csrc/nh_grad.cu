@@ -254,6 +254,7 @@ struct VjpArgs {
   const float* Y;      // (items, n, d)
   const int32_t* idx;  // (items, n)
   const float* Wt;     // (4, N, d)
+  const float4* Wc;    // or null: the same table in chunks, Wc[(a / 4) 4 N + row]
   int Lx, Ly, n;
   int n_img;           // images per sample (items = samples * n_img)
   int samples;
@@ -325,27 +326,32 @@ __global__ void __launch_bounds__(kVjpThreads, 1) pairing_vjp_kernel(VjpArgs a) 
         inv[m] = p;
       }
       __syncthreads();
-      // dY: warp per row p, lanes over q.
+      // dY: lane <-> row p (16 per warp, the two half-warps taking alternate q), so that Y[q] is a
+      // broadcast, the lanes' neighbouring table rows share cache lines (chunked table) and the sums
+      // need one exchange at the end.
       if (a.dY) {
         float* dYi = a.dY + item * n * D;
-        for (int p = warp; p < n; p += kVjpThreads / 32) {
+        for (int p0 = 16 * warp; p0 < n; p0 += 16 * (kVjpThreads / 32)) {
+          const int pl = p0 + (lane & 15), p = pl < n ? pl : n - 1;
           const int mp = modes[p];
           const int sp = mp >> 16, xp = (mp >> 8) & 0xFF, yp = mp & 0xFF;
           float acc[D];
 #pragma unroll
           for (int j = 0; j < D; ++j) acc[j] = 0.0f;
-          for (int q = lane; q < n; q += 32) {
+#pragma unroll 2
+          for (int q = lane >> 4; q < n; q += 2) {
             const float gh = gs[p * NS + q] - gs[q * NS + p];
             const int mq = modes[q];
             const int sq = mq >> 16;
             int dx = xp - ((mq >> 8) & 0xFF), dy = yp - (mq & 0xFF);
             dx += dx < 0 ? Lx : 0;
             dy += dy < 0 ? Ly : 0;
-            const float4* w4 = reinterpret_cast<const float4*>(
-                a.Wt + ((size_t)(2 * sp + sq) * N + dx * Ly + dy) * D);
+            const int row = (2 * sp + sq) * N + dx * Ly + dy;
+            const float4* w4 = a.Wc ? a.Wc + row : reinterpret_cast<const float4*>(a.Wt) + row * (D / 4);
+            const int stride = a.Wc ? 4 * N : 1;
 #pragma unroll
             for (int c = 0; c < D / 4; ++c) {
-              const float4 w = __ldg(w4 + c);
+              const float4 w = __ldg(w4 + c * stride);
               const float4 y = *reinterpret_cast<const float4*>(ys + swz_index<float, D>(q, 4 * c));
               acc[4 * c + 0] = fmaf(gh * w.x, y.x, acc[4 * c + 0]);
               acc[4 * c + 1] = fmaf(gh * w.y, y.y, acc[4 * c + 1]);
@@ -354,37 +360,46 @@ __global__ void __launch_bounds__(kVjpThreads, 1) pairing_vjp_kernel(VjpArgs a) 
             }
           }
 #pragma unroll
-          for (int j = 0; j < D; ++j) {
+          for (int j = 0; j < D; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 16);
+          if (lane < 16 && pl < n)
 #pragma unroll
-            for (int o = 16; o; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
-          }
-          float mine = 0.0f;
-#pragma unroll
-          for (int j = 0; j < D; ++j)
-            if (lane == j) mine = acc[j];
-          if (lane < D) dYi[(size_t)p * D + lane] = mine;
+            for (int j = 0; j < D; ++j) dYi[(size_t)pl * D + j] = acc[j];  // any float alignment
         }
       }
-      // dWt: each (pair, chunk) sums over the rows p; partner q = inv[sq, site_p - r].
-      for (int p = 0; p < n; ++p) {
+      // dWt: each (pair, chunk) sums over the rows p; partner q = inv[sq, site_p - r].  The loads of an
+      // empty partner read row 0 and are not added, so that consecutive rows overlap.
+      auto add_row = [&](int p, float4 (&acc)[kCh]) {
         const int mp = modes[p];
-        const int sp = mp >> 16, xp = (mp >> 8) & 0xFF, yp = mp & 0xFF;
+        const int xp = (mp >> 8) & 0xFF, yp = mp & 0xFF;
         const float4 y1 = *reinterpret_cast<const float4*>(ys + swz_index<float, D>(p, 4 * c_own));
 #pragma unroll
         for (int pi = 0; pi < kCh; ++pi) {
-          if (!p_ok[pi]) continue;
           int x = xp - p_rx[pi], y = yp - p_ry[pi];
           x += x < 0 ? Lx : 0;
           y += y < 0 ? Ly : 0;
-          const int q = inv[p_base[pi] + x * Ly + y];
-          if (q < 0) continue;
-          const float gv = gs[p * NS + q];
-          const float4 y2 = *reinterpret_cast<const float4*>(ys + swz_index<float, D>(q, 4 * c_own));
-          float4& acc = sp ? acc1[pi] : acc0[pi];
-          acc.x = fmaf(gv * y1.x, y2.x, acc.x);
-          acc.y = fmaf(gv * y1.y, y2.y, acc.y);
-          acc.z = fmaf(gv * y1.z, y2.z, acc.z);
-          acc.w = fmaf(gv * y1.w, y2.w, acc.w);
+          const int q = p_ok[pi] ? inv[p_base[pi] + x * Ly + y] : -1;
+          const int qq = q < 0 ? 0 : q;
+          const float gv = gs[p * NS + qq];
+          const float4 y2 = *reinterpret_cast<const float4*>(ys + swz_index<float, D>(qq, 4 * c_own));
+          if (q >= 0) {
+            acc[pi].x = fmaf(gv * y1.x, y2.x, acc[pi].x);
+            acc[pi].y = fmaf(gv * y1.y, y2.y, acc[pi].y);
+            acc[pi].z = fmaf(gv * y1.z, y2.z, acc[pi].z);
+            acc[pi].w = fmaf(gv * y1.w, y2.w, acc[pi].w);
+          }
+        }
+      };
+      // rows of one spin in turn (the modes ascend, so there is one run of each)
+      for (int p = 0; p < n;) {
+        const int sp = modes[p] >> 16;
+        int end = p + 1;
+        while (end < n && (modes[end] >> 16) == sp) ++end;
+        if (sp) {
+#pragma unroll 2
+          for (; p < end; ++p) add_row(p, acc1);
+        } else {
+#pragma unroll 2
+          for (; p < end; ++p) add_row(p, acc0);
         }
       }
       if (a.mode == 0) {  // per-item dWt
@@ -508,49 +523,25 @@ int launch_vjp_t(const VjpArgs& a, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------ CNN VJP
-// One periodic 3x3 cross-correlation of cin planes (stride NS) into cout planes, weights
-// [ci][tap][co] in shared memory, bias (or none), epilogue(co, site, z) stores the result.
+constexpr int kCvThreads = 512;
+
+// One periodic 3x3 cross-correlation of cin planes (stride N + 1) into cout planes, weights
+// [ci][tap][co] in shared memory, no bias; epi(co, site, z) stores the result.
 template <typename Epi>
 __device__ __forceinline__ void conv_planes(const float* in, int cin, int cout, const float* wsm,
-                                            const float* bsm, int Lx, int Ly, Epi epi) {
-  const int N = Lx * Ly, NS = N + 1, half = N / 2, ngroups = cout / 8;
-  for (int task = threadIdx.x; task < ngroups * half; task += kNumThreads) {
-    const int grp = task / half;
-    const int s0 = task - grp * half, s1 = s0 + half;
-    const int x0 = s0 / Ly, y0 = s0 - x0 * Ly;
-    const int x1 = s1 / Ly, y1 = s1 - x1 * Ly;
-    float acc0[8], acc1[8];
+                                            int Lx, int Ly, Epi epi) {
+  const int part = Lx * Ly / 2;
+  for (int task = threadIdx.x; task < (cout / 8) * part; task += kCvThreads) {
+    const int grp = task / part;
+    const int site[2] = {task - grp * part, task - grp * part + part};
+    float acc[2][8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc0[j] = acc1[j] = bsm ? bsm[grp * 8 + j] : 0.0f;
-    for (int ci = 0; ci < cin; ++ci) {
-      const float* inc = in + ci * NS;
+    for (int j = 0; j < 8; ++j) acc[0][j] = acc[1][j] = 0.0f;
+    conv_task<float, 2>(in, cin, cout, wsm, grp, site, Lx, Ly, acc);
 #pragma unroll
-      for (int u = 0; u < 3; ++u) {
-        int xa = x0 + u - 1, xb = x1 + u - 1;
-        xa = xa < 0 ? xa + Lx : (xa >= Lx ? xa - Lx : xa);
-        xb = xb < 0 ? xb + Lx : (xb >= Lx ? xb - Lx : xb);
+    for (int k = 0; k < 2; ++k)
 #pragma unroll
-        for (int v = 0; v < 3; ++v) {
-          int ya = y0 + v - 1, yb = y1 + v - 1;
-          ya = ya < 0 ? ya + Ly : (ya >= Ly ? ya - Ly : ya);
-          yb = yb < 0 ? yb + Ly : (yb >= Ly ? yb - Ly : yb);
-          const float i0 = inc[xa * Ly + ya];
-          const float i1 = inc[xb * Ly + yb];
-          float w8[8];
-          cnn_lds8(wsm + (ci * 9 + u * 3 + v) * cout + grp * 8, w8);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            acc0[j] = fmaf(i0, w8[j], acc0[j]);
-            acc1[j] = fmaf(i1, w8[j], acc1[j]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      epi(grp * 8 + j, s0, acc0[j]);
-      epi(grp * 8 + j, s1, acc1[j]);
-    }
+      for (int j = 0; j < 8; ++j) epi(grp * 8 + j, site[k], acc[k][j]);
   }
 }
 
@@ -575,7 +566,7 @@ struct CnnVjpArgs {
 
 // Shared memory: z planes of layers 0 .. L-2 ((L-1) C NS), the input image (2 NS), two cotangent /
 // activation buffers (2 C NS) and one layer's weights (C C 9).
-__global__ void __launch_bounds__(kNumThreads) cnn_vjp_kernel(CnnVjpArgs a) {
+__global__ void __launch_bounds__(kCvThreads) cnn_vjp_kernel(CnnVjpArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int Lx = a.Lx, Ly = a.Ly, N = Lx * Ly, NS = N + 1, C = a.C, L = a.layers, d = C / 2;
   const int tid = threadIdx.x;
@@ -592,7 +583,7 @@ __global__ void __launch_bounds__(kNumThreads) cnn_vjp_kernel(CnnVjpArgs a) {
       const size_t item = (size_t)smp * a.n_img + g;
       const int sym = a.n_img == 1 ? 0 : g;
       __syncthreads();
-      for (int m = tid; m < 2 * N; m += kNumThreads) {
+      for (int m = tid; m < 2 * N; m += kCvThreads) {
         const int src = sym_map(m, sym, Lx, Ly, N);
         const int ch = m >= N ? 1 : 0;
         img[ch * NS + (m - ch * N)] = base[src] > 0 ? 1.0f : -1.0f;
@@ -603,14 +594,14 @@ __global__ void __launch_bounds__(kNumThreads) cnn_vjp_kernel(CnnVjpArgs a) {
       size_t woff = 0;
       for (int l = 0; l < L - 1; ++l) {
         __syncthreads();
-        for (int i = tid; i < C * cin * 9; i += kNumThreads) wsm[i] = __ldg(a.conv_w_packed + woff + i);
+        for (int i = tid; i < C * cin * 9; i += kCvThreads) wsm[i] = __ldg(a.conv_w_packed + woff + i);
         __syncthreads();
         float* z = zs + (size_t)l * C * NS;
         const float* bl = a.conv_b + l * C;
-        conv_planes(in, cin, C, wsm, nullptr, Lx, Ly,
+        conv_planes(in, cin, C, wsm, Lx, Ly,
                     [&](int co, int s, float v) { z[co * NS + s] = v + __ldg(bl + co); });
         __syncthreads();
-        for (int e = tid; e < C * N; e += kNumThreads) {
+        for (int e = tid; e < C * N; e += kCvThreads) {
           const int co = e / N, s = e - co * N;
           bufA[co * NS + s] = gelu_tanh_dev(z[co * NS + s]);
         }
@@ -622,11 +613,11 @@ __global__ void __launch_bounds__(kNumThreads) cnn_vjp_kernel(CnnVjpArgs a) {
       __syncthreads();
       float* dcur = bufB;
       float* dother = bufA;
-      for (int e = tid; e < C * NS; e += kNumThreads) dcur[e] = 0.0f;
+      for (int e = tid; e < C * NS; e += kCvThreads) dcur[e] = 0.0f;
       __syncthreads();
       const float* dYi = a.dY + item * a.n * d;
       const int32_t* ii = a.idx + item * a.n;
-      for (int e = tid; e < a.n * d; e += kNumThreads) {
+      for (int e = tid; e < a.n * d; e += kCvThreads) {
         const int p = e / d, aa = e - p * d;
         const int m = __ldg(ii + p);
         const int sg = m >= N ? 1 : 0;
@@ -645,53 +636,85 @@ __global__ void __launch_bounds__(kNumThreads) cnn_vjp_kernel(CnnVjpArgs a) {
         const float* ain = img;
         if (l > 0) {
           const float* z = zs + (size_t)(l - 1) * C * NS;
-          for (int e = tid; e < C * N; e += kNumThreads) {
+          for (int e = tid; e < C * N; e += kCvThreads) {
             const int ci = e / N, s = e - ci * N;
             dother[ci * NS + s] = gelu_tanh_dev(z[ci * NS + s]);
           }
           ain = dother;
         }
         __syncthreads();
-        // Weight cotangent: thread owns (4 output channels, 1 input channel) x 9 taps.
+        // Weight cotangent: a task owns (4 output channels, 1 input channel) x 9 taps over a share of
+        // the lattice's rows; with fewer tasks than threads (all but very wide layers) the rows
+        // are split, and the shares are summed in shared memory (the weights' place, not in use).
         const int pairs = (C / 4) * lcin;
-        for (int pr = tid; pr < pairs; pr += kNumThreads) {
+        int split = 1;
+        while (2 * split * pairs <= kCvThreads && 2 * split <= Lx && (2 * split - 1) * pairs * 36 <= C * C * 9)
+          split *= 2;
+        for (int t0 = 0; t0 < pairs * split; t0 += kCvThreads) {
+          const int task = t0 + tid, pr = task % pairs, share = task / pairs;
+          const bool on = task < pairs * split;
           const int ci = pr % lcin, cob = pr / lcin;
           float acc[4][9];
 #pragma unroll
           for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int t = 0; t < 9; ++t) acc[j][t] = 0.0f;
-          const float* ap = ain + ci * NS;
-          const float* dp = dcur + (size_t)(cob * 4) * NS;
-          for (int x = 0; x < Lx; ++x) {
-            const int xm = (x == 0 ? Lx - 1 : x - 1) * Ly, x0 = x * Ly,
-                      xp = (x == Lx - 1 ? 0 : x + 1) * Ly;
-            for (int y = 0; y < Ly; ++y) {
-              const int ym = y == 0 ? Ly - 1 : y - 1, yp = y == Ly - 1 ? 0 : y + 1;
-              const float av[9] = {ap[xm + ym], ap[xm + y], ap[xm + yp],
-                                   ap[x0 + ym], ap[x0 + y], ap[x0 + yp],
-                                   ap[xp + ym], ap[xp + y], ap[xp + yp]};
-              const int s = x0 + y;
+          if (on) {
+            const float* ap = ain + ci * NS;
+            const float* dp = dcur + (size_t)(cob * 4) * NS;
+            for (int x = share; x < Lx; x += split) {
+              const float* r0 = ap + (x == 0 ? Lx - 1 : x - 1) * Ly;
+              const float* r1 = ap + x * Ly;
+              const float* r2 = ap + (x == Lx - 1 ? 0 : x + 1) * Ly;
+              // the window's columns y - 1, y, y + 1 slide along the row
+              float w0[3] = {r0[Ly - 1], r1[Ly - 1], r2[Ly - 1]}, w1[3] = {r0[0], r1[0], r2[0]};
+              for (int y = 0; y < Ly; ++y) {
+                const int yp = y == Ly - 1 ? 0 : y + 1, s = x * Ly + y;
+                const float w2[3] = {r0[yp], r1[yp], r2[yp]};
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const float dv = dp[j * NS + s];
+                for (int j = 0; j < 4; ++j) {
+                  const float dv = dp[j * NS + s];
 #pragma unroll
-                for (int t = 0; t < 9; ++t) acc[j][t] = fmaf(dv, av[t], acc[j][t]);
+                  for (int u = 0; u < 3; ++u) {
+                    acc[j][3 * u] = fmaf(dv, w0[u], acc[j][3 * u]);
+                    acc[j][3 * u + 1] = fmaf(dv, w1[u], acc[j][3 * u + 1]);
+                    acc[j][3 * u + 2] = fmaf(dv, w2[u], acc[j][3 * u + 2]);
+                  }
+                }
+#pragma unroll
+                for (int u = 0; u < 3; ++u) {
+                  w0[u] = w1[u];
+                  w1[u] = w2[u];
+                }
               }
             }
           }
+          if (split > 1) {
+            if (on && share > 0) {
+              float* part = wsm + (size_t)(share - 1) * pairs * 36 + pr;  // [36][pairs]
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int co = cob * 4 + j;
-            float* dst = row + col + ((int64_t)co * lcin + ci) * 9;
+              for (int q = 0; q < 36; ++q) part[q * pairs] = acc[q / 9][q % 9];
+            }
+            __syncthreads();
+          }
+          if (on && share == 0) {
+            for (int sh = 1; sh < split; ++sh) {
+              const float* part = wsm + (size_t)(sh - 1) * pairs * 36 + pr;
 #pragma unroll
-            for (int t = 0; t < 9; ++t) dst[t] = g == 0 ? acc[j][t] : dst[t] + acc[j][t];
+              for (int q = 0; q < 36; ++q) acc[q / 9][q % 9] += part[q * pairs];
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float* dst = row + col + ((int64_t)(cob * 4 + j) * lcin + ci) * 9;
+#pragma unroll
+              for (int t = 0; t < 9; ++t) dst[t] = g == 0 ? acc[j][t] : dst[t] + acc[j][t];
+            }
           }
         }
         // Bias cotangent: warp per output channel.
         {
           const int lane = tid & 31, warp = tid >> 5;
-          for (int co = warp; co < C; co += kNumThreads / 32) {
+          for (int co = warp; co < C; co += kCvThreads / 32) {
             float s = 0.0f;
             for (int e = lane; e < N; e += 32) s += dcur[co * NS + e];
 #pragma unroll
@@ -705,7 +728,7 @@ __global__ void __launch_bounds__(kNumThreads) cnn_vjp_kernel(CnnVjpArgs a) {
         if (l == 0) break;
         // Input cotangent: transposed convolution with flipped taps, times GELU'(z_{l-1}).
         __syncthreads();
-        for (int i = tid; i < C * C * 9; i += kNumThreads) {
+        for (int i = tid; i < C * C * 9; i += kCvThreads) {
           const int cj = i % C;        // output channel of the transposed conv = layer input ci
           const int rest = i / C;      // co * 9 + tap'
           const int co = rest / 9, tp = rest - co * 9;
@@ -713,7 +736,7 @@ __global__ void __launch_bounds__(kNumThreads) cnn_vjp_kernel(CnnVjpArgs a) {
         }
         __syncthreads();
         const float* z = zs + (size_t)(l - 1) * C * NS;
-        conv_planes(dcur, C, C, wsm, nullptr, Lx, Ly, [&](int ci, int s, float v) {
+        conv_planes(dcur, C, C, wsm, Lx, Ly, [&](int ci, int s, float v) {
           dother[ci * NS + s] = v * gelu_tanh_grad_dev(z[ci * NS + s]);
         });
         float* t = dcur;
@@ -751,11 +774,11 @@ int launch_pf_adjoint(const float* F, float* G, int n, int batch, const float* p
 }
 
 int launch_pairing_vjp(const float* G, const float* Y, const int32_t* idx, const float* Wt,
-                       int Lx, int Ly, int d, int n, int n_img, int samples, float* dY,
+                       const float* wt_chunks, int Lx, int Ly, int d, int n, int n_img, int samples, float* dY,
                        float* dWt, float* jac, int64_t ld, int64_t off_w, float theta,
                        cudaStream_t st) {
   if (samples <= 0) return NH_OK;
-  VjpArgs a{G, Y, idx, Wt, Lx, Ly, n, n_img, samples, dY, dWt, jac, ld, off_w, theta,
+  VjpArgs a{G, Y, idx, Wt, reinterpret_cast<const float4*>(wt_chunks), Lx, Ly, n, n_img, samples, dY, dWt, jac, ld, off_w, theta,
             jac ? 1 : 0};
   switch (d) {
     case 8: return launch_vjp_t<8>(a, st);
@@ -787,7 +810,7 @@ int launch_cnn_vjp(const int8_t* spins, int samples, int n_img, const nh_backflo
   CnnVjpArgs a{spins, samples, n_img, p.conv_w, p.conv_w_packed, p.conv_b, p.Lx, p.Ly, C,
                p.layers, p.n_up + p.n_dn, dY, idx, jac, ld};
   ProfScope prof_scope(NH_K_CNN_VJP, st);
-  cnn_vjp_kernel<<<grid, kNumThreads, smem, st>>>(a);
+  cnn_vjp_kernel<<<grid, kCvThreads, smem, st>>>(a);
   return check_launch("cnn_vjp_kernel");
 }
 
