@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(kCvThreads) cnn_vjp_kernel(CnnVjpArgs a) {
       size_t woff = 0;
       for (int l = 0; l < L - 1; ++l) {
         __syncthreads();
-        for (int i = tid; i < C * cin * 9; i += kCvThreads) wsm[i] = __ldg(a.conv_w_packed + woff + i);
+        stage_floats<kCvThreads>(wsm, a.conv_w_packed + woff, C * cin * 9);
         __syncthreads();
         float* z = zs + (size_t)l * C * NS;
         const float* bl = a.conv_b + l * C;
