@@ -45,6 +45,12 @@ __device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
   return r;
 }
+__device__ __forceinline__ float lo2(unsigned long long v) {
+  return __uint_as_float((unsigned)v);
+}
+__device__ __forceinline__ float hi2(unsigned long long v) {
+  return __uint_as_float((unsigned)(v >> 32));
+}
 __device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long a,
                                      unsigned long long b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));

@@ -4,9 +4,9 @@
 //
 // * adjoint_kernel: the cotangent of fermix.slogpf (code/backflow/models.py:210),
 //   G = d log|pf F| / dF = 1/2 F^{-T}, from an in-register Gauss-Jordan inverse of F with implicit
-//   row pivoting (one matrix per 512-thread CTA; thread (warp w, lane c) holds rows w + 16 t and
-//   columns c + 32 u; one barrier per pivot step, the pivot row read from the winning warp's
-//   candidate row in shared memory, as in nh_det.cu).  A per-item scale multiplies G (the image weight of the projection).
+//   row pivoting, eight pivot steps at a time (one matrix per 512-thread CTA; thread (warp w,
+//   lane c) holds rows w + 16 t and columns c + 32 u).  A per-item scale multiplies G (the image
+//   weight of the projection).
 // * pairing_vjp_kernel: the custom VJP of the occupied gather (pf_kernel.py:193-320,354-365):
 //   dY[p, a] = sum_q (G - G^T)[p, q] Wt[blk(p, q), r(p, q), a] Y[q, a] and
 //   dWt[blk, r, a] = sum over the pairs (p, q) with that block and displacement of
@@ -19,6 +19,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "nh_cnn_item.cuh"
 #include "nh_common.cuh"
@@ -28,11 +29,6 @@ namespace {
 
 constexpr int kAdjThreads = 512;  // 16 row groups (warps) x 32 column groups (lanes)
 constexpr int kVjpThreads = 512;
-
-__device__ __forceinline__ unsigned long long pivot_key(float mag, int row) {
-  // |v| >= 0 orders like its bit pattern; ties go to the smaller row.
-  return ((unsigned long long)__float_as_uint(mag) << 32) | (unsigned)(0x7FFFFFFF - row);
-}
 
 // Weight of item (c, g) in d log|psi_P(c)|: sg_g exp(la_g) / sum_h sg_h exp(la_h) (sg, la: the
 // item's signed log-Pfaffian with its fermionic signs folded in); 0 when the sum vanishes.
@@ -60,144 +56,267 @@ struct AdjArgs {
   int32_t* flags;           // (batch,) or null: NH_FLAG_ZERO_PIVOT / NH_FLAG_NONFINITE
 };
 
-// Floats of the region shared by the output tile and the per-warp candidate rows.
-__host__ __device__ constexpr size_t adjoint_region(int n, int np) {
-  return (size_t)n * (n + 1) > (size_t)32 * np ? (size_t)n * (n + 1) : (size_t)32 * np;
-}
+// Blocks of kAdjBlock pivot steps.  The buffers of a block and the output tile share one region.
+constexpr int kAdjBlock = 8;
 
 template <int TC>
-__global__ void __launch_bounds__(kAdjThreads, 1) adjoint_kernel(AdjArgs a) {
-  constexpr int TR = 2 * TC, NP = 32 * TC;
+struct AdjLayout {  // float offsets
+  static constexpr int TR = 2 * TC, NP = 32 * TC, kFs = ((TR + 3) & ~3) + 4;
+  static constexpr int panel = 0, kPs = NP + 4;              // [8][kPs]: the block's columns
+  static constexpr int rows = panel + kAdjBlock * kPs;       // [8][NP]: its pivot rows
+  static constexpr int scaled = rows + kAdjBlock * NP;       // [8][NP]: row k at step k, / pivot
+  static constexpr int mult = scaled + kAdjBlock * NP;       // [8][16][kFs]: -A[i][k] at step k
+  static constexpr int cand = mult + kAdjBlock * 16 * kFs;   // [2][TC][8]: candidates' columns
+  static constexpr int cross = cand + 2 * TC * kAdjBlock;    // [8][8]: mult of the pivot rows
+  static constexpr int mags = cross + kAdjBlock * kAdjBlock;  // [2][8]: their pivots' magnitudes
+  static constexpr int total = mags + 16;
+  __host__ __device__ static constexpr size_t region(int n) {
+    return (size_t)n * (n + 1) > (size_t)total ? (((size_t)n * (n + 1) + 3) & ~(size_t)3) : total;
+  }
+};
+
+// f(t) for a t in [LO, HI) that is the same in all lanes, as a constant: branches by halves, so that
+// an array indexed with it stays in registers.
+template <int LO, int HI, typename Fn>
+__device__ __forceinline__ void with_row(int t, Fn&& f) {
+  if constexpr (HI - LO == 1) {
+    f(std::integral_constant<int, LO>{});
+  } else {
+    constexpr int MID = (LO + HI) / 2;
+    if (t < MID)
+      with_row<LO, MID>(t, f);
+    else
+      with_row<MID, HI>(t, f);
+  }
+}
+
+// Gauss-Jordan inverse in the registers of 512 threads, eight pivot steps at a time.  A step by
+// itself is a chain (maximum of a column, pivot row, reciprocal, multipliers) ending in a barrier of
+// all warps: 2260 cycles at n = 224, where its 98 products per thread take 390.  Here the chain runs
+// on the block's eight columns alone, a row per thread on TC warps; then each thread of those warps
+// takes one column of the eight pivot rows through the same steps, and all 512 threads apply the
+// eight steps to their elements back to back, two rows per packed instruction.  Every element sees
+// the operations of the step-by-step elimination in their order, so the result is bit for bit
+// the same.  2048 matrices of n = 224: 2.88 ms (3.73 step by step).  A block of eight steps takes 15K
+// cycles there: the chain 5.8K (two warp maxima and a barrier, 720 a step), the products 4.4K of
+// 3.1K at the FMA rate, the rest moves columns and pivot rows between registers and shared memory.
+template <int TC>
+__global__ void __launch_bounds__(kAdjThreads, TC <= 4 ? 2 : 1) adjoint_kernel(AdjArgs a) {
+  using L = AdjLayout<TC>;
+  constexpr int TR = L::TR, NP = L::NP, KB = kAdjBlock;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int n = a.n, NS = n + 1;
-  // tile (n, n + 1): G before the coalesced copy.  During the elimination the same region holds
-  // cand [2][16][NP]: each warp's best remaining row of the step, so that the winner's row is
-  // in shared memory by the step's one barrier.
-  float* tile = reinterpret_cast<float*>(smem_raw);
-  float* cand = tile;
-  float* colbuf = tile + adjoint_region(n, NP);        // [2][NP]
-  int* rho = reinterpret_cast<int*>(colbuf + 2 * NP);  // [NP] pivot row of step k
-  int* rhoinv = rho + NP;                              // [NP]
-  unsigned long long* keys = reinterpret_cast<unsigned long long*>(rhoinv + NP);  // [2][16]
-  float* scale_s = reinterpret_cast<float*>(keys + 32);
+  float* tile = reinterpret_cast<float*>(smem_raw);  // (n, n + 1): G before the coalesced copy
+  float* panel = tile + L::panel;
+  float* prows = tile + L::rows;
+  float* scaled = tile + L::scaled;
+  float* mult = tile + L::mult;
+  float* cand = tile + L::cand;
+  float* cross = tile + L::cross;
+  unsigned* mags = reinterpret_cast<unsigned*>(tile + L::mags);
+  int* rho = reinterpret_cast<int*>(tile + L::region(n));  // [NP] pivot row of step k
+  int* rhoinv = rho + NP;                                  // [NP]
+  float* inv_s = reinterpret_cast<float*>(rhoinv + NP);    // [8] 1 / pivot
+  float* scale_s = inv_s + KB;
   int* bad_s = reinterpret_cast<int*>(scale_s + 1);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int* kb_s = bad_s + 1;  // steps of the block before a bad pivot
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   for (int item = blockIdx.x; item < a.batch; item += gridDim.x) {
     const float* F = a.F + (size_t)item * n * n;
-    float A[TR][TC];
+    // A[t][u]: rows warp + 32 t and warp + 32 t + 16, column lane + 32 u
+    unsigned long long A[TC][TC];
 #pragma unroll
-    for (int t = 0; t < TR; ++t) {
-      const int i = warp + 16 * t;
+    for (int t = 0; t < TC; ++t) {
+      const int i0 = warp + 32 * t, i1 = i0 + 16;
 #pragma unroll
       for (int u = 0; u < TC; ++u) {
         const int j = lane + 32 * u;
-        A[t][u] = (i < n && j < n) ? __ldg(F + (size_t)i * n + j) : (i == j ? 1.0f : 0.0f);
+        const float lo = (i0 < n && j < n) ? __ldg(F + (size_t)i0 * n + j) : (i0 == j ? 1.0f : 0.0f);
+        const float hi = (i1 < n && j < n) ? __ldg(F + (size_t)i1 * n + j) : (i1 == j ? 1.0f : 0.0f);
+        A[t][u] = pack2(lo, hi);
       }
     }
-    unsigned used = 0;  // bit t: row warp + 16 t is a pivot row already (or padding)
-#pragma unroll
-    for (int t = 0; t < TR; ++t)
-      if (warp + 16 * t >= n) used |= 1u << t;
-    if (threadIdx.x == 0) {
-      *bad_s = 0;
+    bool used = tid >= n;  // row tid is a pivot row already (or padding)
+    if (tid == 0) {
       float sc = 0.5f;
       if (a.pf_sign) sc = (float)(0.5 * image_weight(a.pf_sign, a.pf_logabs, item, a.n_img));
       *scale_s = sc;
     }
-    __syncthreads();
     int bad = 0;
-    // One barrier per step: the column, key and candidate buffers alternate by parity (a warp
-    // writes step k + 2's copy only after every warp has passed step k + 1's barrier, so after
-    // every read of step k's).  Each warp leaves its best key in a place of its own and reduces all
-    // 16 after the barrier (a 64-bit shared-memory maximum serialised the warps before it).
-#pragma unroll
-    for (int uk = 0; uk < TC; ++uk) {
 #pragma unroll 1
-      for (int lk = 0; lk < 32; ++lk) {
-        const int k = uk * 32 + lk;
-        if (k >= n || bad) break;  // uniform
-        const int par = k & 1;
-        {
-          // Column k of this warp's rows, spread over the lanes (lane t takes row warp + 16 t)
-          // so that the pivot proposal runs on TR lanes instead of the one owning the column.
-          float cv = float(0);
+    for (int K = 0; K < n; K += KB) {
+      const int uk = K >> 5, lk = K & 31;  // the block's columns: lanes lk .. lk + 7, index uk
+      // The block's columns to shared memory.  A warp writes and, at the block's end, reads only
+      // its own rows of it.
+      if (lane >= lk && lane < lk + KB) {
+        float* pc = panel + (lane - lk) * L::kPs + warp;
 #pragma unroll
-          for (int t = 0; t < TR; ++t) {
-            const float v = __shfl_sync(0xffffffffu, A[t][uk], lk);
-            if (lane == t) cv = v;
-          }
-          unsigned long long key = 0ull;
-          if (lane < TR) {
-            colbuf[par * NP + warp + 16 * lane] = cv;
-            if (!((used >> lane) & 1u)) key = pivot_key(fabsf(cv), warp + 16 * lane);
-          }
-          // 64-bit warp maximum as two 32-bit reductions: the magnitude bits, then the row
-          // tie-break among the lanes holding that magnitude.
-          const unsigned hi = (unsigned)(key >> 32);
-          const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-          const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)key : 0u);
-          key = ((unsigned long long)mh << 32) | ml;
-          if (key) {  // this warp's best row goes to its candidate slot
-            const int tl = (0x7FFFFFFF - (int)ml) >> 4;
-            float* cw = cand + (size_t)(par * 16 + warp) * NP;
+        for (int u = 0; u < TC; ++u)
+          if (u == uk) {
 #pragma unroll
-            for (int t = 0; t < TR; ++t)
-              if (t == tl) {
-#pragma unroll
-                for (int u = 0; u < TC; ++u) cw[lane + 32 * u] = A[t][u];
-              }
-          }
-          if (lane == 0) keys[16 * par + warp] = key;
-        }
-        __syncthreads();
-        const unsigned long long kw = keys[16 * par + (lane & 15)];
-        const unsigned wh = __reduce_max_sync(0xffffffffu, (unsigned)(kw >> 32));
-        const unsigned wl =
-            __reduce_max_sync(0xffffffffu, (unsigned)(kw >> 32) == wh ? (unsigned)kw : 0u);
-        const int p = 0x7FFFFFFF - (int)wl;
-        const float mag = __uint_as_float(wh);
-        if ((wh | wl) == 0u || !(mag > 0.0f && mag <= 3.0e38f)) {  // zero column, or non-finite
-          bad = ((wh | wl) == 0u || mag == 0.0f) ? NH_FLAG_ZERO_PIVOT : NH_FLAG_NONFINITE;
-          break;
-        }
-        if (threadIdx.x == 0) rho[k] = p;
-        const float* prow = cand + (size_t)(par * 16 + (p & 15)) * NP;
-        const float inv = 1.0f / prow[k];
-        float r[TC];
-#pragma unroll
-        for (int u = 0; u < TC; ++u) r[u] = prow[lane + 32 * u] * inv;
-#pragma unroll
-        for (int t = 0; t < TR; ++t) {
-          const float f = colbuf[par * NP + warp + 16 * t];
-#pragma unroll
-          for (int u = 0; u < TC; ++u) A[t][u] = fmaf(-f, r[u], A[t][u]);
-        }
-        if (lane == lk) {
-#pragma unroll
-          for (int t = 0; t < TR; ++t) A[t][uk] = -colbuf[par * NP + warp + 16 * t] * inv;
-        }
-        if (warp == (p & 15)) {
-          const int tp = p >> 4;
-          used |= 1u << tp;
-#pragma unroll
-          for (int t = 0; t < TR; ++t)
-            if (t == tp) {
-#pragma unroll
-              for (int u = 0; u < TC; ++u) A[t][u] = r[u];
-              if (lane == lk) A[t][uk] = inv;
+            for (int t = 0; t < TC; ++t) {
+              pc[32 * t] = lo2(A[t][u]);
+              pc[32 * t + 16] = hi2(A[t][u]);
             }
+          }
+      }
+      __syncthreads();
+      // The chain: thread i < NP holds row i of the columns.
+      if (warp < TC) {
+        float v[KB];
+#pragma unroll
+        for (int c = 0; c < KB; ++c) v[c] = panel[c * L::kPs + tid];
+        const int kb = min(KB, n - K);
+        float* mrow = mult + (tid & 15) * L::kFs + (tid >> 4);
+        // One body for all steps (eight copies of it run at the speed of the instruction fetch):
+        // v[0] is the step's column, and each step moves the columns down by one.
+        int done = 0;
+#pragma unroll 1
+        for (; done < kb; ++done) {
+          const int par = done & 1;
+          const float cv = v[0];
+          const float own_inv = 1.0f / cv;  // every row's, beside the search
+          // The warp's largest free row, the first of equals, goes to its candidate slot (|v| >= 0
+          // orders like its bit pattern; a warp without a free row proposes 0, as a zero column).
+          const unsigned mag = used ? 0u : __float_as_uint(fabsf(cv));
+          const unsigned wmag = __reduce_max_sync(0xffffffffu, mag);
+          const int wlane = __ffs(__ballot_sync(0xffffffffu, mag == wmag)) - 1;
+          if (lane == wlane) {
+            float4* cw = reinterpret_cast<float4*>(cand + (par * TC + warp) * KB);
+            cw[0] = make_float4(own_inv, v[1] * own_inv, v[2] * own_inv, v[3] * own_inv);
+            cw[1] = make_float4(v[4] * own_inv, v[5] * own_inv, v[6] * own_inv, v[7] * own_inv);
+            mags[par * 8 + warp] = wmag;
+          }
+          mrow[done * 16 * L::kFs] = -cv;
+          if (TC == 1)
+            __syncwarp();
+          else
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * TC) : "memory");
+          const unsigned m = lane < TC ? mags[par * 8 + lane] : 0u;
+          const unsigned best = __reduce_max_sync(0xffffffffu, m);
+          const int wwarp = __ffs(__ballot_sync(0xffffffffu, m == best)) - 1;
+          if (best == 0u || !(__uint_as_float(best) <= 3.0e38f)) {  // zero column, or non-finite
+            bad = best == 0u ? NH_FLAG_ZERO_PIVOT : NH_FLAG_NONFINITE;
+            break;  // uniform over the TC warps
+          }
+          const bool pivot = warp == wwarp && lane == wlane;
+          const float4* cr = reinterpret_cast<const float4*>(cand + (par * TC + wwarp) * KB);
+          const float4 ra = cr[0], rb = cr[1];
+          const float r[KB] = {ra.x, ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, rb.w};
+          if (pivot) {
+            used = true;
+            rho[K + done] = tid;
+            inv_s[done] = own_inv;
+          }
+#pragma unroll
+          for (int c = 1; c < KB; ++c) v[c - 1] = pivot ? r[c] : fmaf(-cv, r[c], v[c]);
+          v[KB - 1] = pivot ? r[0] : -cv * r[0];
+        }
+#pragma unroll
+        for (int c = 0; c < KB; ++c) panel[((c + done) & (KB - 1)) * L::kPs + tid] = v[c];
+        if (tid == 0) {
+          *kb_s = done;
+          *bad_s = bad;
         }
       }
+      __syncthreads();
+      const int kb = *kb_s;
+      bad = *bad_s;
+      // The pivot rows to shared memory, and their multipliers of the block's steps side by side.
+      const int pl = lane < kb ? rho[K + lane] : 0;  // lane m: pivot row m
+      const unsigned mine = __ballot_sync(0xffffffffu, lane < kb && (pl & 15) == warp);
+      for (unsigned left = mine; left; left &= left - 1) {
+        const int m = __ffs(left) - 1, t = __shfl_sync(0xffffffffu, pl, m) >> 4;
+        float* pr = prows + m * NP + lane;
+        with_row<0, TR>(t, [&](auto tc) {
+          constexpr int tt = decltype(tc)::value;
+#pragma unroll
+          for (int u = 0; u < TC; ++u) pr[32 * u] = tt & 1 ? hi2(A[tt / 2][u]) : lo2(A[tt / 2][u]);
+        });
+      }
+      if (tid < KB * KB) {
+        const int k = tid >> 3, m = (k + tid) & 7;  // in the order of the loop below
+        if (k < kb && m < kb) {
+          const int p = rho[K + m];
+          cross[tid] = mult[(k * 16 + (p & 15)) * L::kFs + (p >> 4)];
+        }
+      }
+      __syncthreads();
+      if (warp < TC) {  // column tid of the pivot rows through the block's steps
+        float x[KB];
+#pragma unroll
+        for (int m = 0; m < KB; ++m) x[m] = prows[m * NP + tid];
+#pragma unroll 1
+        for (int k = 0; k < kb; ++k) {  // x[0] is row k; each step moves the rows down by one
+          const float r = x[0] * inv_s[k];
+          const float4* cm = reinterpret_cast<const float4*>(cross + k * KB);
+          const float4 ca = cm[0], cb = cm[1];
+          const float f[KB] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
+          scaled[k * NP + tid] = r;
+#pragma unroll
+          for (int m = 1; m < KB; ++m) x[m - 1] = fmaf(f[m], r, x[m]);
+          x[KB - 1] = r;
+        }
+#pragma unroll
+        for (int m = 0; m < KB; ++m) prows[((m + kb) & (KB - 1)) * NP + tid] = x[m];
+      }
+      __syncthreads();
+      // Every element through the block's steps (the pivot rows and the block's columns too; they
+      // are replaced below).
+#pragma unroll 1
+      for (int k = 0; k < kb; ++k) {
+        const float* mk = mult + (k * 16 + warp) * L::kFs;
+        const float* sk = scaled + k * NP + lane;
+        unsigned long long r[TC];
+#pragma unroll
+        for (int u = 0; u < TC; ++u) r[u] = pack2(sk[32 * u], sk[32 * u]);
+#pragma unroll
+        for (int t = 0; t < TC; t += 2) {
+          unsigned long long f0, f1 = 0;
+          if (t + 1 < TC) {
+            const ulonglong2 f = *reinterpret_cast<const ulonglong2*>(mk + 2 * t);
+            f0 = f.x, f1 = f.y;
+          } else {
+            f0 = *reinterpret_cast<const unsigned long long*>(mk + 2 * t);
+          }
+#pragma unroll
+          for (int u = 0; u < TC; ++u) fma2(A[t][u], f0, r[u]);
+          if (t + 1 < TC) {
+#pragma unroll
+            for (int u = 0; u < TC; ++u) fma2(A[t + 1][u], f1, r[u]);
+          }
+        }
+      }
+      for (unsigned left = mine; left; left &= left - 1) {
+        const int m = __ffs(left) - 1, t = __shfl_sync(0xffffffffu, pl, m) >> 4;
+        const float* pr = prows + m * NP + lane;
+        with_row<0, TR>(t, [&](auto tc) {
+          constexpr int tt = decltype(tc)::value;
+#pragma unroll
+          for (int u = 0; u < TC; ++u) {
+            const float y = pr[32 * u];
+            A[tt / 2][u] = tt & 1 ? pack2(lo2(A[tt / 2][u]), y) : pack2(y, hi2(A[tt / 2][u]));
+          }
+        });
+      }
+      if (lane >= lk && lane < lk + KB) {
+        const float* pc = panel + (lane - lk) * L::kPs + warp;
+#pragma unroll
+        for (int u = 0; u < TC; ++u)
+          if (u == uk) {
+#pragma unroll
+            for (int t = 0; t < TC; ++t) A[t][u] = pack2(pc[32 * t], pc[32 * t + 16]);
+          }
+      }
+      if (bad) break;  // uniform
+      __syncwarp();    // the next block's columns go where other lanes have read
     }
     // The storage holds X = (P F)^{-1} with logical row k in physical row rho[k], so
     // F^{-1}[i][j] = A[rho[i]][rhoinv[j]] and G[p][q] = 1/2 F^{-1}[q][p]: element (I, J) of the
     // storage goes to G[rho[J]][rhoinv[I]].
-    if (threadIdx.x == 0 && bad) *bad_s = bad;
-    __syncthreads();
-    bad = *bad_s;
     if (!bad)
-      for (int k = threadIdx.x; k < n; k += kAdjThreads) rhoinv[rho[k]] = k;
+      for (int k = tid; k < n; k += kAdjThreads) rhoinv[rho[k]] = k;
     __syncthreads();
     const float sc = bad ? 0.0f : *scale_s;
 #pragma unroll
@@ -208,26 +327,25 @@ __global__ void __launch_bounds__(kAdjThreads, 1) adjoint_kernel(AdjArgs a) {
         const int J = lane + 32 * u;
         if (I < n && J < n) {
           const int dr = bad ? J : rho[J], dc = bad ? I : rhoinv[I];
-          tile[dr * NS + dc] = sc * A[t][u];
+          tile[dr * NS + dc] = sc * (t & 1 ? hi2(A[t / 2][u]) : lo2(A[t / 2][u]));
         }
       }
     }
     __syncthreads();
     float* Gi = a.G + (size_t)item * n * n;
-    for (int e = threadIdx.x; e < n * n; e += kAdjThreads) {
+    for (int e = tid; e < n * n; e += kAdjThreads) {
       const int row = e / n;
       Gi[e] = tile[row * NS + (e - row * n)];
     }
-    if (a.flags && threadIdx.x == 0) a.flags[item] = bad;
+    if (a.flags && tid == 0) a.flags[item] = bad;
     __syncthreads();
   }
 }
 
 template <int TC>
 size_t adjoint_smem(int n) {
-  constexpr int NP = 32 * TC;
-  return sizeof(float) * (adjoint_region(n, NP) + 2 * NP) + sizeof(int) * 2 * NP +
-         sizeof(unsigned long long) * 32 + 16;
+  return sizeof(float) * (AdjLayout<TC>::region(n) + kAdjBlock + 4) +
+         sizeof(int) * 2 * AdjLayout<TC>::NP;
 }
 
 template <int TC>
