@@ -7,8 +7,9 @@
 // (one per group of 16 input channels, 512 columns), added in the epilogue, which keeps the
 // tensor cores' FP32 accumulation chains short (one chain of 216 MMAs left a nearly constant
 // offset of ~8e-4 in log|psi|; four chains, under 2e-4).  Operands are split into BF16 hi + lo
-// and accumulated as hi*hi + hi*lo + lo*hi (about 16 significant bits per product).  One configuration image per CTA at a time (grid-stride), 256 threads: warp w
-// owns tensor-memory lanes 32 (w % 4) .. + 31 of tile w / 4, i.e. one site per thread.
+// and accumulated as hi*hi + hi*lo + lo*hi (about 16 significant bits per product).  One
+// configuration image per CTA at a time (grid-stride), 512 threads: warp w owns tensor-memory lanes
+// 32 (w % 4) .. + 31 of tile (w / 4) % 2, channels 32 (w / 8) .. + 31, i.e. two threads per site.
 //
 // Shared memory (214 KB):
 //   planes  the A operand: 8 + 8 BF16 hi / lo padded planes (nh_tcgen05.cuh layout), holding
@@ -18,10 +19,17 @@
 //   ring    4 slots of one tap's weights (hi + lo, 16 KB, [q][kc][cg][8 co][8 ci] BF16), filled
 //           by bulk copies (no multicast) that complete on full[slot]; the MMAs that read a slot
 //           commit to empty[slot], and the copy of the slice four taps ahead waits for it.
-// Thread 0 issues the MMAs (all 216 of a convolution unrolled, operand descriptors formed once
-// and advanced by constants); thread 32 issues the copies, so that neither waits on the other's
-// instructions.  The weight stream runs ahead across convolutions: the next convolution's first
-// four slices load while the epilogue of the current one runs.
+// One elected lane of warp 0 issues the MMAs (all 216 of a convolution unrolled, operand
+// descriptors formed once and advanced by constants; under a test of the thread index instead of
+// elect.sync each MMA took 58 cycles to issue, now 40); thread 32 issues the copies, so that neither
+// waits on the other's instructions.  The weight stream runs ahead across convolutions: the next
+// convolution's first four slices load while the epilogue of the current one runs.
+//
+// What bounds it: an MMA takes as long as its operands take to leave shared memory (48.7 cycles by
+// itself), 10.5K cycles a convolution, and the epilogue's GELU and split 8K more, one after the
+// other since the planes are both's.  While all threads polled the accumulators' mbarrier the MMAs
+// took about 90 cycles; one thread polls now and the others wait at a barrier.  2048 images of 32
+// convolutions: 8.6 ms at first, 7.6 with the elected lane, 5.7 with the single poller.
 // Epilogues read the accumulators with tcgen05.ld and (a) write u's planes, or (b) add the
 // convolution into x, reduce sum x^2 over the CTA, and write the next h's planes.
 //
@@ -38,7 +46,7 @@ namespace {
 
 using namespace tc;
 
-constexpr int kRtThreads = 256;
+constexpr int kRtThreads = 512;  // two threads per site, 32 channels each
 constexpr int kRtC = 64;
 constexpr int kRtN = kL * kL;                          // 256 sites
 constexpr int kRtPlanes = kRtC / 8;                    // planes per hi / lo
@@ -48,6 +56,7 @@ constexpr int kRtHalfTap = kRtPlanes * 8 * 128;        // 8,192: one of hi / lo 
 constexpr int kRtTapBytes = 2 * kRtHalfTap;            // 16,384
 constexpr int kRtConvBytes = 9 * kRtTapBytes;          // 147,456
 constexpr int kRtSlots = 4;
+constexpr int kRtHalf = kRtC / 2;                      // channels per thread
 constexpr int kRtInts = 2 * kRtN + 2 * kRtN + 4 * kL + 32;  // simg, occl, scan scratch
 constexpr uint32_t kRtIdesc = idesc_bf16(128, 64);
 constexpr int kRtParts = 4;           // partial accumulators per tile (one per 16-ci group)
@@ -105,13 +114,16 @@ __device__ __forceinline__ void issue_tap(uint32_t tmem, uint64_t dAhi, uint64_t
   }
 }
 
-// Write the 64 channels f of this thread's site (lattice x, y) as BF16 hi / lo planes.
-__device__ __forceinline__ void put_channels(unsigned char* planes, int x, int y, const float* f) {
-  uint4 hi[kRtPlanes], lo[kRtPlanes];
+// Write the 32 channels f, from group kc0 of 8 on, of this thread's site (lattice x, y) as BF16 hi /
+// lo planes.
+__device__ __forceinline__ void put_channels(unsigned char* planes, int kc0, int x, int y,
+                                             const float* f) {
+  constexpr int K = kRtHalf / 8;
+  uint4 hi[K], lo[K];
 #pragma unroll
-  for (int kc = 0; kc < kRtPlanes; ++kc) split8(f + 8 * kc, hi + kc, lo + kc);
-  put_site(planes, kRtPlanes, x, y, hi);
-  put_site(planes + kRtPlanes * kPlane, kRtPlanes, x, y, lo);
+  for (int kc = 0; kc < K; ++kc) split8(f + 8 * kc, hi + kc, lo + kc);
+  put_site(planes + kc0 * kPlane, K, x, y, hi);
+  put_site(planes + (kRtPlanes + kc0) * kPlane, K, x, y, lo);
 }
 
 __global__ void __launch_bounds__(kRtThreads, 1) resconv_tc_kernel(RtArgs a) {
@@ -130,8 +142,10 @@ __global__ void __launch_bounds__(kRtThreads, 1) resconv_tc_kernel(RtArgs a) {
   int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
   long long* consumed_total = reinterpret_cast<long long*>(abort_flag + 1);  // at kOffBars + 80
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int quarter = warp & 3, tile = warp >> 2;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // known to be the same in all lanes
+  const int quarter = warp & 3, tile = (warp >> 2) & 1, half = warp >> 3;
+  const int c0 = kRtHalf * half;                   // this thread's first channel
   const int row = 32 * quarter + lane;             // row of this thread's tile
   const int r = 128 * tile + row;                  // column of x
   const int sx = row >> 3, sy = 8 * tile + (row & 7);
@@ -143,16 +157,20 @@ __global__ void __launch_bounds__(kRtThreads, 1) resconv_tc_kernel(RtArgs a) {
                                 : 0;
   const int convs = 2 * a.blocks;
   const long long slices = (long long)my_items * convs * 9;  // weight slices this CTA uses
-  constexpr int kProducer = 32;                              // thread issuing the copies
-  long long loaded = 0;    // slices requested (producer thread)
-  long long consumed = 0;  // slices whose MMAs are issued (thread 0)
+  constexpr int kProducer = 1;  // warp whose first lane issues the copies
+  // The thread that polls for the end of a convolution's MMAs, the others waiting at a barrier: the
+  // polls of all threads took shared-memory cycles from the MMAs' operand reads.
+  constexpr int kWaiter = 64;
+  long long loaded = 0;         // slices requested (producer)
+  long long consumed = 0;       // slices whose MMAs are issued (the electing lane of warp 0)
+  int next_slice = 0;           // loaded modulo the slices of an item (producer)
 
-  auto load_slice = [&](long long sidx) {  // one thread
-    const int slot = (int)(sidx % kRtSlots);
-    const int conv = (int)((sidx / 9) % convs), tap = (int)(sidx % 9);
-    bulk_load(ring + slot * kRtTapBytes,
-              a.wtc + (size_t)conv * kRtConvBytes + (size_t)tap * kRtTapBytes, kRtTapBytes,
+  auto load_slice = [&]() {  // the next slice into its slot (producer)
+    const int slot = (int)(loaded % kRtSlots);
+    bulk_load(ring + slot * kRtTapBytes, a.wtc + (size_t)next_slice * kRtTapBytes, kRtTapBytes,
               full + slot);
+    ++loaded;
+    if (++next_slice == 9 * convs) next_slice = 0;
   };
 
   if (tid == 0) {
@@ -163,9 +181,10 @@ __global__ void __launch_bounds__(kRtThreads, 1) resconv_tc_kernel(RtArgs a) {
     mbar_init(accb, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    for (long long sl = 0; sl < kRtSlots && sl < slices; ++sl) load_slice(sl);
   }
-  loaded = slices < kRtSlots ? slices : kRtSlots;
+  __syncthreads();
+  if (tid == 32 * kProducer)
+    while (loaded < kRtSlots && loaded < slices) load_slice();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
@@ -177,7 +196,7 @@ __global__ void __launch_bounds__(kRtThreads, 1) resconv_tc_kernel(RtArgs a) {
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  const uint32_t t_lane = tmem + ((uint32_t)(32 * quarter) << 16) + 64u * tile;
+  const uint32_t t_lane = tmem + ((uint32_t)(32 * quarter) << 16) + 64u * tile + c0;
   const uint32_t act_hi = smem_u32(planes), act_lo = act_hi + kRtPlanes * kPlane;
   const uint32_t ring0 = smem_u32(ring);
   const uint64_t dAhi = make_desc(act_hi, kPlane, kP * 16);
@@ -188,23 +207,27 @@ __global__ void __launch_bounds__(kRtThreads, 1) resconv_tc_kernel(RtArgs a) {
   uint32_t acc_phase = 0;
   long long conv_seq = 0;  // convolutions processed by this CTA (all threads)
 
-  // Writes h = GELU(RMSNorm(x)) of this thread's site into the planes (all threads call).
+  // Writes h = GELU(RMSNorm(x)) of this thread's channels into the planes (all threads call).  The
+  // sum of a site's 64 squares is one chain, by the threads of its first half.
   auto norm_to_planes = [&]() {
-    float ss = 0.0f;
+    __syncthreads();  // both halves of x
+    if (half == 0) {
+      float ss = 0.0f;
 #pragma unroll 8
-    for (int c = 0; c < kRtC; ++c) ss = fmaf(xs[c * kRtN + r], xs[c * kRtN + r], ss);
+      for (int c = 0; c < kRtC; ++c) ss = fmaf(xs[c * kRtN + r], xs[c * kRtN + r], ss);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if (lane == 0) red[warp] = ss;
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (lane == 0) red[warp] = ss;
+    }
     __syncthreads();
     float tot = 0.0f;
 #pragma unroll
-    for (int w = 0; w < kRtThreads / 32; ++w) tot += red[w];
+    for (int w = 0; w < 8; ++w) tot += red[w];
     const float rn = 1.0f / sqrtf(tot * inv_cn + kRtRmsEps);
-    float f[kRtC];
+    float f[kRtHalf];
 #pragma unroll
-    for (int c = 0; c < kRtC; ++c) f[c] = gelu_fast(xs[c * kRtN + r] * rn);
-    put_channels(planes, sx, sy, f);
+    for (int c = 0; c < kRtHalf; ++c) f[c] = gelu_fast(xs[(c0 + c) * kRtN + r] * rn);
+    put_channels(planes, c0 / 8, sx, sy, f);
   };
 
   for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
@@ -228,7 +251,8 @@ __global__ void __launch_bounds__(kRtThreads, 1) resconv_tc_kernel(RtArgs a) {
     {
       const int occ = (simg[site] > 0 ? 1 : 0) + (simg[kRtN + site] > 0 ? 2 : 0);
 #pragma unroll 8
-      for (int ch = 0; ch < kRtC; ++ch) xs[ch * kRtN + r] = __ldg(a.embed + occ * kRtC + ch);
+      for (int ch = c0; ch < c0 + kRtHalf; ++ch)
+        xs[ch * kRtN + r] = __ldg(a.embed + occ * kRtC + ch);
     }
     norm_to_planes();
 
@@ -237,7 +261,7 @@ __global__ void __launch_bounds__(kRtThreads, 1) resconv_tc_kernel(RtArgs a) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncthreads();  // planes written, accumulators read
-      if (tid == 0) {  // MMA issue: wait for each tap's weights, then its 72 MMAs
+      if (warp == 0 && elect_one()) {  // MMA issue: wait for each tap's weights, then its 72 MMAs
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int tap = 0; tap < 9; ++tap) {
@@ -252,7 +276,7 @@ __global__ void __launch_bounds__(kRtThreads, 1) resconv_tc_kernel(RtArgs a) {
           ++consumed;
         }
         mma_commit(accb);  // arrives once every MMA issued so far has completed
-      } else if (tid == kProducer) {
+      } else if (tid == 32 * kProducer) {
         // Copies: every slice up to the fourth of the next convolution, each into the slot of
         // the slice four back once that slice's MMAs (all of this convolution) have completed.
         const long long upto = (long long)9 * (conv_seq + 1) + kRtSlots;
@@ -263,14 +287,17 @@ __global__ void __launch_bounds__(kRtThreads, 1) resconv_tc_kernel(RtArgs a) {
             *abort_flag = 1;
             break;
           }
-          load_slice(loaded);
-          ++loaded;
+          load_slice();
         }
       }
       ++conv_seq;
-      if (!mbar_wait(accb, acc_phase)) {
-        if (tid == 0) atomicExch(a.err, 4);
-        *abort_flag = 1;
+      if (tid == kWaiter) {
+        if (!mbar_wait(accb, acc_phase)) {
+          atomicExch(a.err, 4);
+          *abort_flag = 1;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       }
       acc_phase ^= 1u;
       __syncthreads();
@@ -279,27 +306,23 @@ __global__ void __launch_bounds__(kRtThreads, 1) resconv_tc_kernel(RtArgs a) {
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      float v[kRtC];
+      float v[kRtHalf];
       tmem_ld32(t_lane, v);
-      tmem_ld32(t_lane + 32, v + 32);
 #pragma unroll
       for (int pc = 1; pc < kRtParts; ++pc) {
         float w[32];
         tmem_ld32(t_lane + 128 * pc, w);
 #pragma unroll
         for (int i = 0; i < 32; ++i) v[i] += w[i];
-        tmem_ld32(t_lane + 128 * pc + 32, w);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) v[32 + i] += w[i];
       }
-      const float* b = a.bias + conv * kRtC;
+      const float* b = a.bias + conv * kRtC + c0;
       if ((conv & 1) == 0) {  // u = GELU(Conv1(h) + b1) into the planes (h is no longer read)
 #pragma unroll
-        for (int ch = 0; ch < kRtC; ++ch) v[ch] = gelu_fast(v[ch] + __ldg(b + ch));
-        put_channels(planes, sx, sy, v);
+        for (int ch = 0; ch < kRtHalf; ++ch) v[ch] = gelu_fast(v[ch] + __ldg(b + ch));
+        put_channels(planes, c0 / 8, sx, sy, v);
       } else {  // x += Conv2(u) + b2, then the next block's h
 #pragma unroll
-        for (int ch = 0; ch < kRtC; ++ch) xs[ch * kRtN + r] += v[ch] + __ldg(b + ch);
+        for (int ch = 0; ch < kRtHalf; ++ch) xs[(c0 + ch) * kRtN + r] += v[ch] + __ldg(b + ch);
         if (conv + 1 < convs) norm_to_planes();
       }
     }
@@ -309,18 +332,19 @@ __global__ void __launch_bounds__(kRtThreads, 1) resconv_tc_kernel(RtArgs a) {
     }
     __syncthreads();
     constexpr int d = kRtC / 2;
-    write_occupied_rows(simg, occl, wbuf, kRtN, a.n, d, g, kL, kL, a.Y + (int64_t)item * a.n * d,
-                        a.idx + (int64_t)item * a.n, a.item_sign + item,
-                        [&](int sg, int aa, int st) {
-                          const int xx = st / kL, yy = st - xx * kL;
-                          const int rr = 128 * (yy >> 3) + 8 * xx + (yy & 7);
-                          return xs[(sg * d + aa) * kRtN + rr] * out_scale;
-                        });
+    auto feat = [&](int sg, int aa, int st) {
+      const int xx = st / kL, yy = st - xx * kL;
+      const int rr = 128 * (yy >> 3) + 8 * xx + (yy & 7);
+      return xs[(sg * d + aa) * kRtN + rr] * out_scale;
+    };
+    write_occupied_rows<float, decltype(feat), kRtThreads>(
+        simg, occl, wbuf, kRtN, a.n, d, g, kL, kL, a.Y + (int64_t)item * a.n * d,
+        a.idx + (int64_t)item * a.n, a.item_sign + item, feat);
   }
   // Copies still in flight (only after an abort): wait for them, bounded, before exiting.
-  if (tid == 0) *consumed_total = consumed;
+  if (warp == 0 && elect_one()) *consumed_total = consumed;
   __syncthreads();
-  if (tid == kProducer) {
+  if (tid == 32 * kProducer) {
     for (long long s = *consumed_total; s < loaded; ++s)
       mbar_wait(full + (s % kRtSlots), (uint32_t)((s / kRtSlots) & 1));
   }
