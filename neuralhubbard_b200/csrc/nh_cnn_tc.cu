@@ -14,13 +14,17 @@
 // accumulates hi*hi + hi*lo + lo*hi (about 16 significant bits per product) for near-FP32
 // features.  The layer-0 input (+-1 occupations) is exact in BF16.  Bias, GELU and the split run
 // in FP32 in the epilogue, which reads the accumulators with tcgen05.ld (warp w % 4 owns lanes
-// 32 (w % 4) .. + 31 of both tiles).
+// 32 (w % 4) .. + 31).
 //
-// Two warp groups of 128 threads run independent image streams in one CTA: each has its own
+// Two warp groups of 256 threads, one site per thread (warps 0-3 of a group: tile 0), run independent image streams in one CTA: each has its own
 // activation planes, bookkeeping, mbarrier, 256 tensor-memory columns (four partial sums of its
 // two 128 x 32 tiles, see issue_layer) and named barrier, and
 // shares the resident weights; while one group's MMAs run, the other converts its accumulators
 // (bias, GELU, hi/lo split) and writes its next planes.
+//
+// What bounds it: the MMAs' operand reads (72 MMAs of 89 / 2 cycles per layer and image, 12.8K
+// cycles an image) beside the epilogues' instructions; two images are in flight to overlap them.
+// 65,536 images: 7.4 ms with 128 threads per group and three MMAs per product, 5.7 ms now.
 //
 // Output: the occupied rows Y (n, d) FP32 of the image configuration, the occupied-mode list and
 // the item sign, like the CUDA-core kernel (mode 1 of nh_cnn.cu).
@@ -44,14 +48,15 @@ namespace {
 
 using namespace tc;
 
-constexpr int kTcThreads = 256;
+constexpr int kTcThreads = 512;
 constexpr int kC = 32;          // channels
-constexpr int kW0Bytes = 2 * 9 * 2 * 4 * 128;    // layer 0: q x tap x kc(2) x cg(4) x 128 B
-constexpr int kW1Bytes = 2 * 9 * 4 * 4 * 128;    // layers 1..3: q x tap x kc(4) x cg(4) x 128 B
+constexpr int kChunkBytes = 2 * 4 * 128;         // 8 input channels of a tap: q x cg(4) x 128 B
+constexpr int kW0Bytes = 9 * 2 * kChunkBytes;    // layer 0: tap x kc(2)
+constexpr int kW1Bytes = 9 * 4 * kChunkBytes;    // layers 1..3: tap x kc(4)
 constexpr int kWBytes = kW0Bytes + 3 * kW1Bytes;
 constexpr int kActBytes = 2 * 4 * kPlane;        // hi and lo, 4 planes each
 constexpr int kWG = 2;                           // independent warp groups per CTA
-constexpr int kWGThreads = kTcThreads / kWG;     // 128
+constexpr int kWGThreads = kTcThreads / kWG;     // 256
 constexpr int kIntsPerWG = 3 * 2 * kL * kL + 4 * kL + 32;  // simg, rowof, occl, scan scratch
 constexpr int kParts = 4;                        // partial sums per tile: (kh, cross)
 constexpr unsigned kTmemCols = 64 * kParts * kWG; // per group: 4 partials x two 128 x 32 tiles
@@ -68,8 +73,9 @@ struct TcArgs {
   int32_t* err;         // error word (0 = ok)
 };
 
-// Instruction descriptor: kind::f16, BF16 x BF16 -> FP32, both K-major, M = 128, N = 32.
-constexpr uint32_t kIdesc = idesc_bf16(128, 32);
+// Instruction descriptors: kind::f16, BF16 x BF16 -> FP32, both K-major, M = 128, N = 32 (one half
+// of the weights) or N = 64 (hi and lo).
+constexpr uint32_t kIdesc = idesc_bf16(128, 32), kIdesc2 = idesc_bf16(128, 64);
 
 // tanh-approximated GELU written as x * sigmoid(2 z), z = sqrt(2/pi) (x + 0.044715 x^3), which is
 // the same function as 0.5 x (1 + tanh z); the exponential is the fast __expf intrinsic.
@@ -79,17 +85,23 @@ __device__ __forceinline__ float gelu_tanh(float x) {
 }
 
 // Issue the MMAs of one layer for both tiles (one thread).
-// Partial sum p = 2 kh + cross of tile h lives at columns 64 p + 32 h of the group's 256: the
-// hi*hi products of the input-channel half kh, and (cross = 1) its hi*lo + lo*hi products, so
-// that every FP32 accumulation chain in the tensor core is short (9 or 18 MMAs) and the small
-// cross terms are not added into the large main sum there.  The epilogue adds the partials.
-__device__ void issue_layer(uint32_t tmem, uint32_t act_hi, uint32_t act_lo, uint32_t w_hi,
-                            uint32_t w_lo, int kchunks, int tap_bytes, bool split_act,
-                            bool split_w) {
-  const uint32_t sbo_a = kP * 16;  // next x-row of the tile
-  const uint32_t lbo_a = kPlane;   // next 8-channel plane
-  const uint32_t lbo_b = 4 * 128;  // next 8-ci chunk of the weights
-  const uint32_t sbo_b = 128;      // next 8-co group of the weights
+// Partial sum p = 2 kh + cross of tile h lives at columns 64 (2 kh + h) + 32 cross of the group's
+// 256: the hi*hi products of the input-channel half kh, and (cross = 1) its hi*lo + lo*hi
+// products, so that every FP32 accumulation chain in the tensor core is short (9 or 18 MMAs) and
+// the small cross terms are not added into the large main sum there.  The epilogue adds the
+// partials.  An MMA takes as long as its operands take to leave shared memory at 128 bytes per
+// cycle (40.7 cycles with N = 32, 48.7 with N = 64, whatever the start's alignment), most of it the
+// activations', so hi*hi and hi*lo are one MMA over the adjacent hi and lo weights: 89 cycles for
+// the three products instead of 122.
+template <int KCHUNKS>
+__device__ __forceinline__ void issue_layer(uint32_t tmem, uint32_t act_hi, uint32_t act_lo,
+                                            uint32_t w, bool split_act, bool split_w) {
+  constexpr int kTapBytes = KCHUNKS * kChunkBytes;
+  // Descriptors formed once and advanced by constants (the address field counts 16-byte units):
+  // next 8-channel plane and next x-row of the tile; next 8-ci chunk and 8-co group of the weights
+  const uint64_t d_ahi = make_desc(act_hi, kPlane, kP * 16);
+  const uint64_t d_alo = make_desc(act_lo, kPlane, kP * 16);
+  const uint64_t d_w = make_desc(w, kChunkBytes, 128);
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
 #pragma unroll
@@ -97,19 +109,12 @@ __device__ void issue_layer(uint32_t tmem, uint32_t act_hi, uint32_t act_lo, uin
       const int dx = tap / 3 - 1, dy = tap % 3 - 1;
       const uint32_t aoff = (uint32_t)pad_off(dx + 1, 8 * h + dy + 1);
 #pragma unroll
-      for (int kh = 0; kh < 2; ++kh) {
-        if (kh >= kchunks / 2) break;
-        const uint32_t d_main = tmem + 64 * (2 * kh) + 32 * h;
-        const uint32_t d_cross = d_main + 64;
-        const uint32_t ao = aoff + 2 * kh * kPlane;
-        const uint32_t bo = tap * tap_bytes + 2 * kh * 4 * 128;
-        const uint64_t ahi = make_desc(act_hi + ao, lbo_a, sbo_a);
-        const uint64_t bhi = make_desc(w_hi + bo, lbo_b, sbo_b);
-        mma_bf16(d_main, ahi, bhi, kIdesc, tap > 0);
-        if (split_w) mma_bf16(d_cross, ahi, make_desc(w_lo + bo, lbo_b, sbo_b), kIdesc, tap > 0);
-        if (split_act)
-          mma_bf16(d_cross, make_desc(act_lo + ao, lbo_a, sbo_a), bhi, kIdesc,
-                   tap > 0 || split_w);
+      for (int kh = 0; kh < KCHUNKS / 2; ++kh) {
+        const uint32_t d_main = tmem + 64 * (2 * kh + h);
+        const uint64_t ao = (aoff + 2 * kh * kPlane) >> 4;
+        const uint64_t bo = (tap * kTapBytes + 2 * kh * kChunkBytes) >> 4;
+        mma_bf16(d_main, d_ahi + ao, d_w + bo, split_w ? kIdesc2 : kIdesc, tap > 0);
+        if (split_act) mma_bf16(d_main + 32, d_alo + ao, d_w + bo, kIdesc, tap > 0 || split_w);
       }
     }
   }
@@ -118,13 +123,13 @@ __device__ void issue_layer(uint32_t tmem, uint32_t act_hi, uint32_t act_lo, uin
 // Accumulators of tile h for this warp's lane quarter: the sum of the partials the layer wrote.
 __device__ __forceinline__ void load_tile(uint32_t tlane, int h, int kchunks, bool cross,
                                           float* v) {
-  tmem_ld32(tlane + 32 * h, v);
+  tmem_ld32(tlane + 64 * h, v);
 #pragma unroll
   for (int p = 1; p < kParts; ++p) {
     const int kh = p >> 1;
     if (kh >= kchunks / 2 || ((p & 1) && !cross)) continue;
     float w[32];
-    tmem_ld32(tlane + 64 * p + 32 * h, w);
+    tmem_ld32(tlane + 64 * (2 * kh + h) + 32 * (p & 1), w);
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] += w[i];
   }
@@ -172,8 +177,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) cnn_tc_kernel(TcArgs a) {
   int* abort_all = reinterpret_cast<int*>(tmem_slot + 1);  // per group
 
   const int tid = threadIdx.x;
-  const int wg = tid / kWGThreads, ltid = tid - wg * kWGThreads;
-  const int lane = ltid & 31, lwid = ltid >> 5;  // lwid = warp % 4: the TMEM lane quarter
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // known to be the same in all lanes
+  const int wg = warp / (kWGThreads / 32), ltid = tid - wg * kWGThreads;
+  const int lane = ltid & 31, lwid = warp % (kWGThreads / 32);  // the TMEM lane quarter
   const int N = kL * kL, M2 = 2 * N;
 
   // Weights resident for the whole launch: one bulk TMA copy of the packed image (16-byte
@@ -231,7 +237,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) cnn_tc_kernel(TcArgs a) {
 
   const int G = a.cl.G;
   const int n_items = (a.cl.n_cfg_dev ? *a.cl.n_cfg_dev : a.cl.n_cfg) * G;
-  for (int item = blockIdx.x * kWG + wg; item < n_items; item += gridDim.x * kWG) {
+  for (int item = wg * gridDim.x + blockIdx.x; item < n_items; item += gridDim.x * kWG) {
     if (*abort_flag) {  // a wait expired earlier: mark the item instead of computing it
       if (ltid == 0) a.item_sign[item] = NAN;
       continue;
@@ -294,19 +300,25 @@ __global__ void __launch_bounds__(kTcThreads, 1) cnn_tc_kernel(TcArgs a) {
     const int total = wbuf[0];
 
     for (int layer = 0; layer < 4; ++layer) {
-      if (ltid == 0) {
+      if (lwid == 0 && elect_one()) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (layer == 0)
-          issue_layer(tmem, act_hi, act_lo, w0, w0 + kW0Bytes / 2, 2, 2 * 4 * 128, false, split);
+          issue_layer<2>(tmem, act_hi, act_lo, w0, false, split);
         else {
           const uint32_t wl = w0 + kW0Bytes + (layer - 1) * kW1Bytes;
-          issue_layer(tmem, act_hi, act_lo, wl, wl + kW1Bytes / 2, 4, 4 * 4 * 128, split, split);
+          issue_layer<4>(tmem, act_hi, act_lo, wl, split, split);
         }
         mma_commit(bar);
       }
-      if (!mbar_wait(bar, phase)) {
-        if (ltid == 0) atomicExch(a.err, 1);
-        *abort_flag = 1;
+      // One thread polls and the others wait at the barrier: the polls of all threads took
+      // shared-memory cycles from the MMAs' operand reads.
+      if (ltid == 32) {
+        if (!mbar_wait(bar, phase)) {
+          atomicExch(a.err, 1);
+          *abort_flag = 1;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       }
       phase ^= 1u;
       wg_sync(wg);
@@ -315,49 +327,38 @@ __global__ void __launch_bounds__(kTcThreads, 1) cnn_tc_kernel(TcArgs a) {
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // Epilogue: warp lwid reads TMEM lanes 32 lwid .. + 31 of both tiles (rows = sites).
-      const int mrow = 32 * lwid + lane;  // row of the 128 x 32 tile
-      const int x = mrow >> 3;
+      // Epilogue: warp lwid reads TMEM lanes 32 (lwid % 4) .. + 31 of tile lwid / 4 (rows = sites).
+      const int h = lwid >> 2, mrow = 32 * (lwid & 3) + lane;  // row of the 128 x 32 tile
+      const uint32_t tlane = tmem + ((uint32_t)(32 * (lwid & 3)) << 16);
+      const int x = mrow >> 3, y = 8 * h + (mrow & 7);
       const float* bl = bsm + layer * kC;
+      float v[32];
+      load_tile(tlane, h, layer == 0 ? 2 : 4, split, v);
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       if (layer < 3) {
-        uint4 hi[2][4], lo[2][4];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          float v[32];
-          load_tile(tmem + ((uint32_t)(32 * lwid) << 16), h, layer == 0 ? 2 : 4, split, v);
-          act_groups(v, bl, hi[h], lo[h]);
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        wg_sync(wg);  // every tile is read before any plane is overwritten
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int y = 8 * h + (mrow & 7);
-          put_site(act, 4, x, y, hi[h]);
-          if (split) put_site(act + 4 * kPlane, 4, x, y, lo[h]);
-        }
+        // The layer's MMAs are complete, so its planes are dead; the next layer's MMAs are issued
+        // after the barrier, so after every tile is read.
+        uint4 hi[4], lo[4];
+        act_groups(v, bl, hi, lo);
+        put_site(act, 4, x, y, hi);
+        if (split) put_site(act + 4 * kPlane, 4, x, y, lo);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         wg_sync(wg);
       } else {
         // Last layer: features y_up = channels 0..15, y_down = 16..31 of occupied modes.
+        const int s = x * kL + y;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          float v[32];
-          load_tile(tmem + ((uint32_t)(32 * lwid) << 16), h, 4, split, v);
-          const int s = x * kL + 8 * h + (mrow & 7);
+        for (int sg = 0; sg < 2; ++sg) {
+          const int row = rowof[sg * N + s];
+          if (row < 0) continue;
+          float4* dst = reinterpret_cast<float4*>(a.Y + ((int64_t)item * a.n + row) * 16);
 #pragma unroll
-          for (int sg = 0; sg < 2; ++sg) {
-            const int row = rowof[sg * N + s];
-            if (row < 0) continue;
-            float4* dst = reinterpret_cast<float4*>(a.Y + ((int64_t)item * a.n + row) * 16);
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-              dst[q] = make_float4(v[16 * sg + 4 * q] + bl[16 * sg + 4 * q],
-                                   v[16 * sg + 4 * q + 1] + bl[16 * sg + 4 * q + 1],
-                                   v[16 * sg + 4 * q + 2] + bl[16 * sg + 4 * q + 2],
-                                   v[16 * sg + 4 * q + 3] + bl[16 * sg + 4 * q + 3]);
-          }
+          for (int q = 0; q < 4; ++q)
+            dst[q] = make_float4(v[16 * sg + 4 * q] + bl[16 * sg + 4 * q],
+                                 v[16 * sg + 4 * q + 1] + bl[16 * sg + 4 * q + 1],
+                                 v[16 * sg + 4 * q + 2] + bl[16 * sg + 4 * q + 2],
+                                 v[16 * sg + 4 * q + 3] + bl[16 * sg + 4 * q + 3]);
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       }
     }
     if (*abort_flag) continue;
@@ -382,7 +383,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) cnn_tc_kernel(TcArgs a) {
                  : "memory");
 }
 
-// Packed weights: per layer, q (hi, lo) x tap x kc x cg x [8 co rows x 8 ci] BF16, the K-major
+// Packed weights: per layer, tap x kc x q (hi, lo) x cg x [8 co rows x 8 ci] BF16, the K-major
 // canonical layout of the B operand (N = co, K = ci); layer 0 pads ci from 2 to 16.
 __global__ void pack_tc_kernel(const float* __restrict__ w, uint16_t* out) {
   const int total = kWBytes / 2;
@@ -401,12 +402,12 @@ __global__ void pack_tc_kernel(const float* __restrict__ w, uint16_t* out) {
       cin = kC;
       off = 18 * kC + (l - 1) * 9 * kC * kC;
     }
-    const int per_q = 9 * kcs * 4 * 64;
-    const int q = r / per_q;
-    int t = r % per_q;
-    const int tap = t / (kcs * 4 * 64);
-    t %= kcs * 4 * 64;
-    const int kc = t / (4 * 64);
+    int t = r;
+    const int tap = t / (kcs * 2 * 4 * 64);
+    t %= kcs * 2 * 4 * 64;
+    const int kc = t / (2 * 4 * 64);
+    t %= 2 * 4 * 64;
+    const int q = t / (4 * 64);
     t %= 4 * 64;
     const int cg = t / 64;
     t %= 64;
@@ -455,7 +456,7 @@ int launch_cnn_tc(const ConfigList& cl, const nh_backflow_params& p, int mode, f
   const int items = cl.n_cfg * cl.G;
   if (items <= 0) return NH_OK;
   int grid = num_sms();
-  if (grid > (items + kWG - 1) / kWG) grid = (items + kWG - 1) / kWG;
+  if (grid > items) grid = items;  // few items: one per SM before a second group's
   TcArgs a{cl, static_cast<const uint16_t*>(p.conv_w_tc), p.conv_b, p.n_up + p.n_dn, mode, Y,
            idx, item_sign, err};
   ProfScope prof_scope(NH_K_CNN_TC, st);
