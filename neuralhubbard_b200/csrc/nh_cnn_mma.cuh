@@ -17,7 +17,7 @@
 // The instruction runs at the DFMA rate (64 FMA per clock and SM, measured), so the gain over
 // scalar code is in operand traffic: a warp loads 6 operands per 8 MMAs of 256 FMA where the
 // scalar loop loads 6 per 16 FMA and thread.  Measured at 16x16, 19,091 images: 15.0 ms scalar,
-// 10.3 ms here (the FMA floor is 8.0 ms).
+// 9.96 ms here (the FMA floor is 8.0 ms).
 #pragma once
 
 #include "nh_cnn_item.cuh"

@@ -152,14 +152,17 @@ __device__ __forceinline__ void put_site(unsigned char* planes, int nplanes, int
 }
 
 // 8 FP32 values -> their BF16 hi parts and the BF16 of the remainders (lo), packed as 16 bytes.
+__device__ __forceinline__ uint32_t bf16_pair(float x, float y) {
+  const __nv_bfloat162 p = __floats2bfloat162_rn(x, y);
+  return (uint32_t)__bfloat16_as_ushort(p.x) | ((uint32_t)__bfloat16_as_ushort(p.y) << 16);
+}
 __device__ __forceinline__ void split8(const float* f, uint4* hi, uint4* lo) {
   uint32_t ph[4], pl[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const uint16_t h0 = bf16_bits(f[2 * j]), h1 = bf16_bits(f[2 * j + 1]);
-    ph[j] = (uint32_t)h0 | ((uint32_t)h1 << 16);
-    pl[j] = (uint32_t)bf16_bits(f[2 * j] - bf16_val(h0)) |
-            ((uint32_t)bf16_bits(f[2 * j + 1] - bf16_val(h1)) << 16);
+    ph[j] = bf16_pair(f[2 * j], f[2 * j + 1]);
+    pl[j] = bf16_pair(f[2 * j] - __uint_as_float(ph[j] << 16),
+                      f[2 * j + 1] - __uint_as_float(ph[j] & 0xFFFF0000u));
   }
   *hi = make_uint4(ph[0], ph[1], ph[2], ph[3]);
   *lo = make_uint4(pl[0], pl[1], pl[2], pl[3]);
