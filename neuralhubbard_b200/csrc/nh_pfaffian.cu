@@ -1,18 +1,17 @@
 // Batched log-Pfaffian (blocked Parlett-Reid LTL^T with partial pivoting), the pairing
 // gather, and the combination of symmetry images.
 //
-// One CTA (256 threads) per antisymmetric n x n matrix, n even, n <= 256; FP32 (two CTAs per
-// SM at n = 224) or FP64 (one CTA per SM, used to recompute ill-conditioned items).  The strict
-// lower triangle lives in shared memory (row i at offset i (i - 1) / 2) and thread t owns
-// physical row t.  A pivot does not move data: it swaps the logical labels of two physical rows,
-// so an elimination step costs two block barriers.  Panel columns are formed lazily (stored
-// column plus the panel's rank-2 terms U V^T - V U^T); at the end of a panel of NB steps the
-// active rows are listed in physical order and the trailing triangle receives the rank-2NB
-// update, one warp per row and one lane per column, the column's U/V in registers and the row's
-// U/V broadcast.  The Pfaffian is the product of the pivots A[k, k+1] times the parity of the
-// relabelling, accumulated in FP64 as mantissa and exponent.  The ratio of the largest to the
-// smallest pivot magnitude estimates the condition number; above cond_tau the item is flagged
-// NH_FLAG_GROWTH (near-nodal) for the FP64 recompute.
+// FP32 matrices of n <= 256 run in pf32_kernel, larger ones in pf32_big_kernel (both described
+// where they stand); pfaffian_kernel below is the FP64 form for dense matrices and for
+// 224 < n <= 236.  One CTA per antisymmetric n x n matrix, n even.  The strict lower triangle lives
+// in shared memory (row i at offset i (i - 1) / 2) or in a slice of global scratch.  A pivot does not
+// move data: it swaps the logical labels of two physical rows, so an elimination step costs two
+// barriers.  Panel columns are formed lazily (stored column plus the panel's rank-2 terms
+// U V^T - V U^T); at the end of a panel of NB steps the active rows are listed in physical order and
+// the trailing triangle receives the rank-2NB update.  The Pfaffian is the product of the pivots
+// A[k, k+1] times the parity of the relabelling, accumulated in FP64 as mantissa and exponent.  The
+// ratio of the largest to the smallest pivot magnitude estimates the condition number; above
+// cond_tau the item is flagged NH_FLAG_GROWTH (near-nodal) for the FP64 recompute.
 //
 // Replaces fermix.slogpf (code/backflow/models.py:210) and, in the gather mode, the Pallas
 // pairing kernel pfsbp_pairing_fwd (code/backflow/pf_kernel.py:156-190) whose formula it
