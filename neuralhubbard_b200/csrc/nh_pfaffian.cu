@@ -359,8 +359,8 @@ __device__ void gather_from_rows(const PfArgs& a, float* Lw, const float* Ys, co
 // memory (a.tri; L2-resident up to n ~ 500), shared memory holding only the panel and the
 // reduction slots.
 template <typename T, int NB, int D, int THREADS = kNumThreads>
-__global__ void __launch_bounds__(THREADS, THREADS > kNumThreads ? 1 : (sizeof(T) == 4 ? 2 : 1))
-    pfaffian_kernel(PfArgs a) {
+__global__ void __launch_bounds__(THREADS, 1) pfaffian_kernel(PfArgs a) {
+  static_assert(sizeof(T) == 8, "FP32 matrices have their own kernels");
   static_assert(NB % Vec<T>::k == 0, "panel width must fill 16-byte vectors");
   constexpr int WARPS = THREADS / 32;
   constexpr bool kGlobalTri = THREADS > kNumThreads;
@@ -378,11 +378,9 @@ __global__ void __launch_bounds__(THREADS, THREADS > kNumThreads ? 1 : (sizeof(T
     Us = Lw + ((tri + 3) & ~3);
   }
   T* Vs = Us + n * NB;            // (n, NB)
-  // FP32: the winner's signed value shares the key slot (its magnitude is the key); FP64 keeps
-  // it separately.  pivs[k/2] = pivot A[k, k+1], negated when that step swapped labels.
-  constexpr int kValSlots = sizeof(T) == 4 ? 0 : WARPS;
-  T* rval = Vs + n * NB;                 // (warps, FP64 only) candidate signed value
-  T* pivs = rval + kValSlots;            // (n / 2) signed pivots, multiplied at the end
+  // pivs[k/2] = pivot A[k, k+1], negated when that step swapped labels.
+  T* rval = Vs + n * NB;                 // (warps) candidate signed value
+  T* pivs = rval + WARPS;                // (n / 2) signed pivots, multiplied at the end
   float* rkey = reinterpret_cast<float*>(pivs + ((n / 2 + 3) & ~3));
   int* rt = reinterpret_cast<int*>(rkey + WARPS);  // (warps) trailing update: ballot counts
   int* rlog = rt + WARPS;
@@ -457,7 +455,7 @@ __global__ void __launch_bounds__(THREADS, THREADS > kNumThreads ? 1 : (sizeof(T
             const unsigned lo = ((0xFFFFu - (unsigned)tid) << 16) |
                                 (signbit(c) ? 0x8000u : 0u) | ((unsigned)my_log & 0x7FFFu);
             cand[wid] = ((unsigned long long)kmax << 32) | lo;
-            if constexpr (sizeof(T) == 8) rval[wid] = c;  // FP64 keeps the signed value
+            rval[wid] = c;
           }
           __syncthreads();  // (1) pivot candidates
           unsigned long long best = 0;
@@ -471,11 +469,7 @@ __global__ void __launch_bounds__(THREADS, THREADS > kNumThreads ? 1 : (sizeof(T
           const float bk = kbest ? __uint_as_float(kbest - 1u) : -1.0f;
           const int r = 0xFFFF - (int)((best >> 16) & 0xFFFFu);
           const int lr = (int)(best & 0x7FFFu);
-          T cr;
-          if constexpr (sizeof(T) == 4)
-            cr = (best & 0x8000u) ? -bk : bk;  // a NaN candidate comes back as an infinite pivot
-          else
-            cr = rval[r >> 5];
+          const T cr = rval[r >> 5];
           if (!(bk > 0.0f)) {
             zero = true;  // exactly singular (or empty) column: pf = 0
           } else {
@@ -532,7 +526,7 @@ __global__ void __launch_bounds__(THREADS, THREADS > kNumThreads ? 1 : (sizeof(T
         // Work units: (64-column block cb, group of RT consecutive rows below its diagonal);
         // lane l updates columns 64 cb + l and 64 cb + 32 + l, so each row's broadcast U/V
         // serves 64 elements.  All loads of a unit precede its stores (stores may alias loads).
-        constexpr int RT = sizeof(T) == 4 ? 2 : 1;
+        constexpr int RT = 1;
         int total = 0;
         for (int cb = 0; 64 * cb + 1 < m; ++cb) total += (m - 64 * cb - 1 + RT - 1) / RT;
         int cb = 0, rem = wid, cur_cb = -1, ib0 = 0, ib1 = 0, pb0 = 0, pb1 = 0;
@@ -658,9 +652,8 @@ __global__ void __launch_bounds__(THREADS, THREADS > kNumThreads ? 1 : (sizeof(T
 template <typename T, int NB, int WARPS = kWarps, bool kGlobalTri = false>
 size_t pf_smem(int n) {
   const size_t tri = (size_t)n * (n - 1) / 2;
-  const size_t val_slots = sizeof(T) == 4 ? 0 : WARPS;
   return sizeof(T) * ((kGlobalTri ? 0 : ((tri + 3) & ~(size_t)3)) + 2 * (size_t)n * NB +
-                      val_slots + ((n / 2 + 3) & ~(size_t)3)) +
+                      WARPS + ((n / 2 + 3) & ~(size_t)3)) +
          sizeof(float) * WARPS + sizeof(int) * (2 * WARPS + (size_t)n + 2);
 }
 
@@ -699,7 +692,7 @@ int launch_pf(const PfArgs& a, cudaStream_t st) {
   int grid = num_sms() * per_sm;
   if (grid > a.n_slots) grid = a.n_slots;
   if (grid <= 0) return NH_OK;
-  ProfScope prof_scope(sizeof(T) == 4 ? NH_K_PFAFFIAN : NH_K_PFAFFIAN64, st);
+  ProfScope prof_scope(NH_K_PFAFFIAN64, st);
   pfaffian_kernel<T, NB, D, THREADS><<<grid, THREADS, smem, st>>>(a);
   return check_launch("pfaffian_kernel");
 }
