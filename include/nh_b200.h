@@ -92,15 +92,17 @@ enum {
  *                log-Pfaffian refined: the same matrix is factorised again in FP64 with the
  *                pivot order of the FP32 factorisation held fixed (no pivot search; a blocked
  *                rank-8 FP64 elimination), which removes the FP32 factorisation error
- *                (NH_FLAG_REFINED).  <= 0: off; 1: every item.  Needs n <= 224; for larger n the
- *                refinement is the pivoted FP64 recompute of cond_tau below.
+ *                (NH_FLAG_REFINED).  <= 0: off; 1: every item.  Needs n <= 224; for larger n it has
+ *                no effect and the refinement is the FP64 recompute of cond_tau below.
  * cond_tau:      an item whose pivot ratio exceeds cond_tau is flagged NH_FLAG_GROWTH and, when
  *                Wt64 is set, its features are recomputed in FP64 (CNN) and its log-Pfaffian is
- *                refined against the FP64 pairing block (NH_FLAG_REFINED; 224 < n <= 236: a
- *                pivoted FP64 Pfaffian); <= 0 disables both.  For projected amplitudes with
- *                cond_tau > 1 an image whose |psi(g s)| is below 1e-3 of |psi_P(s)| is not
- *                recomputed in FP64 (its error cannot move log|psi_P| by more than ~1e-5);
- *                cond_tau <= 1 recomputes every image (the all-FP64 form).
+ *                refined against the FP64 pairing block (NH_FLAG_REFINED), in the pivot order of
+ *                the FP32 factorisation; 224 < n <= 236, and larger n where that order leaves a
+ *                multiplier above 2 or a zero or non-finite pivot: with FP64 partial pivoting.
+ *                <= 0 disables both.  For projected amplitudes with cond_tau > 1 an image whose
+ *                |psi(g s)| is below 1e-3 of |psi_P(s)| is not recomputed in FP64 (its error
+ *                cannot move log|psi_P| by more than ~1e-5); cond_tau <= 1 recomputes every image
+ *                (the all-FP64 form).
  * cancel_tau:    projected amplitudes only: a configuration whose 8 images cancel, i.e.
  *                sum_g |psi(g s)| > cancel_tau |sum_g eta_g psi(g s)|, amplifies the FP32
  *                error of its images by that factor; with cancel_tau > 0 (and Wt64 set) all its

@@ -165,7 +165,8 @@ PipelineBuffers carve_pipeline(void* ws, int max_items, const nh_backflow_params
 // items flagged ill-conditioned or cancelling -> FP64 refinement of the log-Pfaffian with the
 // FP32 pivot order (against the FP64 pairing block for those items, against the item's own FP32
 // block for the others above refine_tau) -> combination of the symmetry images (or a copy for
-// G = 1).  For 224 < n <= 236 the flagged items are recomputed by the pivoted FP64 kernel.
+// G = 1).  For 224 < n <= 236 the flagged items are recomputed by the pivoted FP64 kernel; beyond,
+// those of them for which the FP32 pivot order does not hold in FP64.
 int run_pipeline(const ConfigList& cl, const nh_backflow_params& p, const PipelineBuffers& b,
                  float* sign, double* logabs, int32_t* flags, cudaStream_t st) {
   const int n = p.n_up + p.n_dn, d = p.channels / 2;
@@ -242,10 +243,12 @@ int run_pipeline(const ConfigList& cl, const nh_backflow_params& p, const Pipeli
                      max_items, b.perm, perm_stride(n), b.item_sign, b.pf_sign, b.pf_logabs,
                      b.pf_flags, big ? b.pf_tri : b.slice};
       if ((rc = launch_refine(r, st))) return rc;
-    } else {
+    }
+    if (!refine) {
       PfGatherArgs g64{b.Y64, b.idx64, p.Wt64, p.Lx, p.Ly, d, n, b.count, 1, max_items, b.list,
                        b.item_sign, b.pf_sign, b.pf_logabs, b.pf_flags, 0.0,
                        NH_FLAG_GROWTH | NH_FLAG_REFINED, true, b.pf_tri};
+      g64.only_flag = big ? kFlagRepivot : 0;
       if ((rc = launch_pfaffian_gather(g64, st))) return rc;
     }
   }

@@ -15,11 +15,13 @@ constexpr int kMaxN = 1024;       // sites per lattice supported by the bookkeep
 // image combination): the FP32 pivot ratio exceeds refine_tau, so the item's log-Pfaffian is
 // refined in FP64 with its FP32 pivot order.
 constexpr int kFlagNeedRefine = 1 << 20;
+constexpr int kFlagRepivot = 1 << 21;  // the FP32 pivot order did not serve: factorise with pivoting
 constexpr int kPublicFlags = 0xFFFF;
 // FP64 refinement with the FP32 pivot order (nh_refine.cu): its FP64 triangle lives in shared
 // memory up to kRefineMaxN.  Beyond, the flagged items of the amplitude pipeline are refined with
 // their triangle in global memory where the pipeline has that scratch (pfaffian_scratch_bytes,
-// n > 236), else recomputed by the pivoted FP64 kernel, which also serves dense matrices.
+// n > 236), and those whose order does not hold (kFlagRepivot) again by the pivoted FP64 kernel;
+// else all by that kernel, which also serves dense matrices.
 constexpr int kRefineMaxN = 224;
 constexpr size_t kRefineSmemLimit = 225 * 1024;
 // Backward of the amplitude (nh_grad.cu): the Gauss-Jordan inverse keeps the matrix in registers
@@ -356,6 +358,7 @@ struct PfGatherArgs {
   double refine_tau = 0.0;   // pivot ratio above which kFlagNeedRefine is set (0: never)
   float* ratio = nullptr;    // when set: every item's pivot ratio
   float* wt_chunks = nullptr;  // staged form: 4 N d floats for the FP32 table in chunks
+  int only_flag = 0;           // FP64: when set, items without this flag are left alone
 };
 
 // Launchers (return NH_OK or an error code).

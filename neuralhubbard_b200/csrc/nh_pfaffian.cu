@@ -89,6 +89,7 @@ struct PfArgs {
   int32_t* flags;            // (items,) or null
   double cond_tau;           // flag NH_FLAG_GROWTH when max|piv| > cond_tau min|piv| (0: off)
   int flag_or;               // OR-ed into every written flag
+  int only_flag;             // pfaffian_kernel: when set, items without this flag are left alone
   void* tri;                 // large n: per-CTA lower triangles of T in global memory
   uint16_t* perm;            // or null: per item, logical -> physical row, then the parity
   double refine_tau;         // set kFlagNeedRefine when max|piv| > refine_tau min|piv| (0: off)
@@ -396,6 +397,7 @@ __global__ void __launch_bounds__(THREADS, 1) pfaffian_kernel(PfArgs a) {
   const T* Wt = static_cast<const T*>(a.Wt);
   for (int slot = blockIdx.x; slot < n_work; slot += gridDim.x) {
     const int item = a.slot_item ? a.slot_item[slot] : slot;
+    if (a.only_flag && !(a.flags[item] & a.only_flag)) continue;  // the same in all threads
     __syncthreads();
     if (a.mode == 0) {
       const float* F = a.F + (size_t)item * n * n;
@@ -2252,6 +2254,7 @@ int launch_pfaffian_gather(const PfGatherArgs& g, cudaStream_t st) {
   a.perm = g.perm;
   a.refine_tau = g.refine_tau;
   a.ratio = g.ratio;
+  a.only_flag = g.only_flag;
   if (!g.fp64 && g.n > kNumThreads) {  // pf32_big_kernel gathers from the chunked table
     if (!g.wt_chunks) return fail(NH_ERR_INVALID, "amplitude: n=%d needs the chunked table", g.n);
     if (int rc = launch_wt_chunks(static_cast<const float*>(g.Wt), g.Lx * g.Ly, g.d, g.wt_chunks, st))
