@@ -444,20 +444,24 @@ __global__ void __launch_bounds__(kVjpThreads, 1) pairing_vjp_kernel(VjpArgs a) 
         inv[m] = p;
       }
       __syncthreads();
-      // dY: lane <-> row p (16 per warp, the two half-warps taking alternate q), so that Y[q] is a
-      // broadcast, the lanes' neighbouring table rows share cache lines (chunked table) and the sums
-      // need one exchange at the end.
+      // dY: lane <-> row p (R rows per warp; the warp's 32 / R lane groups take alternate q), so that
+      // Y[q] is a broadcast, the lanes' neighbouring table rows share cache lines (chunked table) and
+      // the sums need few exchanges at the end.  16 rows fill the warps from n = 129 on; below, where
+      // the loop over q is latency, fewer rows per warp keep all of them at work (300 matrices of
+      // n = 56, d = 16: 87.4 us with 16 rows, 58.9 with 4 and the two changes below).
       if (a.dY) {
         float* dYi = a.dY + item * n * D;
-        for (int p0 = 16 * warp; p0 < n; p0 += 16 * (kVjpThreads / 32)) {
-          const int pl = p0 + (lane & 15), p = pl < n ? pl : n - 1;
+        constexpr int WARPS = kVjpThreads / 32;
+        const int R = n <= 4 * WARPS ? 4 : (n <= 8 * WARPS ? 8 : 16);
+        for (int p0 = R * warp; p0 < n; p0 += R * WARPS) {
+          const int pl = p0 + (lane & (R - 1)), p = pl < n ? pl : n - 1;
           const int mp = modes[p];
           const int sp = mp >> 16, xp = (mp >> 8) & 0xFF, yp = mp & 0xFF;
           float acc[D];
 #pragma unroll
           for (int j = 0; j < D; ++j) acc[j] = 0.0f;
 #pragma unroll 2
-          for (int q = lane >> 4; q < n; q += 2) {
+          for (int q = lane / R; q < n; q += 32 / R) {
             const float gh = gs[p * NS + q] - gs[q * NS + p];
             const int mq = modes[q];
             const int sq = mq >> 16;
@@ -477,21 +481,25 @@ __global__ void __launch_bounds__(kVjpThreads, 1) pairing_vjp_kernel(VjpArgs a) 
               acc[4 * c + 3] = fmaf(gh * w.w, y.w, acc[4 * c + 3]);
             }
           }
+          for (int o = 16; o >= R; o >>= 1)
 #pragma unroll
-          for (int j = 0; j < D; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 16);
-          if (lane < 16 && pl < n)
+            for (int j = 0; j < D; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+          if (lane < R && pl < n)
 #pragma unroll
             for (int j = 0; j < D; ++j) dYi[(size_t)pl * D + j] = acc[j];  // any float alignment
         }
       }
       // dWt: each (pair, chunk) sums over the rows p; partner q = inv[sq, site_p - r].  The loads of an
-      // empty partner read row 0 and are not added, so that consecutive rows overlap.
+      // empty partner read row 0 and are not added, so that consecutive rows overlap; passes that
+      // hold no pair of this lattice are left out.
+      const int passes = (2 * N * kCh + kVjpThreads - 1) / kVjpThreads;
       auto add_row = [&](int p, float4 (&acc)[kCh]) {
         const int mp = modes[p];
         const int xp = (mp >> 8) & 0xFF, yp = mp & 0xFF;
         const float4 y1 = *reinterpret_cast<const float4*>(ys + swz_index<float, D>(p, 4 * c_own));
 #pragma unroll
         for (int pi = 0; pi < kCh; ++pi) {
+          if (pi >= passes) break;
           int x = xp - p_rx[pi], y = yp - p_ry[pi];
           x += x < 0 ? Lx : 0;
           y += y < 0 ? Ly : 0;
@@ -507,11 +515,19 @@ __global__ void __launch_bounds__(kVjpThreads, 1) pairing_vjp_kernel(VjpArgs a) 
           }
         }
       };
-      // rows of one spin in turn (the modes ascend, so there is one run of each)
+      // rows of one spin in turn (the modes ascend, so there is one run of each); a run's end is found
+      // by ballots, as a chain of n loads would be a good part of a small matrix's time
       for (int p = 0; p < n;) {
         const int sp = modes[p] >> 16;
-        int end = p + 1;
-        while (end < n && (modes[end] >> 16) == sp) ++end;
+        int end = n;
+        for (int b = p; b < n; b += 32) {
+          const bool other = b + lane < n && (modes[b + lane] >> 16) != sp;
+          const unsigned m = __ballot_sync(0xffffffffu, other);
+          if (m) {
+            end = b + __ffs(m) - 1;
+            break;
+          }
+        }
         if (sp) {
 #pragma unroll 2
           for (; p < end; ++p) add_row(p, acc1);
