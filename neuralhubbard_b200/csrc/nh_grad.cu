@@ -657,15 +657,15 @@ int launch_vjp_t(const VjpArgs& a, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------------ CNN VJP
-constexpr int kCvThreads = 512;
+constexpr size_t kCvTwoCtaSmem = 113 * 1024;
 
 // One periodic 3x3 cross-correlation of cin planes (stride N + 1) into cout planes, weights
 // [ci][tap][co] in shared memory, no bias; epi(co, site, z) stores the result.
-template <typename Epi>
+template <int TH, typename Epi>
 __device__ __forceinline__ void conv_planes(const float* in, int cin, int cout, const float* wsm,
                                             int Lx, int Ly, Epi epi) {
   const int part = Lx * Ly / 2;
-  for (int task = threadIdx.x; task < (cout / 8) * part; task += kCvThreads) {
+  for (int task = threadIdx.x; task < (cout / 8) * part; task += TH) {
     const int grp = task / part;
     const int site[2] = {task - grp * part, task - grp * part + part};
     float acc[2][8];
@@ -700,7 +700,8 @@ struct CnnVjpArgs {
 
 // Shared memory: z planes of layers 0 .. L-2 ((L-1) C NS), the input image (2 NS), two cotangent /
 // activation buffers (2 C NS) and one layer's weights (C C 9).
-__global__ void __launch_bounds__(kCvThreads) cnn_vjp_kernel(CnnVjpArgs a) {
+template <int TH>
+__global__ void __launch_bounds__(TH) cnn_vjp_kernel(CnnVjpArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int Lx = a.Lx, Ly = a.Ly, N = Lx * Ly, NS = N + 1, C = a.C, L = a.layers, d = C / 2;
   const int tid = threadIdx.x;
@@ -717,7 +718,7 @@ __global__ void __launch_bounds__(kCvThreads) cnn_vjp_kernel(CnnVjpArgs a) {
       const size_t item = (size_t)smp * a.n_img + g;
       const int sym = a.n_img == 1 ? 0 : g;
       __syncthreads();
-      for (int m = tid; m < 2 * N; m += kCvThreads) {
+      for (int m = tid; m < 2 * N; m += TH) {
         const int src = sym_map(m, sym, Lx, Ly, N);
         const int ch = m >= N ? 1 : 0;
         img[ch * NS + (m - ch * N)] = base[src] > 0 ? 1.0f : -1.0f;
@@ -728,14 +729,14 @@ __global__ void __launch_bounds__(kCvThreads) cnn_vjp_kernel(CnnVjpArgs a) {
       size_t woff = 0;
       for (int l = 0; l < L - 1; ++l) {
         __syncthreads();
-        stage_floats<kCvThreads>(wsm, a.conv_w_packed + woff, C * cin * 9);
+        stage_floats<TH>(wsm, a.conv_w_packed + woff, C * cin * 9);
         __syncthreads();
         float* z = zs + (size_t)l * C * NS;
         const float* bl = a.conv_b + l * C;
-        conv_planes(in, cin, C, wsm, Lx, Ly,
+        conv_planes<TH>(in, cin, C, wsm, Lx, Ly,
                     [&](int co, int s, float v) { z[co * NS + s] = v + __ldg(bl + co); });
         __syncthreads();
-        for (int e = tid; e < C * N; e += kCvThreads) {
+        for (int e = tid; e < C * N; e += TH) {
           const int co = e / N, s = e - co * N;
           bufA[co * NS + s] = gelu_tanh_dev(z[co * NS + s]);
         }
@@ -747,11 +748,11 @@ __global__ void __launch_bounds__(kCvThreads) cnn_vjp_kernel(CnnVjpArgs a) {
       __syncthreads();
       float* dcur = bufB;
       float* dother = bufA;
-      for (int e = tid; e < C * NS; e += kCvThreads) dcur[e] = 0.0f;
+      for (int e = tid; e < C * NS; e += TH) dcur[e] = 0.0f;
       __syncthreads();
       const float* dYi = a.dY + item * a.n * d;
       const int32_t* ii = a.idx + item * a.n;
-      for (int e = tid; e < a.n * d; e += kCvThreads) {
+      for (int e = tid; e < a.n * d; e += TH) {
         const int p = e / d, aa = e - p * d;
         const int m = __ldg(ii + p);
         const int sg = m >= N ? 1 : 0;
@@ -770,7 +771,7 @@ __global__ void __launch_bounds__(kCvThreads) cnn_vjp_kernel(CnnVjpArgs a) {
         const float* ain = img;
         if (l > 0) {
           const float* z = zs + (size_t)(l - 1) * C * NS;
-          for (int e = tid; e < C * N; e += kCvThreads) {
+          for (int e = tid; e < C * N; e += TH) {
             const int ci = e / N, s = e - ci * N;
             dother[ci * NS + s] = gelu_tanh_dev(z[ci * NS + s]);
           }
@@ -782,9 +783,9 @@ __global__ void __launch_bounds__(kCvThreads) cnn_vjp_kernel(CnnVjpArgs a) {
         // are split, and the shares are summed in shared memory (the weights' place, not in use).
         const int pairs = (C / 4) * lcin;
         int split = 1;
-        while (2 * split * pairs <= kCvThreads && 2 * split <= Lx && (2 * split - 1) * pairs * 36 <= C * C * 9)
+        while (2 * split * pairs <= TH && 2 * split <= Lx && (2 * split - 1) * pairs * 36 <= C * C * 9)
           split *= 2;
-        for (int t0 = 0; t0 < pairs * split; t0 += kCvThreads) {
+        for (int t0 = 0; t0 < pairs * split; t0 += TH) {
           const int task = t0 + tid, pr = task % pairs, share = task / pairs;
           const bool on = task < pairs * split;
           const int ci = pr % lcin, cob = pr / lcin;
@@ -848,7 +849,7 @@ __global__ void __launch_bounds__(kCvThreads) cnn_vjp_kernel(CnnVjpArgs a) {
         // Bias cotangent: warp per output channel.
         {
           const int lane = tid & 31, warp = tid >> 5;
-          for (int co = warp; co < C; co += kCvThreads / 32) {
+          for (int co = warp; co < C; co += TH / 32) {
             float s = 0.0f;
             for (int e = lane; e < N; e += 32) s += dcur[co * NS + e];
 #pragma unroll
@@ -862,7 +863,7 @@ __global__ void __launch_bounds__(kCvThreads) cnn_vjp_kernel(CnnVjpArgs a) {
         if (l == 0) break;
         // Input cotangent: transposed convolution with flipped taps, times GELU'(z_{l-1}).
         __syncthreads();
-        for (int i = tid; i < C * C * 9; i += kCvThreads) {
+        for (int i = tid; i < C * C * 9; i += TH) {
           const int cj = i % C;        // output channel of the transposed conv = layer input ci
           const int rest = i / C;      // co * 9 + tap'
           const int co = rest / 9, tp = rest - co * 9;
@@ -870,7 +871,7 @@ __global__ void __launch_bounds__(kCvThreads) cnn_vjp_kernel(CnnVjpArgs a) {
         }
         __syncthreads();
         const float* z = zs + (size_t)(l - 1) * C * NS;
-        conv_planes(dcur, C, C, wsm, Lx, Ly, [&](int ci, int s, float v) {
+        conv_planes<TH>(dcur, C, C, wsm, Lx, Ly, [&](int ci, int s, float v) {
           dother[ci * NS + s] = v * gelu_tanh_grad_dev(z[ci * NS + s]);
         });
         float* t = dcur;
@@ -885,6 +886,22 @@ size_t cnn_vjp_smem(int N, int C, int L) {
   const size_t NS = (size_t)N + 1;
   return sizeof(float) * ((size_t)(L - 1) * C * NS + ((2 * NS + 3) & ~(size_t)3) +
                           2 * (size_t)C * NS + (size_t)C * C * 9);
+}
+
+template <int TH>
+int launch_cnn_vjp_th(const CnnVjpArgs& a, size_t smem, cudaStream_t st) {
+  static size_t configured = 0;
+  if (smem > 48 * 1024 && smem > configured) {
+    cudaError_t e = cudaFuncSetAttribute(cnn_vjp_kernel<TH>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return check_cuda(e, "cnn vjp smem attribute");
+    configured = smem;
+  }
+  int grid = num_sms() * (smem <= kCvTwoCtaSmem ? 2 : 1);
+  if (grid > a.samples) grid = a.samples;
+  ProfScope prof_scope(NH_K_CNN_VJP, st);
+  cnn_vjp_kernel<TH><<<grid, TH, smem, st>>>(a);
+  return check_launch("cnn_vjp_kernel");
 }
 
 }  // namespace
@@ -932,20 +949,14 @@ int launch_cnn_vjp(const int8_t* spins, int samples, int n_img, const nh_backflo
   if (smem > 227 * 1024)
     return fail(NH_ERR_UNSUPPORTED, "cnn vjp: N = %d, %d channels, %d layers need %zu B", N, C,
                 p.layers, smem);
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    cudaError_t e = cudaFuncSetAttribute(cnn_vjp_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return check_cuda(e, "cnn vjp smem attribute");
-    configured = smem;
-  }
-  int grid = num_sms() * (smem <= 113 * 1024 ? 2 : 1);
-  if (grid > samples) grid = samples;
   CnnVjpArgs a{spins, samples, n_img, p.conv_w, p.conv_w_packed, p.conv_b, p.Lx, p.Ly, C,
                p.layers, p.n_up + p.n_dn, dY, idx, jac, ld};
-  ProfScope prof_scope(NH_K_CNN_VJP, st);
-  cnn_vjp_kernel<<<grid, kCvThreads, smem, st>>>(a);
-  return check_launch("cnn_vjp_kernel");
+  // 512 threads leave room for one CTA per SM (registers), so with more samples than SMs two CTAs of
+  // 256 that shared memory holds are faster: 250 bare samples, 4 layers of 32 channels, whole call:
+  // 3x4 278 -> 232 us, 4x4 322 -> 276, 8x8 487 -> 453, 10x10 721 -> 696; with at most a sample per SM
+  // 512 win (148 samples: 192 against 203, 228 / 243, 331 / 347, 471 / 490).
+  const bool two = smem <= kCvTwoCtaSmem && samples > num_sms();
+  return two ? launch_cnn_vjp_th<256>(a, smem, st) : launch_cnn_vjp_th<512>(a, smem, st);
 }
 
 bool cnn_vjp_supported(const nh_backflow_params& p) {

@@ -63,3 +63,20 @@ def test_jacobian_rectangular(Lx, Ly, up, dn, channels, layers):
     J0 = og.log_jacobian(s, op, symm=False)[2]
     err = np.max(np.abs(J.cpu().numpy() - J0), axis=1) / np.max(np.abs(J0), axis=1)
     assert np.all(err <= 2e-6 * cond + 1e-5), (err, cond)
+
+
+@pytest.mark.parametrize("Lx,Ly,up,dn,channels", [(4, 4, 5, 5, 32), (5, 6, 12, 12, 16),
+                                                  (10, 11, 40, 40, 32), (10, 12, 40, 40, 32)])
+def test_jacobian_many_samples(Lx, Ly, up, dn, channels):
+    """More samples than SMs take the 256-thread form of the CNN cotangents where two CTAs fit (up to
+    10x11): its rows against those of the 512-thread form, which sum the lattice's rows in another
+    split.  FP32 sums of N terms: N eps of the row's largest entry, times ten for the layers."""
+    N = Lx * Ly
+    p = nh.init_params(Lx, Ly, channels=channels, layers=4, std=0.2, seed=N)
+    state = nh.Variational(nh.PfaffianBackflow(Lx, Ly, up, dn, params=p), symm=False)
+    s = olat.random_configs(np.random.default_rng(N), 30, N, up, dn)
+    few = state.jacobian(s)[1].cpu().numpy()
+    many = state.jacobian(np.tile(s, (20, 1)))[1].cpu().numpy()
+    scale = np.max(np.abs(few), axis=1, keepdims=True)
+    assert np.array_equal(many, np.tile(many[:30], (20, 1)))
+    assert np.max(np.abs(many[:30] - few) / scale) <= 10 * N * np.finfo(np.float32).eps
