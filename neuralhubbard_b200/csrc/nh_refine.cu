@@ -893,12 +893,15 @@ int launch_refine_k(const RefineArgs& a, int max_slots, size_t smem, cudaStream_
 }
 
 // Two CTAs of 256 threads per SM where shared memory holds both and there are items for them (small
-// lattices, whose phases are latency-bound), else one of 512.
+// lattices, whose phases are latency-bound), else one of 512.  In-kernel features on the matrix
+// instruction need 512 threads beyond 128 sites; the scalar network (16 channels) runs with either:
+// 290 bare images, whole call, 4x4 159 -> 118 us, 8x8 200 -> 159, 12x14 361 -> 320.
 constexpr size_t kTwoCtaSmem = 111 * 1024;  // dynamic, beside the static arrays
 
 template <int D, int MODE>
 int launch_refine_m(RefineArgs a, int max_slots, cudaStream_t st) {
-  const bool small = MODE != 4 || cnn_mma_fits(a.Lx, a.Ly, a.C, 256);
+  const bool small = MODE != 4 || cnn_mma_fits(a.Lx, a.Ly, a.C, 256) ||
+                     !cnn_mma_fits(a.Lx, a.Ly, a.C, 512);
   const size_t s256 = refine_smem<D>(a, 256);
   if (small && s256 && s256 <= kTwoCtaSmem && max_slots > num_sms())
     return launch_refine_k<D, MODE, 256>(a, max_slots, s256, st);
