@@ -2304,6 +2304,9 @@ int launch_fused_nb(PfArgs a, cudaStream_t st) {
     a.idx_off = (int)idsB;
     a.tail_row = tail;
   }
+  if (smem > 227 * 1024)
+    return fail(NH_ERR_UNSUPPORTED, "fused amplitude: n=%d, N=%d needs %zu B of shared memory", n,
+                N, smem);
   if (a.queue) {
     cudaError_t e = cudaMemsetAsync(a.queue, 0, sizeof(int32_t), st);
     if (e != cudaSuccess) return check_cuda(e, "fused amplitude: clear work counter");

@@ -849,7 +849,8 @@ size_t stage_bytes(int n, int N, int D, int elt, bool wt) {
   return (size_t)elt * n * DP + sizeof(int) * ((n + 3) & ~3) + (wt ? (size_t)elt * 4 * N * DP : 0);
 }
 
-// Shared memory of one launch with TH threads (modes 2, 4: and the staging offsets); 0: too large.
+// Shared memory of one launch with TH threads (modes 2, 4: and the staging offsets, where it is at most
+// kRefineSmemLimit).
 template <int D>
 size_t refine_smem(RefineArgs& a, int TH) {
   const int N = a.Lx * a.Ly, n = a.n, T = tile_rows(n);
@@ -862,7 +863,7 @@ size_t refine_smem(RefineArgs& a, int TH) {
   } else if (a.mode != 0) {
     const size_t y = 8 * (size_t)n * D, inf = (4 * (size_t)n + 15) & ~(size_t)15, wt = 8 * (size_t)N * D;
     const size_t feat = a.mode == 4 ? (features_smem(a.Lx, a.Ly, a.C, 8, TH) + 15) & ~(size_t)15 : 0;
-    if (feat > kRefineSmemLimit) return 0;
+    if (feat > kRefineSmemLimit) return feat;
     a.rows_slice = feat + y + inf > kRefineSmemLimit;
     smem = std::max(smem, a.rows_slice ? std::max(feat, y + inf) : feat + y + inf);
     // One spin block of the table above the tiles' first rows, where it fits at all.
@@ -875,7 +876,7 @@ size_t refine_smem(RefineArgs& a, int TH) {
     a.keep = T;
     while (a.keep > 0 && tile_bytes(a.keep) > (size_t)a.wt_off) --a.keep;
   }
-  return smem <= kRefineSmemLimit ? smem : 0;
+  return smem;
 }
 
 template <int D, int MODE, int TH>
@@ -903,11 +904,11 @@ int launch_refine_m(RefineArgs a, int max_slots, cudaStream_t st) {
   const bool small = MODE != 4 || cnn_mma_fits(a.Lx, a.Ly, a.C, 256) ||
                      !cnn_mma_fits(a.Lx, a.Ly, a.C, 512);
   const size_t s256 = refine_smem<D>(a, 256);
-  if (small && s256 && s256 <= kTwoCtaSmem && max_slots > num_sms())
+  if (small && s256 <= kTwoCtaSmem && max_slots > num_sms())
     return launch_refine_k<D, MODE, 256>(a, max_slots, s256, st);
   const size_t s512 = refine_smem<D>(a, 512);
-  if (!s512)
-    return fail(NH_ERR_UNSUPPORTED, "refine: n=%d does not fit in shared memory", a.n);
+  if (s512 > kRefineSmemLimit)
+    return fail(NH_ERR_UNSUPPORTED, "refine: n=%d needs %zu B of shared memory", a.n, s512);
   return launch_refine_k<D, MODE, 512>(a, max_slots, s512, st);
 }
 
@@ -963,7 +964,8 @@ size_t refine_slice_bytes(int n, int d) {
 int launch_refine(const RefineLaunch& q, cudaStream_t st) {
   const bool big = q.n > kRefineMaxN;  // stored FP64 rows only, tiles in q.slice (refine_big_bytes)
   if (q.n <= 0 || q.n % 2 || q.n > (q.mode == 2 ? kMaxN : kRefineMaxN))
-    return fail(NH_ERR_UNSUPPORTED, "refine: n=%d (even, <= %d)", q.n, kRefineMaxN);
+    return fail(NH_ERR_UNSUPPORTED, "refine: n=%d (even, <= %d)", q.n,
+                q.mode == 2 ? kMaxN : kRefineMaxN);
   if (q.max_slots <= 0) return NH_OK;
   if (q.mode < 0 || q.mode > 4) return fail(NH_ERR_INVALID, "refine: mode %d", q.mode);
   if (q.mode != 0 && !q.slice) return fail(NH_ERR_INVALID, "refine: gather mode needs the slice");

@@ -91,3 +91,13 @@ def test_in_kernel_features(channels, Lx, Ly, up, dn, refine_tau):
 @pytest.mark.parametrize("refine_tau", [0.0, 1.0])
 def test_stored_features(Lx, Ly, up, dn, refine_tau):
     check_forms(32, Lx, Ly, up, dn, refine_tau, 1)
+
+
+@pytest.mark.parametrize("channels,Lx,Ly,ne,kw,message", [
+    (64, 6, 8, 20, dict(cond_tau=1.0), r"refine: n=40 needs \d+ B"),
+    (32, 32, 32, 4, {}, r"fused amplitude: n=8, N=1024 needs \d+ B")])
+def test_refusals_say_what_is_needed(channels, Lx, Ly, ne, kw, message):
+    p = nh.init_params(Lx, Ly, channels=channels, layers=4, std=0.1, seed=1)
+    s = olat.random_configs(np.random.default_rng(1), 2, Lx * Ly, ne, ne)
+    with pytest.raises(nh.NativeLibraryError, match=message):
+        nh.Variational(nh.PfaffianBackflow(Lx, Ly, ne, ne, params=p, **kw))(s)
