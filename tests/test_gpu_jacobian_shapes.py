@@ -13,6 +13,7 @@ import pytest
 import torch
 
 import neuralhubbard_b200 as nh
+from neuralhubbard_b200 import _lib
 from oracle import backflow as obf
 from oracle import gradient as og
 from oracle import lattice as olat
@@ -80,3 +81,27 @@ def test_jacobian_many_samples(Lx, Ly, up, dn, channels):
     scale = np.max(np.abs(few), axis=1, keepdims=True)
     assert np.array_equal(many, np.tile(many[:30], (20, 1)))
     assert np.max(np.abs(many[:30] - few) / scale) <= 10 * N * np.finfo(np.float32).eps
+
+
+@pytest.mark.parametrize("n", [8, 20, 64, 100, 222, 224])
+def test_adjoint_ties_and_nonfinite(n):
+    """Matrices with +-1 everywhere (the pivot searches tie) against the oracle, beside a zero, an
+    infinite and a NaN entry's matrix, which are flagged and leave the others' bits alone."""
+    rng = np.random.default_rng(n)
+    U = np.triu(rng.choice([-1.0, 1.0], size=(5, n, n)), 1)
+    A = (U - np.swapaxes(U, 1, 2)).astype(np.float32)
+    A[2] = 0.0
+    A[3, n - 1, 0], A[3, 0, n - 1] = np.inf, -np.inf
+    A[4, n // 2, 1], A[4, 1, n // 2] = np.nan, np.nan
+    G, fl = nh.slogpf_adjoint(torch.from_numpy(A).to(DEV))
+    alone, _ = nh.slogpf_adjoint(torch.from_numpy(A[:2]).to(DEV))
+    assert torch.equal(G[:2], alone)
+    fl = fl.cpu().numpy()
+    assert np.all(fl[:2] == 0) and fl[2] == _lib.FLAG_ZERO_PIVOT
+    assert np.all(fl[3:] == _lib.FLAG_NONFINITE)
+    assert torch.all(G[2] == 0.0)
+    G0 = og.slogpf_adjoint(A[:2].astype(np.float64))
+    cond = np.linalg.cond(A[:2].astype(np.float64))
+    for b in range(2):
+        scale = np.max(np.abs(G0[b]))
+        assert np.max(np.abs(G[b].cpu().numpy() - G0[b])) <= (2e-6 * cond[b] + 1e-6) * scale
