@@ -285,6 +285,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) cnn_tc_kernel(TcArgs a) {
           rowof[m] = -1;
         }
       }
+      if (total == 0 && ltid == 0) occl[0] = 0;  // no electron: every row reads mode 0
       wg_sync(wg);
       if (ltid == 0) wbuf[0] = total;
     }
