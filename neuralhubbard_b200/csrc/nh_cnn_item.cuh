@@ -23,12 +23,6 @@ __device__ __forceinline__ double gelu_tanh_dev(double x) {
   return 0.5 * x * (1.0 + tanh(k0 * (x + 0.044715 * x * x * x)));
 }
 
-__device__ __forceinline__ void cnn_lds8(const float* p, float* o) {
-  const float4 a = reinterpret_cast<const float4*>(p)[0];
-  const float4 b = reinterpret_cast<const float4*>(p)[1];
-  o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
-  o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
-}
 __device__ __forceinline__ void cnn_lds8(const double* p, double* o) {
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
@@ -131,26 +125,26 @@ __device__ __forceinline__ void conv_task(const T* in, int cin, int cout, const 
     for (int k = 0; k < S; ++k)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        acc[k][2 * j] = __uint_as_float((unsigned)a2[k][j]);
-        acc[k][2 * j + 1] = __uint_as_float((unsigned)(a2[k][j] >> 32));
+        acc[k][2 * j] = lo2(a2[k][j]);
+        acc[k][2 * j + 1] = hi2(a2[k][j]);
       }
-    return;
-  }
+  } else {
 #pragma unroll 1
-  for (int ci = 0; ci < cin; ++ci) {
-    const T* inc = in + ci * NS;
-    const T* wc = wsm + ci * 9 * cout + grp * 8;
+    for (int ci = 0; ci < cin; ++ci) {
+      const T* inc = in + ci * NS;
+      const T* wc = wsm + ci * 9 * cout + grp * 8;
 #pragma unroll
-    for (int u = 0; u < 3; ++u) {
+      for (int u = 0; u < 3; ++u) {
 #pragma unroll
-      for (int v = 0; v < 3; ++v) {
-        T w8[8];
-        cnn_lds8(wc + (u * 3 + v) * cout, w8);
+        for (int v = 0; v < 3; ++v) {
+          T w8[8];
+          cnn_lds8(wc + (u * 3 + v) * cout, w8);
 #pragma unroll
-        for (int k = 0; k < S; ++k) {
-          const T i0 = inc[row[k][u] + col[k][v]];
+          for (int k = 0; k < S; ++k) {
+            const T i0 = inc[row[k][u] + col[k][v]];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) acc[k][j] = fma(i0, w8[j], acc[k][j]);
+            for (int j = 0; j < 8; ++j) acc[k][j] = fma(i0, w8[j], acc[k][j]);
+          }
         }
       }
     }
@@ -215,12 +209,16 @@ __device__ T* cnn_layers(const float* __restrict__ wp, const float* __restrict__
             out[(grp * 8 + j) * NS + site[k]] = act_fn ? gelu_tanh_dev(acc[k][j]) : acc[k][j];
       }
     };
-    if (sizeof(T) == 4 && conv_four_sites(N, C, TH))
-      tasks(Sites<4>{});
-    else if (sizeof(T) == 4 && ngroups * N <= TH)  // small lattices: every thread a task
-      tasks(Sites<1>{});
-    else
+    if constexpr (sizeof(T) == 4) {
+      if (conv_four_sites(N, C, TH))
+        tasks(Sites<4>{});
+      else if (ngroups * N <= TH)  // small lattices: every thread a task
+        tasks(Sites<1>{});
+      else
+        tasks(Sites<2>{});
+    } else {
       tasks(Sites<2>{});
+    }
     wl += C * cin * 9;
     cin = C;
     T* t = in;

@@ -128,7 +128,6 @@ __device__ __forceinline__ int pack_mode(int m, int N, int Ly) {
 __device__ __forceinline__ int tri_off(int i) { return (i * (i - 1)) >> 1; }
 
 // Pivot-search key of a magnitude: FP32, rounded up so that no non-zero value becomes zero.
-__device__ __forceinline__ float to_key_float(float x) { return x; }
 __device__ __forceinline__ float to_key_float(double x) { return __double2float_ru(x); }
 
 template <typename T>
@@ -414,7 +413,7 @@ __global__ void __launch_bounds__(THREADS, 1) pfaffian_kernel(PfArgs a) {
     __syncthreads();
 
     int my_log = tid < n ? tid : -1;
-    int flag = 0, swaps = 0;
+    int flag = 0;
     bool zero = false;
 
     for (int k0 = 0; k0 < n - 1 && !zero; k0 += 2 * NB) {
@@ -506,7 +505,6 @@ __global__ void __launch_bounds__(THREADS, 1) pfaffian_kernel(PfArgs a) {
             }
             if (my_log == k + 2) misc[0] = tid;
             if (tid == 0) pivs[k >> 1] = lr != k + 1 ? -piv : piv;
-            swaps ^= lr != k + 1 ? 1 : 0;
           }
           __syncthreads();  // (2) panel column written, next column's owner known
         }
@@ -608,7 +606,7 @@ __global__ void __launch_bounds__(THREADS, 1) pfaffian_kernel(PfArgs a) {
       // Pfaffian = relabelling parity x product of the pivots, accumulated in FP64 as mantissa
       // and exponent; the pivot ratio flags near-nodal blocks.
       float s = a.item_sign ? a.item_sign[item] : 1.0f;
-      double la, pmax_all = 0.0, pmin_all = 1.0;
+      double la;
       if (isnan(s)) flag |= NH_FLAG_NONFINITE;  // the CNN could not compute this item
       if (zero) {
         s = 0.0f;
@@ -619,7 +617,7 @@ __global__ void __launch_bounds__(THREADS, 1) pfaffian_kernel(PfArgs a) {
         int expo = 0;
         double pmin = INFINITY, pmax = 0.0;
         for (int k = 0; k < n / 2; ++k) {
-          const double pv = (double)pivs[k];
+          const double pv = pivs[k];
           if (pv < 0.0) s = -s;
           const double ap = fabs(pv);
           if (!isfinite(ap)) flag |= NH_FLAG_NONFINITE;
@@ -632,21 +630,11 @@ __global__ void __launch_bounds__(THREADS, 1) pfaffian_kernel(PfArgs a) {
         la = log(mant) + (double)expo * 0.6931471805599453;
         if (!isfinite(la)) flag |= NH_FLAG_NONFINITE;
         if (a.cond_tau > 0.0 && pmax > a.cond_tau * pmin) flag |= NH_FLAG_GROWTH;
-        if (a.refine_tau > 0.0 && pmax > a.refine_tau * pmin) flag |= kFlagNeedRefine;
-        pmax_all = pmax;
-        pmin_all = pmin;
       }
       if (s == 0.0f) la = -INFINITY;
       a.sign[item] = s;
       a.logabs[item] = la;
       if (a.flags) a.flags[item] = flag | a.flag_or;
-      if (a.ratio) a.ratio[item] = zero ? INFINITY : (float)(pmax_all / pmin_all);
-    }
-    // Pivot order for the FP64 refinement: every row's final logical label, and the parity.
-    if (a.perm && !zero) {
-      uint16_t* pr = a.perm + (size_t)item * perm_stride(n);
-      if (tid < n) pr[my_log] = (uint16_t)tid;
-      if (tid == 0) pr[n] = (uint16_t)swaps;
     }
   }
 }
@@ -2178,8 +2166,7 @@ int launch_pf_tc(const PfArgs& a, int32_t* err, cudaStream_t st) {
 bool pfaffian64_fits(int n) { return pf_smem<double, 2>(n) <= 227 * 1024; }
 
 bool pfaffian_needs_scratch(int n, bool fp64) {
-  if (n > kNumThreads) return true;
-  return fp64 ? pf_smem<double, 2>(n) > 227 * 1024 : pf_smem<float, 4>(n) > 227 * 1024;
+  return n > kNumThreads || (fp64 && !pfaffian64_fits(n));
 }
 
 size_t pfaffian_scratch_bytes(int n) {

@@ -89,54 +89,39 @@ struct RefineArgs {
   bool rows_slice;  // mode 4: no room for Y above the CNN, its rows pass through the slice
 };
 
-template <typename T>
-struct Vec2;
-template <>
-struct Vec2<float> {
-  static constexpr int k = 4;
-  using V = float4;
-};
-template <>
-struct Vec2<double> {
-  static constexpr int k = 2;
-  using V = double2;
-};
-
-// Phase 1 of modes 1 and 3: logical lower triangle A[p][q] = F[perm p][perm q] of one item into the CTA's slice
-// (element type T).  Warp <-> 32 consecutive logical columns q (their features in registers
+// Phase 1 of modes 1 and 3: logical lower triangle A[p][q] = F[perm p][perm q] of one item, FP32, into
+// the CTA's slice.  Warp <-> 32 consecutive logical columns q (their features in registers
 // when small), rows p > q in turn (the row's features broadcast); each element reads one Wt row.
-template <typename T, int D, int TH, int kRegBytes = 64>
-__device__ void gather_permuted(const RefineArgs& a, const T* Yg, const int32_t* ig,
-                                const uint16_t* perm, unsigned char* smem, T* slice) {
+template <int D, int TH>
+__device__ void gather_permuted(const RefineArgs& a, const float* Yg, const int32_t* ig,
+                                const uint16_t* perm, unsigned char* smem, float* slice) {
   const int n = a.n, N = a.Lx * a.Ly;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  constexpr int DP = D + (sizeof(T) == 4 ? 4 : 2);
-  constexpr int VK = Vec2<T>::k;
-  using V = typename Vec2<T>::V;
-  const T* Wg = static_cast<const T*>(a.Wt);
-  T* ys = reinterpret_cast<T*>(smem);                    // (n, DP)
-  int* info = reinterpret_cast<int*>(ys + n * DP);       // (n) spin << 16 | x << 8 | y
-  T* wts = reinterpret_cast<T*>(info + ((n + 3) & ~3));  // (4 N, DP) when staged
+  constexpr int DP = D + 4, VK = 4;
+  const float* Wg = static_cast<const float*>(a.Wt);
+  float* ys = reinterpret_cast<float*>(smem);                    // (n, DP)
+  int* info = reinterpret_cast<int*>(ys + n * DP);               // (n) spin << 16 | x << 8 | y
+  float* wts = reinterpret_cast<float*>(info + ((n + 3) & ~3));  // (4 N, DP) when staged
   // Row r of the source (D values, 16-byte vectors) to row r of the padded staging copy; several
   // vectors in flight per thread.  Read-only tables (nc) take the non-coherent path; the rows,
-  // which modes 3 and 4 write in this kernel, plain loads.
-  auto stage = [&](const T* src, T* dst, int rows, bool nc) {
+  // which mode 3 writes in this kernel, plain loads.
+  auto stage = [&](const float* src, float* dst, int rows, bool nc) {
     constexpr int VPR = D / VK;  // vectors per row
     const int nv = rows * VPR;
     for (int v0 = tid; v0 < nv; v0 += 4 * TH) {
-      V buf[4];
+      float4 buf[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int v = v0 + u * TH;
-        if (v < nv) buf[u] = nc ? __ldg(reinterpret_cast<const V*>(src) + v)
-                                : reinterpret_cast<const V*>(src)[v];
+        if (v < nv) buf[u] = nc ? __ldg(reinterpret_cast<const float4*>(src) + v)
+                                : reinterpret_cast<const float4*>(src)[v];
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int v = v0 + u * TH;
         if (v < nv) {
           const int r = v / VPR;
-          *reinterpret_cast<V*>(dst + r * DP + (v - r * VPR) * VK) = buf[u];
+          *reinterpret_cast<float4*>(dst + r * DP + (v - r * VPR) * VK) = buf[u];
         }
       }
     }
@@ -153,8 +138,8 @@ __device__ void gather_permuted(const RefineArgs& a, const T* Yg, const int32_t*
   for (int qb = 0; 32 * qb + 1 < n; ++qb) total += n - 32 * qb - 1;
   int qb = 0, rem = wid, cur = -1, j = 0, infj = 0;
   // The column's features stay in registers when they are small, else they are read per element.
-  constexpr bool kRegs = D * sizeof(T) <= kRegBytes;
-  T yj[kRegs ? D : 1];
+  constexpr bool kRegs = D <= 16;
+  float yj[kRegs ? D : 1];
 #pragma unroll 1
   for (int u = wid; u < total; u += (TH / 32), rem += (TH / 32)) {
     while (rem >= n - 32 * qb - 1) {
@@ -169,7 +154,7 @@ __device__ void gather_permuted(const RefineArgs& a, const T* Yg, const int32_t*
       if constexpr (kRegs) {
 #pragma unroll
         for (int c = 0; c < D; c += VK)
-          *reinterpret_cast<V*>(yj + c) = *reinterpret_cast<const V*>(ys + j * DP + c);
+          *reinterpret_cast<float4*>(yj + c) = *reinterpret_cast<const float4*>(ys + j * DP + c);
       }
     }
     const int p = 32 * qb + 1 + rem;
@@ -184,22 +169,22 @@ __device__ void gather_permuted(const RefineArgs& a, const T* Yg, const int32_t*
     const int r = (2 * (ih >> 16) + (il >> 16)) * N + dx * a.Ly + dy;
     // yi[c] * yj[c] equals the FP32 gather's row-times-column product bit for bit (the product
     // commutes); the accumulation order over c is the gather's.
-    const T* yi = ys + i * DP;
-    const T* wr = a.stage_wt ? wts + r * DP : Wg + (size_t)r * D;
-    T acc = T(0);
+    const float* yi = ys + i * DP;
+    const float* wr = a.stage_wt ? wts + r * DP : Wg + (size_t)r * D;
+    float acc = 0.0f;
 #pragma unroll
     for (int c = 0; c < D; c += VK) {
-      T vi[VK], vw[VK], vj[VK];
-      *reinterpret_cast<V*>(vi) = *reinterpret_cast<const V*>(yi + c);
+      float vi[VK], vw[VK], vj[VK];
+      *reinterpret_cast<float4*>(vi) = *reinterpret_cast<const float4*>(yi + c);
       if (a.stage_wt)
-        *reinterpret_cast<V*>(vw) = *reinterpret_cast<const V*>(wr + c);
+        *reinterpret_cast<float4*>(vw) = *reinterpret_cast<const float4*>(wr + c);
       else
-        *reinterpret_cast<V*>(vw) = __ldg(reinterpret_cast<const V*>(wr + c));
+        *reinterpret_cast<float4*>(vw) = __ldg(reinterpret_cast<const float4*>(wr + c));
       if constexpr (kRegs) {
 #pragma unroll
         for (int k = 0; k < VK; ++k) vj[k] = yj[c + k];
       } else {
-        *reinterpret_cast<V*>(vj) = *reinterpret_cast<const V*>(ys + j * DP + c);
+        *reinterpret_cast<float4*>(vj) = *reinterpret_cast<const float4*>(ys + j * DP + c);
       }
 #pragma unroll
       for (int k = 0; k < VK; ++k) acc = fma(vi[k] * vj[k], vw[k], acc);
@@ -573,7 +558,7 @@ __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArg
         Yg = sl;
         ig = reinterpret_cast<const int32_t*>(sl + n * D);
       }
-      gather_permuted<float, D, TH>(a, Yg, ig, perm_s, smem, sl);
+      gather_permuted<D, TH>(a, Yg, ig, perm_s, smem, sl);
       __syncthreads();  // slice written; the staging area is dead
       for (int p = wid; p < n; p += WARPS)
         for (int q = lane; q < p; q += 32)

@@ -126,9 +126,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
 __device__ __forceinline__ uint16_t bf16_bits(float x) {
   return __bfloat16_as_ushort(__float2bfloat16_rn(x));
 }
-__device__ __forceinline__ float bf16_val(uint16_t b) {
-  return __bfloat162float(__ushort_as_bfloat16(b));
-}
 
 // Byte offset of padded position (X, Y) inside a plane.
 __device__ __forceinline__ int pad_off(int X, int Y) { return (X * kP + Y) * 16; }
