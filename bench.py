@@ -413,7 +413,7 @@ def measure_local_energy(args, dev, st) -> dict:
         del graph, e, state, model
         torch.cuda.empty_cache()
     out["setup"] = ("4096 uniformly random configurations at 8x8 and 16x16, 256 at 24x24 (n = "
-                    "504, large-lattice path: 40 ms of amplitudes per sample), unprojected "
+                    "504, large-lattice path: 65 ms of amplitudes per sample), unprojected "
                     "amplitudes, t = 1, t' = -0.2, U = 8; one CUDA-graph replay of the whole call")
     return out
 
@@ -690,7 +690,7 @@ def measure_large(args, dev, st, q) -> dict:
     e1.record(st)
     torch.cuda.synchronize()
     out["amplitudes_per_s"] = 512 * IMAGES / (e0.elapsed_time(e1) / 1e3)
-    out["note"] = ("tau_int is not measured at 32x32 within the bench (about 2.4 s per step with "
+    out["note"] = ("tau_int is not measured at 32x32 within the bench (about 0.85 s per step with "
                    "4096 chains); the proposal is trained at 16x16 (its backward kernel holds "
                    "the activations of up to 559 sites in shared memory) and transferred")
     return out

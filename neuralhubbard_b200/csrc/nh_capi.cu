@@ -899,8 +899,8 @@ int nh_pairing_occ_vjp(const float* Y, const int32_t* idx, const float* Wt, cons
     return fail(NH_ERR_INVALID, "pairing_occ_vjp: bad arguments");
   if (Lx < 1 || Ly < 1 || 2 * Lx * Ly > 512 || n > kGradMaxN)
     return fail(NH_ERR_UNSUPPORTED, "pairing_occ_vjp: lattice %dx%d, n = %d", Lx, Ly, n);
-  return launch_pairing_vjp(G, Y, idx, Wt, nullptr, Lx, Ly, d, n, 1, batch, dY, dWt, nullptr, 0, 0, 0.0f,
-                            static_cast<cudaStream_t>(stream));
+  return launch_pairing_vjp(G, Y, idx, Wt, nullptr, Lx, Ly, d, n, 1, batch, dY, dWt, nullptr, 0, 0,
+                            0.0f, static_cast<cudaStream_t>(stream));
 }
 
 int64_t nh_param_count(const nh_backflow_params* p) {
@@ -967,8 +967,8 @@ int nh_log_jacobian(const int8_t* spins, int batch, int n_symm, const nh_backflo
       return rc;
     float* jrow = jac + (size_t)c0 * P;
     // run_pipeline's staged Pfaffian (n <= 224, FP32) left the table in chunks
-    if ((rc = launch_pairing_vjp(Fbuf, b.Y, b.idx, q.Wt, b.wt_chunks, q.Lx, q.Ly, d, n, n_symm, m, dYbuf,
-                                 nullptr, jrow, P, off_w, theta, st)))
+    if ((rc = launch_pairing_vjp(Fbuf, b.Y, b.idx, q.Wt, b.wt_chunks, q.Lx, q.Ly, d, n, n_symm, m,
+                                 dYbuf, nullptr, jrow, P, off_w, theta, st)))
       return rc;
     if ((rc = launch_cnn_vjp(sp, m, n_symm, q, dYbuf, b.idx, jrow, P, st))) return rc;
   }

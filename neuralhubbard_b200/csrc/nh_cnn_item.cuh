@@ -1,5 +1,5 @@
-// The backflow CNN of one item (configuration x symmetry image) by one 256-thread block: the
-// device function behind cnn_kernel (nh_cnn.cu) and the fused kernels that compute an item's
+// The backflow CNN of one item (configuration x symmetry image) by one block of 128 to 512 threads:
+// the device function behind cnn_kernel (nh_cnn.cu) and the fused kernels that compute an item's
 // features and consume them in the same block (the amplitude/Pfaffian kernel of the persistent
 // local energy, nh_pfaffian.cu, and the FP64 refinement, nh_refine.cu).
 //
@@ -71,10 +71,10 @@ struct Sites {
   static constexpr int value = S;
 };
 
-// One task of a periodic 3x3 cross-correlation: S sites x 8 output channels (group grp of cout / 8) of
-// cin planes of stride N + 1, weights [ci][tap][co] in shared memory, accumulated in order of
-// (ci, tap) onto acc.  With four sites a thread issues 32 FMAs (16 packed) per 4 loads of inputs and
-// two broadcast 16-byte weight loads (two cycles of the load port each).
+// One task of a periodic 3x3 cross-correlation: S sites x 8 output channels (group grp of cout / 8)
+// of cin planes of stride N + 1, weights [ci][tap][co] in shared memory, accumulated in order of
+// (ci, tap) onto acc.  With four sites a thread issues 32 FMAs (16 packed) per 4 loads of inputs
+// and two broadcast 16-byte weight loads (two cycles of the load port each).
 template <typename T, int S>
 __device__ __forceinline__ void conv_task(const T* in, int cin, int cout, const T* wsm, int grp,
                                           const int (&site)[S], int Lx, int Ly, T (&acc)[S][8]) {

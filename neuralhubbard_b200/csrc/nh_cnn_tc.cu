@@ -1,7 +1,7 @@
 // Backflow CNN forward on the 5th-generation tensor cores (tcgen05, sm_100a): the chosen form.
 //
-// The 3x3 periodic convolutions run as implicit GEMMs D[site, co] += A[site + tap, ci] W[tap][ci, co]
-// with BF16 operands in shared memory and FP32 accumulators in tensor memory.  The activations
+// The 3x3 periodic convolutions run as implicit GEMMs D[site, co] += A[site + tap, ci] W[tap][ci,
+// co] with BF16 operands in shared memory and FP32 accumulators in tensor memory.  The activations
 // of one configuration live in a padded plane: site (x, y) sits at padded position
 // (x + 1, y + 1) of an (Lx + 2) x (Ly + 2) grid whose border repeats the periodic neighbours, and
 // each padded site holds 8 channels in 16 bytes ("core-matrix rows"), one plane per group of 8
@@ -16,16 +16,16 @@
 // in FP32 in the epilogue, which reads the accumulators with tcgen05.ld (warp w % 4 owns lanes
 // 32 (w % 4) .. + 31).
 //
-// Two warp groups of 256 threads, one site per thread (warps 0-3 of a group: tile 0), run independent image streams in one CTA: each has its own
-// activation planes, bookkeeping, mbarrier, 256 tensor-memory columns (four partial sums of its
-// two 128 x 32 tiles, see issue_layer) and named barrier, and
-// shares the resident weights; while one group's MMAs run, the other converts its accumulators
-// (bias, GELU, hi/lo split) and writes its next planes.
+// Two warp groups of 256 threads, one site per thread (warps 0-3 of a group: tile 0), run
+// independent image streams in one CTA: each has its own activation planes, bookkeeping, mbarrier,
+// 256 tensor-memory columns (four partial sums of its two 128 x 32 tiles, see issue_layer) and named
+// barrier, and shares the resident weights; while one group's MMAs run, the other converts its
+// accumulators (bias, GELU, hi/lo split) and writes its next planes.
 //
-// What bounds it: the MMAs' operand reads (72 MMAs of 89 / 2 cycles per layer and image, 12.8K
-// cycles an image) beside the epilogues' instructions; two images are in flight to overlap them.
-// 65,536 images: 7.4 ms with 128 threads per group and three MMAs per product, 5.7 without, 5.3 with
-// the BF16 conversions in pairs.
+// What bounds it: the MMAs' operand reads (an image's layers 1 to 3 issue 72 MMAs of 89 / 2 cycles
+// each, layer 0 18 of 49: 10.5K of the 23.7K cycles that an image takes) beside the epilogues'
+// instructions; two images are in flight to overlap them.  65,536 images: 7.4 ms with 128 threads
+// per group and three MMAs per product, 5.7 without, 5.3 with the BF16 conversions in pairs.
 //
 // Output: the occupied rows Y (n, d) FP32 of the image configuration, the occupied-mode list and
 // the item sign, like the CUDA-core kernel (mode 1 of nh_cnn.cu).

@@ -494,9 +494,9 @@ int launch_pf_adjoint(const float* F, float* G, int n, int batch, const float* p
 // jac[sample * ld + off_w + (3 N d W values, theta)].  wt_chunks: Wt in chunks of four a
 // (launch_pfaffian_staged leaves it in its buffer), or null.
 int launch_pairing_vjp(const float* G, const float* Y, const int32_t* idx, const float* Wt,
-                       const float* wt_chunks, int Lx, int Ly, int d, int n, int n_img, int samples, float* dY,
-                       float* dWt, float* jac, int64_t ld, int64_t off_w, float theta,
-                       cudaStream_t st);
+                       const float* wt_chunks, int Lx, int Ly, int d, int n, int n_img,
+                       int samples, float* dY, float* dWt, float* jac, int64_t ld, int64_t off_w,
+                       float theta, cudaStream_t st);
 // Convolution weight and bias cotangents of every sample's images, summed into jac[sample * ld].
 int launch_cnn_vjp(const int8_t* spins, int samples, int n_img, const nh_backflow_params& p,
                    const float* dY, const int32_t* idx, float* jac, int64_t ld, cudaStream_t st);

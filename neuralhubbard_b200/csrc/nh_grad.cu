@@ -469,7 +469,8 @@ __global__ void __launch_bounds__(kVjpThreads, 1) pairing_vjp_kernel(VjpArgs a) 
             dx += dx < 0 ? Lx : 0;
             dy += dy < 0 ? Ly : 0;
             const int row = (2 * sp + sq) * N + dx * Ly + dy;
-            const float4* w4 = a.Wc ? a.Wc + row : reinterpret_cast<const float4*>(a.Wt) + row * (D / 4);
+            const float4* w4 =
+                a.Wc ? a.Wc + row : reinterpret_cast<const float4*>(a.Wt) + row * (D / 4);
             const int stride = a.Wc ? 4 * N : 1;
 #pragma unroll
             for (int c = 0; c < D / 4; ++c) {
@@ -489,8 +490,8 @@ __global__ void __launch_bounds__(kVjpThreads, 1) pairing_vjp_kernel(VjpArgs a) 
             for (int j = 0; j < D; ++j) dYi[(size_t)pl * D + j] = acc[j];  // any float alignment
         }
       }
-      // dWt: each (pair, chunk) sums over the rows p; partner q = inv[sq, site_p - r].  The loads of an
-      // empty partner read row 0 and are not added, so that consecutive rows overlap; passes that
+      // dWt: each (pair, chunk) sums over the rows p; partner q = inv[sq, site_p - r].  The loads of
+      // an empty partner read row 0 and are not added, so that consecutive rows overlap; passes that
       // hold no pair of this lattice are left out.
       const int passes = (2 * N * kCh + kVjpThreads - 1) / kVjpThreads;
       auto add_row = [&](int p, float4 (&acc)[kCh]) {
@@ -515,8 +516,8 @@ __global__ void __launch_bounds__(kVjpThreads, 1) pairing_vjp_kernel(VjpArgs a) 
           }
         }
       };
-      // rows of one spin in turn (the modes ascend, so there is one run of each); a run's end is found
-      // by ballots, as a chain of n loads would be a good part of a small matrix's time
+      // rows of one spin in turn (the modes ascend, so there is one run of each); a run's end is
+      // found by ballots, as a chain of n loads would be a good part of a small matrix's time
       for (int p = 0; p < n;) {
         const int sp = modes[p] >> 16;
         int end = n;
@@ -783,7 +784,8 @@ __global__ void __launch_bounds__(TH) cnn_vjp_kernel(CnnVjpArgs a) {
         // are split, and the shares are summed in shared memory (the weights' place, not in use).
         const int pairs = (C / 4) * lcin;
         int split = 1;
-        while (2 * split * pairs <= TH && 2 * split <= Lx && (2 * split - 1) * pairs * 36 <= C * C * 9)
+        while (2 * split * pairs <= TH && 2 * split <= Lx &&
+               (2 * split - 1) * pairs * 36 <= C * C * 9)
           split *= 2;
         for (int t0 = 0; t0 < pairs * split; t0 += TH) {
           const int task = t0 + tid, pr = task % pairs, share = task / pairs;
@@ -925,12 +927,12 @@ int launch_pf_adjoint(const float* F, float* G, int n, int batch, const float* p
 }
 
 int launch_pairing_vjp(const float* G, const float* Y, const int32_t* idx, const float* Wt,
-                       const float* wt_chunks, int Lx, int Ly, int d, int n, int n_img, int samples, float* dY,
-                       float* dWt, float* jac, int64_t ld, int64_t off_w, float theta,
+                       const float* wt_chunks, int Lx, int Ly, int d, int n, int n_img,
+                       int samples, float* dY, float* dWt, float* jac, int64_t ld, int64_t off_w, float theta,
                        cudaStream_t st) {
   if (samples <= 0) return NH_OK;
-  VjpArgs a{G, Y, idx, Wt, reinterpret_cast<const float4*>(wt_chunks), Lx, Ly, n, n_img, samples, dY, dWt, jac, ld, off_w, theta,
-            jac ? 1 : 0};
+  VjpArgs a{G, Y, idx, Wt, reinterpret_cast<const float4*>(wt_chunks), Lx, Ly, n, n_img,
+            samples, dY, dWt, jac, ld, off_w, theta, jac ? 1 : 0};
   switch (d) {
     case 8: return launch_vjp_t<8>(a, st);
     case 16: return launch_vjp_t<16>(a, st);

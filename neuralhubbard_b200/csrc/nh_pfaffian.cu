@@ -2,16 +2,17 @@
 // gather, and the combination of symmetry images.
 //
 // FP32 matrices of n <= 256 run in pf32_kernel, larger ones in pf32_big_kernel (both described
-// where they stand); pfaffian_kernel below is the FP64 form for dense matrices and for
-// 224 < n <= 236.  One CTA per antisymmetric n x n matrix, n even.  The strict lower triangle lives
-// in shared memory (row i at offset i (i - 1) / 2) or in a slice of global scratch.  A pivot does not
-// move data: it swaps the logical labels of two physical rows, so an elimination step costs two
-// barriers.  Panel columns are formed lazily (stored column plus the panel's rank-2 terms
-// U V^T - V U^T); at the end of a panel of NB steps the active rows are listed in physical order and
-// the trailing triangle receives the rank-2NB update.  The Pfaffian is the product of the pivots
-// A[k, k+1] times the parity of the relabelling, accumulated in FP64 as mantissa and exponent.  The
-// ratio of the largest to the smallest pivot magnitude estimates the condition number; above
-// cond_tau the item is flagged NH_FLAG_GROWTH (near-nodal) for the FP64 recompute.
+// where they stand); pfaffian_kernel below is the FP64 form for dense matrices, for 224 < n <= 236
+// and beyond for the blocks whose FP32 pivot order does not hold in FP64.  One CTA per antisymmetric
+// n x n matrix, n even.  The strict lower triangle lives in shared memory (row i at offset
+// i (i - 1) / 2) or in a slice of global scratch.  A pivot does not move data: it swaps the logical
+// labels of two physical rows, so an elimination step costs two barriers.  Panel columns are formed
+// lazily (stored column plus the panel's rank-2 terms U V^T - V U^T); at the end of a panel of NB
+// steps the active rows are listed in physical order and the trailing triangle receives the
+// rank-2NB update.  The Pfaffian is the product of the pivots A[k, k+1] times the parity of the
+// relabelling, accumulated in FP64 as mantissa and exponent.  The ratio of the largest to the
+// smallest pivot magnitude estimates the condition number; above cond_tau the item is flagged
+// NH_FLAG_GROWTH (near-nodal) for the FP64 recompute.
 //
 // Replaces fermix.slogpf (code/backflow/models.py:210) and, in the gather mode, the Pallas
 // pairing kernel pfsbp_pairing_fwd (code/backflow/pf_kernel.py:156-190) whose formula it
@@ -689,8 +690,10 @@ int launch_pf(const PfArgs& a, cudaStream_t st) {
 
 // ------------------------------------------------------------------ FP32, n <= 256
 // The factorisation of pfaffian_kernel (same operations in the same order, so the same bits) for
-// the matrices that fit in shared memory, organised around what bounds them: the 112 pivot steps
-// of n = 224 are latency, the trailing updates shared-memory traffic.
+// the matrices that fit in shared memory, organised around what bounds them.  At n = 224, two CTAs
+// per SM, a matrix is resident for 371K cycles: 148K in the panels (112 pivot steps of latency, the
+// larger part of the block waiting), 111K in the gather and 109K in the trailing updates (both on
+// the shared-memory port, shared with the neighbour), 3K in the tail.
 //  * The active rows are compacted at the end of every panel (alist, clog: physical row and
 //    logical label in physical order), and a panel is run by ceil(m / 32) warps behind a named
 //    barrier of their own: warps without active rows do not repeat the step's work, and the last
@@ -1293,8 +1296,8 @@ __device__ __forceinline__ void bb_panel(const float* Lw, float4* Us, float4* Vs
 // One unit of the trailing update: RT rows from ia0 on the lane's two columns (physical rows pb,
 // panel values ub / vb).  FULL: every row exists and reaches both columns of every lane.
 template <int RT, bool FULL>
-__device__ __forceinline__ void bb_unit(float* Lw, const float4* Us, const float4* Vs, const int* offs,
-                                        int n, int m, int ia0, int col, const int (&pb)[2],
+__device__ __forceinline__ void bb_unit(float* Lw, const float4* Us, const float4* Vs,
+                                        const int* offs, int n, int m, int ia0, int col, const int (&pb)[2],
                                         const float4 (&ub)[2][kBbQuads],
                                         const float4 (&vb)[2][kBbQuads]) {
   float acc[RT][2];
@@ -1304,7 +1307,8 @@ __device__ __forceinline__ void bb_unit(float* Lw, const float4* Us, const float
     off[r] = offs[FULL ? ia0 + r : min(ia0 + r, m - 1)];
 #pragma unroll
     for (int h = 0; h < 2; ++h)
-      acc[r][h] = FULL || (ia0 + r < m && col + 32 * h < ia0 + r) ? __ldcg(Lw + off[r] + pb[h]) : 0.0f;
+      acc[r][h] = FULL || (ia0 + r < m && col + 32 * h < ia0 + r) ? __ldcg(Lw + off[r] + pb[h])
+                                                                  : 0.0f;
   }
 #pragma unroll
   for (int r = 0; r < RT; ++r) {
@@ -1488,8 +1492,8 @@ int launch_pf32_big(const PfArgs& a, cudaStream_t st) {
   return check_launch("pf32_big_kernel");
 }
 
-// FP32: pf32_kernel up to 256 rows, pf32_big_kernel beyond; FP64: one CTA per SM, beyond shared memory
-// (n > 236) the triangle in global memory.
+// FP32: pf32_kernel up to 256 rows, pf32_big_kernel beyond; FP64: one CTA per SM, beyond shared
+// memory (n > 236) the triangle in global memory.
 template <typename T, int D>
 int launch_pf_pick(const PfArgs& a, cudaStream_t st) {
   if (a.n <= kNumThreads) {
@@ -2202,7 +2206,8 @@ int launch_pfaffian_from_F(const float* F, int n, int batch, const int32_t* list
 // Wt (rows, d) to chunks of four a: Wc[(a / 4) rows + row].
 __global__ void wt_chunk_kernel(const float4* __restrict__ Wt, int rows, int chunks,
                                 float4* __restrict__ Wc) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < rows * chunks; e += gridDim.x * blockDim.x) {
+  const int step = gridDim.x * blockDim.x;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < rows * chunks; e += step) {
     const int c = e / rows, row = e - c * rows;
     Wc[e] = __ldg(Wt + (size_t)row * chunks + c);
   }

@@ -6,9 +6,11 @@
 // again in FP64 with that order held fixed (static pivoting): with no pivot search the
 // elimination is blocked into panels of 4 steps (8 logical columns) whose trailing update is a
 // rank-8 FP64 product, and it returns the FP64 pivots x_t, so log|pf| = sum_t log|x_t| and
-// sign(pf) = item sign x parity x prod_t sign(x_t).  Because the FP32 pivots bound every
-// multiplier by ~1, the fixed order is as stable as partial pivoting; the result carries FP64
-// rounding only, against ~1e-4 for the FP32 factorisation of an ill-conditioned block.
+// sign(pf) = item sign x parity x prod_t sign(x_t).  The FP32 pivots bound the multipliers of the
+// FP32 matrix by 1, and those of the FP64 one stay there (kMaxMultiplier says how far) unless the
+// FP32 run broke down or its last columns were rounding noise, so the fixed order is as stable as
+// partial pivoting; the result carries FP64 rounding only, against ~1e-4 for the FP32 factorisation
+// of an ill-conditioned block.
 //
 // The matrix is refined against its own FP32 entries (the bits the FP32 kernel factorised, so
 // the result is log|pf| of that FP32 matrix to FP64 accuracy) or against the FP64 matrix
@@ -21,9 +23,10 @@
 // lower triangle in shared memory, stored as 8 x 8 FP64 tiles (tile (I, J <= I) at index
 // I (I + 1) / 2 + J; 16-byte chunks swizzled inside a tile, see toff); phase 2 eliminates panels of
 // 8 columns: one warp factorises the 8 x 8 pivot block, the panel rows are multiplied by the inverse
-// of its unit factor, and the trailing tiles take P W^T, all as m8n8k4 FP64 products.  The next panel's column is
-// updated first, so that its pivot block (a serial chain) is factorised by warp 0 while the other
-// warps update the rest.  n <= kRefineMaxN (224: the tiles take 203 KB).
+// of its unit factor, and the trailing tiles take P W^T, all as m8n8k4 FP64 products.  The next
+// panel's column is updated first, so that its pivot block (a serial chain) is factorised by warp 0
+// while the other warps update the rest.  n <= kRefineMaxN (224: the tiles take 203 KB); larger
+// matrices in refine_big_kernel.
 #include <cooperative_groups.h>
 #include <math.h>
 
@@ -89,9 +92,9 @@ struct RefineArgs {
   bool rows_slice;  // mode 4: no room for Y above the CNN, its rows pass through the slice
 };
 
-// Phase 1 of modes 1 and 3: logical lower triangle A[p][q] = F[perm p][perm q] of one item, FP32, into
-// the CTA's slice.  Warp <-> 32 consecutive logical columns q (their features in registers
-// when small), rows p > q in turn (the row's features broadcast); each element reads one Wt row.
+// Phase 1 of modes 1 and 3: logical lower triangle A[p][q] = F[perm p][perm q] of one item, FP32,
+// into the CTA's slice.  Warp <-> 32 consecutive logical columns q (their features in registers when
+// small), rows p > q in turn (the row's features broadcast); each element reads one Wt row.
 template <int D, int TH>
 __device__ void gather_permuted(const RefineArgs& a, const float* Yg, const int32_t* ig,
                                 const uint16_t* perm, unsigned char* smem, float* slice) {
@@ -411,7 +414,8 @@ __device__ __forceinline__ double2* acc_ptr(double* t) {
 // an MMA operand.  Writes Li (that inverse, a swizzled tile), the reciprocal pivots xinv and the
 // pivots to piv[0, w / 2).  d: the lane's two elements.  The loop stays rolled (the code runs on one
 // warp).  Returns whether a multiplier of this lane's row is beyond kMaxMultiplier.
-__device__ __forceinline__ bool factor_block(double2 d, int w, double* Li, double* xinv, double* piv) {
+__device__ __forceinline__ bool factor_block(double2 d, int w, double* Li, double* xinv,
+                                             double* piv) {
   const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
   // entries outside the strict lower triangle of the w rows hold no data
   double b0 = (r < w && 2 * q < r) ? d.x : 0.0, b1 = (r < w && 2 * q + 1 < r) ? d.y : 0.0;
@@ -423,7 +427,8 @@ __device__ __forceinline__ bool factor_block(double2 d, int w, double* Li, doubl
     const double x = -__shfl_sync(full, b0, (2 * t + 1) * 4 + t);  // B[k][k+1] = -B[k+1][k]
     const double inv = 1.0 / x;
     // B[r][k], B[r][k+1] of this row and of the rows 2q, 2q + 1 (this lane's columns)
-    const double xr = __shfl_sync(full, b0, (lane & 28) + t), yr = __shfl_sync(full, b1, (lane & 28) + t);
+    const double xr = __shfl_sync(full, b0, (lane & 28) + t);
+    const double yr = __shfl_sync(full, b1, (lane & 28) + t);
     const double x0 = __shfl_sync(full, b0, 8 * q + t), y0 = __shfl_sync(full, b1, 8 * q + t);
     const double x1 = __shfl_sync(full, b0, 8 * q + 4 + t), y1 = __shfl_sync(full, b1, 8 * q + 4 + t);
     const double f0 = __shfl_sync(full, e0, 8 * t + q), f1 = __shfl_sync(full, e1, 8 * t + q);
@@ -537,7 +542,8 @@ __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArg
     if (tid == 0) nu_s = 0;
     __syncthreads();
     // Phase 1: the permuted lower triangle in FP64 tiles.
-    unsigned char* slb = static_cast<unsigned char*>(a.slice) + (size_t)blockIdx.x * slice_stride(n, D);
+    unsigned char* slb =
+        static_cast<unsigned char*>(a.slice) + (size_t)blockIdx.x * slice_stride(n, D);
     if constexpr (MODE == 0) {
       const float* F = a.F + (size_t)item * n * n;
       for (int p = wid; p < n; p += WARPS) {
@@ -672,7 +678,8 @@ __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArg
       }
       __syncthreads();
     }
-    if (wid == 0) write_result(a, item, pr[n] & 1, [&](int t) { return Wb[(t >> 2) * 64 + (t & 3)]; });
+    if (wid == 0)
+      write_result(a, item, pr[n] & 1, [&](int t) { return Wb[(t >> 2) * 64 + (t & 3)]; });
   }
 }
 
@@ -682,10 +689,9 @@ __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArg
 // W tiles of a panel travel, written by their owner into every CTA's shared memory (two panels'
 // worth, by parity), so a panel costs one cluster barrier.  Every CTA factorises the pivot block
 // itself, and every warp forms the one foreign W tile that the next column needs.  The order is the
-// FP32 matrix's, so the multipliers of the FP64 one are watched (kMaxMultiplier): an item that exceeds
-// them is marked kFlagRepivot and factorised again with pivoting.  What bounds it
-// is the L2 traffic of the trailing tiles (1 KB per tile update) and, at the end, the panels'
-// latency.  Replaces the pivoted FP64 factorisation with its triangle in global memory, one CTA
+// FP32 matrix's, so the multipliers of the FP64 one are watched (kMaxMultiplier): an item beyond the
+// bound is marked kFlagRepivot and factorised again with pivoting.  What bounds it is the L2 traffic
+// of the trailing tiles (1 KB per tile update) and, at the end, the panels' latency.  Replaces the pivoted FP64 factorisation with its triangle in global memory, one CTA
 // per item: 44 items at n = 896 12.25 -> 2.62 ms, 98 at n = 504 3.33 -> 1.37 ms.
 constexpr int kBigTh = 512;
 constexpr int kBigCl = 4;
@@ -742,7 +748,8 @@ __global__ void __cluster_dims__(kBigCl, 1, 1) __launch_bounds__(kBigTh, 1)
     }
     if (!a.rows_slice) {  // rows staged in shared memory
       const double2* src = reinterpret_cast<const double2*>(Yg);
-      for (int v = tid; v < n * (D / 2); v += kBigTh) reinterpret_cast<double2*>(Ys)[v] = __ldg(src + v);
+      for (int v = tid; v < n * (D / 2); v += kBigTh)
+        reinterpret_cast<double2*>(Ys)[v] = __ldg(src + v);
     }
     __syncthreads();
     for (int p = tid; p < n; p += kBigTh) {
@@ -762,8 +769,8 @@ __global__ void __cluster_dims__(kBigCl, 1, 1) __launch_bounds__(kBigTh, 1)
     __syncthreads();
     for (int p = 0; p + 1 < T; ++p) {
       double* Wp = Wl + (size_t)(p & 1) * T * 64;
-      // (1) this CTA's rows I > p: W_I and P_I from tile (I, p), then tile (I, p + 1).  W of row p + 1
-      // comes from that row's own tile (its owner does not overwrite it).
+      // (1) this CTA's rows I > p: W_I and P_I from tile (I, p), then tile (I, p + 1).  W of row
+      // p + 1 comes from that row's own tile (its owner does not overwrite it).
       {
         const Operand li = load_operand(Li);
         const double inv = xinv[lane & 3];
@@ -834,8 +841,8 @@ size_t stage_bytes(int n, int N, int D, int elt, bool wt) {
   return (size_t)elt * n * DP + sizeof(int) * ((n + 3) & ~3) + (wt ? (size_t)elt * 4 * N * DP : 0);
 }
 
-// Shared memory of one launch with TH threads (modes 2, 4: and the staging offsets, where it is at most
-// kRefineSmemLimit).
+// Shared memory of one launch with TH threads (modes 2, 4: and the staging offsets, where it is at
+// most kRefineSmemLimit).
 template <int D>
 size_t refine_smem(RefineArgs& a, int TH) {
   const int N = a.Lx * a.Ly, n = a.n, T = tile_rows(n);
@@ -846,7 +853,8 @@ size_t refine_smem(RefineArgs& a, int TH) {
     smem = std::max(smem, stage_bytes(n, N, D, 4, a.stage_wt));
     if (a.mode == 3) smem = std::max(smem, features_smem(a.Lx, a.Ly, a.C, 4, TH));
   } else if (a.mode != 0) {
-    const size_t y = 8 * (size_t)n * D, inf = (4 * (size_t)n + 15) & ~(size_t)15, wt = 8 * (size_t)N * D;
+    const size_t y = 8 * (size_t)n * D, inf = (4 * (size_t)n + 15) & ~(size_t)15;
+    const size_t wt = 8 * (size_t)N * D;
     const size_t feat = a.mode == 4 ? (features_smem(a.Lx, a.Ly, a.C, 8, TH) + 15) & ~(size_t)15 : 0;
     if (feat > kRefineSmemLimit) return feat;
     a.rows_slice = feat + y + inf > kRefineSmemLimit;
@@ -901,7 +909,8 @@ int launch_refine_m(RefineArgs a, int max_slots, cudaStream_t st) {
 template <int D>
 int launch_refine_big(RefineArgs a, int max_slots, cudaStream_t st) {
   const int N = a.Lx * a.Ly, n = a.n, T = tile_rows(n);
-  const size_t inf = (4 * (size_t)n + 15) & ~(size_t)15, y = 8 * (size_t)n * D, wt = 8 * (size_t)N * D;
+  const size_t inf = (4 * (size_t)n + 15) & ~(size_t)15, y = 8 * (size_t)n * D;
+  const size_t wt = 8 * (size_t)N * D;
   const size_t lim = 200 * 1024;
   a.rows_slice = inf + y > lim;  // rows read from global memory
   a.stage_wt = !a.rows_slice && inf + y + wt <= lim;
