@@ -269,6 +269,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) cnn_tc_kernel(TcArgs a) {
         if (lane >= o) x += y;
       }
       if (lane == 31) wbuf[lwid] = x;
+      if (ltid == 0) occl[0] = 0;  // without electrons every row reads mode 0
       wg_sync(wg);
       int before = 0, total = 0;
       for (int w = 0; w < kWGThreads / 32; ++w) {
@@ -285,7 +286,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) cnn_tc_kernel(TcArgs a) {
           rowof[m] = -1;
         }
       }
-      if (total == 0 && ltid == 0) occl[0] = 0;  // no electron: every row reads mode 0
       wg_sync(wg);
       if (ltid == 0) wbuf[0] = total;
     }

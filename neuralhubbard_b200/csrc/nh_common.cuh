@@ -182,10 +182,10 @@ __device__ void write_occupied_rows(const int* simg, int* occl, int* wbuf, int N
   int cnt = 0;
   for (int m = m0; m < m0 + per && m < M2; ++m) cnt += simg[m] > 0;
   int total;
+  if (tid == 0) occl[0] = 0;  // without electrons every row reads mode 0
   int pos = block_scan<TH>(cnt, wbuf, &total);
   for (int m = m0; m < m0 + per && m < M2; ++m)
     if (simg[m] > 0) occl[pos++] = m;
-  if (total == 0 && tid == 0) occl[0] = 0;  // no electron: every row reads mode 0
   __syncthreads();
   const int E = 16 / (int)sizeof(T), K = d / E;  // swizzled rows: K 16-byte chunks of E values
   for (int o = tid; o < n * d; o += TH) {

@@ -413,7 +413,8 @@ __device__ __forceinline__ double2* acc_ptr(double* t) {
 // the identity give the inverse of the block's unit lower factor, which the panel solve uses as
 // an MMA operand.  Writes Li (that inverse, a swizzled tile), the reciprocal pivots xinv and the
 // pivots to piv[0, w / 2).  d: the lane's two elements.  The loop stays rolled (the code runs on one
-// warp).  Returns whether a multiplier of this lane's row is beyond kMaxMultiplier.
+// warp).  CHECK: returns whether a multiplier of this lane's row is beyond kMaxMultiplier.
+template <bool CHECK>
 __device__ __forceinline__ bool factor_block(double2 d, int w, double* Li, double* xinv,
                                              double* piv) {
   const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
@@ -435,7 +436,7 @@ __device__ __forceinline__ bool factor_block(double2 d, int w, double* Li, doubl
     const double g0 = __shfl_sync(full, e0, 8 * t + 4 + q), g1 = __shfl_sync(full, e1, 8 * t + 4 + q);
     const double yi = yr * inv, xi = xr * inv;
     if (r >= 2 * t + 2) {
-      grew |= r < w && !(fabs(xi) <= kMaxMultiplier);
+      if (CHECK) grew |= r < w && !(fabs(xi) <= kMaxMultiplier);
       if (2 * q >= 2 * t + 2) {
         b0 = fma(yi, x0, fma(-xi, y0, b0));
         b1 = fma(yi, x1, fma(-xi, y1, b1));
@@ -611,7 +612,7 @@ __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArg
 
     // Phase 2: static-pivot blocked elimination.  The pivots of panel p are kept in the W tile of
     // tile row p, which no later step reads or writes.
-    if (wid == 0) factor_block(*acc_ptr(S), min(kPW, n), Li, xinv, Wb);
+    if (wid == 0) factor_block<false>(*acc_ptr(S), min(kPW, n), Li, xinv, Wb);
     __syncthreads();
     for (int p = 0; p + 1 < T; ++p) {
       // (1) tile rows I > p: W_I = -S_(I, p) Li^T (the forward substitution of every row as one
@@ -641,8 +642,8 @@ __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArg
       __syncthreads();
       // (3) warp 0: the next pivot block; the others: the remaining tiles, 2 x 2 at a time.
       if (wid == 0) {
-        factor_block(*acc_ptr(S + (size_t)(tile_base(p + 1) + p + 1) * 64),
-                     min(kPW, n - 8 * (p + 1)), Li, xinv, Wb + (p + 1) * 64);
+        factor_block<false>(*acc_ptr(S + (size_t)(tile_base(p + 1) + p + 1) * 64),
+                            min(kPW, n - 8 * (p + 1)), Li, xinv, Wb + (p + 1) * 64);
       } else if (wid & 3) {
         // not the warps of warp 0's scheduler, whose chain would queue behind their products
         constexpr int NW = WARPS - WARPS / 4;
@@ -765,7 +766,7 @@ __global__ void __cluster_dims__(kBigCl, 1, 1) __launch_bounds__(kBigTh, 1)
     cluster.sync();  // every tile written; the staging areas are dead in every CTA
     const int o = toff(lane >> 2, 2 * (lane & 3));  // this lane's elements of a tile
     bool grew = false;  // of this lane's multipliers
-    if (wid == 0) grew = factor_block(ldcg2(S + o), min(kPW, n), Li, xinv, piv);
+    if (wid == 0) grew = factor_block<true>(ldcg2(S + o), min(kPW, n), Li, xinv, piv);
     __syncthreads();
     for (int p = 0; p + 1 < T; ++p) {
       double* Wp = Wl + (size_t)(p & 1) * T * 64;
@@ -802,8 +803,8 @@ __global__ void __cluster_dims__(kBigCl, 1, 1) __launch_bounds__(kBigTh, 1)
       // (2) warp 0: the next pivot block; the others: this CTA's rows over the columns p + 2 .. I,
       // strips of kStrip tiles of one row with all loads in flight.
       if (wid == 0) {
-        grew |= factor_block(ldcg2(S + (size_t)(tile_base(p + 1) + p + 1) * 64 + o),
-                             min(kPW, n - 8 * (p + 1)), Li, xinv, piv + 4 * (p + 1));
+        grew |= factor_block<true>(ldcg2(S + (size_t)(tile_base(p + 1) + p + 1) * 64 + o),
+                                   min(kPW, n - 8 * (p + 1)), Li, xinv, piv + 4 * (p + 1));
       } else {
         constexpr int kStrip = 6, NW = kBigWarps - 1;
         int I = p + 2 + ((rank - (p + 2)) & (kBigCl - 1)), rem = wid - 1;
