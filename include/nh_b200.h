@@ -98,7 +98,7 @@ enum {
  *                Wt64 is set, its features are recomputed in FP64 (CNN) and its log-Pfaffian is
  *                refined against the FP64 pairing block (NH_FLAG_REFINED), in the pivot order of
  *                the FP32 factorisation; 224 < n <= 236, and larger n where that order leaves a
- *                multiplier above 2 or a zero or non-finite pivot: with FP64 partial pivoting.
+ *                multiplier of 2 or more or a zero or non-finite pivot: with FP64 partial pivoting.
  *                <= 0 disables both.  For projected amplitudes with cond_tau > 1 an image whose
  *                |psi(g s)| is below 1e-3 of |psi_P(s)| is not recomputed in FP64 (its error
  *                cannot move log|psi_P| by more than ~1e-5); cond_tau <= 1 recomputes every image

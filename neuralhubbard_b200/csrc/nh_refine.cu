@@ -7,7 +7,7 @@
 // elimination is blocked into panels of 4 steps (8 logical columns) whose trailing update is a
 // rank-8 FP64 product, and it returns the FP64 pivots x_t, so log|pf| = sum_t log|x_t| and
 // sign(pf) = item sign x parity x prod_t sign(x_t).  The FP32 pivots bound the multipliers of the
-// FP32 matrix by 1, and those of the FP64 one stay there (kMaxMultiplier says how far) unless the
+// FP32 matrix by 1, and those of the FP64 one stay there (beyond_bound says how far) unless the
 // FP32 run broke down or its last columns were rounding noise, so the fixed order is as stable as
 // partial pivoting; the result carries FP64 rounding only, against ~1e-4 for the FP32 factorisation
 // of an ill-conditioned block.
@@ -399,7 +399,10 @@ size_t features_smem(int Lx, int Ly, int C, int elt, int TH) {
 // there in FP64 too: at n = 240 and 504 at most 1.0001 over blocks of pivot ratio up to 2e7.  It
 // leaves 1 where a column of FP32 Schur complements is at its rounding noise (3.6 seen at a ratio of
 // 3e10) and is unbounded where the FP32 run met infinities.
-constexpr double kMaxMultiplier = 2.0;
+__device__ __forceinline__ bool beyond_bound(double m) {  // |m| >= 2 (its high word), or NaN
+  constexpr int kMaxMultiplier = 0x40000000;
+  return (__double2hiint(m) & 0x7FFFFFFF) >= kMaxMultiplier;
+}
 
 // A lane's two elements of a tile in the MMA accumulator layout.
 __device__ __forceinline__ double2* acc_ptr(double* t) {
@@ -413,16 +416,15 @@ __device__ __forceinline__ double2* acc_ptr(double* t) {
 // the identity give the inverse of the block's unit lower factor, which the panel solve uses as
 // an MMA operand.  Writes Li (that inverse, a swizzled tile), the reciprocal pivots xinv and the
 // pivots to piv[0, w / 2).  d: the lane's two elements.  The loop stays rolled (the code runs on one
-// warp).  CHECK: returns whether a multiplier of this lane's row is beyond kMaxMultiplier.
+// warp).  CHECK: a multiplier beyond the bound sets *grew.
 template <bool CHECK>
-__device__ __forceinline__ bool factor_block(double2 d, int w, double* Li, double* xinv,
-                                             double* piv) {
+__device__ __forceinline__ void factor_block(double2 d, int w, double* Li, double* xinv,
+                                             double* piv, int* grew = nullptr) {
   const int lane = threadIdx.x & 31, r = lane >> 2, q = lane & 3;
   // entries outside the strict lower triangle of the w rows hold no data
   double b0 = (r < w && 2 * q < r) ? d.x : 0.0, b1 = (r < w && 2 * q + 1 < r) ? d.y : 0.0;
   double e0 = r == 2 * q ? 1.0 : 0.0, e1 = r == 2 * q + 1 ? 1.0 : 0.0;
   const unsigned full = 0xffffffffu;
-  bool grew = false;
 #pragma unroll 1
   for (int t = 0; 2 * t < w; ++t) {
     const double x = -__shfl_sync(full, b0, (2 * t + 1) * 4 + t);  // B[k][k+1] = -B[k+1][k]
@@ -436,7 +438,7 @@ __device__ __forceinline__ bool factor_block(double2 d, int w, double* Li, doubl
     const double g0 = __shfl_sync(full, e0, 8 * t + 4 + q), g1 = __shfl_sync(full, e1, 8 * t + 4 + q);
     const double yi = yr * inv, xi = xr * inv;
     if (r >= 2 * t + 2) {
-      if (CHECK) grew |= r < w && !(fabs(xi) <= kMaxMultiplier);
+      if (CHECK && r < w && beyond_bound(xi)) *grew = 1;
       if (2 * q >= 2 * t + 2) {
         b0 = fma(yi, x0, fma(-xi, y0, b0));
         b1 = fma(yi, x1, fma(-xi, y1, b1));
@@ -450,7 +452,6 @@ __device__ __forceinline__ bool factor_block(double2 d, int w, double* Li, doubl
     }
   }
   *reinterpret_cast<double2*>(Li + toff(r, 2 * q)) = make_double2(e0, e1);
-  return grew;
 }
 
 // Tile update C += P W^T: P and W are 8 x 8 tiles (rows x panel columns).
@@ -690,10 +691,12 @@ __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArg
 // W tiles of a panel travel, written by their owner into every CTA's shared memory (two panels'
 // worth, by parity), so a panel costs one cluster barrier.  Every CTA factorises the pivot block
 // itself, and every warp forms the one foreign W tile that the next column needs.  The order is the
-// FP32 matrix's, so the multipliers of the FP64 one are watched (kMaxMultiplier): an item beyond the
+// FP32 matrix's, so the multipliers of the FP64 one are watched (beyond_bound): an item beyond the
 // bound is marked kFlagRepivot and factorised again with pivoting.  What bounds it is the L2 traffic
-// of the trailing tiles (1 KB per tile update) and, at the end, the panels' latency.  Replaces the pivoted FP64 factorisation with its triangle in global memory, one CTA
-// per item: 44 items at n = 896 12.25 -> 2.62 ms, 98 at n = 504 3.33 -> 1.37 ms.
+// of the trailing tiles (1 KB per tile update) and, at the end, the panels' latency.  Replaces the
+// pivoted FP64 factorisation with its triangle in global memory, one CTA per item: 44 items at
+// n = 896 12.25 -> 2.64 ms, 98 at n = 504 3.33 -> 1.38 ms, of which the check and the launch that
+// looks for marked items are 22 and 8 us.
 constexpr int kBigTh = 512;
 constexpr int kBigCl = 4;
 constexpr int kBigWarps = kBigTh / 32;
@@ -721,7 +724,7 @@ __global__ void __cluster_dims__(kBigCl, 1, 1) __launch_bounds__(kBigTh, 1)
   __shared__ double piv[kMaxN / 2];
   __shared__ uint16_t iperm[kMaxN];
   __shared__ int nu_s;
-  __shared__ int grew_s;  // rank 0's: a multiplier of the item was beyond kMaxMultiplier
+  __shared__ int grew_s;  // rank 0's: a multiplier of the item was beyond the bound
   const int n = a.n, T = tile_rows(n), N = a.Lx * a.Ly;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   // Elimination: W tiles of two panels, then this CTA's P tiles (rows rank, rank + kBigCl, ...).
@@ -765,8 +768,7 @@ __global__ void __cluster_dims__(kBigCl, 1, 1) __launch_bounds__(kBigTh, 1)
                             nullptr, S, rank * kBigWarps + wid, kBigCl * kBigWarps);
     cluster.sync();  // every tile written; the staging areas are dead in every CTA
     const int o = toff(lane >> 2, 2 * (lane & 3));  // this lane's elements of a tile
-    bool grew = false;  // of this lane's multipliers
-    if (wid == 0) grew = factor_block<true>(ldcg2(S + o), min(kPW, n), Li, xinv, piv);
+    if (wid == 0) factor_block<true>(ldcg2(S + o), min(kPW, n), Li, xinv, piv, &grew_s);
     __syncthreads();
     for (int p = 0; p + 1 < T; ++p) {
       double* Wp = Wl + (size_t)(p & 1) * T * 64;
@@ -788,7 +790,7 @@ __global__ void __cluster_dims__(kBigCl, 1, 1) __launch_bounds__(kBigTh, 1)
           const double2 sv = ldcg2(row + p * 64 + o), cv = ldcg2(row + (p + 1) * 64 + o);
           const double2 w = tile_mma(make_double2(0.0, 0.0), to_operand(sv), li);
           const double2 pv = make_double2(-w.y * inv, w.x * inv);
-          grew |= 8 * I + (lane >> 2) < n && !(fabs(pv.y) <= kMaxMultiplier);
+          if (beyond_bound(pv.y) && 8 * I + (lane >> 2) < n) *grew0 = 1;
           *reinterpret_cast<double2*>(Pl + (I / kBigCl) * 64 + o) = pv;
 #pragma unroll
           for (int r = 0; r < kBigCl; ++r)
@@ -798,13 +800,12 @@ __global__ void __cluster_dims__(kBigCl, 1, 1) __launch_bounds__(kBigTh, 1)
           __stcg(reinterpret_cast<double2*>(row + (p + 1) * 64 + o), nv);
         }
       }
-      if (grew) *grew0 = 1;
       cluster.sync();  // W complete everywhere, column p + 1 updated
       // (2) warp 0: the next pivot block; the others: this CTA's rows over the columns p + 2 .. I,
       // strips of kStrip tiles of one row with all loads in flight.
       if (wid == 0) {
-        grew |= factor_block<true>(ldcg2(S + (size_t)(tile_base(p + 1) + p + 1) * 64 + o),
-                                   min(kPW, n - 8 * (p + 1)), Li, xinv, piv + 4 * (p + 1));
+        factor_block<true>(ldcg2(S + (size_t)(tile_base(p + 1) + p + 1) * 64 + o),
+                           min(kPW, n - 8 * (p + 1)), Li, xinv, piv + 4 * (p + 1), &grew_s);
       } else {
         constexpr int kStrip = 6, NW = kBigWarps - 1;
         int I = p + 2 + ((rank - (p + 2)) & (kBigCl - 1)), rem = wid - 1;
@@ -831,8 +832,7 @@ __global__ void __cluster_dims__(kBigCl, 1, 1) __launch_bounds__(kBigTh, 1)
       __syncthreads();  // Li ready, this CTA's rows updated
     }
     if (rank == 0 && wid == 0)
-      write_result(a, item, pr[n] & 1, [&](int t) { return piv[t]; }, true,
-                   __any_sync(0xffffffffu, grew) || grew_s != 0);
+      write_result(a, item, pr[n] & 1, [&](int t) { return piv[t]; }, true, grew_s != 0);
     cluster.sync();  // no CTA starts the next item's gather over tiles still being read
   }
 }
