@@ -28,6 +28,7 @@
 // while the other warps update the rest.  n <= kRefineMaxN (224: the tiles take 203 KB); larger
 // matrices in refine_big_kernel.
 #include <cooperative_groups.h>
+#include <limits.h>
 #include <math.h>
 
 #include <algorithm>
@@ -78,7 +79,8 @@ struct RefineArgs {
   int Lx, Ly, D;
   bool stage_wt;  // Wt (modes 2, 4: one spin block of it) fits in shared memory with the rows
   const int32_t* list;   // slot -> item
-  const int32_t* count;  // device number of slots
+  const int32_t* count;  // device number of slots; beyond [min_count, max_count] nothing is done
+  int min_count, max_count;
   const uint16_t* perm;  // per item: perm[0, n) logical -> physical, [n] relabelling parity
   int perm_stride;       // uint16 per item
   const float* item_sign;  // (items,) or null
@@ -530,6 +532,7 @@ __global__ void __launch_bounds__(TH, TH <= 256 ? 2 : 1) refine_kernel(RefineArg
   double* S = reinterpret_cast<double*>(smem);
   double* Wb = S + (size_t)tile_base(T) * 64;  // W tiles of the current panel, one per tile row
   const int n_work = *a.count;
+  if (n_work < a.min_count || n_work > a.max_count) return;
   for (int slot = blockIdx.x; slot < n_work; slot += gridDim.x) {
     const int item = a.list[slot];
     const uint16_t* pr = a.perm + (size_t)item * a.perm_stride;
@@ -889,17 +892,26 @@ int launch_refine_k(const RefineArgs& a, int max_slots, size_t smem, cudaStream_
 
 // Two CTAs of 256 threads per SM where shared memory holds both and there are items for them (small
 // lattices, whose phases are latency-bound), else one of 512.  In-kernel features on the matrix
-// instruction need 512 threads beyond 128 sites; the scalar network (16 channels) runs with either:
-// 290 bare images, whole call, 4x4 159 -> 118 us, 8x8 200 -> 159, 12x14 361 -> 320.
+// instruction need 512 threads beyond 128 sites.  The scalar network (16 channels) runs with either,
+// and there the number of listed items decides on the device, both forms being launched (3 us): 290
+// bare images, all listed, whole call with 512 and with 256 threads: 4x4 159 and 118 us, 8x8 200 and
+// 159, 12x14 361 and 320; 320 images of 40 projected configurations, a third of them listed: 8x8 167
+// and 178, 12x12 270 and 299.
 constexpr size_t kTwoCtaSmem = 111 * 1024;  // dynamic, beside the static arrays
 
 template <int D, int MODE>
 int launch_refine_m(RefineArgs a, int max_slots, cudaStream_t st) {
-  const bool small = MODE != 4 || cnn_mma_fits(a.Lx, a.Ly, a.C, 256) ||
-                     !cnn_mma_fits(a.Lx, a.Ly, a.C, 512);
+  const bool scalar = MODE == 4 && !cnn_mma_fits(a.Lx, a.Ly, a.C, 512);
+  const bool small = MODE != 4 || scalar || cnn_mma_fits(a.Lx, a.Ly, a.C, 256);
   const size_t s256 = refine_smem<D>(a, 256);
-  if (small && s256 <= kTwoCtaSmem && max_slots > num_sms())
-    return launch_refine_k<D, MODE, 256>(a, max_slots, s256, st);
+  a.max_count = INT_MAX;
+  if (small && s256 <= kTwoCtaSmem && max_slots > num_sms()) {
+    a.min_count = scalar ? num_sms() + 1 : 0;
+    const int rc = launch_refine_k<D, MODE, 256>(a, max_slots, s256, st);
+    if (rc || !scalar) return rc;
+    a.min_count = 0;
+    a.max_count = num_sms();
+  }
   const size_t s512 = refine_smem<D>(a, 512);
   if (s512 > kRefineSmemLimit)
     return fail(NH_ERR_UNSUPPORTED, "refine: n=%d needs %zu B of shared memory", a.n, s512);

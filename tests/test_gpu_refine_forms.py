@@ -101,3 +101,22 @@ def test_refusals_say_what_is_needed(channels, Lx, Ly, ne, kw, message):
     s = olat.random_configs(np.random.default_rng(1), 2, Lx * Ly, ne, ne)
     with pytest.raises(nh.NativeLibraryError, match=message):
         nh.Variational(nh.PfaffianBackflow(Lx, Ly, ne, ne, params=p, **kw))(s)
+
+
+@pytest.mark.parametrize("Lx,Ly,up,dn", [(8, 8, 28, 26), (12, 14, 71, 69)])
+def test_few_of_many_listed(Lx, Ly, up, dn):
+    """16 channels, more images than SMs of which fewer than SMs are listed: the 512-thread form then,
+    as for few images; the same bits either way, and both lists' lengths occur."""
+    N = Lx * Ly
+    p = nh.init_params(Lx, Ly, channels=16, layers=4, std=0.1, seed=N)
+    s = olat.random_configs(np.random.default_rng(N + 1), 6, N, up, dn)
+    seen = set()
+    for tau in (1.0, 5.0, 10.0, 20.0, 40.0, 80.0, 160.0, 320.0):
+        state = nh.Variational(nh.PfaffianBackflow(Lx, Ly, up, dn, params=p, cond_tau=tau),
+                               symm=False)
+        few, many = state(s), state(np.tile(s, (50, 1)))
+        assert torch.equal(few.sign.repeat(50), many.sign)
+        assert torch.equal(few.logabs.repeat(50), many.logabs)
+        assert torch.equal(few.flags.repeat(50), many.flags)
+        seen.add(int((few.flags & _lib.FLAG_REFINED != 0).sum()))
+    assert seen & {1, 2} and seen & {3, 4, 5, 6}, seen
